@@ -87,6 +87,28 @@ __host__ __device__ inline int tc_off(int r, int k) {
 __host__ __device__ inline int tc_off_mn(int n, int k) {
   return (n >> 3) * kTcGroup + (k >> 3) * 64 + (k & 7) * 8 + (n & 7);
 }
+// FP64 tensor-core MMA (mma.sync m8n8k4, the full-rate FP64 path of sm_100a): lane
+// (g = lane / 4, t = lane % 4) supplies A[g][t] and B[t][g] and accumulates C[g][2t] and
+// C[g][2t + 1].  One instruction does 256 multiply-adds, so the small channel GEMMs are no longer
+// bound by instruction issue and shared-memory loads.
+__device__ __forceinline__ void dmma_884(double (&c)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+      : "+d"(c[0]), "+d"(c[1])
+      : "d"(a), "d"(b));
+}
+
+// C (16 x 8) += A (16 x 16) B (16 x 8) in FP64, lane layout (g = lane / 4, t = lane % 4):
+// a[i] = A[g + 8 (i % 2)][t + 4 (i / 2)], b[i] = B[t + 4 i][g],
+// c = {C[g][2t], C[g][2t + 1], C[g + 8][2t], C[g + 8][2t + 1]}.
+__device__ __forceinline__ void dmma_16816(double (&c)[4], const double (&a)[8],
+                                           const double (&b)[4]) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, "
+      "{%4,%5,%6,%7,%8,%9,%10,%11}, {%12,%13,%14,%15}, {%0,%1,%2,%3};"
+      : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+      : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(a[4]), "d"(a[5]), "d"(a[6]), "d"(a[7]),
+        "d"(b[0]), "d"(b[1]), "d"(b[2]), "d"(b[3]));
+}
+
 // x -> nt bf16 terms, each the round-to-nearest of what the previous ones leave (the
 // remainders are exact in double).
 // bf16 bits of a double h that has at most 8 significant bits: sign, exponent rebased from
