@@ -8,81 +8,68 @@
 
 namespace ccd {
 
-// pp-ladder tiling.  V_pppp is antisymmetric in both pair indices (calcTBME is
-// f(p,q,r,s) - f(p,q,s,r)), so D[ab,ij] = 1/2 sum_cd V[ab,cd] T[cd,ij] is evaluated as
-// sum_{c<d} V[ab,cd] T[cd,ij] over rows a<=b and mirrored to the b>a rows with a sign flip:
-// one quarter of the V bytes and flops of the full product.
+// Packed amplitudes.  The amplitudes are antisymmetric, t_ab,ij = -t_ab,ji = -t_ba,ij = t_ba,ji,
+// and so are V and D, so the solver iterates on one element in four: the quads (u, w) of a
+// channel, u = strict particle pair a < b (pk of them), w = strict hole pair i < j (hk), row-major
+// [u][w] with row stride hs.  T, V_hhpp and D use this layout (channel block at q_off, rows
+// padded to a multiple of kBK with zeros).
 //
-// Operand tiles are stored in HBM already in their shared-memory image so that one bulk copy
-// (TMA) moves a whole stage:
-//   thin channels (hh <= 8, nb in {2, 4, 8}, one row per consumer thread):
-//     A tiles [rows][kBK] row-major, column XOR-swizzled by (row & 15): a warp reading 16
-//             consecutive rows at one k hits 16 distinct bank pairs;
-//     B tiles [kBK][nb] k-major, read as warp broadcasts;
-//   mid and wide channels (nb = 8*C, FP64 MMA fragments):
-//     A tiles [kBK][as] k-major, as = rows rounded up to 8, plus 4;
-//     B tiles [kBK][bs] k-major, bs = nb + 4;
-//     strides of 4 mod 8 doubles put the 4 k-rows of an FP64 MMA fragment load (m16n8k16 in
-//     the ladder) on distinct banks.
+// pp ladder.  D[ab,ij] = sum_{c<d} V[ab,cd] T[cd,ij] over the quads: V is the pk x pk packed
+// matrix (1/4 of V_pppp), T the packed amplitudes themselves (16 consecutive rows are one
+// contiguous B stage).  A stages are stored in HBM in their shared-memory image so that one bulk
+// copy (TMA) moves each:
+//   thin channels (hk <= 4, hs in {1, 2, 4}; two consumer threads per row):
+//     [rows][kBK] row-major, column XOR-swizzled by (row & 15): a warp reading two k of 16
+//     consecutive rows takes the minimum of two wavefronts;
+//   wider channels (FP64 MMA fragments): [kBK][as] k-major, as = rows rounded up to 8, plus 4,
+//     and hs = 4 mod 8: with strides of 4 mod 8 doubles the 4 k-rows of an m16n8k16 fragment
+//     load fall on distinct banks.
 // The last row tile of a channel is stored compact (only its real rows, rounded up to 8).
 constexpr int kBK = 16;        // K depth of one pipeline stage
-constexpr int kStages = 4;     // bulk-copy pipeline depth
-constexpr int kMaxCG = 9;      // column groups of 8 -> up to 72 hh columns
-constexpr int kLadderConsumers = 128;
+constexpr int kStages = 5;     // bulk-copy pipeline depth
+constexpr int kMaxHH = 72;     // hole pairs of a channel (ordered)
+constexpr int kMaxCG = 5;      // column groups of 8 strict hole pairs (hk <= 36)
+constexpr int kLadderConsumers = 256;                  // 8 warps of 16 rows
 constexpr int kLadderThreads = kLadderConsumers + 32;  // + 1 producer warp
-// Mid and wide classes: 8 consumer warps of 16 rows each (two CTAs per SM).
-constexpr int kLadderConsumersMMA = 256;
-__host__ __device__ constexpr int ladder_threads(int cls) {
-  return (cls == 0 ? kLadderConsumers : kLadderConsumersMMA) + 32;
-}
-constexpr int kMaxBM = 128;
-constexpr int kMaxNB = 8 * kMaxCG;
+constexpr int kMaxBM = 128;    // rows per tile
+constexpr int kMaxNB = 36;     // largest row stride hs of the packed amplitudes
 constexpr int kMaxAS = kMaxBM + 4;  // A stage row stride bound (doubles)
-constexpr int kMaxBS = kMaxNB + 4;  // B stage row stride bound (doubles)
 
 __host__ __device__ inline int swzA(int row, int k) { return row * kBK + (k ^ (row & 15)); }
-// Padded column count of a channel with hh hole pairs.
-__host__ __device__ inline int ladder_nb(int hh) {
-  return hh <= 2 ? 2 : hh <= 4 ? 4 : 8 * ((hh + 7) / 8);
+// Row stride of the packed layout for hk strict hole pairs.
+__host__ __device__ inline int quad_hs(int hk) {
+  return hk <= 2 ? hk : hk <= 4 ? 4 : 8 * ((hk + 3) / 8) + 4;
 }
-// Rows per tile: thin channels one row per consumer thread; mid and wide ones (nb >= 16)
-// 16 rows x nb columns per consumer warp.
-__host__ __device__ inline int ladder_bm(int nb) { return kLadderConsumers; }
-// A chunks of mid and wide channels are k-major (row stride `arows`, see above); thin ones are
-// row-major and XOR-swizzled (one row per thread).
-__host__ __device__ inline bool ladder_kmajor(int nb) { return nb >= 16; }
-// A row stride (doubles per k row of an A chunk) of a row tile with `rows` real rows.
-__host__ __device__ inline int ladder_arows(int nb, int rows) {
-  return ladder_kmajor(nb) ? ((rows + 7) & ~7) + 4 : rows;
+// Column classes: 0 thin, 1 mid (hs 12, 20), 2 wide (hs 28, 36).
+__host__ __device__ inline int ladder_class(int hs) { return hs <= 4 ? 0 : hs <= 20 ? 1 : 2; }
+__host__ __device__ inline bool ladder_kmajor(int hs) { return hs > 4; }
+// Doubles per k row of an A chunk (k-major) or rows of it (thin) for a tile of `rows` rows.
+__host__ __device__ inline int ladder_arows(int hs, int rows) {
+  return ladder_kmajor(hs) ? ((rows + 7) & ~7) + 4 : rows;
 }
-// A image of row tile mt starts at mt * ladder_arows(nb, kMaxBM) * nk * kBK (full tiles).
-__host__ __device__ inline int ladder_arows_full(int nb) { return ladder_arows(nb, kMaxBM); }
-// B row stride (doubles per k row of a B chunk).
-__host__ __device__ inline int ladder_bs(int nb) { return ladder_kmajor(nb) ? nb + 4 : nb; }
-__host__ __device__ inline int ladder_aoff(int nb, int arows, int r, int k) {
-  return ladder_kmajor(nb) ? k * arows + r : swzA(r, k);
-}
+// A image of row tile mt starts at mt * ladder_arows_full(hs) * nk * kBK (full tiles).
+__host__ __device__ inline int ladder_arows_full(int hs) { return ladder_arows(hs, kMaxBM); }
 
 // Mixed-precision pp-ladder images (tensor-core operands, ccd_tc.cuh).  A K chunk of a
 // 128-row tile holds kTcKC bf16 per row in 8 x 8 core matrices, K-major, no swizzle:
 //   element (r, k) -> (r / 8) * kTcGroup + (k / 8) * 64 + (r % 8) * 8 + k % 8.
 constexpr int kTcKC = 32;                    // K depth of one chunk (bf16 elements)
 constexpr int kTcBM = 128;                   // rows per tile = UMMA M
-constexpr int kTcMaxNB = 80;                 // padded columns = UMMA N (multiple of 16)
+constexpr int kTcMaxNB = 48;                 // padded columns = UMMA N (multiple of 16)
 constexpr int kTcThreads = 192;
 constexpr int kTcAPlane = kTcBM * kTcKC;     // bf16 elements of one A term per stage (8 KB)
-constexpr int kTcBPlane = kTcMaxNB * kTcKC;  // one B term per stage (5 KB)
+constexpr int kTcBPlane = kTcMaxNB * kTcKC;  // one B term per stage (3 KB)
 constexpr int kTcGroup = 8 * kTcKC;          // bf16 elements of one 8-row group of a chunk
 
-// Padded UMMA N for hh columns.
-__host__ __device__ inline int tc_nb(int hh) { return 16 * ((hh + 15) / 16); }
+// Padded UMMA N for hk columns.
+__host__ __device__ inline int tc_nb(int hk) { return 16 * ((hk + 15) / 16); }
 // Offset of element (r, k) inside a chunk image (bf16 units), 0 <= k < kTcKC: K-major core
-// matrices (8 rows of 8 consecutive k), used for the A operands.
+// matrices (8 rows of 8 consecutive k), used for the A operand (V).
 __host__ __device__ inline int tc_off(int r, int k) {
   return (r >> 3) * kTcGroup + (k >> 3) * 64 + (r & 7) * 8 + (k & 7);
 }
-// The B operands (N = hh columns) in MN-major core matrices (8 k-rows of 8 consecutive n):
-// neighbouring columns are neighbouring bytes, as the assembly and hh ladder write them.  Same
+// The B operand (T, N = hk columns) in MN-major core matrices (8 k-rows of 8 consecutive n):
+// neighbouring columns are neighbouring bytes, as the assembly writes them.  Same
 // 8 x 8 block positions as tc_off, so the shared-memory descriptors are the same.
 __host__ __device__ inline int tc_off_mn(int n, int k) {
   return (n >> 3) * kTcGroup + (k >> 3) * 64 + (k & 7) * 8 + (n & 7);
@@ -148,55 +135,60 @@ __device__ __forceinline__ void split_bf16_n(double x, __nv_bfloat16 (&out)[NT])
   for (int p = 0; p < NT; ++p) out[p] = bf16_of_short(split_bf16_step(x));
 }
 
-// One pp-ladder work tile: packed rows [mt*bm, mt*bm+rows) of channel `ch`, V-part K chunks
-// [kc0, kc0+nks).  Tiles of one row block that split K write partial sums; the last one to
-// finish (ticket on counter `group`) adds them in segment order.  The segment with seg ==
-// nseg-1 also runs the T X chunks.
+// One pp-ladder work tile: packed rows [128 mt, 128 mt + rows) of channel `ch`, K chunks
+// [kc0, kc0 + nks).  Tiles of one row block that split K write separate planes of the channel's
+// D partials (LadderChan), which the assembly adds in segment order.
 struct LadderTile {
-  int32_t ch, mt, kc0, nks, nkc, nkh, nb, bm, rows, pr, hh, seg, nseg, group;
-  int64_t v_base;    // A tiles of V:  + mt*arows_full*nkc*kBK + kc * arows*kBK
-  int64_t tkt_base;  // B tiles of T:  + kc * kBK*bs
-  int64_t tmt_base;  // A tiles of T (rows a<=b, K = hh): + mt*bm*nkh*kBK + kh * rows*kBK
-  int64_t xt_base;   // B tiles of X/2: + kh * kBK*bs
-  int64_t t_off;     // offset of the channel's pp x hh block in the t2 layout
-  int64_t row_off;   // offset into rowmap / mirror
-  int64_t part_base; // partial sums of this row block: nseg * bm * nb doubles
+  int32_t ch, mt, kc0, nks;
+  int32_t rows, hk, hs, nb;  // nb: UMMA N (tensor-core tiles)
+  int64_t a_base;  // first A chunk: + c * ladder_arows(hs, rows) * kBK (tensor core: see there)
+  int64_t b_base;  // first B chunk: + c * kBK * hs
+  int64_t out;     // D of the tile's first row: + u_local * hs
 };
 
-// Per active regular channel.
+// Where the ladder leaves D of a channel: nseg planes of `plane` doubles from `base`, each in
+// the packed layout; D is their sum in plane order.
+struct LadderChan {
+  int64_t base;
+  int32_t nseg, plane;
+};
+
+// Per active regular channel.  A channel without quads (pk or hk zero) has no ladder tile, hh
+// unit or assembly item: its amplitudes are zero.
 struct ChanInfo {
-  int32_t pp, hh, nb, nkc, nkh, nmt, bm, pr, pk, nhht;
+  int32_t pp, hh, pk, hk;
+  int32_t hs, nkc, nmt, nhht;  // packed row stride, K chunks, row tiles, hh-ladder slices
   int64_t t_off;     // pphh block offset (reference t2 layout)
-  int64_t pp_off;    // offset into pp_pairs / pp_swap / pk_idx / r
-  int64_t hh_off;    // offset into hh_pairs / hh_swap / s
-  int64_t x_off;     // hh x hh block offset (V_hhhh and X)
-  int64_t tkt_base, tmt_base, xt_base, vkt_base;
-  int64_t row_off;   // offset into rowmap / mirror (pr entries)
-  int64_t pk_off;    // offset into kcol (pk entries)
-  int64_t part_off;  // hh-ladder partial products: nhht * hh*hh doubles
-  int64_t hht0;      // first hh-ladder tile of the channel
+  int64_t pp_off;    // offset into pp_pairs / pp_swap / prow
+  int64_t hh_off;    // offset into hh_pairs / hh_swap / hcol
+  int64_t vhh_off;   // hh x hh block offset (V_hhhh)
+  int64_t q_off;     // packed block: 16 nkc x hs doubles (T, V_hhpp)
+  int64_t x_off;     // X: hk x hs
+  int64_t vkt_base;  // A tiles of V
+  int64_t pk_off;    // strict particle pairs: offset into kcol / quad rows / r (pk entries)
+  int64_t qcol_off;  // strict hole pairs: offset into quad columns / s (hk entries)
   // Mixed-precision operand images (bf16 terms, tensor-core layout; see ccd_tc.cuh):
-  // nbt = UMMA N, nkct / nkht = 32-deep K chunks of V T / T X.
-  int32_t nbt, nkct, nkht, pad_tc;
-  int64_t vtc_base, tkt_tc_base, tmt_tc_base, xt_tc_base;
-  // Fused assembly: hk = strict hole pairs (i < j); quad tables from qrow_off (pk strict
-  // packed rows a < b) and qcol_off (hk entries).
-  int32_t hk, pad_q;
-  int64_t qrow_off, qcol_off;
+  // nbt = UMMA N, nkct = 32-deep K chunks of V T.
+  int32_t nbt, nkct;
+  int64_t vtc_base, tkt_tc_base;
 };
 
-// hh-ladder unit: rows [k0, k0+rows) of channel ch (slice idx), a chunk of P rows.
+// hh-ladder unit: rows [k0, k0+rows) of channel ch (slice idx).
 struct HHTile {
-  int32_t ch, k0, idx, rows, chunk, pad;
+  int32_t ch, k0, idx, rows;
+};
+// One element of X = V_hhhh + P: P's partials part[k * stride], k < nslices, the V_hhhh element
+// and where X (and, on the diagonal, s) goes (s < 0: off the diagonal).
+struct HHOut {
+  int64_t part;
+  int32_t nslices, stride, v, x, s, pad;
 };
 
-// Fused assembly, static data of strict packed row u (a < b) of a channel (index
-// qrow_off + u): offsets of rows ab and ba inside the channel block (ab * hh, ba * hh), the
-// operand-image indices of row ab (pk_idx: K index, packed row), particle indices a - np,
-// b - np, and e_a, e_b ...
+// Fused assembly, static data of strict packed row u (a < b) of a channel (index pk_off + u):
+// particle indices a - np, b - np, e_a, e_b, and the offsets of rows ab and ba inside the
+// channel block (ab * hh, ba * hh) ...
 struct QuadRow {
   int32_t o_ab, o_ba;
-  int32_t qx, qy;
   int32_t pa, pb;
   double ea, eb;
 };
@@ -207,11 +199,11 @@ struct QuadCol {
   double eij;
 };
 // Work item of the fused assembly: quads [q0, q1) (q = u * hk + w) of active channel ch, with
-// the channel's hk, block offset and table offsets (so a thread's table reads depend on the
-// item alone).
+// what its threads need of the channel (so their table reads depend on the item alone).
 struct QuadItem {
   int32_t ch, q0, q1, hk;
-  int64_t t_off, qrow_off, qcol_off;
+  int32_t hs, pad;
+  int64_t q_off, x_off, pk_off, qcol_off;
 };
 
 // Per active modified channel.
@@ -228,7 +220,8 @@ struct ElemRange {
   int64_t e0, e1;
 };
 
-// Kernel ids of the start-time trace (Control::trace_*).
+// Kernel ids of the start-time trace (Control::trace_*).  The FP64 ladder records every class
+// under kTrLadderThin; LadderMid, LadderWide, Retile and Reduce are unused.
 enum TraceKernel {
   kTrRingSmall = 0, kTrRingMid, kTrRingLarge, kTrHHSmall, kTrHHTiled, kTrOneBody, kTrLadderThin,
   kTrLadderMid, kTrLadderWide, kTrLadderTC, kTrAssemble, kTrLoopCtl, kTrEnergy, kTrRetile,
@@ -250,10 +243,8 @@ struct Control {
   int32_t error;         // bit flags, see kErr*
   int32_t active;        // 1 while a solve is running (0: kernels run unconditionally)
   int32_t phase;         // mixed-precision solve: 1 = split-bf16 ladder, 2 = FP64 polish
-  int32_t retile;        // the FP64 ladder operand tiles are stale (a mixed iteration ran)
-  int32_t inject;        // test-only fault: 1 = the first FP64 pp-ladder CTA of each class
-                         // withholds its first stage (its bounded waits run out)
-  int32_t pad0;
+  int32_t inject;        // test-only fault: 1 = the first FP64 pp-ladder CTA withholds its
+                         // first stage (its bounded waits run out)
   double polish_rel;     // phase 1 -> 2 once |dE| <= max(tol, polish_rel * |E|)
   int64_t polish_iters;  // iterations run in phase 2
   int64_t stop_at;       // device solve loop: one graph launch runs while iterations < stop_at

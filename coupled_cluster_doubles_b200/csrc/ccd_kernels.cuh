@@ -1,9 +1,9 @@
 // CCD iteration kernels for sm_100a (FP64 path).
 //
 // Reference correspondence (calc.cpp / Chain.hpp of justinlietz/coupled_cluster_doubles):
-//   pp_ladder_kernel        D = 0.5 T X + 0.5 V_pppp T              calc.cpp:162-202
-//                           (antisymmetry-packed, FP64 FMA pipe)
-//   hh_mma_kernel           X = V_hhhh + 0.5 V_hhpp T                calc.cpp:141-160
+//   pp_ladder_kernel        V_pppp T part of D = 0.5 T X + 0.5 V T   calc.cpp:162-202
+//                           (antisymmetry-packed; the assembly adds T X)
+//   hh_ladder_kernel        X = V_hhhh + 0.5 V_hhpp T                calc.cpp:141-160
 //   ring_*_kernel           Y = V_hphp + 0.5 V_hpph T'; R = T' Y     calc.cpp:264-313
 //   onebody_tables_kernel   calcChannelT2Diff_h2pp_h1 / _p2_p1hh     calc.cpp:9-25, 73-89
 //   onebody_fused_kernel    the same dot products, read from the ladder intermediates
@@ -71,21 +71,6 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t
       "l"(src), "r"(bytes), "r"(bar)
       : "memory");
 }
-// sum_k a[k*sa] * b[k*sb] for k < n with four interleaved partial sums (more independent FMA
-// chains in flight), combined in a fixed order.
-__device__ __forceinline__ double dot4(const double *a, int sa, const double *b, int sb, int n) {
-  double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-  int k = 0;
-  for (; k + 4 <= n; k += 4) {
-    s0 = fma(a[k * sa], b[k * sb], s0);
-    s1 = fma(a[(k + 1) * sa], b[(k + 1) * sb], s1);
-    s2 = fma(a[(k + 2) * sa], b[(k + 2) * sb], s2);
-    s3 = fma(a[(k + 3) * sa], b[(k + 3) * sb], s3);
-  }
-  for (; k < n; ++k) s0 = fma(a[k * sa], b[k * sb], s0);
-  return (s0 + s1) + (s2 + s3);
-}
-
 // Programmatic dependent launch: wait until the preceding kernel of the stream has completed
 // (its writes are visible), then allow the next kernel to begin launching once every CTA of
 // this grid is resident.  Both are no-ops for kernels launched without the PDL attribute.
@@ -123,154 +108,103 @@ __device__ __forceinline__ bool skip_iteration(const Control *ctl, int gate, int
 }
 
 // ------------------------------------------------------------------------------------------
-// pp ladder + hh-ladder output in FP64 (FMA pipe for thin channels, FP64 MMA for the rest):
-//   D[ab,:] = sum_{c<d} V[ab,cd] T[cd,:] + T[ab,:] (X/2)     for packed rows a <= b,
-//   D[ba,:] = -D[ab,:]                                        (antisymmetry of V and T).
-// Warp 4 is the producer: one lane streams pre-tiled A/B stages with bulk copies (TMA, no
-// multicast) into a kStages-deep shared-memory ring guarded by mbarriers.  The 128 consumer
-// threads run register-blocked DFMAs (thin channels: V rows from shared memory conflict-free
-// by an XOR swizzle, T / X columns as warp broadcasts) or FP64 MMAs (mid and wide channels).  K runs over the c<d pairs (V T) and then over
-// hh (T X) with the same pipeline.  Row blocks whose K is split over several tiles write
-// partial sums that ladder_reduce_kernel adds in segment order (deterministic).
+// pp ladder in FP64 (FMA pipe for thin channels, FP64 MMA for the rest) over the packed quads:
+//   D[u, w] = sum_c V[u, c] T[c, w]        (u = a<b, c = c<d, w = i<j)
+// Half of the hole columns and none of the a = b rows of the full antisymmetry-packed product,
+// and no T X: the product needs only the amplitudes, so it starts at the head of an iteration
+// beside the hh ladder and the ring instead of behind the hh ladder (the assembly adds T X).
+// It streams V once and is bound by that: one CTA per SM leaves registers and shared memory
+// for the other streams' kernels, and its five 17-22 KB stages (85-108 KB in flight) still
+// cover HBM's latency.
+// One producer warp: a lane claims tiles from a launch-wide counter (list sorted by class, wide
+// first, then by decreasing work: longest-first list scheduling that adapts to CTAs starting
+// late behind another stream's kernels) and streams pre-tiled A/B stages with bulk copies (TMA,
+// no multicast) into a kStages-deep shared-memory ring guarded by mbarriers, across tile
+// boundaries; beside each stage it leaves the tile's description for the consumers.  The 8
+// consumer warps run DFMAs (thin: two threads a row, T as broadcasts) or m16n8k16 FP64 MMAs.
+// All classes share one launch (EG N=54 |n|^2 <= 36, 566 MB of V: the three launches of the
+// hh-wide columns took 181 us one after another).
 // ------------------------------------------------------------------------------------------
 
-// Stores the finished values of packed row u_local (cols [c0, c0+n)), or its partial sum.
-struct LadderOut {
-  const LadderTile &tile;
-  const int32_t *rowmap, *mirror;
-  double *d, *part;
-  // N is a compile-time count so that v stays in registers (every index is a constant).
-  template <int N>
-  __device__ __forceinline__ void row(int u_local, int c0, const double (&v)[N]) const {
-    if (u_local >= tile.rows) return;
-    if (tile.nseg > 1) {
-      double *pp = part + tile.part_base + ((int64_t)tile.seg * tile.bm + u_local) * tile.nb + c0;
+// What the consumers need of the tile a stage belongs to.
+struct StageInfo {
+  int64_t out;
+  int32_t rows, hk, hs, nks;  // nks: K chunks of the tile; 0: no more tiles
+};
+
+// Thin tiles (hs = NB in {1, 2, 4}): two consumer threads per packed row, even and odd k.
+template <int NB>
+__device__ __forceinline__ void thin_chunk(const double *A, const double *B, int tid,
+                                           double (&acc)[NB]) {
+  const int row = tid >> 1, odd = tid & 1;
 #pragma unroll
-      for (int j = 0; j < N; ++j) pp[j] = v[j];
-      return;
-    }
-    const int u = tile.mt * tile.bm + u_local;
-    const int ab = rowmap[tile.row_off + u], mir = mirror[tile.row_off + u];
-    double *dr = d + tile.t_off + (int64_t)ab * tile.hh;
-    double *mr = d + tile.t_off + (int64_t)mir * tile.hh;
+  for (int j = 0; j < kBK / 2; ++j) {
+    const int k = 2 * j + odd;
+    const double a = A[swzA(row, k)];
+    if constexpr (NB == 1) {
+      acc[0] = fma(a, B[k], acc[0]);
+    } else {
+      const double2 *bp = reinterpret_cast<const double2 *>(B + k * NB);
 #pragma unroll
-    for (int j = 0; j < N; ++j) {
-      if (c0 + j < tile.hh) {
-        dr[c0 + j] = v[j];
-        if (mir >= 0) mr[c0 + j] = -v[j];
+      for (int q = 0; q < NB / 2; ++q) {
+        const double2 b = bp[q];
+        acc[2 * q] = fma(a, b.x, acc[2 * q]);
+        acc[2 * q + 1] = fma(a, b.y, acc[2 * q + 1]);
       }
     }
   }
-};
-
-// Split-K partial sums of a row block, added in segment order by ladder_reduce_kernel after the
-// ladder: item = (first tile of the row block, first row of a kRedRows-row chunk).
-struct RedItem {
-  int32_t tile, r0;
-};
-constexpr int kRedRows = 16;
-
-// D rows of split row blocks: sum of the segments' partials in segment order (deterministic),
-// written to row ab and negated to its mirror ba.  Fully parallel over (row block, row chunk).
-__global__ void __launch_bounds__(256)
-ladder_reduce_kernel(const RedItem *__restrict__ items, const LadderTile *__restrict__ tiles,
-                     const int32_t *__restrict__ rowmap, const int32_t *__restrict__ mirror,
-                     double *__restrict__ d, const double *__restrict__ part, const Control *ctl,
-                     int gate) {
-  if (skip_iteration(ctl, gate, kTrReduce)) return;
-  const RedItem it = items[blockIdx.x];
-  const LadderTile tile = tiles[it.tile];
-  const int nr = min(kRedRows, tile.rows - it.r0), n = nr * tile.nb;
-  for (int e = threadIdx.x; e < n; e += blockDim.x) {
-    const int u_local = it.r0 + e / tile.nb, col = e % tile.nb;
-    if (col >= tile.hh) continue;
-    // Eight segments' loads in flight together, then added in segment order.
-    const double *pc = part + tile.part_base + (int64_t)u_local * tile.nb + col;
-    const int64_t seg_stride = (int64_t)tile.bm * tile.nb;
-    double v = 0.0;
-    int sg = 0;
-    for (; sg + 8 <= tile.nseg; sg += 8) {
-      double x[8];
-#pragma unroll
-      for (int k = 0; k < 8; ++k) x[k] = pc[(int64_t)(sg + k) * seg_stride];
-#pragma unroll
-      for (int k = 0; k < 8; ++k) v += x[k];
-    }
-    for (; sg < tile.nseg; ++sg) v += pc[(int64_t)sg * seg_stride];
-    const int u = tile.mt * tile.bm + u_local;
-    const int ab = rowmap[tile.row_off + u], mir = mirror[tile.row_off + u];
-    d[tile.t_off + (int64_t)ab * tile.hh + col] = v;
-    if (mir >= 0) d[tile.t_off + (int64_t)mir * tile.hh + col] = -v;
-  }
-  trace_end(ctl, kTrReduce);
 }
 
-// Thin channels (nb in {2,4,8}): consumer thread = one packed row, all nb columns.
-// bstage: doubles between consecutive B stages (the producer's layout).
+// The consumer side of one tile: its chunks from the stage ring, then its D rows.  gc: chunks
+// this CTA has consumed so far.  False: a wait ran out (the tile's rows stay unwritten).
 template <int NB>
-__device__ __forceinline__ bool consume_thin(const LadderTile &tile, const double *As,
-                                             const double *Bs, int bstage, uint64_t *bars,
-                                             int tid, const LadderOut &out, int32_t *err,
-                                             int gc0) {
-  const int lane = tid & 31;
+__device__ __forceinline__ bool consume_thin(const StageInfo &ti, const double *As,
+                                             const double *Bs, uint64_t *bars, int tid, int gc,
+                                             double *__restrict__ d) {
   double acc[NB];
 #pragma unroll
   for (int j = 0; j < NB; ++j) acc[j] = 0.0;
-  const int nchunks = tile.nks + tile.nkh;
-  for (int c = 0; c < nchunks; ++c) {
-    const int gch = gc0 + c, s = gch % kStages;  // chunk number gch of this CTA
-    if (!mbar_wait(smem_u32(&bars[s]), (gch / kStages) & 1)) {
-      atomicOr(err, kErrTimeout);
-      return false;
-    }
-    const double *A = As + s * (kMaxAS * kBK);
-    const double *B = Bs + s * bstage;
-#pragma unroll
-    for (int k = 0; k < kBK; ++k) {
-      const double a = A[swzA(tid, k)];
-      const double2 *bp = reinterpret_cast<const double2 *>(B + k * NB);
-#pragma unroll
-      for (int j = 0; j < NB / 2; ++j) {
-        const double2 b = bp[j];
-        acc[2 * j] = fma(a, b.x, acc[2 * j]);
-        acc[2 * j + 1] = fma(a, b.y, acc[2 * j + 1]);
-      }
-    }
+  for (int c = 0; c < ti.nks; ++c) {
+    const int g = gc + c, s = g % kStages;
+    if (!mbar_wait(smem_u32(&bars[s]), (g / kStages) & 1)) return false;
+    if ((tid >> 1) < ti.rows)
+      thin_chunk<NB>(As + s * (kMaxAS * kBK), Bs + s * (kBK * kMaxNB), tid, acc);
     __syncwarp();
-    if (lane == 0) mbar_arrive(smem_u32(&bars[kStages + s]));
+    if ((tid & 31) == 0) mbar_arrive(smem_u32(&bars[kStages + s]));
   }
-  out.row<NB>(tid, 0, acc);
+#pragma unroll
+  for (int j = 0; j < NB; ++j) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], 1);
+  if (!(tid & 1) && (tid >> 1) < ti.rows) {
+    double *o = d + ti.out + (int64_t)(tid >> 1) * NB;
+#pragma unroll
+    for (int j = 0; j < NB; ++j)
+      if (j < ti.hk) o[j] = acc[j];
+  }
   return true;
 }
 
-// Mid and wide channels (nb = 8*C, C = 2..9) on the FP64 MMA: consumer warp w owns tile rows
-// [16w, 16w + 16), one m16n8k16 per 8-column tile and stage (kBK = 16), 4*C accumulators per
-// lane.  A (k-major, row stride ar) and B (k-major, row stride bs) fragments come from the
-// stage conflict-free: both strides are 4 mod 8 doubles.  A warp whose lower 8-row half has
-// no rows feeds zeros there instead of reading past the tile.
+// Wider tiles on the FP64 MMA: consumer warp w owns tile rows [16w, 16w + 16), one m16n8k16
+// per 8-column tile and stage (kBK = 16), 4 C accumulators per lane.  A (k-major, row stride
+// ar) and B (k-major, row stride hs) fragments come from the stage conflict-free: both strides
+// are 4 mod 8 doubles.  A warp whose lower 8-row half has no rows feeds zeros there instead of
+// reading past the tile; columns past hk (the stage's next row, or stale) are not stored.
 template <int C>
-__device__ __forceinline__ bool consume_mma(const LadderTile &tile, const double *As,
-                                            const double *Bs, int bstage, uint64_t *bars,
-                                            int tid, const LadderOut &out, int32_t *err,
-                                            int gc0) {
+__device__ __forceinline__ bool consume_mma(const StageInfo &ti, const double *As,
+                                            const double *Bs, uint64_t *bars, int tid, int gc,
+                                            double *__restrict__ d) {
   static_assert(kBK == 16, "one m16n8k16 K step per stage");
-  constexpr int NB = 8 * C, BS = NB + 4;
   const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  const int ar = ladder_arows(NB, tile.rows);
-  const int halves = min(2, max(0, ((tile.rows + 7) >> 3) - 2 * warp));  // 8-row halves with rows
+  const int ar = ladder_arows(ti.hs, ti.rows), hs = ti.hs;
+  const int halves = min(2, max(0, ((ti.rows + 7) >> 3) - 2 * warp));  // 8-row halves with rows
   double acc[C][4];
 #pragma unroll
   for (int j = 0; j < C; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0;
-  const int nchunks = tile.nks + tile.nkh;
-  for (int c = 0; c < nchunks; ++c) {
-    const int gch = gc0 + c, s = gch % kStages;  // chunk number gch of this CTA
-    if (!mbar_wait(smem_u32(&bars[s]), (gch / kStages) & 1)) {
-      atomicOr(err, kErrTimeout);
-      return false;
-    }
+  for (int c = 0; c < ti.nks; ++c) {
+    const int gch = gc + c, s = gch % kStages;
+    if (!mbar_wait(smem_u32(&bars[s]), (gch / kStages) & 1)) return false;
     if (halves > 0) {
       const double *A = As + s * (kMaxAS * kBK) + t * ar + 16 * warp + g;
-      const double *B = Bs + s * bstage + t * BS + g;
+      const double *B = Bs + s * (kBK * kMaxNB) + t * hs + g;
       double a[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i)
@@ -279,46 +213,37 @@ __device__ __forceinline__ bool consume_mma(const LadderTile &tile, const double
       for (int j = 0; j < C; ++j) {
         double b[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) b[q] = B[4 * q * BS + 8 * j];
+        for (int q = 0; q < 4; ++q) b[q] = B[4 * q * hs + 8 * j];
         dmma_16816(acc[j], a, b);
       }
     }
     __syncwarp();
     if (lane == 0) mbar_arrive(smem_u32(&bars[kStages + s]));
   }
-  if (halves > 0) {
 #pragma unroll
-    for (int j = 0; j < C; ++j) {
-      const double lo[2] = {acc[j][0], acc[j][1]}, hi[2] = {acc[j][2], acc[j][3]};
-      out.row<2>(16 * warp + g, 8 * j + 2 * t, lo);
-      if (halves > 1) out.row<2>(16 * warp + 8 + g, 8 * j + 2 * t, hi);
+  for (int j = 0; j < C; ++j)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int r = 16 * warp + g + 8 * (q >> 1), col = 8 * j + 2 * t + (q & 1);
+      if (r < ti.rows && col < ti.hk) d[ti.out + (int64_t)r * hs + col] = acc[j][q];
     }
-  }
   return true;
 }
 
-// Column classes: CLS 0 = thin (nb <= 8), 1 = mid (nb 16..32), 2 = wide (nb 40..72).  Separate
-// instantiations keep the register budget of narrow channels independent of the 72-column case.
-// Persistent CTAs: CTA b runs tiles cta_off[b] .. cta_off[b+1] (a balanced assignment made on the
-// host); the producer streams K chunks through the stage ring across tile boundaries and the
-// consumers write each tile's rows when its last chunk is done.
-template <int CLS>
-__global__ void __launch_bounds__(ladder_threads(CLS), CLS == 0 ? 3 : CLS == 1 ? 2 : 1)
-pp_ladder_kernel(const LadderTile *__restrict__ tiles, const int32_t *__restrict__ cta_off,
-                 const double *__restrict__ v_t, const double *__restrict__ t_kt,
-                 const double *__restrict__ t_mt, const double *__restrict__ x_t,
-                 const int32_t *__restrict__ rowmap, const int32_t *__restrict__ mirror,
-                 double *__restrict__ d, double *part, const Control *ctl, int32_t *err,
-                 int gate) {
-  if (skip_iteration(ctl, gate, kTrLadderThin + CLS)) return;
+constexpr size_t kLadderSmem =
+    (size_t)kStages * (kMaxAS * kBK + kBK * kMaxNB) * 8 + kStages * sizeof(StageInfo) +
+    2 * kStages * 8 + kBK * 8;  // slack: the last B stage's fragment loads past hs
+__global__ void __launch_bounds__(kLadderThreads)
+pp_ladder_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *sched,
+                 const double *__restrict__ v_t, const double *tq0, const double *tq1,
+                 double *__restrict__ d, const Control *ctl, int32_t *err, int gate) {
+  if (skip_iteration(ctl, gate, kTrLadderThin)) return;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   double *As = reinterpret_cast<double *>(smem_raw);
   double *Bs = As + kStages * kMaxAS * kBK;
-  constexpr bool WIDE = CLS > 0;
-  constexpr int kConsumerWarps = (ladder_threads(CLS) - 32) / 32;
-  const int bstage = WIDE ? kBK * kMaxBS : kBK * 8;
-  uint64_t *bars = reinterpret_cast<uint64_t *>(Bs + kStages * bstage);
-  const int t_begin = cta_off[blockIdx.x], t_end = cta_off[blockIdx.x + 1];
+  StageInfo *info = reinterpret_cast<StageInfo *>(Bs + kStages * kBK * kMaxNB + kBK);
+  uint64_t *bars = reinterpret_cast<uint64_t *>(info + kStages);  // full, then empty
+  constexpr int kConsumerWarps = kLadderConsumers / 32;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
@@ -331,127 +256,103 @@ pp_ladder_kernel(const LadderTile *__restrict__ tiles, const int32_t *__restrict
 
   if (warp == kConsumerWarps) {
     if (lane == 0) {
+      const double *t_q = ctl->parity ? tq1 : tq0;
       int gc = 0;  // chunks issued by this CTA
       bool stop = false;
       // Test-only fault (ccdgpu_inject_wait_timeout): CTA 0 never fills its first stage, so
       // its consumers' bounded waits run out, then this producer's wait for that stage does.
       const bool withhold = ctl->inject != 0 && blockIdx.x == 0;
-      for (int ti = t_begin; ti < t_end && !stop; ++ti) {
+      auto free_stage = [&]() {  // the stage of chunk gc may be filled
+        if (gc < kStages ||
+            mbar_wait(smem_u32(&bars[kStages + gc % kStages]), ((gc / kStages) - 1) & 1))
+          return true;
+        atomicOr(err, kErrTimeout);
+        return false;
+      };
+      int ti = blockIdx.x;  // the first tile needs no claim (grid <= n_tiles)
+      while (ti < n_tiles && !stop) {
         const LadderTile tile = tiles[ti];
-        const int ar = ladder_arows(tile.nb, tile.rows);
-        const int bs = ladder_bs(tile.nb), af = ladder_arows_full(tile.nb);
-        const uint32_t abytes = ar * kBK * 8, bbytes = kBK * bs * 8;
-        const int nchunks = tile.nks + tile.nkh;
-        const int64_t vtile = tile.v_base + (int64_t)tile.mt * af * tile.nkc * kBK;
-        const int64_t ttile = tile.tmt_base + (int64_t)tile.mt * af * tile.nkh * kBK;
-        for (int c = 0; c < nchunks; ++c, ++gc) {
+        // The next claim's latency hides behind this tile.
+        ti = (int)gridDim.x + atomicAdd(&sched[0], 1);
+        const uint32_t abytes = ladder_arows(tile.hs, tile.rows) * kBK * 8;
+        const uint32_t bbytes = kBK * tile.hs * 8;
+        const double *asrc = v_t + tile.a_base, *bsrc = t_q + tile.b_base;
+        for (int c = 0; c < tile.nks; ++c, ++gc) {
           const int s = gc % kStages;
-          if (gc >= kStages &&
-              !mbar_wait(smem_u32(&bars[kStages + s]), ((gc / kStages) - 1) & 1)) {
-            atomicOr(err, kErrTimeout);
+          if (!free_stage()) {
             stop = true;
             break;
           }
           if (withhold && gc == 0) continue;
-          const double *asrc, *bsrc;
-          if (c < tile.nks) {
-            const int kc = tile.kc0 + c;
-            asrc = v_t + vtile + (int64_t)kc * ar * kBK;
-            bsrc = t_kt + tile.tkt_base + (int64_t)kc * kBK * bs;
-          } else {
-            const int kh = c - tile.nks;
-            asrc = t_mt + ttile + (int64_t)kh * ar * kBK;
-            bsrc = x_t + tile.xt_base + (int64_t)kh * kBK * bs;
-          }
+          if (c == 0) info[s] = StageInfo{tile.out, tile.rows, tile.hk, tile.hs, tile.nks};
           const uint32_t full = smem_u32(&bars[s]);
           mbar_expect_tx(full, abytes + bbytes);
-          bulk_g2s(smem_u32(As + s * kMaxAS * kBK), asrc, abytes, full);
-          bulk_g2s(smem_u32(Bs + s * bstage), bsrc, bbytes, full);
+          bulk_g2s(smem_u32(As + s * kMaxAS * kBK), asrc + c * (abytes / 8), abytes, full);
+          bulk_g2s(smem_u32(Bs + s * kBK * kMaxNB), bsrc + c * (bbytes / 8), bbytes, full);
         }
+      }
+      if (!stop && free_stage()) {  // the end marker
+        info[gc % kStages].nks = 0;
+        mbar_arrive(smem_u32(&bars[gc % kStages]));
+      }
+      // The last producer to finish (each has made its last claim) resets the counters for
+      // the next launch.
+      __threadfence();
+      if (atomicAdd(&sched[1], 1) == (int)gridDim.x - 1) {
+        sched[0] = 0;
+        sched[1] = 0;
+        __threadfence();
       }
     }
     return;
   }
   const int tid = threadIdx.x;
   int gc = 0;
-  for (int ti = t_begin; ti < t_end; ++ti) {
-    const LadderTile tile = tiles[ti];
-    const LadderOut out{tile, rowmap, mirror, d, part};
+  for (;;) {
+    // The first chunk's stage describes the tile.
+    const int s = gc % kStages;
+    if (!mbar_wait(smem_u32(&bars[s]), (gc / kStages) & 1)) {
+      atomicOr(err, kErrTimeout);
+      break;
+    }
+    const StageInfo ti = info[s];
+    if (ti.nks == 0) break;
     bool ok = true;
-    if (!WIDE) {
-      switch (tile.nb) {
-        case 2: ok = consume_thin<2>(tile, As, Bs, bstage, bars, tid, out, err, gc); break;
-        case 4: ok = consume_thin<4>(tile, As, Bs, bstage, bars, tid, out, err, gc); break;
-        default: ok = consume_thin<8>(tile, As, Bs, bstage, bars, tid, out, err, gc); break;
+    if (ti.hs <= 4) {
+      switch (ti.hs) {
+        case 1: ok = consume_thin<1>(ti, As, Bs, bars, tid, gc, d); break;
+        case 2: ok = consume_thin<2>(ti, As, Bs, bars, tid, gc, d); break;
+        default: ok = consume_thin<4>(ti, As, Bs, bars, tid, gc, d); break;
       }
     } else {
-#define CCD_WIDE8_CASE(n) \
-  case n: ok = consume_mma<n>(tile, As, Bs, bstage, bars, tid, out, err, gc); break;
-      if (CLS == 1) {
-        switch (tile.nb / 8) { CCD_WIDE8_CASE(2) CCD_WIDE8_CASE(3) CCD_WIDE8_CASE(4) default: break; }
-      } else {
-        switch (tile.nb / 8) {
-          CCD_WIDE8_CASE(5) CCD_WIDE8_CASE(6) CCD_WIDE8_CASE(7) CCD_WIDE8_CASE(8) CCD_WIDE8_CASE(9)
-          default: break;
-        }
-      }
-#undef CCD_WIDE8_CASE
-    }
-    if (!ok) break;  // a timed-out tile leaves its row block unfinished (error already set)
-    gc += tile.nks + tile.nkh;
-  }
-  trace_end(ctl, kTrLadderThin + CLS);
-}
-
-// ------------------------------------------------------------------------------------------
-// Register-tiled outer-product micro-GEMM for the small per-channel FP64 products:
-//   acc[i][j] += sum_k A[k*lda + r0 + i] * B[k*ldb + c0 + j],   i, j < TM.
-// Both operands are k-row major in shared memory, so a thread reads its TM-wide slices with
-// 16-byte loads (TM even: lda, ldb and r0, c0 even).  Slices may run past the valid rows or
-// columns (and past the last row into padding); those accumulators are never stored.
-// ------------------------------------------------------------------------------------------
-template <int TM>
-__device__ __forceinline__ void opgemm(const double *__restrict__ A, int lda,
-                                       const double *__restrict__ B, int ldb, int K, int r0,
-                                       int c0, double (&acc)[TM][TM]) {
-  const double *a = A + r0, *b = B + c0;
-#pragma unroll 2
-  for (int k = 0; k < K; ++k) {
-    double av[TM], bv[TM];
-    if constexpr (TM % 2 == 0) {
-#pragma unroll
-      for (int i = 0; i < TM / 2; ++i) {
-        const double2 x = *reinterpret_cast<const double2 *>(a + 2 * i);
-        const double2 y = *reinterpret_cast<const double2 *>(b + 2 * i);
-        av[2 * i] = x.x;
-        av[2 * i + 1] = x.y;
-        bv[2 * i] = y.x;
-        bv[2 * i + 1] = y.y;
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < TM; ++i) {
-        av[i] = a[i];
-        bv[i] = b[i];
+      switch ((ti.hk + 7) / 8) {
+        case 1: ok = consume_mma<1>(ti, As, Bs, bars, tid, gc, d); break;
+        case 2: ok = consume_mma<2>(ti, As, Bs, bars, tid, gc, d); break;
+        case 3: ok = consume_mma<3>(ti, As, Bs, bars, tid, gc, d); break;
+        case 4: ok = consume_mma<4>(ti, As, Bs, bars, tid, gc, d); break;
+        default: ok = consume_mma<5>(ti, As, Bs, bars, tid, gc, d); break;
       }
     }
-#pragma unroll
-    for (int i = 0; i < TM; ++i)
-#pragma unroll
-      for (int j = 0; j < TM; ++j) acc[i][j] = fma(av[i], bv[j], acc[i][j]);
-    a += lda;
-    b += ldb;
+    if (!ok) {  // a timed-out tile leaves its rows unfinished
+      atomicOr(err, kErrTimeout);
+      break;
+    }
+    gc += ti.nks;
   }
+  trace_end(ctl, kTrLadderThin);
 }
-__host__ __device__ inline int even_up(int n) { return (n + 1) & ~1; }
 
-// cp.async (8- and 4-byte) global -> shared copies, committed and waited for by group.
+// cp.async (4-, 8- and 16-byte) global -> shared copies, committed and waited for by group.
 __device__ __forceinline__ void cp_async8(void *dst, const void *src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src)
                : "memory");
 }
 __device__ __forceinline__ void cp_async4(void *dst, const void *src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src)
                : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() {
@@ -463,305 +364,222 @@ __device__ __forceinline__ void cp_async_wait() {
 }
 
 // ------------------------------------------------------------------------------------------
-// hh ladder intermediate (calc.cpp:141-160 and the one-body sums of calc.cpp:18-20, 82-84):
-//   P = V_hhpp T (K = pp),  X = V_hhhh + 0.5 P  (reference layout, and X/2 as B tiles),
-//   s[IJ] = P[IJ][IJ],  r[AB] = sum_IJ V[IJ][AB] T[AB][IJ].
-// V_hhpp is held transposed (pp x hh), so a K slice of V and of T are contiguous row ranges.
-// hh_mma_kernel: one warp per (slice of kHHRows pp rows, chunk of P rows) on the FP64 MMA,
-// fragments loaded straight from global memory (8 consecutive columns of 4 rows per load);
-// rows past the slice and columns past hh read as zero.  The warp of chunk 0 also forms the
-// row dots r from the same fragments.  Each slice writes its partial P; hh_reduce_kernel adds
-// the partials in slice order (deterministic) and finishes X, its operand tiles and s.
+// hh ladder intermediate (calc.cpp:141-160 and the one-body sums of calc.cpp:18-20, 82-84) over
+// the packed quads:
+//   X[kl, ij] = V_hhhh[kl, ij] + P[kl, ij],  P = sum_u V[u, kl] T[u, ij]   (k<l, i<j, u = a<b;
+//               0.5 of the sum over all ordered pairs ab),
+//   s[ij] = P[ij][ij],  r[u] = sum_ij V[u, ij] T[u, ij],
+// a quarter of the reads and an eighth of the products of the ordered pairs.  V_hhpp is held in
+// the packed layout of T, so a K slice of either is one contiguous range.
+// hh_ladder_kernel: CTAs of two kinds in one launch.
+//   hk <= 8: a warp per slice of kHHRows rows, its m8n8k4 fragments loaded straight from global
+//   memory (8 consecutive columns of 4 rows a load, all loads of the slice in flight at once);
+//   wider: a CTA per slice of kHHRowsL rows, both ranges copied to shared memory (16-byte
+//   cp.async; the row stride hs is 4 mod 8 doubles, conflict-free for the fragments) and P on
+//   m16n8k16, warp w taking items of one 16-row tile by kHHNC 8-column tiles.
+// Both form the row dots r, and write the slice's partial P, which hh_reduce_kernel adds in
+// slice order (deterministic).  Bound by latency: 12 MB of operands at EG N=54 |n|^2 <= 36,
+// where the ordered pairs' 47 MB and hh^2 outputs took 15 + 19 us.
 // ------------------------------------------------------------------------------------------
-constexpr int kHHWarps = 8;
-constexpr int kHHRows = 32;  // pp rows of one K slice
+constexpr int kHHRows = 32;       // packed rows of a warp's slice (hk <= 8)
+constexpr int kHHRowsL = 64;      // ... of a CTA's slice
+constexpr int kHHThreads = 256;
+constexpr int kHHNC = 2;
+__host__ __device__ inline int hh_rows(int hk) { return hk <= 8 ? kHHRows : kHHRowsL; }
+// Slack: fragment loads of the rows and columns past hk in the last row.
+constexpr size_t kHHSmem = (2 * (size_t)kHHRowsL * kMaxNB + 16) * sizeof(double);
 
-// X, its X/2 operand tiles (FP64 and, for a mixed iteration, bf16 terms) and s from one
-// finished element P[kl][ij].
-__device__ __forceinline__ void hh_finish(const ChanInfo &ch, int kl, int ij, double p,
-                                          const double *__restrict__ v_hhhh, double *x_ref,
-                                          double *x_t, double *s_out, __nv_bfloat16 *xt_tc,
-                                          int64_t xt_tc_stride, int nt) {
-  const int hh = ch.hh, idx = kl * hh + ij;
-  const double x = v_hhhh[ch.x_off + idx] + 0.5 * p;
-  x_ref[ch.x_off + idx] = x;
-  const int bs = ladder_bs(ch.nb);
-  x_t[ch.xt_base + (int64_t)(kl / kBK) * kBK * bs + (kl % kBK) * bs + ij] = 0.5 * x;
-  if (nt) {
-    const int64_t o =
-        ch.xt_tc_base + (int64_t)(kl >> 5) * (ch.nbt >> 3) * kTcGroup + tc_off_mn(ij, kl & 31);
-    if (nt == 3) {
-      __nv_bfloat16 hv[3];
-      split_bf16_n<3>(0.5 * x, hv);
-#pragma unroll
-      for (int q = 0; q < 3; ++q) xt_tc[q * xt_tc_stride + o] = hv[q];
-    } else {
-      __nv_bfloat16 hv[2];
-      split_bf16_n<2>(0.5 * x, hv);
-#pragma unroll
-      for (int q = 0; q < 2; ++q) xt_tc[q * xt_tc_stride + o] = hv[q];
-    }
-  }
-  if (kl == ij) s_out[ch.hh_off + ij] = p;
-}
-
-// NMAX = column tiles of 8 held per warp: 2 for hh <= 16 (MC = 2 row tiles per warp, the whole
-// P), kMaxCG for the rest (MC = 1 row tile per warp).
-template <int NMAX>
-__global__ void __launch_bounds__(kHHWarps * 32, NMAX <= 2 ? 4 : 2)
-hh_mma_kernel(const HHTile *__restrict__ tiles, int n, const ChanInfo *__restrict__ chans,
-              const double *__restrict__ v_pphh, const double *tbuf0, const double *tbuf1,
-              double *__restrict__ part, double *__restrict__ r_out, const Control *ctl,
-              int gate) {
-  if (skip_iteration(ctl, gate, NMAX <= 2 ? kTrHHSmall : kTrHHTiled)) return;
-  const int u = blockIdx.x * kHHWarps + (threadIdx.x >> 5);
-  if (u >= n) return;
-  const HHTile tt = tiles[u];
-  const ChanInfo ch = chans[tt.ch];
-  const double *t_old = ctl->parity ? tbuf1 : tbuf0;
-  const int hh = ch.hh, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  constexpr int MC = NMAX <= 2 ? 2 : 1;
-  const int h8 = (hh + 7) >> 3, mc0 = MC * tt.chunk, mc = min(MC, h8 - mc0);
-  const bool do_dot = tt.chunk == 0;
-  const double *vb = v_pphh + ch.t_off + (int64_t)tt.k0 * hh;
-  const double *tb = t_old + ch.t_off + (int64_t)tt.k0 * hh;
-  double acc[MC][NMAX][2];
-#pragma unroll
-  for (int m = 0; m < MC; ++m)
-#pragma unroll
-    for (int c = 0; c < NMAX; ++c) acc[m][c][0] = acc[m][c][1] = 0.0;
-  // hh <= 16: all kHHRows / 4 steps unrolled, so that every fragment load of the slice is issued
-  // at once (rows past the slice read as zero); wider hh: two steps at a time (registers).
+__device__ __forceinline__ void hh_warp_unit(const HHTile &tt, const ChanInfo &ch,
+                                             const double *__restrict__ vq, const double *tq,
+                                             double *__restrict__ part,
+                                             double *__restrict__ r_out) {
+  const int hk = ch.hk, hs = ch.hs, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int64_t base = ch.q_off + (int64_t)tt.k0 * hs + g;
   constexpr int kSteps = kHHRows / 4;
-#pragma unroll(NMAX <= 2 ? kSteps : 2)
+  double a[kSteps], b[kSteps], acc[2] = {0.0, 0.0};
+#pragma unroll
   for (int k4 = 0; k4 < kSteps; ++k4) {
     const int k = 4 * k4 + t;
-    const bool kin = k < tt.rows;
-    const double *vr = vb + (int64_t)k * hh, *tr = tb + (int64_t)k * hh;
-    double a[MC], b[NMAX];
-#pragma unroll
-    for (int m = 0; m < MC; ++m) {
-      const int col = (mc0 + m) * 8 + g;
-      a[m] = (kin && col < hh) ? vr[col] : 0.0;
-    }
-#pragma unroll
-    for (int c = 0; c < NMAX; ++c) {
-      const int col = c * 8 + g;
-      b[c] = (kin && col < hh) ? tr[col] : 0.0;
-    }
-#pragma unroll
-    for (int m = 0; m < MC; ++m)
-#pragma unroll
-      for (int c = 0; c < NMAX; ++c)
-        if (m < mc && c < h8) dmma_884(acc[m][c], a[m], b[c]);
-    if (do_dot) {
-      // Row k: lane partial over columns 8c + g, then a fixed butterfly over g.
-      double d = 0.0;
-#pragma unroll
-      for (int c = 0; c < NMAX; ++c) {
-        const int col = c * 8 + g;
-        const double v = c < MC ? a[c] : ((kin && col < hh) ? vr[col] : 0.0);
-        d = fma(v, b[c], d);
-      }
-      d += __shfl_xor_sync(0xffffffffu, d, 4);
-      d += __shfl_xor_sync(0xffffffffu, d, 8);
-      d += __shfl_xor_sync(0xffffffffu, d, 16);
-      if (g == 0 && kin) r_out[ch.pp_off + tt.k0 + k] = d;
-    }
+    const bool in = k < tt.rows && g < hk;
+    a[k4] = in ? vq[base + k * hs] : 0.0;
+    b[k4] = in ? tq[base + k * hs] : 0.0;
   }
-  double *pb = part + ch.part_off + (int64_t)tt.idx * hh * hh;
 #pragma unroll
-  for (int m = 0; m < MC; ++m)
+  for (int k4 = 0; k4 < kSteps; ++k4) {
+    dmma_884(acc, a[k4], b[k4]);
+    double d = a[k4] * b[k4];  // row dot: a fixed butterfly over the columns
+    d += __shfl_xor_sync(0xffffffffu, d, 4);
+    d += __shfl_xor_sync(0xffffffffu, d, 8);
+    d += __shfl_xor_sync(0xffffffffu, d, 16);
+    if (g == 0 && 4 * k4 + t < tt.rows) r_out[ch.pk_off + tt.k0 + 4 * k4 + t] = d;
+  }
 #pragma unroll
-    for (int c = 0; c < NMAX; ++c) {
-      const int kl = (mc0 + m) * 8 + g, ij = c * 8 + 2 * t;
-      if (m < mc && c < h8 && kl < hh) {
-        if (ij < hh) pb[kl * hh + ij] = acc[m][c][0];
-        if (ij + 1 < hh) pb[kl * hh + ij + 1] = acc[m][c][1];
-      }
-    }
-  trace_end(ctl, NMAX <= 2 ? kTrHHSmall : kTrHHTiled);
+  for (int q = 0; q < 2; ++q)
+    if (g < hk && 2 * t + q < hk) part[g * hk + 2 * t + q] = acc[q];
 }
 
-// Channels with hh > 16: one CTA per K slice of kHHRowsL pp rows.  The slice's rows of V_pphh
-// and T (two contiguous ranges of rows * hh doubles) go to shared memory with cp.async, all in
-// flight at once, at a row stride of hh rounded up to 16, plus 4 (4 mod 16 doubles:
-// conflict-free fragment loads); rows up to the next multiple of 16 and columns up to the
-// padded width are zero.  P = V^T T runs on the FP64 m16n8k16 MMA: warp w takes items of one
-// 16-row tile of P by kHHNC 8-column tiles, at most four k-steps per slice, so T is read from
-// HBM once per slice and the accumulator chains are short; the warps then form the slice's
-// row dots r (lanes over the columns, a fixed butterfly).  Partial P per slice as for
-// hh_mma_kernel.
-constexpr int kHHRowsL = 64;
-constexpr int kHHSliceThreads = 256;
-constexpr int kHHNC = 4;
-__host__ __device__ inline int hh_slice_ld(int hh) { return ((hh + 15) & ~15) + 4; }
-__host__ __device__ inline size_t hh_slice_smem(int hh) {
-  return (size_t)2 * kHHRowsL * hh_slice_ld(hh) * sizeof(double);
-}
-__global__ void __launch_bounds__(kHHSliceThreads, 3)
-hh_slice_kernel(const HHTile *__restrict__ tiles, const ChanInfo *__restrict__ chans,
-                const double *__restrict__ v_pphh, const double *tbuf0, const double *tbuf1,
-                double *__restrict__ part, double *__restrict__ r_out, const Control *ctl,
-                int gate) {
-  if (skip_iteration(ctl, gate, kTrHHTiled)) return;
-  extern __shared__ __align__(16) double hs_smem[];
-  const HHTile tt = tiles[blockIdx.x];
-  const ChanInfo &ch = chans[tt.ch];
-  const double *t_old = ctl->parity ? tbuf1 : tbuf0;
-  const int hh = ch.hh, ld = hh_slice_ld(hh), hh16 = ld - 4;
-  const int rows = tt.rows, rows16 = (rows + 15) & ~15;
-  double *Vs = hs_smem, *Ts = hs_smem + kHHRowsL * ld;
-  const int64_t base = ch.t_off + (int64_t)tt.k0 * hh;
-  const double *vb = v_pphh + base, *tb = t_old + base;
-  // A warp per row, lanes over the columns (no integer division); columns [hh, hh16) and rows
-  // [rows, rows16) are zero.
+__device__ __forceinline__ void hh_cta_unit(const HHTile &tt, const ChanInfo &ch,
+                                            const double *__restrict__ vq, const double *tq,
+                                            double *__restrict__ part,
+                                            double *__restrict__ r_out, double *sm) {
+  const int hk = ch.hk, hs = ch.hs, rows = tt.rows, rows16 = (rows + 15) & ~15;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  for (int k = warp; k < rows16; k += kHHSliceThreads / 32) {
-    for (int c = lane; c < hh16; c += 32) {
-      if (k < rows && c < hh) {
-        cp_async8(Vs + k * ld + c, vb + (int64_t)k * hh + c);
-        cp_async8(Ts + k * ld + c, tb + (int64_t)k * hh + c);
-      } else {
-        Vs[k * ld + c] = 0.0;
-        Ts[k * ld + c] = 0.0;
-      }
-    }
+  double *Vs = sm, *Ts = sm + rows16 * hs;
+  const int64_t base = ch.q_off + (int64_t)tt.k0 * hs;
+  // Rows up to the next multiple of 16 are the block's zero padding, which is copied too.
+  for (int e = 2 * threadIdx.x; e < rows16 * hs; e += 2 * kHHThreads) {
+    cp_async16(Vs + e, vq + base + e);
+    cp_async16(Ts + e, tq + base + e);
   }
   cp_async_commit();
   cp_async_wait<0>();
   __syncthreads();
-  double *pb = part + ch.part_off + (int64_t)tt.idx * hh * hh;
-  const int n8 = (hh + 7) >> 3, nch = (n8 + kHHNC - 1) / kHHNC, items = (hh16 >> 4) * nch;
-  for (int it = warp; it < items; it += kHHSliceThreads / 32) {
+  const int n8 = (hk + 7) >> 3, nch = (n8 + kHHNC - 1) / kHHNC, items = ((hk + 15) >> 4) * nch;
+  for (int it = warp; it < items; it += kHHThreads / 32) {
     const int mt = it / nch, n0 = (it - mt * nch) * kHHNC;
     double acc[kHHNC][4];
 #pragma unroll
     for (int n = 0; n < kHHNC; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.0;
-    for (int k16 = 0; k16 < rows16 / 16; ++k16) {
+    for (int k16 = 0; k16 < rows16; k16 += 16) {
       double a[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i)  // A[kl][k] = V[k][kl]
-        a[i] = Vs[(16 * k16 + t + 4 * (i / 2)) * ld + 16 * mt + g + 8 * (i % 2)];
+        a[i] = Vs[(k16 + t + 4 * (i / 2)) * hs + 16 * mt + g + 8 * (i % 2)];
 #pragma unroll
       for (int n = 0; n < kHHNC; ++n) {
         if (n0 + n >= n8) break;
         double b[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) b[q] = Ts[(16 * k16 + t + 4 * q) * ld + 8 * (n0 + n) + g];
+        for (int q = 0; q < 4; ++q) b[q] = Ts[(k16 + t + 4 * q) * hs + 8 * (n0 + n) + g];
         dmma_16816(acc[n], a, b);
       }
     }
 #pragma unroll
     for (int n = 0; n < kHHNC; ++n) {
       if (n0 + n >= n8) break;
-      const int ij = 8 * (n0 + n) + 2 * t;
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int kl = 16 * mt + g + 8 * h;
-        if (kl < hh) {
-          if (ij < hh) pb[kl * hh + ij] = acc[n][2 * h];
-          if (ij + 1 < hh) pb[kl * hh + ij + 1] = acc[n][2 * h + 1];
-        }
+      for (int q = 0; q < 4; ++q) {
+        const int kl = 16 * mt + g + 8 * (q >> 1), ij = 8 * (n0 + n) + 2 * t + (q & 1);
+        if (kl < hk && ij < hk) part[kl * hk + ij] = acc[n][q];
       }
     }
   }
-  for (int k = warp; k < rows; k += kHHSliceThreads / 32) {
+  for (int k = warp; k < rows; k += kHHThreads / 32) {
     double d = 0.0;
-    for (int c = lane; c < hh; c += 32) d = fma(Vs[k * ld + c], Ts[k * ld + c], d);
+    for (int c = lane; c < hk; c += 32) d = fma(Vs[k * hs + c], Ts[k * hs + c], d);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-    if (lane == 0) r_out[ch.pp_off + tt.k0 + k] = d;
+    if (lane == 0) r_out[ch.pk_off + tt.k0 + k] = d;
   }
-  __syncthreads();
-  trace_end(ctl, kTrHHTiled);
 }
 
-// Item = 256 consecutive elements P[kl][ij] (row-major) of channel ch, from idx0.
-struct HHRed {
-  int32_t ch, idx0;
-};
-__global__ void __launch_bounds__(256)
-hh_reduce_kernel(const HHRed *__restrict__ items, const ChanInfo *__restrict__ chans,
-                 const double *__restrict__ v_hhhh, const double *__restrict__ part,
-                 double *__restrict__ x_ref, double *__restrict__ x_t, double *__restrict__ s_out,
-                 __nv_bfloat16 *__restrict__ xt_tc, int64_t xt_tc_stride, int nt,
+// Units [0, n_cta) one per CTA, then n_warp units, one per warp of the following CTAs.
+__global__ void __launch_bounds__(kHHThreads, 4)
+hh_ladder_kernel(const HHTile *__restrict__ tiles, int n_cta, int n_warp,
+                 const ChanInfo *__restrict__ chans, const double *__restrict__ vq,
+                 const double *tq0, const double *tq1, double *__restrict__ part,
+                 const int64_t *__restrict__ part_off, double *__restrict__ r_out,
                  const Control *ctl, int gate) {
+  const int tr = (int)blockIdx.x < n_cta ? kTrHHTiled : kTrHHSmall;
+  if (skip_iteration(ctl, gate, tr)) return;
+  extern __shared__ __align__(16) double hh_smem[];
+  const bool wide = (int)blockIdx.x < n_cta;
+  const int w = ((int)blockIdx.x - n_cta) * (kHHThreads / 32) + (int)(threadIdx.x >> 5);
+  if (!wide && w >= n_warp) return;
+  const HHTile tt = tiles[wide ? (int)blockIdx.x : n_cta + w];
+  const ChanInfo &ch = chans[tt.ch];
+  const double *tq = ctl->parity ? tq1 : tq0;
+  double *pb = part + part_off[tt.ch] + (int64_t)tt.idx * ch.hk * ch.hk;
+  if (wide) hh_cta_unit(tt, ch, vq, tq, pb, r_out, hh_smem);
+  else hh_warp_unit(tt, ch, vq, tq, pb, r_out);
+  trace_end(ctl, tr);
+}
+
+// X and s: one thread per element of every channel's P (a flat list, so that channels of one
+// hole pair do not take a CTA each), the slices' partials added in slice order with a block of
+// loads in flight ahead of the additions.
+__global__ void __launch_bounds__(128)
+hh_reduce_kernel(const HHOut *__restrict__ outs, int n, const double *__restrict__ v_hhhh,
+                 const double *__restrict__ part, double *__restrict__ x,
+                 double *__restrict__ s_out, const Control *ctl, int gate) {
   if (skip_iteration(ctl, gate, kTrHHReduce)) return;
-  const HHRed it = items[blockIdx.x];
-  const ChanInfo ch = chans[it.ch];
-  const int hh = ch.hh, nout = hh * hh, idx = it.idx0 + threadIdx.x;
-  if (idx >= nout) return;
-  const double *pb = part + ch.part_off + idx;
-  // Eight interleaved partial sums over the slices (their loads independent, so they are in
-  // flight together), combined in a fixed order.
-  double acc[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  const int i = blockIdx.x * 128 + threadIdx.x;
+  if (i >= n) return;
+  const HHOut o = outs[i];
+  const double *pb = part + o.part;
+  const double vh = __ldg(v_hhhh + o.v);
+  double p = 0.0;
   int sl = 0;
-  // Sixteen slices' loads in flight together, then added to the same partial sums in the same
-  // order as the eight-slice rounds below.
-  for (; sl + 16 <= ch.nhht; sl += 16) {
-    double x[16];
+  for (; sl + 8 <= o.nslices; sl += 8) {
+    double y[8];
 #pragma unroll
-    for (int k = 0; k < 16; ++k) x[k] = __ldcg(pb + (int64_t)(sl + k) * nout);
+    for (int k = 0; k < 8; ++k) y[k] = __ldcg(pb + (int64_t)(sl + k) * o.stride);
 #pragma unroll
-    for (int k = 0; k < 16; ++k) acc[k & 7] += x[k];
+    for (int k = 0; k < 8; ++k) p += y[k];
   }
-  for (; sl + 8 <= ch.nhht; sl += 8) {
+  {
+    double y[8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) acc[k] += __ldcg(pb + (int64_t)(sl + k) * nout);
+    for (int k = 0; k < 8; ++k)
+      y[k] = sl + k < o.nslices ? __ldcg(pb + (int64_t)(sl + k) * o.stride) : 0.0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) p += y[k];
   }
-  for (; sl < ch.nhht; ++sl) acc[0] += __ldcg(pb + (int64_t)sl * nout);
-  const double p =
-      ((acc[0] + acc[1]) + (acc[2] + acc[3])) + ((acc[4] + acc[5]) + (acc[6] + acc[7]));
-  hh_finish(ch, idx / hh, idx - (idx / hh) * hh, p, v_hhhh, x_ref, x_t, s_out, xt_tc,
-            xt_tc_stride, nt);
+  x[o.x] = vh + p;
+  if (o.s >= 0) s_out[o.s] = p;
   trace_end(ctl, kTrHHReduce);
 }
 
 // ------------------------------------------------------------------------------------------
 // Ring term: Y = V_hphp + 0.5 V_hpph T', R = T' Y per modified channel (calc.cpp:264-313).
-// T' is read from the phhp slab (t2Old_phhp; the fused assembly keeps it current); V_hpph is
-// held transposed per channel (Vt[k][i] = V_hpph[i][k], k < ph', i < hp').  Result
-// layout: fused path (inv != null) scatters R into pphh order, out[inv[p]] = R[p] (inv =
-// inverse of the ai_jb table), so the assembly reads R_ai,jb / R_aj,ib / R_bi,ja / R_bj,ia from
-// the channel's own block; table path (inv == null) writes t2Diff_phhp, out[p] = R[p].
+// T' is read from the phhp slab (t2Old_phhp); V_hpph is held transposed per channel
+// (Vt[k][i] = V_hpph[i][k], k < ph', i < hp').  Result layout: fused path (dst != null) stores
+// R[p] at out[dst[p]], the four terms of a quad side by side (dst < 0: a = b or i = j, in no
+// quad), so that the assembly reads them as one 32-byte word; table path (dst == null) writes
+// t2Diff_phhp, out[p] = R[p].
 // Channels with ph', hp' <= kRingSmall run one per warp; larger ones one per CTA, grouped by
 // padded size (ring16_kernel).
 // ------------------------------------------------------------------------------------------
 constexpr int kRingSmall = 16;
+constexpr int kRingMax = 80;  // largest ph', hp'
 
-// T' for the ring on the fused path: the phhp slab gathered from the current amplitudes,
-// phhp[p] = t[inv[p]] (inv = inverse of the ai_jb table, a permutation of the n elements), at
-// the head of the ring stream: coalesced index loads and slab stores, scattered reads of t
-// (which the previous assembly has just written, so mostly L2 hits).  Eight elements per
-// thread, all their loads in flight together.  gate < 0: run outside the iteration gating
-// (a read of the slab after a solve).
+// dst[p] of the fused path: 4 * (packed position of the quad) + k, k = 0: (ab, ij), 1: (ab, ji),
+// 2: (ba, ij), 3: (ba, ji); -1 outside every quad.  The amplitude there is +t, -t, -t, +t.
+__device__ __forceinline__ double ring_amplitude(const double *tq, int32_t dst) {
+  if (dst < 0) return 0.0;
+  const double t = __ldcg(tq + (dst >> 2));
+  return ((dst & 3) == 1 || (dst & 3) == 2) ? -t : t;
+}
+
+// T' for the ring on the fused path: the phhp slab gathered from the packed amplitudes, at the
+// head of the ring stream: coalesced index loads and slab stores, scattered reads of an array a
+// quarter of the slab's size (which the previous assembly has just written, so mostly L2 hits).
+// Eight elements per thread, all their loads in flight together.  gate < 0: run outside the
+// iteration gating (a read of the slab after a solve).
 constexpr int kGatherPer = 8;
 __global__ void __launch_bounds__(256)
-phhp_gather_kernel(const int32_t *__restrict__ inv, int64_t n, const double *tbuf0,
-                   const double *tbuf1, double *__restrict__ phhp, const Control *ctl, int gate) {
+phhp_gather_kernel(const int32_t *__restrict__ dst, int64_t n, const double *tq0,
+                   const double *tq1, double *__restrict__ phhp, const Control *ctl, int gate) {
   if (gate >= 0) {
     if (skip_iteration(ctl, gate, kTrGather)) return;
   } else {
     pdl_enter();
   }
-  const double *__restrict__ t = ctl->parity ? tbuf1 : tbuf0;
+  const double *__restrict__ t = ctl->parity ? tq1 : tq0;
   const int64_t p0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * kGatherPer;
   if (p0 >= n) return;
-  int32_t idx[kGatherPer];
   double v[kGatherPer];
   if (p0 + kGatherPer <= n) {
-    const int4 a = __ldg(reinterpret_cast<const int4 *>(inv + p0));
-    const int4 b = __ldg(reinterpret_cast<const int4 *>(inv + p0) + 1);
-    idx[0] = a.x; idx[1] = a.y; idx[2] = a.z; idx[3] = a.w;
-    idx[4] = b.x; idx[5] = b.y; idx[6] = b.z; idx[7] = b.w;
+    const int4 a = __ldg(reinterpret_cast<const int4 *>(dst + p0));
+    const int4 b = __ldg(reinterpret_cast<const int4 *>(dst + p0) + 1);
+    const int32_t idx[kGatherPer] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
-    for (int k = 0; k < kGatherPer; ++k) v[k] = __ldcg(t + idx[k]);
+    for (int k = 0; k < kGatherPer; ++k) v[k] = ring_amplitude(t, idx[k]);
     double2 *o = reinterpret_cast<double2 *>(phhp + p0);
 #pragma unroll
     for (int k = 0; k < kGatherPer / 2; ++k) o[k] = make_double2(v[2 * k], v[2 * k + 1]);
   } else {
-    for (int64_t p = p0; p < n; ++p) phhp[p] = __ldcg(t + inv[p]);
+    for (int64_t p = p0; p < n; ++p) phhp[p] = ring_amplitude(t, dst[p]);
   }
   if (gate >= 0) trace_end(ctl, kTrGather);
 }
@@ -805,13 +623,13 @@ __host__ __device__ inline int ring_pad8(int n) { return (n + 7) & ~7; }
 // Channels with ph', hp' <= kRingSmall, one per warp (kRingSmallWarps per CTA), the same two
 // products on the FP64 MMA: the warp's stage is padded to P, H in {8, 16} with zeros and a row
 // stride of 20 doubles (4 mod 8: conflict-free fragment loads); R goes straight to global
-// memory (scattered through the inverse ai_jb table on the fused path).
+// memory (through dst on the fused path).
 constexpr int kRingSmallWarps = 4;
 constexpr int kRingSmallLd = kRingSmall + 4;
 __global__ void __launch_bounds__(kRingSmallWarps * 32)
 ring_small_kernel(const ModInfo *__restrict__ mods, int n, const double *__restrict__ v_hpph,
                   const double *__restrict__ v_hphp, const double *__restrict__ t_phhp,
-                  const int32_t *__restrict__ inv, double *__restrict__ out, const Control *ctl,
+                  const int32_t *__restrict__ dst, double *__restrict__ out, const Control *ctl,
                   int gate) {
   if (skip_iteration(ctl, gate, kTrRingSmall)) return;
   __shared__ __align__(16) double buf[kRingSmallWarps][3 * kRingSmall * kRingSmallLd];
@@ -841,8 +659,8 @@ ring_small_kernel(const ModInfo *__restrict__ mods, int n, const double *__restr
     else Ys[r * ld + c] = 0.0;
   }
   int32_t *Is = ibuf[w];  // scatter destinations (fused path), staged with the operands
-  if (inv)
-    for (int p = lane; p < ph * hp; p += 32) cp_async4(Is + p, inv + m.m_off + p);
+  if (dst)
+    for (int p = lane; p < ph * hp; p += 32) cp_async4(Is + p, dst + m.m_off + p);
   cp_async_commit();
   cp_async_wait<0>();
   __syncwarp();
@@ -853,7 +671,8 @@ ring_small_kernel(const ModInfo *__restrict__ mods, int n, const double *__restr
   warp_mma_gemm<2>(Ts, ld, 1, Ys, ld, P / 8, H / 8, H / 4, 0, 1, [&](int r, int c, double v) {
     if (r < ph && c < hp) {
       const int p = r * hp + c;
-      out[inv ? (int64_t)Is[p] : m.m_off + p] = v;
+      const int64_t o = dst ? (int64_t)Is[p] : m.m_off + p;
+      if (o >= 0) out[o] = v;
     }
   });
   trace_end(ctl, kTrRingSmall);
@@ -934,7 +753,7 @@ template <int PAD>
 __global__ void __launch_bounds__(32 * ring16_warps(PAD), ring16_ctas(PAD))
 ring16_kernel(const ModInfo *__restrict__ mods, const double *__restrict__ v_hpph,
               const double *__restrict__ v_hphp, const double *__restrict__ t_phhp,
-              const int32_t *__restrict__ inv, double *__restrict__ out, const Control *ctl,
+              const int32_t *__restrict__ dst, double *__restrict__ out, const Control *ctl,
               int gate) {
   if (skip_iteration(ctl, gate, PAD <= 32 ? kTrRingMid : kTrRingLarge)) return;
   extern __shared__ __align__(16) double r16[];
@@ -993,18 +812,18 @@ ring16_kernel(const ModInfo *__restrict__ mods, const double *__restrict__ v_hpp
         [&](int r, int c, double v, int) { Ys[r * ld + c] = 0.5 * v + Ys[r * ld + c]; });
   }
   __syncthreads();
-  // R = T' Y, stored for r < ph', c < hp' (through the inverse ai_jb table on the fused path);
+  // R = T' Y, stored for r < ph', c < hp' (through dst on the fused path);
   // the destinations are loaded before the MMAs, so the stores do not wait on them.
-  int32_t dst[4 * kRing16NC];
+  int32_t to[4 * kRing16NC];
   ring16_gemm<PAD, 1>(
       Ts, Ys, warp,
       [&](int slot, int r, int c) {
         const int32_t p = (int32_t)(m.m_off + (int64_t)r * hp + c);
-        dst[slot] = (r < ph && c < hp) ? (inv ? __ldg(inv + p) : p) : -1;
+        to[slot] = (r < ph && c < hp) ? (dst ? __ldg(dst + p) : p) : -1;
         return 0.0;
       },
       [&](int, int, double v, int slot) {
-        if (dst[slot] >= 0) out[dst[slot]] = v;
+        if (to[slot] >= 0) out[to[slot]] = v;
       });
   trace_end(ctl, PAD <= 32 ? kTrRingMid : kTrRingLarge);
 }
@@ -1060,7 +879,8 @@ onebody_tables_kernel(int np, const int64_t *__restrict__ o_h, const int64_t *__
   }
 }
 
-// Fused path: x_k and y_a as segmented sums of the ladder-kernel by-products s and r.
+// Fused path: x_k and y_a as segmented sums of the hh ladder's by-products s and r over the
+// strict pairs that hold the orbital; twice, for the two orders of the summed pair.
 // One warp per orbital, lane-strided partial sums and a fixed shuffle tree.
 __global__ void onebody_fused_kernel(int np, int nsp, const int64_t *__restrict__ list_off,
                                      const int32_t *__restrict__ list, const double *__restrict__ s,
@@ -1088,75 +908,39 @@ __global__ void onebody_fused_kernel(int np, int nsp, const int64_t *__restrict_
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
   if (lane == 0) {
-    if (hole) xh[w] = v;
-    else yp[w - np] = v;
+    if (hole) xh[w] = 2.0 * v;
+    else yp[w - np] = 2.0 * v;
   }
   trace_end(ctl, kTrOneBody);
 }
 
-// Writes one amplitude into the ladder operand tiles: the B tiles of V T (rows c<d) and the A
-// tiles of T X (rows a<=b, compact last row tile).  pk_idx[AB] = (K index or -1, packed row
-// or -1).
-__device__ __forceinline__ void write_t_tiles_q(const ChanInfo &ch, int2 q, int ij, double t,
-                                                double *t_kt, double *t_mt) {
-  const int bs = ladder_bs(ch.nb);
-  if (q.x >= 0) t_kt[ch.tkt_base + (int64_t)(q.x / kBK) * kBK * bs + (q.x % kBK) * bs + ij] = t;
-  if (q.y >= 0) {
-    const int mt = q.y / ch.bm, rows = min(ch.bm, ch.pr - mt * ch.bm);
-    const int ar = ladder_arows(ch.nb, rows);
-    t_mt[ch.tmt_base + (int64_t)mt * ladder_arows_full(ch.nb) * ch.nkh * kBK +
-         (int64_t)(ij / kBK) * ar * kBK +
-         ladder_aoff(ch.nb, ar, q.y - mt * ch.bm, ij % kBK)] = t;
-  }
-}
-__device__ __forceinline__ void write_t_tiles(const ChanInfo &ch, const int2 *__restrict__ pk_idx,
-                                              int ab, int ij, double t, double *t_kt,
-                                              double *t_mt) {
-  write_t_tiles_q(ch, pk_idx[ch.pp_off + ab], ij, t, t_kt, t_mt);
-}
-
-// The same amplitude into the mixed-precision operand images: nt bf16 terms of T in the
-// tensor-core chunk layout (tc_off), V T operand B (K = c<d pair) and T X operand A (rows a<=b,
-// compact last 128-row tile, K = hh).
+// One packed amplitude t of quad (u, w) into the mixed-precision operand image: nt bf16 terms
+// of T as the B operand of V T in the tensor-core chunk layout (K = u).
 template <int NT>
-__device__ __forceinline__ void write_t_tiles_tc_n(const ChanInfo &ch, int2 q, int ij, double t,
-                                                   __nv_bfloat16 *tkt_tc, int64_t tkt_stride,
-                                                   __nv_bfloat16 *tmt_tc, int64_t tmt_stride) {
+__device__ __forceinline__ void write_t_image_n(const ChanInfo &ch, int u, int w, double t,
+                                                __nv_bfloat16 *img, int64_t stride) {
   __nv_bfloat16 hv[NT];
   split_bf16_n<NT>(t, hv);
-  if (q.x >= 0) {
-    const int64_t o =
-        ch.tkt_tc_base + (int64_t)(q.x >> 5) * (ch.nbt >> 3) * kTcGroup + tc_off_mn(ij, q.x & 31);
+  const int64_t o =
+      ch.tkt_tc_base + (int64_t)(u >> 5) * (ch.nbt >> 3) * kTcGroup + tc_off_mn(w, u & 31);
 #pragma unroll
-    for (int p = 0; p < NT; ++p) tkt_tc[p * tkt_stride + o] = hv[p];
-  }
-  if (q.y >= 0) {
-    const int mt = q.y >> 7, r = q.y & 127;
-    const int rg = (min(kTcBM, ch.pr - mt * kTcBM) + 7) >> 3;
-    const int64_t o = ch.tmt_tc_base + (int64_t)mt * kTcBM * ch.nkht * kTcKC +
-                      (int64_t)(ij >> 5) * rg * kTcGroup + tc_off(r, ij & 31);
-#pragma unroll
-    for (int p = 0; p < NT; ++p) tmt_tc[p * tmt_stride + o] = hv[p];
-  }
+  for (int p = 0; p < NT; ++p) img[p * stride + o] = hv[p];
 }
-__device__ __forceinline__ void write_t_tiles_tc(const ChanInfo &ch, int2 q, int ij, double t,
-                                                 int nt, __nv_bfloat16 *tkt_tc,
-                                                 int64_t tkt_stride, __nv_bfloat16 *tmt_tc,
-                                                 int64_t tmt_stride) {
-  if (q.x < 0 && q.y < 0) return;  // row ba of a mirrored pair: in neither image
-  if (nt == 3) write_t_tiles_tc_n<3>(ch, q, ij, t, tkt_tc, tkt_stride, tmt_tc, tmt_stride);
-  else write_t_tiles_tc_n<2>(ch, q, ij, t, tkt_tc, tkt_stride, tmt_tc, tmt_stride);
+__device__ __forceinline__ void write_t_image(const ChanInfo &ch, int u, int w, double t, int nt,
+                                              __nv_bfloat16 *img, int64_t stride) {
+  if (nt == 3) write_t_image_n<3>(ch, u, w, t, img, stride);
+  else write_t_image_n<2>(ch, u, w, t, img, stride);
 }
 
 // ------------------------------------------------------------------------------------------
 // Fused assembly (calc.cpp:384-418 plus the remaps folded in):
-//   value = V + D + R_ai,jb - R_aj,ib - R_bi,ja + R_bj,ia          (4 gathers from R in phhp layout)
+//   value = V + D + R_ai,jb - R_aj,ib - R_bi,ja + R_bj,ia          (4 ring terms, read side by side)
 //         + 0.5 x_i t_ab,ji - 0.5 x_j t_ab,ij                       (h2pp_h1 gathers, algebraically)
 //         + (-0.5 y_b) t_ab,ij - (-0.5 y_a) t_ba,ij                 (p2_p1hh gathers, algebraically)
 //   t_new = mixing value/(e_i+e_j-e_a-e_b) + (1-mixing) t_old;  E += V t_new
-// and the next iteration's ladder operand tiles are written in the same pass (the ring's phhp
-// slab is gathered from t_new by phhp_gather_kernel at the head of the next iteration's ring
-// stream: mapToDistributed ai_jb as a coalesced write instead of a scattered one here).
+// with D = V_pppp T from the ladder's planes plus 0.5 T X = sum_{k<l} T[u, kl] X[kl, w], formed
+// here: hk multiply-adds per quad on operands that L1 holds (T's row is one broadcast per k),
+// instead of a K extension of the ladder that made it wait for the hh ladder.
 // ------------------------------------------------------------------------------------------
 constexpr int kAsmThreads = 256;
 constexpr int kAsmPerThread = 2;  // table path: elements per thread of an ElemRange
@@ -1173,27 +957,20 @@ __device__ __forceinline__ void loop_set_condition(const Control *ctl,
   cudaGraphSetConditional(cond, (more && (body_mixed ? mixed_phase : !mixed_phase)) ? 1u : 0u);
 }
 
-// Work is organised over quads (u, w): strict packed row u (a < b) of a channel and strict hole
-// pair w (i < j).  The amplitudes are antisymmetric, t_ab,ij = -t_ab,ji = -t_ba,ij = t_ba,ji,
-// and so are V, D and the combination of the four R terms; the fused path keeps them exactly
-// so (the ladders write D[ba] = -D[ab]; a quad writes its four elements as +t, -t, -t, +t), and
-// rows a = b or columns i = j hold zeros that no iteration changes.  One thread computes the
-// quad's element (ab, ij) from V, D, t at (ab, ij) and R at the four positions, and writes all
-// four elements and the operand-image entries of rows ab (row ba is in neither image).  The energy gains 4 V t_new per quad.
-// Persistent CTAs stride over work items of up to kQuadPerItem quads of one channel; a thread
-// takes one quad of an item and issues all its loads before the first store.
-// In a mixed iteration (nt > 0) only the bf16 operand images are written; retile_kernel
-// rebuilds the FP64 tiles if FP64 iterations follow.
+// Work is organised over quads (u, w); one thread computes one quad from V, D and t at its
+// packed position and the four ring terms, and writes the new packed amplitude (and, in a mixed
+// iteration, its bf16 terms).  The energy gains 4 V t_new per quad.  Persistent CTAs stride over
+// work items of up to kQuadPerItem quads of one channel; a thread takes one quad of an item and
+// issues all its loads before the store.  EG N=54 |n|^2 <= 36: 64 bytes a quad against 136 when
+// the ordered pairs were kept (four amplitudes written, D and R read in their layout).
 constexpr int kQuadPerItem = kAsmThreads;  // one quad per thread and item
 constexpr int kAsmCTAsPerSM = 3;
 
-// One thread's quad of a work item: where its four elements sit in the channel block, its
-// operand-image indices, one-body indices and denominator.  ok = false: no quad (past the
-// item or past the last item).
+// One thread's quad of a work item.  ok = false: no quad (past the item or past the last item).
 struct QuadRef {
-  int32_t o_ab, o_ba, c_ij, c_ji, qx, qy, pa, pb, i, j, ch;
+  int32_t u, w, hk, hs, pa, pb, i, j, ch;
   bool ok;
-  int64_t t_off;
+  int64_t q_off, x_off;
   double den;
 };
 __device__ __forceinline__ void quad_fetch(const QuadItem *__restrict__ items, int n_items,
@@ -1210,14 +987,29 @@ __device__ __forceinline__ void quad_fetch(const QuadItem *__restrict__ items, i
   const int hk = item.hk;
   const uint32_t magic = hk > 1 ? 0xFFFFFFFFu / (uint32_t)hk + 1u : 0u;
   const int u = hk > 1 ? (int)__umulhi((uint32_t)q, magic) : q, w = q - u * hk;
-  const QuadRow rw = qrows[item.qrow_off + u];
+  const QuadRow rw = qrows[item.pk_off + u];
   const QuadCol cl = qcols[item.qcol_off + w];
-  r.o_ab = rw.o_ab; r.o_ba = rw.o_ba; r.qx = rw.qx; r.qy = rw.qy; r.pa = rw.pa; r.pb = rw.pb;
-  r.c_ij = cl.c_ij; r.c_ji = cl.c_ji; r.i = cl.i; r.j = cl.j;
+  r.u = u; r.w = w; r.hk = hk; r.hs = item.hs;
+  r.pa = rw.pa; r.pb = rw.pb; r.i = cl.i; r.j = cl.j;
   r.den = cl.eij - rw.ea - rw.eb;
   r.ch = item.ch;
-  r.t_off = item.t_off;
+  r.q_off = item.q_off;
+  r.x_off = item.x_off;
   r.ok = true;
+}
+
+// D of quad (u, w): the ladder's planes in order, then T X.
+__device__ __forceinline__ double quad_d(const LadderChan &lc, const double *__restrict__ dp,
+                                         const double *__restrict__ t_row,
+                                         const double *__restrict__ x, int hk, int hs, int u,
+                                         int w) {
+  const double *p = dp + lc.base + (int64_t)u * hs + w;
+  double d = __ldcg(p);
+  for (int s = 1; s < lc.nseg; ++s) d += __ldcg(p + (int64_t)s * lc.plane);
+  double tx = 0.0;
+#pragma unroll 4
+  for (int k = 0; k < hk; ++k) tx = fma(t_row[k], x[k * hs + w], tx);
+  return d + tx;
 }
 
 // value of element (ab, ij) (calc.cpp:384-418) with t_ab,ji = -t and t_ba,ij = -t:
@@ -1245,14 +1037,13 @@ __device__ __forceinline__ double quad_value(double v, double dm, double r1, dou
 template <bool LOOP>
 __global__ void __launch_bounds__(kAsmThreads, kAsmCTAsPerSM)
 assemble_fused_kernel(const QuadItem *__restrict__ items, int n_items,
-                      const ChanInfo *__restrict__ chans, const QuadRow *__restrict__ qrows,
-                      const QuadCol *__restrict__ qcols, const double *__restrict__ v_pphh,
-                      const double *__restrict__ dmat, const double *__restrict__ d_ring,
-                      const double *__restrict__ xh, const double *__restrict__ yp,
-                      double *tbuf0, double *tbuf1, double *__restrict__ t_kt,
-                      double *__restrict__ t_mt, double *__restrict__ epart, int32_t *ticket,
-                      Control *ctl, __nv_bfloat16 *__restrict__ tkt_tc, int64_t tkt_tc_stride,
-                      __nv_bfloat16 *__restrict__ tmt_tc, int64_t tmt_tc_stride, int nt,
+                      const ChanInfo *__restrict__ chans, const LadderChan *__restrict__ lchans,
+                      const QuadRow *__restrict__ qrows, const QuadCol *__restrict__ qcols,
+                      const double *__restrict__ vq, const double *__restrict__ dp,
+                      const double *__restrict__ x, const double *__restrict__ r_quad,
+                      const double *__restrict__ xh, const double *__restrict__ yp, double *tq0,
+                      double *tq1, double *__restrict__ epart, int32_t *ticket, Control *ctl,
+                      __nv_bfloat16 *__restrict__ tkt_tc, int64_t tkt_tc_stride, int nt,
                       cudaGraphConditionalHandle cond, int loop_body, int gate) {
   // loop_body: 0 outside the device solve loop, 1 / 2 last kernel of its FP64 / mixed body,
   // where the CTA that applies the stop rule also sets the loop condition.  A skipped body
@@ -1264,8 +1055,8 @@ assemble_fused_kernel(const QuadItem *__restrict__ items, int n_items,
       if (blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(cond, 0u);
     return;
   }
-  const double *__restrict__ t_old = ctl->parity ? tbuf1 : tbuf0;
-  double *__restrict__ t_new = ctl->parity ? tbuf0 : tbuf1;
+  const double *__restrict__ t_old = ctl->parity ? tq1 : tq0;
+  double *__restrict__ t_new = ctl->parity ? tq0 : tq1;
   const double mixing = ctl->mixing;
   double corr = 0.0;
   // Two-stage pipeline over the CTA's items: the next item's header and this thread's row and
@@ -1274,43 +1065,29 @@ assemble_fused_kernel(const QuadItem *__restrict__ items, int n_items,
   quad_fetch(items, n_items, qrows, qcols, blockIdx.x, nx);
   for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
     const QuadRef cu = nx;
-    double tv = 0.0, vv = 0.0, dv = 0.0, rv[4] = {0.0, 0.0, 0.0, 0.0}, xs[2] = {0.0, 0.0},
-           ys[2] = {0.0, 0.0};
-    int32_t pos[4];
-    pos[0] = cu.o_ab + cu.c_ij;
-    pos[1] = cu.o_ab + cu.c_ji;
-    pos[2] = cu.o_ba + cu.c_ij;
-    pos[3] = cu.o_ba + cu.c_ji;
+    double tv = 0.0, vv = 0.0, dv = 0.0, xs[2] = {0.0, 0.0}, ys[2] = {0.0, 0.0};
+    double2 r01 = make_double2(0.0, 0.0), r23 = r01;
+    const int64_t p = cu.q_off + (int64_t)cu.u * cu.hs + cu.w;
     if (cu.ok) {
-      const int64_t p0 = cu.t_off + pos[0];
-      tv = t_old[p0];
-      vv = __ldg(v_pphh + p0);
-      dv = __ldcg(dmat + p0);
-#pragma unroll
-      for (int m = 0; m < 4; ++m) rv[m] = __ldcg(d_ring + cu.t_off + pos[m]);
+      tv = t_old[p];
+      vv = __ldg(vq + p);
+      const double2 *rp = reinterpret_cast<const double2 *>(r_quad + 4 * p);
+      r01 = __ldcg(rp);
+      r23 = __ldcg(rp + 1);
       // The one-body sums are small arrays every quad reads: through L1 (an L2-only load
       // would send every warp to the same few L2 slices).
       xs[0] = xh[cu.i];
       xs[1] = xh[cu.j];
       ys[0] = yp[cu.pa];
       ys[1] = yp[cu.pb];
+      dv = quad_d(lchans[cu.ch], dp, t_old + p - cu.w, x + cu.x_off, cu.hk, cu.hs, cu.u, cu.w);
     }
     quad_fetch(items, n_items, qrows, qcols, it + gridDim.x, nx);
     if (!cu.ok) continue;
-    const double t1 = quad_value(vv, dv, rv[0], rv[1], rv[2], rv[3], tv, xs[0], xs[1], ys[0],
+    const double t1 = quad_value(vv, dv, r01.x, r01.y, r23.x, r23.y, tv, xs[0], xs[1], ys[0],
                                  ys[1], cu.den, mixing);
-    const double sg[4] = {t1, -t1, -t1, t1};
-#pragma unroll
-    for (int m = 0; m < 4; ++m) t_new[cu.t_off + pos[m]] = sg[m];
-    const ChanInfo &ch = chans[cu.ch];
-    const int2 qa = make_int2(cu.qx, cu.qy);
-    if (nt) {
-      write_t_tiles_tc(ch, qa, cu.c_ij, t1, nt, tkt_tc, tkt_tc_stride, tmt_tc, tmt_tc_stride);
-      write_t_tiles_tc(ch, qa, cu.c_ji, -t1, nt, tkt_tc, tkt_tc_stride, tmt_tc, tmt_tc_stride);
-    } else {
-      write_t_tiles_q(ch, qa, cu.c_ij, t1, t_kt, t_mt);
-      write_t_tiles_q(ch, qa, cu.c_ji, -t1, t_kt, t_mt);
-    }
+    t_new[p] = t1;
+    if (nt) write_t_image(chans[cu.ch], cu.u, cu.w, t1, nt, tkt_tc, tkt_tc_stride);
     corr += 4.0 * (vv * t1);
   }
   const double sum = block_sum<kAsmThreads>(corr, scratch);
@@ -1327,33 +1104,97 @@ assemble_fused_kernel(const QuadItem *__restrict__ items, int n_items,
   energy_reduce(epart, gridDim.x, ctl, 3, nullptr);
   if (threadIdx.x == 0) {
     *ticket = 0;
-    if (nt) ctl->retile = 1;  // the FP64 ladder tiles were not written this iteration
     if constexpr (LOOP) loop_set_condition(ctl, cond, loop_body == 2);
   }
 }
 
-// Rebuilds the FP64 ladder operand tiles from the current amplitudes after mixed iterations
-// (they write only the bf16 images); a no-op unless ctl->retile is set.  First kernel of every
-// FP64 iteration of the fused path and of the FP64 ladder stage.
+// ---- Between the packed amplitudes and the reference's layout ----------------------------
+
+// D of the ladder in the reference layout (t2Diff_pphh), from the ladder's planes, X and the
+// amplitudes they were computed from (buffer parity ^ flip): a quad's four elements as
+// +D, -D, -D, +D; rows a = b and columns i = j stay zero.
+__global__ void __launch_bounds__(kAsmThreads)
+expand_d_kernel(const QuadItem *__restrict__ items, const ChanInfo *__restrict__ chans,
+                const LadderChan *__restrict__ lchans, const QuadRow *__restrict__ qrows,
+                const QuadCol *__restrict__ qcols, const double *__restrict__ dp,
+                const double *__restrict__ x, const double *tq0, const double *tq1, int flip,
+                const Control *ctl, double *__restrict__ d) {
+  const QuadItem item = items[blockIdx.x];
+  const int q = item.q0 + threadIdx.x;
+  if (q >= item.q1) return;
+  const int u = q / item.hk, w = q - u * item.hk;
+  const double *t = (ctl->parity ^ flip) ? tq1 : tq0;
+  const double v = quad_d(lchans[item.ch], dp, t + item.q_off + (int64_t)u * item.hs,
+                          x + item.x_off, item.hk, item.hs, u, w);
+  const QuadRow rw = qrows[item.pk_off + u];
+  const QuadCol cl = qcols[item.qcol_off + w];
+  double *o = d + chans[item.ch].t_off;
+  o[rw.o_ab + cl.c_ij] = v;
+  o[rw.o_ab + cl.c_ji] = -v;
+  o[rw.o_ba + cl.c_ij] = -v;
+  o[rw.o_ba + cl.c_ji] = v;
+}
+
+// Quad of element (ab, ij): prow[ab] = 2 u (a < b), 2 u + 1 (a > b) or -1 (a = b), hcol[ij]
+// alike; sign flips once per exchanged pair.  False: in no quad.
+__device__ __forceinline__ bool quad_of(const ChanInfo &ch, const int32_t *__restrict__ prow,
+                                        const int32_t *__restrict__ hcol, int ab, int ij, int &u,
+                                        int &w, bool &neg) {
+  const int r = prow[ch.pp_off + ab], c = hcol[ch.hh_off + ij];
+  u = r >> 1;
+  w = c >> 1;
+  neg = ((r ^ c) & 1) != 0;
+  return r >= 0 && c >= 0;
+}
+
+// Packed amplitudes -> t2_pphh in the reference's order (coalesced stores).
 __global__ void __launch_bounds__(256)
-retile_kernel(const ElemRange *__restrict__ ranges, const ChanInfo *__restrict__ chans,
-              const int2 *__restrict__ pk_idx, const double *tbuf0, const double *tbuf1,
-              double *__restrict__ t_kt, double *__restrict__ t_mt, Control *ctl, int gate) {
-  if (skip_iteration(ctl, gate, kTrRetile) || !ctl->retile) return;
+expand_t_kernel(const ElemRange *__restrict__ ranges, const ChanInfo *__restrict__ chans,
+                const int32_t *__restrict__ prow, const int32_t *__restrict__ hcol,
+                const double *tq0, const double *tq1, const Control *ctl,
+                double *__restrict__ t2) {
   const ElemRange rg = ranges[blockIdx.x];
-  const ChanInfo ch = chans[rg.ch];
-  const double *t = ctl->parity ? tbuf1 : tbuf0;
+  const ChanInfo &ch = chans[rg.ch];
+  const double *t = ctl->parity ? tq1 : tq0;
   for (int64_t e = rg.e0 + threadIdx.x; e < rg.e1; e += blockDim.x) {
     const int64_t loc = e - ch.t_off;
     const int ab = (int)(loc / ch.hh), ij = (int)(loc - (int64_t)ab * ch.hh);
-    write_t_tiles(ch, pk_idx, ab, ij, t[e], t_kt, t_mt);
+    int u, w;
+    bool neg;
+    double v = 0.0;
+    if (quad_of(ch, prow, hcol, ab, ij, u, w, neg)) {
+      v = t[ch.q_off + (int64_t)u * ch.hs + w];
+      if (neg) v = -v;
+    }
+    t2[e] = v;
   }
 }
 
-// Clears the retile flag once every retile CTA has read it (single thread, after retile).
-__global__ void retile_done_kernel(Control *ctl) {
-  pdl_enter();
-  if (threadIdx.x == 0) ctl->retile = 0;
+// A value of the packed layout from its (ab, ij) elements of the reference layout (V_hhpp).
+__global__ void __launch_bounds__(kAsmThreads)
+pack_quads_kernel(const QuadItem *__restrict__ items, const ChanInfo *__restrict__ chans,
+                  const QuadRow *__restrict__ qrows, const QuadCol *__restrict__ qcols,
+                  const double *__restrict__ src, double *__restrict__ out) {
+  const QuadItem item = items[blockIdx.x];
+  const int q = item.q0 + threadIdx.x;
+  if (q >= item.q1) return;
+  const int u = q / item.hk, w = q - u * item.hk;
+  out[item.q_off + (int64_t)u * item.hs + w] =
+      src[chans[item.ch].t_off + qrows[item.pk_off + u].o_ab + qcols[item.qcol_off + w].c_ij];
+}
+
+// The bf16 operand image of a mixed handle's tensor-core ladder from the packed amplitudes,
+// before a mixed iteration that follows something other than a mixed iteration.
+__global__ void __launch_bounds__(kAsmThreads)
+t_image_kernel(const QuadItem *__restrict__ items, const ChanInfo *__restrict__ chans,
+               const double *tq0, const double *tq1, const Control *ctl,
+               __nv_bfloat16 *__restrict__ img, int64_t stride, int nt) {
+  const QuadItem item = items[blockIdx.x];
+  const int q = item.q0 + threadIdx.x;
+  if (q >= item.q1) return;
+  const int u = q / item.hk, w = q - u * item.hk;
+  const double *t = ctl->parity ? tq1 : tq0;
+  write_t_image(chans[item.ch], u, w, t[item.q_off + (int64_t)u * item.hs + w], nt, img, stride);
 }
 
 // Table path assembly: exactly calcChannelT2_pphh over the eight gathered chains.
@@ -1407,22 +1248,34 @@ __global__ void gather8_kernel(int64_t n_t, const int32_t *__restrict__ flat,
   }
 }
 
-// Chain::set + the five mapToDistributed scatters, plus the ladder operand tiles.
+// Chain::set + the five mapToDistributed scatters, plus the packed amplitudes (buffer `parity`
+// of the control block).  An element that is not a number or infinite anywhere (also where no
+// quad reads it) makes its quad, or the first quad of all, not a number, so that the next
+// iteration reports it: `mark` is that second pass, launched after the first.
 __global__ void map_to_kernel(const ElemRange *__restrict__ ranges, const ChanInfo *__restrict__ chans,
-                              const int2 *__restrict__ pk_idx, const int32_t *__restrict__ flat,
-                              int64_t n_t,
+                              const int32_t *__restrict__ prow, const int32_t *__restrict__ hcol,
+                              const int32_t *__restrict__ flat, int64_t n_t,
                               const double *__restrict__ t2, double *__restrict__ t2_old,
                               double *__restrict__ old_h2pp_h1, double *__restrict__ old_h1pp_h2,
                               double *__restrict__ old_p1_p2hh, double *__restrict__ old_p2_p1hh,
-                              double *__restrict__ old_phhp, double *__restrict__ t_kt,
-                              double *__restrict__ t_mt, int with_3body,
-                              __nv_bfloat16 *__restrict__ tkt_tc, int64_t tkt_tc_stride,
-                              __nv_bfloat16 *__restrict__ tmt_tc, int64_t tmt_tc_stride, int nt) {
+                              double *__restrict__ old_phhp, double *tq0, double *tq1,
+                              int with_3body, const Control *ctl, int mark) {
   const ElemRange rg = ranges[blockIdx.x];
-  const ChanInfo ch = chans[rg.ch];
+  const ChanInfo &ch = chans[rg.ch];
+  double *tq = ctl->parity ? tq1 : tq0;
   for (int64_t e = rg.e0 + threadIdx.x; e < rg.e1; e += blockDim.x) {
     const double t = t2[e];
-    t2_old[e] = t;
+    if (mark && isfinite(t)) continue;
+    const int64_t loc = e - ch.t_off;
+    const int ab = (int)(loc / ch.hh), ij = (int)(loc - (int64_t)ab * ch.hh);
+    int u, w;
+    bool neg;
+    const bool in = quad_of(ch, prow, hcol, ab, ij, u, w, neg);
+    if (mark) {
+      tq[in ? ch.q_off + (int64_t)u * ch.hs + w : 0] = __longlong_as_double(0x7ff8000000000000ll);
+      continue;
+    }
+    if (t2_old != t2) t2_old[e] = t;
     if (with_3body) {
       old_h2pp_h1[flat[1 * n_t + e]] = t;  // jab_i
       old_h1pp_h2[flat[0 * n_t + e]] = t;  // iab_j
@@ -1430,11 +1283,8 @@ __global__ void map_to_kernel(const ElemRange *__restrict__ ranges, const ChanIn
       old_p2_p1hh[flat[3 * n_t + e]] = t;  // b_aij
     }
     old_phhp[flat[4 * n_t + e]] = t;       // ai_jb
-    const int64_t loc = e - ch.t_off;
-    const int ab = (int)(loc / ch.hh), ij = (int)(loc - (int64_t)ab * ch.hh);
-    write_t_tiles(ch, pk_idx, ab, ij, t, t_kt, t_mt);
-    if (nt) write_t_tiles_tc(ch, pk_idx[ch.pp_off + ab], ij, t, nt, tkt_tc, tkt_tc_stride,
-                             tmt_tc, tmt_tc_stride);
+    if (in && prow[ch.pp_off + ab] == 2 * u && hcol[ch.hh_off + ij] == 2 * w)
+      tq[ch.q_off + (int64_t)u * ch.hs + w] = t;
   }
 }
 

@@ -27,37 +27,40 @@ __global__ void transpose_hhpp_kernel(const ElemRange *__restrict__ ranges,
   }
 }
 
-// Packed, tiled V_pppp: one CTA per packed row u of one channel.  vraw holds each channel's
-// packed rows (a <= b) in u order, pp values each, from vraw_off[channel].
-// items[i] = (active channel, packed row); kcol[pk_off + w] = pp index of the w-th c<d pair.
-__global__ void tile_v_kernel(const ChanInfo *__restrict__ chans, const int2 *__restrict__ items,
-                              const int32_t *__restrict__ rowmap, const int32_t *__restrict__ kcol,
+// Packed, tiled V_pppp: one CTA per packed row u (a < b) of one channel.  vraw holds each
+// channel's rows a <= b in order, pp values each, from vraw_off[channel].
+// items[i] = (active channel, packed row, its row among the rows a <= b);
+// kcol[pk_off + w] = pp index of the w-th c<d pair.
+__global__ void tile_v_kernel(const ChanInfo *__restrict__ chans, const int4 *__restrict__ items,
+                              const int32_t *__restrict__ kcol,
                               const int64_t *__restrict__ vraw_off, const double *__restrict__ vraw,
                               double *__restrict__ v_t) {
-  const int2 it = items[blockIdx.x];
+  const int4 it = items[blockIdx.x];
   const ChanInfo ch = chans[it.x];
   const int u = it.y;
-  const double *src = vraw + vraw_off[it.x] + (int64_t)u * ch.pp;  // packed row u
-  const int mt = u / ch.bm, rows = min(ch.bm, ch.pr - mt * ch.bm);
-  const int ar = ladder_arows(ch.nb, rows);
-  const int64_t tb = ch.vkt_base + (int64_t)mt * ladder_arows_full(ch.nb) * ch.nkc * kBK;
-  for (int w = threadIdx.x; w < ch.pk; w += blockDim.x)
-    v_t[tb + (int64_t)(w / kBK) * ar * kBK + ladder_aoff(ch.nb, ar, u - mt * ch.bm, w % kBK)] =
+  const double *src = vraw + vraw_off[it.x] + (int64_t)it.z * ch.pp;
+  const int mt = u / kMaxBM, r = u % kMaxBM, rows = min(kMaxBM, ch.pk - mt * kMaxBM);
+  const int ar = ladder_arows(ch.hs, rows);
+  const int64_t tb = ch.vkt_base + (int64_t)mt * ladder_arows_full(ch.hs) * ch.nkc * kBK;
+  for (int w = threadIdx.x; w < ch.pk; w += blockDim.x) {
+    const int k = w % kBK;
+    v_t[tb + (int64_t)(w / kBK) * ar * kBK + (ladder_kmajor(ch.hs) ? k * ar + r : swzA(r, k))] =
         src[kcol[ch.pk_off + w]];
+  }
 }
 
 // Packed V_pppp as nt bf16 terms in the tensor-core chunk images of the mixed-precision
 // ladder (128-row tiles, 32-deep K chunks, compact last tile); one CTA per packed row.
-__global__ void tile_v_tc_kernel(const ChanInfo *__restrict__ chans, const int2 *__restrict__ items,
-                                 const int32_t *__restrict__ rowmap, const int32_t *__restrict__ kcol,
+__global__ void tile_v_tc_kernel(const ChanInfo *__restrict__ chans, const int4 *__restrict__ items,
+                                 const int32_t *__restrict__ kcol,
                                  const int64_t *__restrict__ vraw_off, const double *__restrict__ vraw,
                                  __nv_bfloat16 *__restrict__ v_tc, int64_t stride, int nt) {
-  const int2 it = items[blockIdx.x];
+  const int4 it = items[blockIdx.x];
   const ChanInfo ch = chans[it.x];
   const int u = it.y;
-  const double *src = vraw + vraw_off[it.x] + (int64_t)u * ch.pp;  // packed row u
+  const double *src = vraw + vraw_off[it.x] + (int64_t)it.z * ch.pp;
   const int mt = u >> 7, r = u & 127;
-  const int rg = (min(kTcBM, ch.pr - mt * kTcBM) + 7) >> 3;
+  const int rg = (min(kTcBM, ch.pk - mt * kTcBM) + 7) >> 3;
   const int64_t tb = ch.vtc_base + (int64_t)mt * kTcBM * ch.nkct * kTcKC;
   for (int w = threadIdx.x; w < ch.pk; w += blockDim.x) {
     __nv_bfloat16 hv[3];
@@ -69,7 +72,7 @@ __global__ void tile_v_tc_kernel(const ChanInfo *__restrict__ chans, const int2 
 
 // ---- V_pppp generated on the device from the model (CCDGPU_V_ON_THE_FLY) ----------------
 // The antisymmetrised <ab|v|cd> of SPBasis::calcTBME, evaluated for every packed element of the
-// pp ladder (rows a <= b, columns c < d) and written straight into its operand images, so the
+// pp ladder (rows a < b, columns c < d) and written straight into its operand images, so the
 // host never builds or uploads V_pppp.
 struct ModelDev {
   int32_t kind, stride;
@@ -167,7 +170,7 @@ __global__ void gen_v_hhhh_kernel(const ChanInfo *__restrict__ chans,
   const ChanInfo ch = chans[blockIdx.x];
   for (int e = threadIdx.x; e < ch.hh * ch.hh; e += blockDim.x) {
     const int2 ij = hh_pairs[ch.hh_off + e / ch.hh], kl = hh_pairs[ch.hh_off + e % ch.hh];
-    v_hhhh[ch.x_off + e] = tbme_dev(m, ij.x, ij.y, kl.x, kl.y);
+    v_hhhh[ch.vhh_off + e] = tbme_dev(m, ij.x, ij.y, kl.x, kl.y);
   }
 }
 
@@ -294,25 +297,25 @@ __global__ void normal_order_kernel(ModelDev m, const double *__restrict__ bare,
 // V_pppp generated straight into the ladders' operand images, one CTA per image chunk, so that
 // each CTA writes one contiguous block (the chunk's elements in image order; padding rows and
 // K columns past pk get zeros).  FP64 ladder: items (channel, row tile, 16-deep K chunk), block
-// of ar x kBK doubles, k-major (mid and wide classes) or XOR-swizzled rows (thin class).  The
+// of ar x kBK doubles, k-major (wider channels) or XOR-swizzled rows (thin class).  The
 // tensor-core images of mixed handles come with the FP64 tiles from gen_v_both_chunks_kernel.
 template <bool EG>  // EG: the electron gas's orbital-code path only (fewer registers)
 __global__ void __launch_bounds__(256)
 gen_v_chunks_kernel(const ChanInfo *__restrict__ chans, const int4 *__restrict__ items,
-                    const int32_t *__restrict__ rowmap, const int32_t *__restrict__ kcol,
-                    const int2 *__restrict__ pp_pairs, ModelDev m, double *__restrict__ v_t) {
+                    const int32_t *__restrict__ kcol, const int2 *__restrict__ pp_pairs,
+                    ModelDev m, double *__restrict__ v_t) {
   __shared__ uint2 s_ab[kMaxBM];  // electron gas: orbital codes of the chunk's rows (a, b)
   __shared__ uint2 s_cd[kBK];     // ... and of its K columns (c, d)
   const int4 it = items[blockIdx.x];
   const ChanInfo ch = chans[it.x];
   const int mt = it.y, kc = it.z;
-  const int rows = min(ch.bm, ch.pr - mt * ch.bm), ar = ladder_arows(ch.nb, rows);
-  const bool kmajor = ladder_kmajor(ch.nb);
-  double *out = v_t + ch.vkt_base + (int64_t)mt * ladder_arows_full(ch.nb) * ch.nkc * kBK +
+  const int rows = min(kMaxBM, ch.pk - mt * kMaxBM), ar = ladder_arows(ch.hs, rows);
+  const bool kmajor = ladder_kmajor(ch.hs);
+  double *out = v_t + ch.vkt_base + (int64_t)mt * ladder_arows_full(ch.hs) * ch.nkc * kBK +
                 (int64_t)kc * ar * kBK;
   if (EG) {  // the codes once per chunk, not once per element
     for (int r = threadIdx.x; r < rows; r += blockDim.x) {
-      const int2 ab = pp_pairs[ch.pp_off + rowmap[ch.row_off + mt * ch.bm + r]];
+      const int2 ab = pp_pairs[ch.pp_off + kcol[ch.pk_off + mt * kMaxBM + r]];
       s_ab[r] = make_uint2(m.ocode[ab.x], m.ocode[ab.y]);
     }
     for (int k = threadIdx.x; k < kBK; k += blockDim.x) {
@@ -333,13 +336,13 @@ gen_v_chunks_kernel(const ChanInfo *__restrict__ chans, const int4 *__restrict__
       r = e >> 4;
       k = (e & 15) ^ (r & 15);  // swzA(r, k) = 16 r + (k ^ (r & 15))
     }
-    const int u = mt * ch.bm + r, w = kc * kBK + k;
+    const int u = mt * kMaxBM + r, w = kc * kBK + k;
     double v = 0.0;
     if (r < rows && w < ch.pk) {
       if constexpr (EG) {
         v = eg_tbme_code(m, s_ab[r].x, s_ab[r].y, s_cd[k].x, s_cd[k].y);
       } else {
-        const int2 ab = pp_pairs[ch.pp_off + rowmap[ch.row_off + u]];
+        const int2 ab = pp_pairs[ch.pp_off + kcol[ch.pk_off + u]];
         const int2 cd = pp_pairs[ch.pp_off + kcol[ch.pk_off + w]];
         v = tbme_dev(m, ab.x, ab.y, cd.x, cd.y);
       }
@@ -350,7 +353,7 @@ gen_v_chunks_kernel(const ChanInfo *__restrict__ chans, const int4 *__restrict__
 
 // Mixed handles with generated V: both images from one evaluation of each element.  Items are
 // the tensor-core chunks (channel, 128-row tile, 32-deep K chunk); the FP64 ladder's row tiles
-// are also 128 rows (ladder_bm), so a chunk covers FP64 K chunks 2 kc and 2 kc + 1 of the same
+// are also 128 rows, so a chunk covers FP64 K chunks 2 kc and 2 kc + 1 of the same
 // rows.  The CTA evaluates its 128 x 32 elements once into shared memory (k-major, row stride
 // kGenLd; zero past the channel's rows and columns), four per thread at a time, then writes
 // the NT bf16 terms of each element in the tensor core's K-major core-matrix order (8 x 8
@@ -362,7 +365,7 @@ constexpr int kGenLd = kTcBM + 4;
 template <int NT, bool EG>
 __global__ void __launch_bounds__(256)
 gen_v_both_chunks_kernel(const ChanInfo *__restrict__ chans, const int4 *__restrict__ items,
-                         const int32_t *__restrict__ rowmap, const int32_t *__restrict__ kcol,
+                         const int32_t *__restrict__ kcol,
                          const int2 *__restrict__ pp_pairs, ModelDev m, double *__restrict__ v_t,
                          __nv_bfloat16 *__restrict__ v_tc, int64_t tc_stride) {
   __shared__ uint2 s_ab[kTcBM];
@@ -371,10 +374,10 @@ gen_v_both_chunks_kernel(const ChanInfo *__restrict__ chans, const int4 *__restr
   const int4 it = items[blockIdx.x];
   const ChanInfo ch = chans[it.x];
   const int mt = it.y, kc = it.z;
-  const int rows = min(kTcBM, ch.pr - mt * kTcBM), rg = (rows + 7) >> 3;
+  const int rows = min(kTcBM, ch.pk - mt * kTcBM), rg = (rows + 7) >> 3;
   if (EG) {
     for (int r = threadIdx.x; r < rows; r += blockDim.x) {
-      const int2 ab = pp_pairs[ch.pp_off + rowmap[ch.row_off + mt * kTcBM + r]];
+      const int2 ab = pp_pairs[ch.pp_off + kcol[ch.pk_off + mt * kTcBM + r]];
       s_ab[r] = make_uint2(m.ocode[ab.x], m.ocode[ab.y]);
     }
     for (int k = threadIdx.x; k < kTcKC; k += blockDim.x) {
@@ -400,7 +403,7 @@ gen_v_both_chunks_kernel(const ChanInfo *__restrict__ chans, const int4 *__restr
         if constexpr (EG) {
           v[q] = eg_tbme_code(m, s_ab[r].x, s_ab[r].y, s_cd[k].x, s_cd[k].y);
         } else {
-          const int2 ab = pp_pairs[ch.pp_off + rowmap[ch.row_off + mt * kTcBM + r]];
+          const int2 ab = pp_pairs[ch.pp_off + kcol[ch.pk_off + mt * kTcBM + r]];
           const int2 cd = pp_pairs[ch.pp_off + kcol[ch.pk_off + w]];
           v[q] = tbme_dev(m, ab.x, ab.y, cd.x, cd.y);
         }
@@ -424,12 +427,12 @@ gen_v_both_chunks_kernel(const ChanInfo *__restrict__ chans, const int4 *__restr
     for (int p = 0; p < NT; ++p) v_tc[p * tc_stride + base + e] = hv[p];
   }
   // FP64 chunks 2 kc and 2 kc + 1, as gen_v_chunks_kernel (rows past `rows` are zero).
-  const int ar = ladder_arows(ch.nb, rows);
-  const bool kmajor = ladder_kmajor(ch.nb);
+  const int ar = ladder_arows(ch.hs, rows);
+  const bool kmajor = ladder_kmajor(ch.hs);
   for (int h = 0; h < 2; ++h) {
     const int kc64 = 2 * kc + h;
     if (kc64 >= ch.nkc) break;
-    double *out = v_t + ch.vkt_base + (int64_t)mt * ladder_arows_full(ch.nb) * ch.nkc * kBK +
+    double *out = v_t + ch.vkt_base + (int64_t)mt * ladder_arows_full(ch.hs) * ch.nkc * kBK +
                   (int64_t)kc64 * ar * kBK;
     for (int e = threadIdx.x; e < ar * kBK; e += blockDim.x) {
       int r, k;
@@ -445,30 +448,24 @@ gen_v_both_chunks_kernel(const ChanInfo *__restrict__ chans, const int4 *__restr
   }
 }
 
-// The fused assembly's row table (one CTA per active channel): for each packed row u with
-// a < b (row ab, mirror row ba), at the row's index among those rows (its K index qx), the
-// offsets of rows ab and ba in the channel block, its operand-image indices, the particle
-// indices and energies.
+// The fused assembly's row table (one CTA per active channel): per packed row u (a < b) the
+// offsets of rows ab and ba in the channel block, the particle indices and energies.
 __global__ void __launch_bounds__(256)
-quad_rows_kernel(const ChanInfo *__restrict__ chans, const int32_t *__restrict__ rowmap,
-                 const int32_t *__restrict__ mirror, const int2 *__restrict__ pk_idx,
-                 const int2 *__restrict__ pp_pairs, const double *__restrict__ eps, int np,
-                 QuadRow *__restrict__ out) {
+quad_rows_kernel(const ChanInfo *__restrict__ chans, const int32_t *__restrict__ kcol,
+                 const int32_t *__restrict__ pp_swap, const int2 *__restrict__ pp_pairs,
+                 const double *__restrict__ eps, int np, QuadRow *__restrict__ out) {
   const ChanInfo ch = chans[blockIdx.x];
-  for (int u = threadIdx.x; u < ch.pr; u += blockDim.x) {
-    const int ab = rowmap[ch.row_off + u], ba = mirror[ch.row_off + u];
-    if (ba < 0) continue;  // a = b: zero row
-    const int2 q = pk_idx[ch.pp_off + ab], pab = pp_pairs[ch.pp_off + ab];
+  for (int u = threadIdx.x; u < ch.pk; u += blockDim.x) {
+    const int ab = kcol[ch.pk_off + u], ba = pp_swap[ch.pp_off + ab];
+    const int2 pab = pp_pairs[ch.pp_off + ab];
     QuadRow r;
     r.o_ab = ab * ch.hh;
     r.o_ba = ba * ch.hh;
-    r.qx = q.x;
-    r.qy = q.y;
     r.pa = pab.x - np;
     r.pb = pab.y - np;
     r.ea = eps[pab.x];
     r.eb = eps[pab.y];
-    out[ch.qrow_off + q.x] = r;
+    out[ch.pk_off + u] = r;
   }
 }
 
@@ -648,18 +645,20 @@ __global__ void transpose_hpph_kernel(const ModInfo *__restrict__ mods,
   }
 }
 
-// Fused-path ring tables.  inv[ai_jb(e)] = e turns the phhp slab position of every amplitude
-// back into its pphh element, so the ring can read T' from the amplitudes and write R in pphh
-// order.  The other three ring maps of loadMaps are ai_jb composed with the swaps i<->j and
-// a<->b (load.cpp:469-526 builds all four from the same (a,i),(j,b) pairing); this is checked
-// here, since the fused assembly reads R_aj,ib, R_bi,ja and R_bj,ia at (ab,ji), (ba,ij) and
-// (ba,ji) of the pphh-ordered R.
+// Fused-path ring table.  dst[ai_jb(e)] of amplitude e: 4 x the packed position of its quad
+// plus 0 (ab, ij), 1 (ab, ji), 2 (ba, ij) or 3 (ba, ji); -1 for a = b or i = j.  The ring reads
+// T' through it and writes R into the quads' four terms.  The other three ring maps of loadMaps
+// are ai_jb composed with the swaps i<->j and a<->b (load.cpp:469-526 builds all four from the
+// same (a,i),(j,b) pairing); this is checked here, since the fused assembly takes R_aj,ib,
+// R_bi,ja and R_bj,ia from the terms 1, 2 and 3.
 __global__ void ring_maps_kernel(const ElemRange *__restrict__ ranges,
                                  const ChanInfo *__restrict__ chans,
                                  const int32_t *__restrict__ pp_swap,
                                  const int32_t *__restrict__ hh_swap,
+                                 const int32_t *__restrict__ prow,
+                                 const int32_t *__restrict__ hcol,
                                  const int32_t *__restrict__ flat, int64_t n_t,
-                                 int32_t *__restrict__ inv, int32_t *err) {
+                                 int32_t *__restrict__ dst, int32_t *err) {
   const ElemRange rg = ranges[blockIdx.x];
   const ChanInfo ch = chans[rg.ch];
   for (int64_t e = rg.e0 + threadIdx.x; e < rg.e1; e += blockDim.x) {
@@ -670,7 +669,10 @@ __global__ void ring_maps_kernel(const ElemRange *__restrict__ ranges,
     const int64_t e_ba = ch.t_off + (int64_t)ps * ch.hh + ij;
     const int64_t e_baji = ch.t_off + (int64_t)ps * ch.hh + hs;
     const int32_t f = flat[4 * n_t + e];
-    inv[f] = (int32_t)e;
+    const int r = prow[ch.pp_off + ab], c = hcol[ch.hh_off + ij];
+    dst[f] = r < 0 || c < 0 ? -1
+                            : (int32_t)(4 * (ch.q_off + (int64_t)(r >> 1) * ch.hs + (c >> 1)) +
+                                        2 * (r & 1) + (c & 1));
     if (flat[5 * n_t + e] != flat[4 * n_t + e_ji] || flat[6 * n_t + e] != flat[4 * n_t + e_ba] ||
         flat[7 * n_t + e] != flat[4 * n_t + e_baji])
       atomicOr(err, kErrRingMaps);

@@ -1,9 +1,9 @@
 // Mixed-precision pp ladder on the 5th-generation tensor cores (tcgen05, sm_100a).
 //
-//   D[ab,:] = sum_{c<d} V[ab,cd] T[cd,:] + T[ab,:] (X/2)        packed rows a <= b
+//   D[u,:] = sum_c V[u,c] T[c,:]        packed rows u = a<b, c = c<d, columns i<j
 //
-// is the same antisymmetry-packed product as pp_ladder_kernel (calc.cpp:162-202), with every
-// operand split into NT bf16 terms, x = x_0 + x_1 (+ x_2), each term the bf16 rounding of what
+// is the same antisymmetry-packed product as pp_ladder_kernel (calc.cpp:162-202), with both
+// operands split into NT bf16 terms, x = x_0 + x_1 (+ x_2), each term the bf16 rounding of what
 // the previous ones leave.  The products x_p y_q with p + q < NT are summed by
 // tcgen05.mma.kind::f16 (bf16 inputs, FP32 accumulator in tensor memory): NT = 2 carries
 // about 17 significant bits per operand, NT = 3 about 25.  The ladder is the only mixed
@@ -12,9 +12,9 @@
 //
 // Operand images.  A 128-row x 32-deep K chunk of one term is stored in HBM exactly as the
 // tensor core reads it from shared memory: non-swizzled canonical layouts made of 8 x 8 "core
-// matrices" (128 contiguous bytes), K-major for A (V, and T rows for T X):
+// matrices" (128 contiguous bytes), K-major for A (V):
 //   element (r, k) of a chunk -> (r / 8) * 256 + (k / 8) * 64 + (r % 8) * 8 + k % 8   (bf16)
-// and MN-major for B (T for V T, X/2): element (n, k) -> (n / 8) * 256 + (k / 8) * 64 +
+// and MN-major for B (T): element (n, k) -> (n / 8) * 256 + (k / 8) * 64 +
 // (k % 8) * 8 + n % 8 (tc_off / tc_off_mn in ccd_device.cuh).  One 1-D bulk copy per term moves
 // a stage, and both smem descriptors use LBO = 128 bytes (next core matrix along K) and
 // SBO = 512 bytes (next 8-row / 8-column group).  The last row tile of a channel is compact (only its ceil(rows/8) row groups are
@@ -38,10 +38,12 @@
 
 namespace ccd {
 
-__host__ __device__ constexpr int tc_stages(int nt) { return nt == 2 ? 4 : 3; }
+// 110 KB and 99 KB of stages: one CTA per SM beside the ring's and the hh ladder's CTAs.
+__host__ __device__ constexpr int tc_stages(int nt) { return nt == 2 ? 5 : 3; }
 __host__ __device__ constexpr size_t tc_stage_bytes(int nt) {
   return (size_t)nt * (kTcAPlane + kTcBPlane) * 2;
 }
+constexpr int kTcEpilogue = 128;  // threads that read the accumulator back
 // V_pppp generated inside the ladder (electron gas): generator warps.
 constexpr int kTcGenWarps = 4;
 __host__ __device__ constexpr int tc_threads(bool gen) {
@@ -157,7 +159,7 @@ __device__ __forceinline__ bool consumers_all(bool v) {
       "{ .reg .pred p, q; setp.ne.u32 p, %1, 0; bar.red.and.pred q, 1, %2, p; "
       "selp.u32 %0, 1, 0, q; }"
       : "=r"(r)
-      : "r"((uint32_t)v), "n"(kLadderConsumers)
+      : "r"((uint32_t)v), "n"(kTcEpilogue)
       : "memory");
   return r != 0;
 }
@@ -175,15 +177,15 @@ __device__ __forceinline__ void tc_drain(const uint64_t *full, int issued, int s
 // tile in a small shared-memory queue that the MMA thread, the epilogue warps and (GEN) the
 // generator warps follow.  The producer streams K chunks through the S-stage ring without a
 // break at tile boundaries; the MMA thread accumulates tile number lt of the CTA into
-// tensor-memory buffer lt & 1 (two 128-column accumulators), so that the epilogue warps read
+// tensor-memory buffer lt & 1 (two 64-column accumulators), so that the epilogue warps read
 // tile lt back while tile lt + 1 is loaded and multiplied.  Barriers: full / empty per stage,
 // acc_full / acc_empty per accumulator (tcgen05.commit, and one arrival per epilogue warp),
 // tq_full / tq_empty per queue slot.  Every wait is bounded and checks the CTA's abort flag.
 // Tiles are bm = 128 rows, nb = UMMA N columns, K chunks of kTcKC; image arrays hold NT planes
 // each, plane p at base + p * stride.  A mixed-phase kernel (gate 1 of skip_iteration).
-constexpr uint32_t kTcAccCols = 128;  // columns of one accumulator buffer (nb <= kTcMaxNB)
+constexpr uint32_t kTcAccCols = 64;   // columns of one accumulator buffer (nb <= kTcMaxNB)
 constexpr int kTcTQ = 4;              // slots of a CTA's queue of claimed tiles
-constexpr int kTcGrid = 2 * 148;      // persistent grid: two CTAs on each of the 148 SMs
+constexpr int kTcGrid = 148;          // persistent grid: one CTA on each SM
 // GEN (electron gas, V generated in the ladder): warps 6 .. 6 + kTcGenWarps - 1 write the V
 // operand planes of every V T chunk into the stage (fence.proxy.async, then one arrival per
 // warp on the stage's full barrier, for every chunk); the producer copies only the B planes of
@@ -193,10 +195,7 @@ __global__ void __launch_bounds__(tc_threads(GEN), GEN ? 2 : 1)
 pp_ladder_tc_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *sched,
                     const __nv_bfloat16 *__restrict__ v_tc, int64_t v_stride,
                     const __nv_bfloat16 *__restrict__ tkt_tc, int64_t tkt_stride,
-                    const __nv_bfloat16 *__restrict__ tmt_tc, int64_t tmt_stride,
-                    const __nv_bfloat16 *__restrict__ xt_tc, int64_t xt_stride,
-                    const int32_t *__restrict__ rowmap, const int32_t *__restrict__ mirror,
-                    double *__restrict__ d, double *part, const Control *ctl, int32_t *err,
+                    double *__restrict__ d, const Control *ctl, int32_t *err,
                     const ChanInfo *__restrict__ chans, const VGenRow *__restrict__ vg_rows,
                     const uint32_t *__restrict__ vg_cols, const double *__restrict__ vg_tab) {
   if (skip_iteration(ctl, 1, kTrLadderTC)) return;
@@ -228,12 +227,12 @@ pp_ladder_tc_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&acc_full[b]), 1);
-      mbar_init(smem_u32(&acc_empty[b]), kLadderConsumers / 32);
+      mbar_init(smem_u32(&acc_empty[b]), kTcEpilogue / 32);
     }
     mbar_init(smem_u32(done), 1);
     for (int q = 0; q < kTcTQ; ++q) {
       mbar_init(smem_u32(&tq_full[q]), 1);
-      mbar_init(smem_u32(&tq_empty[q]), 1 + kLadderConsumers / 32 + (GEN ? kTcGenWarps : 0));
+      mbar_init(smem_u32(&tq_empty[q]), 1 + kTcEpilogue / 32 + (GEN ? kTcGenWarps : 0));
     }
     abort_flag = 0;
     issued_chunks = 0;
@@ -284,12 +283,10 @@ pp_ladder_tc_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *
         mbar_arrive(smem_u32(&tq_full[slot]));
         if (ti < 0) break;
         const LadderTile tile = tiles[ti];
-        const int nchunks = tile.nks + tile.nkh;
+        const int nchunks = tile.nks;
         const int rg = (tile.rows + 7) >> 3;  // stored row groups of the A chunks
         const int ng = tile.nb >> 3;          // row groups of a B chunk
         const uint32_t abytes = (uint32_t)rg * kTcGroup * 2, bbytes = (uint32_t)ng * kTcGroup * 2;
-        const int64_t vtile = tile.v_base + (int64_t)tile.mt * kTcBM * tile.nkc * kTcKC;
-        const int64_t ttile = tile.tmt_base + (int64_t)tile.mt * kTcBM * tile.nkh * kTcKC;
         for (int c = 0; c < nchunks; ++c, ++gc) {
           const int s = gc % S;
           if (read_flag(&abort_flag) ||
@@ -298,29 +295,15 @@ pp_ladder_tc_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *
             stop = true;
             break;
           }
-          const __nv_bfloat16 *asrc, *bsrc;
-          int64_t as, bs;
-          if (c < tile.nks) {
-            const int kc = tile.kc0 + c;
-            asrc = v_tc + vtile + (int64_t)kc * rg * kTcGroup;
-            bsrc = tkt_tc + tile.tkt_base + (int64_t)kc * ng * kTcGroup;
-            as = v_stride;
-            bs = tkt_stride;
-          } else {
-            const int kh = c - tile.nks;
-            asrc = tmt_tc + ttile + (int64_t)kh * rg * kTcGroup;
-            bsrc = xt_tc + tile.xt_base + (int64_t)kh * ng * kTcGroup;
-            as = tmt_stride;
-            bs = xt_stride;
-          }
+          const __nv_bfloat16 *asrc = v_tc + tile.a_base + (int64_t)c * rg * kTcGroup;
+          const __nv_bfloat16 *bsrc = tkt_tc + tile.b_base + (int64_t)c * ng * kTcGroup;
           const uint32_t fb = smem_u32(&full[s]);
           const uint32_t sa = base + s * kStageBytes, sb = sa + NT * kTcAPlane * 2;
-          const bool copy_a = !GEN || c >= tile.nks;  // GEN: the generator warps write V
-          mbar_expect_tx(fb, NT * ((copy_a ? abytes : 0u) + bbytes));
+          mbar_expect_tx(fb, NT * ((GEN ? 0u : abytes) + bbytes));  // GEN: V is generated
 #pragma unroll
           for (int p = 0; p < NT; ++p) {
-            if (copy_a) bulk_g2s(sa + p * kTcAPlane * 2, asrc + p * as, abytes, fb);
-            bulk_g2s(sb + p * kTcBPlane * 2, bsrc + p * bs, bbytes, fb);
+            if (!GEN) bulk_g2s(sa + p * kTcAPlane * 2, asrc + p * v_stride, abytes, fb);
+            bulk_g2s(sb + p * kTcBPlane * 2, bsrc + p * tkt_stride, bbytes, fb);
           }
         }
       }
@@ -348,7 +331,7 @@ pp_ladder_tc_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *
         tc_fence_after();
         const uint32_t acc = tmem + buf * kTcAccCols;
         const uint32_t idesc = tc_idesc(tile.nb);
-        const int nchunks = tile.nks + tile.nkh;
+        const int nchunks = tile.nks;
         bool ok = true;
         for (int c = 0; c < nchunks; ++c, ++gc) {
           const int s = gc % S;
@@ -396,7 +379,7 @@ pp_ladder_tc_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *
       }
       if (ti < 0) break;
       const LadderTile tile = tiles[ti];
-      const int nchunks = tile.nks + tile.nkh;
+      const int nchunks = tile.nks;
       const int64_t pk_off = chans[tile.ch].pk_off;
       const int pk = chans[tile.ch].pk;
       VGenRow rw[RG];
@@ -405,7 +388,7 @@ pp_ladder_tc_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *
         const int r = 8 * (gw + i * kTcGenWarps) + (lane >> 2);
         // Rows past the tile: zero momenta, so the index stays inside the table (their
         // accumulator rows are never read).
-        rw[i] = r < tile.rows ? vg_rows[tile.row_off + (int64_t)tile.mt * kTcBM + r]
+        rw[i] = r < tile.rows ? vg_rows[pk_off + (int64_t)tile.mt * kTcBM + r]
                               : VGenRow{kVGenZero, kVGenZero};
       }
       // Column codes of a chunk; K padding (w >= pk) gets weight 0.
@@ -431,7 +414,7 @@ pp_ladder_tc_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *
           stop = true;
           break;
         }
-        if (c < tile.nks) {
+        {
           unsigned char *sa = stage0 + s * kStageBytes;
 #pragma unroll
           for (int i = 0; i < RG; ++i) {
@@ -480,17 +463,15 @@ pp_ladder_tc_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *
       if (!ok) fail();
       // One decision for all four warps (tcgen05.ld is warp-collective).
       if (!consumers_all(ok && !read_flag(&abort_flag))) break;
-      if (tile.nks + tile.nkh > 0) {
-        const LadderOut out{tile, rowmap, mirror, d, part};
-        const uint32_t lane_addr = tmem + buf * kTcAccCols + ((uint32_t)(warp * 32) << 16);
-        for (int c0 = 0; c0 < tile.nb; c0 += 16) {
-          float v[16];
-          tc_ld16(lane_addr + c0, v);
-          double dv[16];
+      const uint32_t lane_addr = tmem + buf * kTcAccCols + ((uint32_t)(warp * 32) << 16);
+      double *o = d + tile.out + (int64_t)tid * tile.hs;
+      for (int c0 = 0; c0 < tile.nb; c0 += 16) {
+        float v[16];
+        tc_ld16(lane_addr + c0, v);
+        if (tid < tile.rows)
 #pragma unroll
-          for (int i = 0; i < 16; ++i) dv[i] = (double)v[i];
-          out.row<16>(tid, c0, dv);
-        }
+          for (int i = 0; i < 16; ++i)
+            if (c0 + i < tile.hk) o[c0 + i] = (double)v[i];
       }
       tc_fence_before();
       __syncwarp();

@@ -57,15 +57,12 @@ struct ccdgpu_handle {
   cudaEvent_t ev[10] = {};
   uint64_t nch = 0, nsp = 0, np = 0, npart = 0;
   int64_t n_t = 0, n_m = 0, n_h = 0, n_p = 0;
-  int n_hh_small = 0;  // hh-ladder units of channels with hh <= 16 (first in hh_tiles)
-  size_t hh_slice_smem = 0;  // dynamic shared memory of hh_slice_kernel (largest hh > 16)
-  int n_hh_red = 0;    // hh-ladder reduction items
-  int n_act = 0, n_mod = 0, n_mod_small = 0, n_mod_mid = 0, n_tiles = 0, n_hh_tiles = 0;
+  int n_hh_cta = 0, n_hh_warp = 0;  // hh-ladder units: one per CTA (hk > 8) first, then per warp
+  int n_hh_out = 0;    // hh-ladder reduction outputs
+  int n_act = 0, n_mod = 0, n_mod_small = 0, n_mod_mid = 0, n_tiles = 0;
   int n_ranges = 0;
   int n_asm_blocks = 0;  // fused assembly CTAs (persistent, striding over quad_items)
-  int n_cls[3] = {0, 0, 0};  // pp-ladder tiles per column class (thin, mid, wide), in that order
-  size_t ladder_smem_thin = 0;
-  size_t ladder_smem = 0, hh_smem = 0;
+  int n_cls[3] = {0, 0, 0};  // FP64 pp-ladder tiles per column class (thin, mid, wide)
   int n_mod_pad[4] = {0, 0, 0, 0};  // ring channels by padded size 32, 48, 64, 80 (after small)
   bool have_3body = false;
   std::vector<DevBuf> allocs;
@@ -74,10 +71,10 @@ struct ccdgpu_handle {
   ModInfo *mods = nullptr;        // small (n_mod_small), then by padded size 32 .. 80
   LadderTile *tiles = nullptr;
   HHTile *hh_tiles = nullptr;
-  HHRed *hh_red = nullptr;
-  int32_t *rowmap = nullptr, *mirror = nullptr;
-  int2 *pk_idx = nullptr;
-  double *part = nullptr, *lpart = nullptr;
+  HHOut *hh_out = nullptr;
+  int64_t *hh_part_off = nullptr;  // per channel: its hh-ladder partials (nhht * hk * hk)
+  int32_t *prow = nullptr, *hcol = nullptr;  // pp / hh pair -> 2 u (+ 1 when a > b), -1
+  double *part = nullptr;
   ElemRange *ranges = nullptr;
   QuadItem *quad_items = nullptr;  // fused assembly: work items of quads (u, w)
   QuadRow *quad_rows = nullptr;    // fused assembly: per strict packed row / hole pair tables
@@ -89,15 +86,23 @@ struct ccdgpu_handle {
   int64_t *list_off = nullptr;
   int32_t *list = nullptr;
   double *eps = nullptr, *v_pphh = nullptr, *v_hhhh = nullptr, *v_t = nullptr;
+  // Packed layout (quads): amplitudes (ping-pong by the control block's parity), V_hhpp, and
+  // the four ring terms of each quad.
+  double *tq[2] = {nullptr, nullptr}, *vq = nullptr, *r_quad = nullptr;
+  int64_t n_q = 0;
   double *v_hpph = nullptr, *v_hphp = nullptr;
   double *t[2] = {nullptr, nullptr}, *dmat = nullptr, *old_phhp = nullptr, *r_phhp = nullptr;
-  double *x = nullptr, *x_t = nullptr, *t_kt = nullptr, *t_mt = nullptr;
+  // t[0] of the fused path holds the amplitudes in the reference order only while slab_current
+  // (it is expanded when they are read); dmat likewise holds t2Diff_pphh unless d_from names
+  // the iteration kind (1 FP64, 2 mixed) whose ladder planes it is expanded from when read.
+  bool slab_current = true;
+  int d_from = 0;
+  double *x = nullptr;
   double *s = nullptr, *r = nullptr, *xh = nullptr, *yp = nullptr, *epart = nullptr;
   int32_t *flat = nullptr;
-  int32_t *inv4 = nullptr;   // phhp position -> pphh element (inverse of the ai_jb table)
+  int32_t *ring_dst = nullptr;  // fused path: phhp position -> 4 x packed position + term, -1
   double create_ms[5] = {};   // ccdgpu_profile::ms_create
   double loop_graph_ms = 0;   // ccdgpu_profile::ms_loop_graph
-  double *d_ring = nullptr;  // fused path: ring result R in pphh order
   int64_t *o_h = nullptr, *o_p = nullptr;
   double *v_h_hpp = nullptr, *v_phh_p = nullptr;
   double *old_h1pp_h2 = nullptr, *old_h2pp_h1 = nullptr, *diff_h2pp_h1 = nullptr;
@@ -120,7 +125,6 @@ struct ccdgpu_handle {
   bool inject_next_step = false;  // ccdgpu_inject_wait_timeout armed for the next step
   ccdgpu_profile prof{};
   double flops = 0, v_bytes = 0, v_packed_bytes = 0, ladder_flops = 0, ladder_bytes = 0;
-  int64_t n_tkt = 0, n_tmt = 0;
   int64_t launches = 0;
 
   // pp-ladder work lists (make_ladder_tiles), in their own allocation so the autotuner can
@@ -131,27 +135,26 @@ struct ccdgpu_handle {
   ccdgpu_schedule schedule{};
   void *tile_mem = nullptr;
   size_t tile_bytes = 0;
-  RedItem *red_fp = nullptr, *red_tc = nullptr;  // split-K reduction items
-  int32_t *tc_sched = nullptr;  // tensor-core ladder: tile counter, exit ticket (zero between launches)
-  int tc_grid = 0;
-  int32_t *fp_cta_off = nullptr;  // FP64 ladder classes: tile ranges of their persistent CTAs
-  int fp_grid[3] = {0, 0, 0}, fp_off_base[3] = {0, 0, 0};
-  int n_red_fp = 0, n_red_tc = 0, n_red_cls[3] = {0, 0, 0};
+  LadderChan *lchans = nullptr, *tc_lchans = nullptr;  // D planes per channel
+  double *d_planes = nullptr, *tc_planes = nullptr;
+  // Tile counter and exit ticket of the FP64 ladder, then of the tensor-core ladder (zero
+  // between launches).
+  int32_t *sched = nullptr;
 
   // Mixed precision (nt bf16 terms per operand; 0 for an FP64 handle).
   int nt = 0;
   int n_tc_tiles = 0;
   LadderTile *tc_tiles = nullptr;
   int32_t *kcol = nullptr;  // pp index of the w-th c<d pair of each channel (pk_off + w)
-  double *tc_part = nullptr;
-  __nv_bfloat16 *v_tc = nullptr, *tkt_tc = nullptr, *tmt_tc = nullptr, *xt_tc = nullptr;
+  __nv_bfloat16 *v_tc = nullptr, *tkt_tc = nullptr;
+  bool tc_stale = false;  // tkt_tc is not the image of the current amplitudes
   // Electron gas with V generated on the device: the tensor-core ladder generates its V
   // planes itself (no v_tc images) from these per-row / per-K-column codes and the q^2 table.
   bool tc_gen = false;
   VGenRow *vg_rows = nullptr;
   uint32_t *vg_cols = nullptr;
   double *vg_tab = nullptr;
-  int64_t n_vtc = 0, n_tkttc = 0, n_tmttc = 0, n_xttc = 0;  // plane strides (elements)
+  int64_t n_vtc = 0, n_tkttc = 0;  // plane strides (elements)
   size_t tc_smem = 0;
   double ladder_bytes_tc = 0;
   cudaGraphExec_t graph_tc = nullptr;
@@ -759,189 +762,97 @@ int upload_runs(ccdgpu_handle *h, T *dst, const std::vector<const T *> &src,
   return copy_runs_to_device(h, reinterpret_cast<char *>(dst), rs, rl);
 }
 
-// pp-ladder work tiles for a schedule (split factors of K per column class), in their own
-// device allocation; drops captured graphs, which hold the old lists.
-//   FP64 ladder: thin row blocks stream at full bandwidth on their own, so K is split only when
-//   there are fewer of them than SMs (up to thin_split_mul tiles per SM); mid/wide tiles are
-//   compute-latency bound per CTA, so K is split into segments of at least four chunks until
-//   the class has about wide_split_mul tiles per SM.
-//   Tensor-core ladder: each CTA is bandwidth bound, so K is split until there are about
-//   tc_split_mul tiles per SM.
-// Split row blocks are reduced after the ladder by ladder_reduce_kernel (segment order, so
-// deterministic), one item per (row block, 16-row chunk), FP64 items grouped by class.
-// Longest-processing-time assignment of tiles[lo, hi) to G persistent CTAs: sorted by cost,
-// largest first, each tile goes to the CTA with the least work so far; the range is rewritten
-// grouped by CTA and the CTAs' ranges are appended to `off` (absolute indices, G + 1 entries).
-template <class Cost>
-void lpt_group(std::vector<LadderTile> &tiles, size_t lo, size_t hi, int G, Cost cost,
-               std::vector<int32_t> &off) {
-  // Costs once; (-cost, position) pairs sorted ascending give the order of a stable sort by
-  // decreasing cost.
-  const size_t n = hi - lo;
-  std::vector<std::pair<int64_t, int32_t>> order(n);
-  for (size_t i = 0; i < n; i++) order[i] = {-cost(tiles[lo + i]), (int32_t)i};
-  std::sort(order.begin(), order.end());
-  std::priority_queue<std::pair<int64_t, int>, std::vector<std::pair<int64_t, int>>,
-                      std::greater<std::pair<int64_t, int>>> load;
-  for (int b = 0; b < G; b++) load.push({0, b});
-  std::vector<int32_t> owner(n), count(G + 1, 0);
-  for (size_t i = 0; i < n; i++) {
-    auto [w, b] = load.top();
-    load.pop();
-    owner[i] = b;
-    count[b + 1]++;
-    load.push({w - order[i].first, b});
-  }
-  // Each CTA's tiles in the order they were assigned, CTA after CTA.
-  for (int b = 0; b < G; b++) count[b + 1] += count[b];
-  std::vector<LadderTile> placed(n);
-  std::vector<int32_t> next(count.begin(), count.end() - 1);
-  for (size_t i = 0; i < n; i++) placed[next[owner[i]]++] = tiles[lo + order[i].second];
-  std::copy(placed.begin(), placed.end(), tiles.begin() + lo);
-  for (int b = 0; b <= G; b++) off.push_back((int32_t)(lo + count[b]));
-}
+int materialize_d(ccdgpu_handle *h);
 
+// pp-ladder work tiles for a schedule (split factors of K per column class), in their own
+// device allocation with the D planes they write; drops captured graphs, which hold the old
+// lists.  Row blocks stream at full bandwidth on their own, so K is split (into segments of at
+// least four chunks) only until a class has about its split factor's number of tiles per SM:
+// thin ones when there are fewer blocks than SMs, up to thin_split_mul tiles per SM; mid and
+// wide ones, compute bound per CTA, to about wide_split_mul (mid_split_mul); the tensor-core
+// ladder to about tc_split_mul.  Each segment writes its own plane of the channel's D, which the
+// assembly adds in segment order (deterministic).
+// The persistent CTAs claim tiles in list order from a launch-wide counter: FP64 tiles by class,
+// wide first (the longest work per byte), then by decreasing cost, the tensor-core tiles by
+// decreasing cost.  Cost = bytes streamed per K chunk x chunks, plus two chunks' worth for the
+// pipeline fill and the epilogue.
 int make_ladder_tiles(ccdgpu_handle *h, const ccdgpu_schedule &sch) {
+  if (int rc = materialize_d(h)) return rc;  // it reads the planes that go away here
   const std::vector<ChanInfo> &chans = h->host_chans;
-  auto cls_of = [](int nb) { return nb <= 8 ? 0 : nb <= 32 ? 1 : 2; };
-  int64_t blocks[3] = {0, 0, 0};
-  for (const ChanInfo &a : chans) blocks[cls_of(a.nb)] += a.nmt;
   const int64_t kSMs = 148;
   const int mid_mul = sch.mid_split_mul > 0 ? sch.mid_split_mul : sch.wide_split_mul;
-  auto want_of = [&](int64_t mul, int64_t b) {
-    return (int)std::min<int64_t>(64, std::max<int64_t>(1, ceil_div(mul * kSMs, std::max<int64_t>(b, 1))));
+  int64_t blocks[3] = {0, 0, 0}, tc_blocks = 0;
+  for (const ChanInfo &a : chans) {
+    if (a.nmt) blocks[ladder_class(a.hs)] += a.nmt;
+    tc_blocks += a.nmt;
+  }
+  auto want_of = [&](int64_t mul, int64_t b, int64_t most) {
+    return (int)std::min<int64_t>(most, std::max<int64_t>(1, ceil_div(mul * kSMs, std::max<int64_t>(b, 1))));
   };
-  const int want_cls[3] = {
-      blocks[0] >= kSMs ? 1 : (int)std::min<int64_t>(8, ceil_div(sch.thin_split_mul * kSMs, std::max<int64_t>(blocks[0], 1))),
-      want_of(mid_mul, blocks[1]), want_of(sch.wide_split_mul, blocks[2])};
-  std::vector<LadderTile> tiles;
-  int64_t lpart_tot = 0;
-  int32_t groups = 0;
-  for (int ai = 0; ai < h->n_act; ai++) {
-    const ChanInfo &a = chans[ai];
-    const int want = want_cls[cls_of(a.nb)];
-    const int min_chunks = 4;
-    const int nseg = std::max(1, std::min(want, a.nkc / min_chunks));
-    for (int mt = 0; mt < a.nmt; mt++) {
-      const int rows = std::min(a.bm, a.pr - mt * a.bm);
-      const int64_t pbase = lpart_tot;
-      if (nseg > 1) lpart_tot += (int64_t)nseg * a.bm * a.nb;
-      for (int sg = 0; sg < nseg; sg++) {
-        LadderTile tl{};
-        tl.ch = ai; tl.mt = mt;
-        tl.kc0 = (int)((int64_t)a.nkc * sg / nseg);
-        tl.nks = (int)((int64_t)a.nkc * (sg + 1) / nseg) - tl.kc0;
-        tl.nkc = a.nkc;
-        tl.nkh = (sg == nseg - 1) ? a.nkh : 0;
-        tl.nb = a.nb; tl.bm = a.bm; tl.rows = rows; tl.pr = a.pr; tl.hh = a.hh;
-        tl.seg = sg; tl.nseg = nseg; tl.group = groups;
-        tl.v_base = a.vkt_base; tl.tkt_base = a.tkt_base; tl.tmt_base = a.tmt_base;
-        tl.xt_base = a.xt_base; tl.t_off = a.t_off; tl.row_off = a.row_off;
-        tl.part_base = pbase;
-        tiles.push_back(tl);
-      }
-      groups++;
-    }
-  }
-  // Thin channels first, then mid and wide ones; each class runs on persistent CTAs (3, 2 and
-  // 1 per SM) with a balanced (LPT) assignment.  Cost = bytes per 16-deep chunk x chunks, plus
-  // two chunks' worth for the pipeline fill and the epilogue.
-  {  // stable by class: three passes
-    std::vector<LadderTile> by_cls;
-    by_cls.reserve(tiles.size());
-    for (int k = 0; k < 3; k++)
-      for (const LadderTile &t : tiles)
-        if (cls_of(t.nb) == k) by_cls.push_back(t);
-    tiles.swap(by_cls);
-  }
-  std::vector<int32_t> fp_cta_off;
-  {
-    auto fp_cost = [](const LadderTile &x) {
-      return (int64_t)(x.nks + x.nkh + 2) * (ladder_arows(x.nb, x.rows) + ladder_bs(x.nb));
-    };
-    size_t lo = 0;
-    const int slots[3] = {3 * 148, 2 * 148, 148};
-    for (int k = 0; k < 3; k++) {
-      size_t hi = lo;
-      while (hi < tiles.size() && cls_of(tiles[hi].nb) == k) hi++;
-      h->fp_off_base[k] = (int)fp_cta_off.size();
-      h->fp_grid[k] = (int)std::min<size_t>(hi - lo, slots[k]);
-      if (hi > lo) lpt_group(tiles, lo, hi, h->fp_grid[k], fp_cost, fp_cta_off);
-      lo = hi;
-    }
-  }
-  std::vector<LadderTile> tc_tiles;
-  int64_t tcpart_tot = 0;
-  int32_t tc_groups = 0;
-  if (h->nt) {
-    int64_t blocks = 0;
-    for (const ChanInfo &a : chans) blocks += ceil_div(a.pr, kTcBM);
-    const int want = (int)std::min<int64_t>(32, std::max<int64_t>(1, ceil_div(sch.tc_split_mul * kSMs, blocks)));
+  const int want_cls[3] = {blocks[0] >= kSMs ? 1 : want_of(sch.thin_split_mul, blocks[0], 8),
+                           want_of(mid_mul, blocks[1], 64),
+                           want_of(sch.wide_split_mul, blocks[2], 64)};
+  const int want_tc = want_of(sch.tc_split_mul, tc_blocks, 32);
+  struct Key {
+    int64_t cost;
+    int32_t cls, pos;
+  };
+  auto make = [&](bool tc, std::vector<LadderTile> &out, std::vector<LadderChan> &lchans,
+                  int64_t &planes) {
+    std::vector<LadderTile> tiles;
+    std::vector<Key> keys;
+    lchans.assign(h->n_act, LadderChan{0, 1, 0});
+    planes = 0;
     for (int ai = 0; ai < h->n_act; ai++) {
       const ChanInfo &a = chans[ai];
-      const int nmt = (int)ceil_div(a.pr, kTcBM);
-      const int nseg = std::max(1, std::min(want, a.nkct / 4));
-      for (int mt = 0; mt < nmt; mt++) {
-        const int rows = std::min(kTcBM, a.pr - mt * kTcBM);
-        const int64_t pbase = tcpart_tot;
-        if (nseg > 1) tcpart_tot += (int64_t)nseg * kTcBM * a.nbt;
+      if (!a.nmt) continue;
+      const int nk = tc ? a.nkct : a.nkc;
+      const int want = tc ? want_tc : want_cls[ladder_class(a.hs)];
+      const int nseg = std::max(1, std::min(want, nk / 4));
+      const int64_t plane = (int64_t)a.nkc * kBK * a.hs;
+      lchans[ai] = LadderChan{planes, nseg, (int32_t)plane};
+      for (int mt = 0; mt < a.nmt; mt++) {
+        const int rows = std::min(kMaxBM, a.pk - mt * kMaxBM);
         for (int sg = 0; sg < nseg; sg++) {
-          LadderTile tl{};
-          tl.ch = ai; tl.mt = mt;
-          tl.kc0 = (int)((int64_t)a.nkct * sg / nseg);
-          tl.nks = (int)((int64_t)a.nkct * (sg + 1) / nseg) - tl.kc0;
-          tl.nkc = a.nkct;
-          tl.nkh = (sg == nseg - 1) ? a.nkht : 0;
-          tl.nb = a.nbt; tl.bm = kTcBM; tl.rows = rows; tl.pr = a.pr; tl.hh = a.hh;
-          tl.seg = sg; tl.nseg = nseg; tl.group = tc_groups;
-          tl.v_base = a.vtc_base; tl.tkt_base = a.tkt_tc_base; tl.tmt_base = a.tmt_tc_base;
-          tl.xt_base = a.xt_tc_base; tl.t_off = a.t_off; tl.row_off = a.row_off;
-          tl.part_base = pbase;
-          tc_tiles.push_back(tl);
+          LadderTile t{};
+          t.ch = ai; t.mt = mt; t.rows = rows;
+          t.kc0 = (int)((int64_t)nk * sg / nseg);
+          t.nks = (int)((int64_t)nk * (sg + 1) / nseg) - t.kc0;
+          t.hk = a.hk; t.hs = a.hs; t.nb = a.nbt;
+          t.out = planes + sg * plane + (int64_t)mt * kMaxBM * a.hs;
+          int64_t cost;
+          if (tc) {
+            const int rg = (rows + 7) / 8, ng = a.nbt / 8;
+            t.a_base = a.vtc_base + (int64_t)mt * kTcBM * nk * kTcKC + (int64_t)t.kc0 * rg * kTcGroup;
+            t.b_base = a.tkt_tc_base + (int64_t)t.kc0 * ng * kTcGroup;
+            cost = (int64_t)(t.nks + 2) * (8 * rg + a.nbt);
+          } else {
+            const int ar = ladder_arows(a.hs, rows);
+            t.a_base = a.vkt_base + ((int64_t)mt * ladder_arows_full(a.hs) * nk + (int64_t)t.kc0 * ar) * kBK;
+            t.b_base = a.q_off + (int64_t)t.kc0 * kBK * a.hs;
+            cost = (int64_t)(t.nks + 2) * (ar + a.hs);
+          }
+          keys.push_back(Key{cost, tc ? 0 : 2 - ladder_class(a.hs), (int32_t)tiles.size()});
+          tiles.push_back(t);
         }
-        tc_groups++;
       }
+      planes += nseg * plane;
     }
-    // The persistent CTAs claim tiles in list order from a launch-wide counter: sorted by
-    // decreasing cost, that is longest-first list scheduling.  Cost = bytes streamed per
-    // 32-deep chunk x chunks, plus two chunks' worth for the pipeline fill and the epilogue.
-    auto tc_cost = [](const LadderTile &x) {
-      return (int64_t)(x.nks + x.nkh + 2) * (((x.rows + 7) & ~7) + x.nb);
-    };
-    // (-cost, position) pairs sorted ascending: the order of a stable sort by decreasing cost.
-    std::vector<std::pair<int64_t, int32_t>> ord(tc_tiles.size());
-    for (size_t i = 0; i < tc_tiles.size(); i++) ord[i] = {-tc_cost(tc_tiles[i]), (int32_t)i};
-    std::sort(ord.begin(), ord.end());
-    std::vector<LadderTile> sorted(tc_tiles.size());
-    for (size_t i = 0; i < ord.size(); i++) sorted[i] = tc_tiles[ord[i].second];
-    tc_tiles.swap(sorted);
-  }
-  // Reduction items of split row blocks.
-  auto red_items = [](const std::vector<LadderTile> &tl, std::vector<RedItem> &out, int *per_cls,
-                      bool by_class, int (*cls)(int)) {
-    std::vector<std::vector<RedItem>> parts(by_class ? 3 : 1);
-    std::vector<char> seen;
-    for (size_t i = 0; i < tl.size(); i++) {
-      const LadderTile &t = tl[i];
-      if (t.nseg <= 1) continue;
-      if ((size_t)t.group >= seen.size()) seen.resize(t.group + 1, 0);
-      if (seen[t.group]) continue;
-      seen[t.group] = 1;
-      for (int r0 = 0; r0 < t.rows; r0 += kRedRows)
-        parts[by_class ? cls(t.nb) : 0].push_back({(int32_t)i, r0});
-    }
-    for (size_t k = 0; k < parts.size(); k++) {
-      if (per_cls) per_cls[k] = (int)parts[k].size();
-      out.insert(out.end(), parts[k].begin(), parts[k].end());
-    }
+    std::sort(keys.begin(), keys.end(), [](const Key &x, const Key &y) {
+      return x.cls != y.cls ? x.cls < y.cls : x.cost != y.cost ? x.cost > y.cost : x.pos < y.pos;
+    });
+    out.resize(tiles.size());
+    for (size_t i = 0; i < keys.size(); i++) out[i] = tiles[keys[i].pos];
   };
-  std::vector<RedItem> red_fp, red_tc;
-  red_items(tiles, red_fp, h->n_red_cls, true, [](int nb) { return nb <= 8 ? 0 : nb <= 32 ? 1 : 2; });
-  red_items(tc_tiles, red_tc, nullptr, false, nullptr);
-  // Device copies: one allocation, counters zeroed, written on s3, which s0 then waits for.
-  // A schedule that replaces another first waits for the handle's work in flight (the old
-  // lists may be in use); the first one, made in create while the set-up kernels run on s0,
-  // has nothing to wait for, so create's host work goes on beside them.
+  std::vector<LadderTile> tiles, tc_tiles;
+  std::vector<LadderChan> lchans, tc_lchans;
+  int64_t planes = 0, tc_planes = 0;
+  make(false, tiles, lchans, planes);
+  if (h->nt) make(true, tc_tiles, tc_lchans, tc_planes);
+  // Device copies: one allocation, written on s3, which s0 then waits for.  A schedule that
+  // replaces another first waits for the handle's work in flight (the old lists may be in use);
+  // the first one, made in create while the set-up kernels run on s0, has nothing to wait for,
+  // so create's host work goes on beside them.
   const bool first = h->tile_mem == nullptr;
   if (!first) {
     CK(cudaStreamSynchronize(h->s0));
@@ -956,54 +867,42 @@ int make_ladder_tiles(ccdgpu_handle *h, const ccdgpu_schedule &sch) {
   h->tile_mem = nullptr;
   h->tile_bytes = 0;
   h->tiles = h->tc_tiles = nullptr;
-  h->lpart = h->tc_part = nullptr;
-  h->fp_cta_off = nullptr;
-  h->tc_sched = nullptr;
-  h->red_fp = h->red_tc = nullptr;
+  h->lchans = h->tc_lchans = nullptr;
+  h->d_planes = h->tc_planes = nullptr;
+  h->sched = nullptr;
   h->n_tiles = h->n_tc_tiles = 0;
   Arena ar;
-  ar.add(&h->tiles, tiles.size()); ar.add(&h->lpart, lpart_tot);
-  ar.add(&h->tc_tiles, tc_tiles.size());
-  ar.add(&h->fp_cta_off, fp_cta_off.size()); ar.add(&h->tc_sched, 2);
-  ar.add(&h->tc_part, tcpart_tot);
-  ar.add(&h->red_fp, red_fp.size()); ar.add(&h->red_tc, red_tc.size());
+  ar.add(&h->tiles, tiles.size()); ar.add(&h->tc_tiles, tc_tiles.size());
+  ar.add(&h->lchans, lchans.size()); ar.add(&h->tc_lchans, tc_lchans.size());
+  ar.add(&h->sched, 4);
+  ar.add(&h->d_planes, planes); ar.add(&h->tc_planes, tc_planes);
   CK(dev_alloc(ar.used, &h->tile_mem, &h->tile_bytes));
-  CK(cudaMemsetAsync(h->tile_mem, 0, ar.used, h->s3));
   for (auto &r : ar.reqs) *r.first = static_cast<char *>(h->tile_mem) + r.second;
-  if (!tiles.empty())
-    CK(cudaMemcpyAsync(h->tiles, tiles.data(), tiles.size() * sizeof(LadderTile),
-                       cudaMemcpyHostToDevice, h->s3));
-  if (!tc_tiles.empty())
-    CK(cudaMemcpyAsync(h->tc_tiles, tc_tiles.data(), tc_tiles.size() * sizeof(LadderTile),
-                       cudaMemcpyHostToDevice, h->s3));
-  if (!fp_cta_off.empty())
-    CK(cudaMemcpyAsync(h->fp_cta_off, fp_cta_off.data(), fp_cta_off.size() * sizeof(int32_t),
-                       cudaMemcpyHostToDevice, h->s3));
-  h->tc_grid = (int)std::min<size_t>(tc_tiles.size(), kTcGrid);
-  if (!red_fp.empty())
-    CK(cudaMemcpyAsync(h->red_fp, red_fp.data(), red_fp.size() * sizeof(RedItem),
-                       cudaMemcpyHostToDevice, h->s3));
-  if (!red_tc.empty())
-    CK(cudaMemcpyAsync(h->red_tc, red_tc.data(), red_tc.size() * sizeof(RedItem),
-                       cudaMemcpyHostToDevice, h->s3));
-  h->n_red_fp = (int)red_fp.size();
-  h->n_red_tc = (int)red_tc.size();
+  // The planes are written in full (where the assembly reads them) by every ladder.
+  CK(cudaMemsetAsync(h->sched, 0, 4 * sizeof(int32_t), h->s3));
+  auto up = [&](auto *dst, const auto &v) -> int {
+    if (v.empty()) return CCDGPU_OK;
+    return cuda_status(cudaMemcpyAsync(dst, v.data(), v.size() * sizeof(v[0]),
+                                       cudaMemcpyHostToDevice, h->s3));
+  };
+  if (int rc = up(h->tiles, tiles)) return rc;
+  if (int rc = up(h->tc_tiles, tc_tiles)) return rc;
+  if (int rc = up(h->lchans, lchans)) return rc;
+  if (int rc = up(h->tc_lchans, tc_lchans)) return rc;
   CK(cudaEventRecord(h->ev_fork2, h->s3));
   CK(cudaStreamWaitEvent(h->s0, h->ev_fork2, 0));
   if (!first) CK(cudaStreamSynchronize(h->s0));
   h->n_tiles = (int)tiles.size();
   h->n_cls[0] = h->n_cls[1] = h->n_cls[2] = 0;
-  for (const LadderTile &t : tiles) h->n_cls[cls_of(t.nb)]++;
+  for (const LadderTile &t : tiles) h->n_cls[ladder_class(t.hs)]++;
   h->n_tc_tiles = (int)tc_tiles.size();
   h->schedule = sch;
   return CCDGPU_OK;
 }
 
 using TcKernel = void (*)(const LadderTile *, int, int32_t *, const __nv_bfloat16 *, int64_t,
-                         const __nv_bfloat16 *, int64_t, const __nv_bfloat16 *, int64_t,
-                         const __nv_bfloat16 *, int64_t, const int32_t *, const int32_t *,
-                         double *, double *, const Control *, int32_t *, const ChanInfo *,
-                         const VGenRow *, const uint32_t *, const double *);
+                         const __nv_bfloat16 *, int64_t, double *, const Control *, int32_t *,
+                         const ChanInfo *, const VGenRow *, const uint32_t *, const double *);
 TcKernel tc_kernel_of(int nt, bool gen) {
   if (nt == 2) return gen ? pp_ladder_tc_kernel<2, true> : pp_ladder_tc_kernel<2, false>;
   return gen ? pp_ladder_tc_kernel<3, true> : pp_ladder_tc_kernel<3, false>;
@@ -1013,8 +912,9 @@ TcKernel tc_kernel_of(int nt, bool gen) {
 // (first-touch page faults of ~20 MB of fresh vectors were most of a warm create's host time
 // on the largest bases), later creates only clear them.
 struct BuildScratch {
-  std::vector<int32_t> rowmap, mirror, kcol, pp_swap, hh_swap, list;
-  std::vector<int2> pk_idx, pp_pairs, hh_pairs, vrows, mod_ph, mod_hp, mod_dims;
+  std::vector<int32_t> rowmap, kcol, pp_swap, hh_swap, prow, hcol, qrow, list;
+  std::vector<int2> pp_pairs, hh_pairs, mod_ph, mod_hp, mod_dims;
+  std::vector<int4> vrows;
   std::vector<QuadCol> quad_cols;
   std::vector<QuadItem> quad_items;
   std::vector<ElemRange> ranges;
@@ -1082,23 +982,26 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   for (uint64_t c = 0; c < nch; c++) {
     const int64_t pp = D[c].pp, hh = D[c].hh;
     if (!pp || !hh) continue;
-    if (hh > 8 * kMaxCG || pp > (1 << 20)) return CCDGPU_ERR_UNSUPPORTED;
+    if (hh > kMaxHH || pp > (1 << 20)) return CCDGPU_ERR_UNSUPPORTED;
     if (!P->chan_maps[c].pp || !P->chan_maps[c].hh) return CCDGPU_ERR_INVALID_ARGUMENT;
     act_chan.push_back(c);
     a_pp_off.push_back(a_pp_off.back() + pp);
     a_hh_off.push_back(a_hh_off.back() + hh);
   }
   const int n_act = (int)act_chan.size();
-  std::vector<int32_t> &rowmap = bs.rowmap, &mirror = bs.mirror, &kcol = bs.kcol;
-  std::vector<int2> &pk_idx = bs.pk_idx, &pp_pairs = bs.pp_pairs, &hh_pairs = bs.hh_pairs,
-                    &vrows = bs.vrows;
-  std::vector<int32_t> &pp_swap = bs.pp_swap, &hh_swap = bs.hh_swap;
+  std::vector<int32_t> &rowmap = bs.rowmap, &kcol = bs.kcol;
+  std::vector<int2> &pp_pairs = bs.pp_pairs, &hh_pairs = bs.hh_pairs;
+  std::vector<int4> &vrows = bs.vrows;
+  std::vector<int32_t> &pp_swap = bs.pp_swap, &hh_swap = bs.hh_swap, &prow = bs.prow,
+                       &hcol = bs.hcol, &qrow = bs.qrow;
   pp_pairs.resize(a_pp_off[n_act]);
   pp_swap.resize(a_pp_off[n_act]);
-  pk_idx.resize(a_pp_off[n_act]);
+  prow.resize(a_pp_off[n_act]);
+  qrow.resize(a_pp_off[n_act]);
   hh_pairs.resize(a_hh_off[n_act]);
   hh_swap.resize(a_hh_off[n_act]);
-  std::vector<int32_t> a_pr(n_act), a_pk(n_act);
+  hcol.resize(a_hh_off[n_act]);
+  std::vector<int32_t> a_pr(n_act), a_pk(n_act), a_hk(n_act);
   std::atomic<int> bad{0};
   const int host_threads = std::max(1, std::min(omp_get_max_threads(), 16));
 #pragma omp parallel num_threads(host_threads)
@@ -1126,6 +1029,7 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
       }
       a_pr[ai] = pr;
       a_pk[ai] = pk;
+      int hk = 0;
       for (int64_t k = 0; k < hh; k++) {
         const uint64_t i = hm[k].p, j = hm[k].q;
         const int sw = (i < np && j < np) ? find_pair(hm, hh, j, i) : -1;
@@ -1135,124 +1039,122 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
         }
         hh_pairs[hoff + k] = make_int2((int)i, (int)j);
         hh_swap[hoff + k] = sw;
+        hcol[hoff + k] = i < j ? 2 * hk++ : -1;  // the mirrors in the second pass
       }
+      a_hk[ai] = hk;
     }
   }
   if (bad) return bad;
-  std::vector<int64_t> a_row_off(n_act + 1, 0), a_pk_off(n_act + 1, 0);
+  std::vector<int64_t> a_row_off(n_act + 1, 0), a_pk_off(n_act + 1, 0), a_vrow_off(n_act + 1, 0);
   for (int ai = 0; ai < n_act; ai++) {
     a_row_off[ai + 1] = a_row_off[ai] + a_pr[ai];
     a_pk_off[ai + 1] = a_pk_off[ai] + a_pk[ai];
+    a_vrow_off[ai + 1] = a_vrow_off[ai] + (a_hk[ai] ? a_pk[ai] : 0);
   }
-  rowmap.resize(a_row_off[n_act]);
-  mirror.resize(a_row_off[n_act]);
+  rowmap.resize(on_the_fly ? 0 : a_row_off[n_act]);  // rows a <= b, as V_pppp is uploaded
   // Row items of the stored-V tiling kernels (not needed when V_pppp is generated).
-  vrows.resize(on_the_fly ? 0 : a_row_off[n_act]);
+  vrows.resize(on_the_fly ? 0 : a_vrow_off[n_act]);
   kcol.resize(a_pk_off[n_act]);
 #pragma omp parallel for num_threads(host_threads) schedule(dynamic, 4)
   for (int ai = 0; ai < n_act; ai++) {
     const int64_t pp = D[act_chan[ai]].pp, off = a_pp_off[ai];
-    int32_t *rm = rowmap.data() + a_row_off[ai], *mr = mirror.data() + a_row_off[ai];
-    int2 *vr = on_the_fly ? nullptr : vrows.data() + a_row_off[ai];
+    const int64_t hh = D[act_chan[ai]].hh, hoff = a_hh_off[ai];
+    int32_t *rm = on_the_fly ? nullptr : rowmap.data() + a_row_off[ai];
+    int4 *vr = on_the_fly || !a_hk[ai] ? nullptr : vrows.data() + a_vrow_off[ai];
     int32_t *kc = kcol.data() + a_pk_off[ai];
     int pr = 0, pk = 0;
     for (int64_t k = 0; k < pp; k++) {
       const int a = pp_pairs[off + k].x, b = pp_pairs[off + k].y;
-      int2 q = make_int2(-1, -1);
-      if (a < b) { q.x = pk; kc[pk++] = (int32_t)k; }
-      if (a <= b) {
-        q.y = pr;
-        rm[pr] = (int32_t)k;
-        mr[pr] = a < b ? pp_swap[off + k] : -1;
-        if (vr) vr[pr] = make_int2(ai, pr);
-        pr++;
+      prow[off + k] = qrow[off + k] = -1;
+      if (a < b) {
+        if (vr) vr[pk] = make_int4(ai, pk, pr, 0);
+        prow[off + k] = 2 * pk;
+        qrow[off + k] = (int32_t)(a_pk_off[ai] + pk);
+        kc[pk++] = (int32_t)k;
       }
-      pk_idx[off + k] = q;
+      if (rm && a <= b) rm[pr] = (int32_t)k;
+      pr += a <= b;
     }
+    for (int64_t k = 0; k < pp; k++)
+      if (pp_pairs[off + k].x > pp_pairs[off + k].y) {
+        prow[off + k] = prow[off + pp_swap[off + k]] + 1;
+        qrow[off + k] = qrow[off + pp_swap[off + k]];
+      }
+    for (int64_t k = 0; k < hh; k++)
+      if (hh_pairs[hoff + k].x > hh_pairs[hoff + k].y)
+        hcol[hoff + k] = hcol[hoff + hh_swap[hoff + k]] + 1;
   }
   std::vector<HHTile> hh_tiles;
-  std::vector<HHRed> hh_red;
-  int64_t x_tot = 0, tkt = 0, tmt = 0, xt = 0, vt = 0, part_tot = 0;
+  int64_t vhh_tot = 0, x_tot = 0, q_tot = 0, vt = 0, part_tot = 0, qcol_tot = 0;
   int64_t vraw_tot = 0;
-  int64_t vtc = 0, tkttc = 0, tmttc = 0, xttc = 0;
-  std::vector<int64_t> vraw_off;
-  int maxhh = 1;
+  int64_t vtc = 0, tkttc = 0;
+  std::vector<int64_t> vraw_off, hh_part_off;
   for (int ai = 0; ai < n_act; ai++) {
     const uint64_t c = act_chan[ai];
     const int64_t pp = D[c].pp, hh = D[c].hh;
-    const int pr = a_pr[ai], pk = a_pk[ai];
+    const int pk = a_pk[ai], hk = a_hk[ai];
     ChanInfo ci{};
     ci.pp = (int)pp; ci.hh = (int)hh;
-    ci.nb = ladder_nb((int)hh);
-    ci.bm = ladder_bm(ci.nb);
-    ci.row_off = a_row_off[ai];
+    ci.pk = pk; ci.hk = hk;
+    ci.hs = quad_hs(hk);
     ci.pk_off = a_pk_off[ai];
-    ci.pp_off = a_pp_off[ai]; ci.hh_off = a_hh_off[ai]; ci.x_off = x_tot;
-    ci.pr = pr; ci.pk = pk;
-    ci.nkc = (int)ceil_div(pk, kBK);
-    ci.nkh = (int)ceil_div(hh, kBK);
-    ci.nmt = (int)ceil_div(pr, ci.bm);
-    const int hh_rows = hh <= 16 ? kHHRows : kHHRowsL;  // K slice of the hh ladder
-    ci.nhht = (int)ceil_div(pp, hh_rows);
+    ci.pp_off = a_pp_off[ai]; ci.hh_off = a_hh_off[ai];
     ci.t_off = o_t[c];
-    ci.tkt_base = tkt; ci.tmt_base = tmt; ci.xt_base = xt; ci.vkt_base = vt;
-    ci.part_off = part_tot;
-    ci.hht0 = (int64_t)hh_tiles.size();
-    ci.nbt = tc_nb(ci.hh);
-    ci.nkct = (int)ceil_div(pk, kTcKC);
-    ci.nkht = (int)ceil_div(hh, kTcKC);
-    ci.vtc_base = vtc; ci.tkt_tc_base = tkttc; ci.tmt_tc_base = tmttc; ci.xt_tc_base = xttc;
-    vtc += (int64_t)ci.nkct * kTcGroup * ceil_div(pr, 8);
-    tmttc += (int64_t)ci.nkht * kTcGroup * ceil_div(pr, 8);
-    tkttc += (int64_t)ci.nkct * (ci.nbt / 8) * kTcGroup;
-    xttc += (int64_t)ci.nkht * (ci.nbt / 8) * kTcGroup;
-    const int nb = ci.nb;
-    x_tot += hh * hh;
-    tkt += (int64_t)ci.nkc * kBK * ladder_bs(nb);
-    // Full row tiles at their A stride, then the compact last one.
-    const int64_t arows_tot = (int64_t)(ci.nmt - 1) * ladder_arows_full(ci.nb) +
-                              ladder_arows(ci.nb, ci.pr - (ci.nmt - 1) * ci.bm);
-    tmt += (int64_t)ci.nkh * arows_tot * kBK;
-    xt += (int64_t)ci.nkh * kBK * ladder_bs(nb);
-    vt += (int64_t)ci.nkc * arows_tot * kBK;
-    part_tot += (int64_t)ci.nhht * hh * hh;
+    ci.vhh_off = vhh_tot; ci.x_off = x_tot; ci.q_off = q_tot; ci.vkt_base = vt;
+    ci.qcol_off = qcol_tot;
+    ci.vtc_base = vtc; ci.tkt_tc_base = tkttc;
+    hh_part_off.push_back(part_tot);
+    vhh_tot += hh * hh;
+    qcol_tot += hk;
+    if (pk && hk) {
+      ci.nkc = (int)ceil_div(pk, kBK);
+      ci.nmt = (int)ceil_div(pk, kMaxBM);
+      const int rows = hh_rows(hk);  // K slice of the hh ladder
+      ci.nhht = (int)ceil_div(pk, rows);
+      ci.nbt = tc_nb(hk);
+      ci.nkct = (int)ceil_div(pk, kTcKC);
+      vtc += (int64_t)ci.nkct * kTcGroup * ceil_div(pk, 8);
+      tkttc += (int64_t)ci.nkct * (ci.nbt / 8) * kTcGroup;
+      x_tot += hk * ci.hs;
+      q_tot += (int64_t)ci.nkc * kBK * ci.hs;
+      // Full row tiles at their A stride, then the compact last one.
+      const int64_t arows_tot = (int64_t)(ci.nmt - 1) * ladder_arows_full(ci.hs) +
+                                ladder_arows(ci.hs, pk - (ci.nmt - 1) * kMaxBM);
+      vt += (int64_t)ci.nkc * arows_tot * kBK;
+      part_tot += (int64_t)ci.nhht * hk * hk;
+      for (int t = 0; t < ci.nhht; t++)
+        hh_tiles.push_back({ai, t * rows, t, std::min(rows, pk - t * rows)});
+    }
     vraw_off.push_back(vraw_tot);
-    if (!on_the_fly) vraw_tot += (int64_t)ci.pr * pp;  // packed rows (a <= b) only
-    maxhh = std::max<int>(maxhh, (int)hh);
-    // hh ladder: hh <= 16, one warp unit per K slice (the whole P); wider hh, one CTA unit per
-    // K slice of kHHRowsL rows (every P row tile, hh_slice_kernel).
-    for (int t = 0; t < ci.nhht; t++)
-      hh_tiles.push_back({ai, t * hh_rows, t,
-                          (int)std::min<int64_t>(hh_rows, pp - (int64_t)t * hh_rows), 0, 0});
-    for (int64_t i0 = 0; i0 < hh * hh; i0 += 256) hh_red.push_back({ai, (int32_t)i0});
+    if (!on_the_fly) vraw_tot += (int64_t)a_pr[ai] * pp;  // rows a <= b only
     chans.push_back(ci);
   }
+  if (q_tot * 4 >= INT32_MAX) return CCDGPU_ERR_UNSUPPORTED;  // ring_dst is 32-bit
+  h->n_q = q_tot;
   const int64_t pp_tot = a_pp_off[n_act], hh_tot = a_hh_off[n_act];
   h->n_act = n_act;
-  h->n_hh_tiles = (int)hh_tiles.size();
-  h->n_hh_red = (int)hh_red.size();
-  // Channels with hh <= 16 first (their own launch), then the rest; largest units
-  // (rows x hh^2) first within each, so the short ones fill in behind them.
-  // A stable sort by (class, -cost): the units come channel by channel as runs of equal cost
-  // (the full slices, then a shorter last one), so the runs are stably sorted and expanded,
-  // which gives the same order as sorting the units themselves.
+  // hh-ladder units: one per CTA (hk > 8) first, then one per warp; within each the largest
+  // (rows x hk^2) first, so that the short ones fill in behind them.  A stable sort by (class,
+  // -cost): the units come channel by channel as runs of equal cost (the full slices, then a
+  // shorter last one), so the runs are stably sorted and expanded, which gives the same order as
+  // sorting the units themselves.
   {
     struct Run {
       int32_t first, n;
-      bool wide;
+      bool warp;
       int64_t cost;
     };
     std::vector<Run> runs;
     for (int32_t i = 0; i < (int32_t)hh_tiles.size(); i++) {
       const HHTile &t = hh_tiles[i];
-      const int64_t hh = chans[t.ch].hh, cost = (int64_t)t.rows * hh * hh;
+      const int64_t hk = chans[t.ch].hk, cost = (int64_t)t.rows * hk * hk;
       if (!runs.empty() && hh_tiles[runs.back().first].ch == t.ch && runs.back().cost == cost)
         runs.back().n++;
       else
-        runs.push_back(Run{i, 1, hh > 16, cost});
+        runs.push_back(Run{i, 1, hk <= 8, cost});
     }
     std::stable_sort(runs.begin(), runs.end(), [](const Run &x, const Run &y) {
-      if (x.wide != y.wide) return !x.wide;
+      if (x.warp != y.warp) return y.warp;
       return x.cost > y.cost;
     });
     std::vector<HHTile> sorted;
@@ -1261,11 +1163,9 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
       sorted.insert(sorted.end(), hh_tiles.begin() + r.first, hh_tiles.begin() + r.first + r.n);
     hh_tiles.swap(sorted);
   }
-  for (const HHTile &t : hh_tiles) h->n_hh_small += chans[t.ch].hh <= 16 ? 1 : 0;
-  for (const ChanInfo &a : chans)
-    if (a.hh > 16) h->hh_slice_smem = std::max(h->hh_slice_smem, hh_slice_smem(a.hh));
-  // Per orbital w, the pair elements whose first index is w, ascending (particles: pp
-  // elements, holes: hh elements): a counting sort.  The pp elements (first index a particle)
+  for (const HHTile &t : hh_tiles) (chans[t.ch].hk > 8 ? h->n_hh_cta : h->n_hh_warp)++;
+  // Per orbital w, the strict pairs that hold w, in the order of the ordered pairs whose first
+  // index is w (particles: rows of r, holes: entries of s): a counting sort.  The pp elements (first index a particle)
   // are split into one contiguous range per host thread: per-thread bucket counts, then each
   // thread places its range from its own start in every bucket, so a bucket keeps ascending
   // element order.  The hh elements (first index a hole, buckets of their own) follow serially.
@@ -1282,11 +1182,11 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
       const int t = omp_get_thread_num();
       const int64_t lo = pp_tot * t / team, hi = pp_tot * (t + 1) / team;
       int64_t *c = cnt.data() + (size_t)t * nsp;
-      for (int64_t e = lo; e < hi; e++) c[pp_pairs[e].x]++;
+      for (int64_t e = lo; e < hi; e++) c[pp_pairs[e].x] += qrow[e] >= 0;
 #pragma omp barrier
 #pragma omp single
       {
-        for (int64_t e = 0; e < hh_tot; e++) list_off[hh_pairs[e].x + 1]++;
+        for (int64_t e = 0; e < hh_tot; e++) list_off[hh_pairs[e].x + 1] += hcol[e] >= 0;
         for (uint64_t w = 0; w < nsp; w++) {
           int64_t s = 0;
           for (int u = 0; u < team; u++) s += cnt[(size_t)u * nsp + w];
@@ -1303,11 +1203,14 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
           }
         }
       }
-      for (int64_t e = lo; e < hi; e++) list[c[pp_pairs[e].x]++] = (int32_t)e;
+      for (int64_t e = lo; e < hi; e++)
+        if (qrow[e] >= 0) list[c[pp_pairs[e].x]++] = qrow[e];
     }
     std::vector<int64_t> &cur = bs.o_m_scratch;
     cur.assign(list_off.begin(), list_off.end() - 1);
-    for (int64_t e = 0; e < hh_tot; e++) list[cur[hh_pairs[e].x]++] = (int32_t)e;
+    for (const ChanInfo &a : chans)
+      for (int64_t e = a.hh_off; e < a.hh_off + a.hh; e++)
+        if (hcol[e] >= 0) list[cur[hh_pairs[e].x]++] = (int32_t)(a.qcol_off + (hcol[e] >> 1));
   }
   h->n_list = list_off[nsp];
 
@@ -1329,7 +1232,7 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     const int64_t ph = MD[c].ph, hp = MD[c].hp;
     mod_dims[c] = make_int2((int)ph, (int)hp);
     if (!ph || !hp) continue;
-    if (ph > kTcMaxNB || hp > kTcMaxNB) return CCDGPU_ERR_UNSUPPORTED;  // ring register tiles
+    if (ph > kRingMax || hp > kRingMax) return CCDGPU_ERR_UNSUPPORTED;  // ring tiles
     ModInfo m{};
     m.ph = (int)ph; m.hp = (int)hp; m.m_off = o_m[c]; m.y_off = y_tot;
     if (gen_v) {
@@ -1415,12 +1318,9 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   quad_items.clear();
   // Rows: the packed rows with a < b (pk of them per channel), filled in parallel below;
   // columns (i < j) and work items here.
-  int64_t qrows_tot = 0;
+  std::vector<HHOut> hh_out;
   for (int ai = 0; ai < h->n_act; ai++) {
-    ChanInfo &a = chans[ai];
-    a.qrow_off = qrows_tot;
-    qrows_tot += a.pk;
-    a.qcol_off = (int64_t)quad_cols.size();
+    const ChanInfo &a = chans[ai];
     for (int j = 0; j < a.hh; j++) {
       const int2 pij = hh_pairs[a.hh_off + j];
       if (pij.x >= pij.y) continue;  // i = j: zero column; i > j: the mirror of (j, i)
@@ -1429,14 +1329,21 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
       c.eij = P->sp_energy[pij.x] + P->sp_energy[pij.y];
       quad_cols.push_back(c);
     }
-    a.hk = (int)((int64_t)quad_cols.size() - a.qcol_off);
     const int64_t nq = (int64_t)a.pk * a.hk;
     if (nq >= ((int64_t)1 << 31) / 2) return CCDGPU_ERR_UNSUPPORTED;
     for (int64_t q = 0; q < nq; q += kQuadPerItem)
       quad_items.push_back({ai, (int32_t)q, (int32_t)std::min<int64_t>(nq, q + kQuadPerItem),
-                            a.hk, a.t_off, a.qrow_off, a.qcol_off});
+                            a.hk, a.hs, 0, a.q_off, a.x_off, a.pk_off, a.qcol_off});
+    const QuadCol *qc = quad_cols.data() + a.qcol_off;
+    for (int kl = 0; nq && kl < a.hk; kl++)
+      for (int ij = 0; ij < a.hk; ij++)
+        hh_out.push_back({hh_part_off[ai] + kl * a.hk + ij, a.nhht, a.hk * a.hk,
+                          (int32_t)(a.vhh_off + (int64_t)qc[kl].c_ij * a.hh + qc[ij].c_ij),
+                          (int32_t)(a.x_off + kl * a.hs + ij),
+                          kl == ij ? (int32_t)(a.qcol_off + ij) : -1, 0});
   }
-  h->n_quad_rows = qrows_tot;  // built on the device (quad_rows_kernel)
+  h->n_hh_out = (int)hh_out.size();
+  h->n_quad_rows = a_pk_off[n_act];  // built on the device (quad_rows_kernel)
 
   h->host_chans = chans;
   h->n_quad_items = (int)quad_items.size();
@@ -1450,27 +1357,23 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     lf += 2.0 * a.pp * a.pp * a.hh;
     fl += 2.0 * a.pp * a.pp * a.hh + 4.0 * a.pp * a.hh * (double)a.hh;
     vb += 8.0 * a.pp * a.pp;
-    vbp += 8.0 * a.pr * (double)a.pk;
+    if (a.hk) vbp += 8.0 * a.pk * (double)a.pk;
   }
   for (const ModInfo &m : mods) fl += 4.0 * m.ph * (double)m.hp * m.hp;
   h->flops = fl; h->ladder_flops = lf; h->v_bytes = vb; h->v_packed_bytes = vbp;
-  // Bytes one pp-ladder launch must move: packed V, the T operand rows (c<d for V T, a<=b
-  // for T X), X, and D written in full.
+  // Bytes one pp-ladder launch must move: packed V, the packed amplitudes in and D out.
   double lb = vbp;
-  for (const ChanInfo &a : chans)
-    lb += 8.0 * ((double)a.pk * a.hh + (double)a.pr * a.hh + (double)a.hh * a.hh + (double)a.pp * a.hh);
+  for (const ChanInfo &a : chans) lb += 16.0 * (double)a.pk * a.hk;
   h->ladder_bytes = lb;
   double lbt = 0;
   for (const ChanInfo &a : chans)
-    lbt += 2.0 * h->nt * ((double)a.pr * a.pk + (double)a.pk * a.hh + (double)a.pr * a.hh +
-                          (double)a.hh * a.hh) + 8.0 * a.pp * (double)a.hh;
+    if (a.hk)
+      lbt += 2.0 * h->nt * ((double)a.pk * a.pk + (double)a.pk * a.hk) + 8.0 * a.pk * (double)a.hk;
   h->ladder_bytes_tc = lbt;
-  h->n_tkt = tkt;
-  h->n_tmt = tmt;
 
   // Tensor-core ladder with V generated in the kernel (electron gas, on-the-fly V, momenta
-  // |n_i| <= 6 so that q^2 <= 432): per packed row u (rowmap order) the codes of a and b, per K
-  // index w (kcol order) the code of c (momentum bytes biased by 64, spin in byte 3), and the
+  // |n_i| <= 6 so that q^2 <= 432): per packed row u the codes of a and b, per K
+  // index w the code of c (momentum bytes biased by 64, spin in byte 3), and the
   // direct term by q^2.
   std::vector<VGenRow> vg_rows;
   std::vector<uint32_t> vg_cols;
@@ -1487,16 +1390,14 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
         return (uint32_t)(q[0] + 64) | ((uint32_t)(q[1] + 64) << 8) |
                ((uint32_t)(q[2] + 64) << 16) | ((uint32_t)(q[3] > 0 ? kVGenSpin : 0) << 24);
       };
-      vg_rows.resize(rowmap.size());
+      vg_rows.resize(kcol.size());
       vg_cols.resize(kcol.size());
-      for (const ChanInfo &a : chans) {
-        for (int u = 0; u < a.pr; u++) {
-          const int2 ab = pp_pairs[a.pp_off + rowmap[a.row_off + u]];
-          vg_rows[a.row_off + u] = VGenRow{code(ab.x), code(ab.y)};
+      for (const ChanInfo &a : chans)
+        for (int u = 0; u < a.pk; u++) {
+          const int2 ab = pp_pairs[a.pp_off + kcol[a.pk_off + u]];
+          vg_rows[a.pk_off + u] = VGenRow{code(ab.x), code(ab.y)};
+          vg_cols[a.pk_off + u] = code(ab.x);
         }
-        for (int w = 0; w < a.pk; w++)
-          vg_cols[a.pk_off + w] = code(pp_pairs[a.pp_off + kcol[a.pk_off + w]].x);
-      }
       // w(q^2) = e^2 / L^3 * 4 pi / (2 pi / L)^2 q^2, zero for q = 0 (ElectronGasSPBasis.cpp:
       // 453-466 as a function of q^2).
       const double L = M->params[0], e_sq = M->params[1];
@@ -1505,11 +1406,9 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
         const double rel = (2 * M_PI / L) * (2 * M_PI / L) * q2;
         vg_tab[q2] = e_sq / (L * L * L) * 4 * M_PI / rel;
       }
-      // The ladder then moves no V bytes: the T and X operand images and D.
+      // The ladder then moves no V bytes: the T operand image and D.
       double lbg = 0;
-      for (const ChanInfo &a : chans)
-        lbg += 2.0 * h->nt * ((double)a.pk * a.hh + (double)a.pr * a.hh + (double)a.hh * a.hh) +
-               8.0 * a.pp * (double)a.hh;
+      for (const ChanInfo &a : chans) lbg += (2.0 * h->nt + 8.0) * a.pk * (double)a.hk;
       h->ladder_bytes_tc = lbg;
     }
   }
@@ -1518,26 +1417,28 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   h->create_ms[0] = ms_since(t_build);
   Arena ar;
   ar.add(&h->chans, chans.size()); ar.add(&h->mods, mods.size());
-  ar.add(&h->hh_tiles, hh_tiles.size()); ar.add(&h->hh_red, hh_red.size());
+  ar.add(&h->hh_tiles, hh_tiles.size()); ar.add(&h->hh_out, hh_out.size());
+  ar.add(&h->hh_part_off, hh_part_off.size());
   ar.add(&h->ranges, ranges.size());
   ar.add(&h->pp_pairs, pp_pairs.size()); ar.add(&h->hh_pairs, hh_pairs.size());
   ar.add(&h->pp_swap, pp_swap.size()); ar.add(&h->hh_swap, hh_swap.size());
   ar.add(&h->list_off, list_off.size()); ar.add(&h->list, list.size());
-  ar.add(&h->rowmap, rowmap.size()); ar.add(&h->mirror, mirror.size());
-  ar.add(&h->pk_idx, pk_idx.size());
+  ar.add(&h->prow, prow.size()); ar.add(&h->hcol, hcol.size());
   ar.add(&h->part, part_tot);
+  ar.add(&h->tq[0], q_tot); ar.add(&h->tq[1], q_tot); ar.add(&h->vq, q_tot);
 
   ar.add(&h->eps, nsp);
   // Generated V images are written in full (padding included) by the V generators.
-  ar.add(&h->v_pphh, n_t); ar.add(&h->v_hhhh, x_tot);
+  ar.add(&h->v_pphh, n_t); ar.add(&h->v_hhhh, vhh_tot);
   if (on_the_fly) ar.add_unset(&h->v_t, vt);
   else ar.add(&h->v_t, vt);
   ar.add(&h->v_hpph, h->n_m); ar.add(&h->v_hphp, y_tot);
-  ar.add(&h->flat, (size_t)8 * n_t); ar.add(&h->inv4, n_t); ar.add(&h->d_ring, n_t); ar.add(&h->o_h, o_h.size()); ar.add(&h->o_p, o_p.size());
+  ar.add(&h->flat, (size_t)8 * n_t); ar.add(&h->ring_dst, n_t); ar.add(&h->r_quad, 4 * q_tot);
+  ar.add(&h->o_h, o_h.size()); ar.add(&h->o_p, o_p.size());
   ar.add(&h->t[0], n_t); ar.add(&h->t[1], n_t); ar.add(&h->dmat, n_t);
   ar.add(&h->old_phhp, h->n_m); ar.add(&h->r_phhp, h->n_m);
-  ar.add(&h->x, x_tot); ar.add(&h->x_t, xt); ar.add(&h->t_kt, tkt); ar.add(&h->t_mt, tmt);
-  ar.add(&h->s, hh_tot); ar.add(&h->r, pp_tot); ar.add(&h->xh, np); ar.add(&h->yp, h->npart);
+  ar.add(&h->x, x_tot);
+  ar.add(&h->s, quad_cols.size()); ar.add(&h->r, h->n_quad_rows); ar.add(&h->xh, np); ar.add(&h->yp, h->npart);
   ar.add(&h->quad_items, quad_items.size());
   ar.add(&h->quad_rows, h->n_quad_rows); ar.add(&h->quad_cols, quad_cols.size());
   ar.add(&h->kcol, kcol.size());  // V tiling at create
@@ -1546,7 +1447,6 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   if (h->nt) {
     auto round_up = [](int64_t n) { return std::max<int64_t>(256, (n + 255) / 256 * 256); };
     h->n_vtc = round_up(vtc); h->n_tkttc = round_up(tkttc);
-    h->n_tmttc = round_up(tmttc); h->n_xttc = round_up(xttc);
     if (h->tc_gen) {
       h->n_vtc = 0;  // V planes generated in the ladder
       ar.add(&h->vg_rows, vg_rows.size()); ar.add(&h->vg_cols, vg_cols.size());
@@ -1557,7 +1457,6 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
       ar.add(&h->v_tc, (size_t)h->nt * h->n_vtc);
     }
     ar.add(&h->tkt_tc, (size_t)h->nt * h->n_tkttc);
-    ar.add(&h->tmt_tc, (size_t)h->nt * h->n_tmttc); ar.add(&h->xt_tc, (size_t)h->nt * h->n_xttc);
   }
   if (h->have_3body) {
     ar.add(&h->v_h_hpp, h->n_h); ar.add(&h->v_phh_p, h->n_p);
@@ -1573,7 +1472,8 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   double *vraw = nullptr, *hhpp_raw = nullptr, *hpph_raw = nullptr;
   RawIndex *raw_idx = nullptr;
   int32_t *counts = nullptr;
-  int2 *d_vrows = nullptr, *d_mod_dims = nullptr;
+  int2 *d_mod_dims = nullptr;
+  int4 *d_vrows = nullptr;
   int4 *d_gv_items = nullptr, *d_gvt_items = nullptr;
   // Generated V_pppp: one item per operand-image chunk (channel, row tile, K chunk).
   // Counted per channel, then filled in parallel, each channel at its offset.
@@ -1587,7 +1487,7 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     for (int ai = 0; ai < h->n_act; ai++) {
       const ChanInfo &a = chans[ai];
       go[ai + 1] = go[ai] + (tc_images ? 0 : (int64_t)a.nmt * a.nkc);
-      gto[ai + 1] = gto[ai] + (tc_images ? (int64_t)ceil_div(a.pr, kTcBM) * a.nkct : 0);
+      gto[ai + 1] = gto[ai] + (tc_images ? (int64_t)a.nmt * a.nkct : 0);
     }
     gv_items.resize(go[h->n_act]);
     gvt_items.resize(gto[h->n_act]);
@@ -1600,7 +1500,7 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
           for (int kc = 0; kc < a.nkc; kc++) *g++ = make_int4(ai, mt, kc, 0);
       int4 *gt = gvt_items.data() + gto[ai];
       if (tc_images)
-        for (int mt = 0; mt < (int)ceil_div(a.pr, kTcBM); mt++)
+        for (int mt = 0; mt < a.nmt; mt++)
           for (int kc = 0; kc < a.nkct; kc++) *gt++ = make_int4(ai, mt, kc, 0);
     }
   }
@@ -1762,7 +1662,8 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     return CCDGPU_OK;
   };
   TRY(put(h->chans, chans)); TRY(put(h->mods, mods));
-  TRY(put(h->hh_tiles, hh_tiles)); TRY(put(h->hh_red, hh_red)); TRY(put(h->ranges, ranges)); TRY(put(h->quad_items, quad_items));
+  TRY(put(h->hh_tiles, hh_tiles)); TRY(put(h->hh_out, hh_out)); TRY(put(h->hh_part_off, hh_part_off));
+  TRY(put(h->ranges, ranges)); TRY(put(h->quad_items, quad_items));
   TRY(put(h->quad_cols, quad_cols));
 
   TRY(put(h->kcol, kcol));
@@ -1772,7 +1673,7 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   TRY(put(h->pp_pairs, pp_pairs)); TRY(put(h->hh_pairs, hh_pairs));
   TRY(put(h->pp_swap, pp_swap)); TRY(put(h->hh_swap, hh_swap));
   TRY(put(h->list_off, list_off)); TRY(put(h->list, list));
-  TRY(put(h->rowmap, rowmap)); TRY(put(h->mirror, mirror)); TRY(put(h->pk_idx, pk_idx));
+  TRY(put(h->prow, prow)); TRY(put(h->hcol, hcol));
   TRY(put(h->o_h, o_h)); TRY(put(h->o_p, o_p));
   TRY(put(d_vrows, vrows)); TRY(put(d_vraw_off, vraw_off));
   TRY(put(d_gv_items, gv_items)); TRY(put(d_gvt_items, gvt_items));
@@ -1791,9 +1692,9 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
       const ChanInfo &a = chans[ai];
       if ((!on_the_fly && !P->v_pppp[c]) || (!gen_v && (!P->v_hhpp[c] || !P->v_hhhh[c])))
         return CCDGPU_ERR_INVALID_ARGUMENT;
-      if (!on_the_fly)  // the rows a <= b of V_pppp, the only ones the ladder reads
-        for (int u = 0; u < a.pr; u++) {
-          sp.push_back(P->v_pppp[c] + (int64_t)rowmap[a.row_off + u] * a.pp);
+      if (!on_the_fly)  // the rows a <= b of V_pppp (the ladder reads those with a < b)
+        for (int u = 0; u < a_pr[ai]; u++) {
+          sp.push_back(P->v_pppp[c] + (int64_t)rowmap[a_row_off[ai] + u] * a.pp);
           np2.push_back(a.pp);
         }
       if (!gen_v) {
@@ -1844,9 +1745,8 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   // Device layout transforms.
   h->create_ms[1] = ms_since(t_build) - h->create_ms[0];
   if (h->n_quad_rows) {
-    quad_rows_kernel<<<(unsigned)h->n_act, 256, 0, h->s0>>>(h->chans, h->rowmap, h->mirror,
-                                                           h->pk_idx, h->pp_pairs, h->eps,
-                                                           (int)np, h->quad_rows);
+    quad_rows_kernel<<<(unsigned)h->n_act, 256, 0, h->s0>>>(
+        h->chans, h->kcol, h->pp_swap, h->pp_pairs, h->eps, (int)np, h->quad_rows);
     CK(cudaGetLastError());
   }
   if (gen_v && !mod_gen.empty()) {
@@ -1869,6 +1769,11 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
                                                             h->v_pphh);
     }
     CK(cudaGetLastError());
+    if (h->n_quad_items) {
+      pack_quads_kernel<<<h->n_quad_items, kAsmThreads, 0, h->s0>>>(
+          h->quad_items, h->chans, h->quad_rows, h->quad_cols, h->v_pphh, h->vq);
+      CK(cudaGetLastError());
+    }
     if (derive_tables || gen_v3) {
       pair_sizes_kernel<<<(unsigned)chans.size(), 256, 0, h->s0>>>(
           h->chans, h->pp_pairs, h->hh_pairs, (int)np, (int)h->npart, d_hblk, d_pblk);
@@ -1908,17 +1813,18 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     check_counts_kernel<<<std::max(nb, 1), 256, 0, h->s0>>>(counts, 5 * n_t, h->err);
     CK(cudaGetLastError());
     ring_maps_kernel<<<h->n_ranges, 256, 0, h->s0>>>(h->ranges, h->chans, h->pp_swap, h->hh_swap,
-                                                     h->flat, n_t, h->inv4, h->err);
+                                                     h->prow, h->hcol, h->flat, n_t, h->ring_dst,
+                                                     h->err);
     CK(cudaGetLastError());
   }
-  if (a_row_off[n_act] > 0) {
+  if (a_vrow_off[n_act] > 0) {
     if (on_the_fly) {
       // FP64 tiles, and the bf16 images unless the tensor-core ladder generates its own V: one
       // CTA per image chunk; with bf16 images, one CTA per tensor-core chunk writes both.
       if (!gv_items.empty()) {
         auto kern64 = md.ocode ? gen_v_chunks_kernel<true> : gen_v_chunks_kernel<false>;
         kern64<<<(unsigned)gv_items.size(), 256, 0, h->s0>>>(
-            h->chans, d_gv_items, h->rowmap, h->kcol, h->pp_pairs, md, h->v_t);
+            h->chans, d_gv_items, h->kcol, h->pp_pairs, md, h->v_t);
         CK(cudaGetLastError());
       }
       if (h->nt && !h->tc_gen && !gvt_items.empty()) {
@@ -1926,18 +1832,18 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
                                            : gen_v_both_chunks_kernel<2, true>)
                              : (h->nt == 3 ? gen_v_both_chunks_kernel<3, false>
                                            : gen_v_both_chunks_kernel<2, false>);
-        kern<<<(unsigned)gvt_items.size(), 256, 0, h->s0>>>(h->chans, d_gvt_items, h->rowmap,
-                                                           h->kcol, h->pp_pairs, md, h->v_t,
-                                                           h->v_tc, h->n_vtc);
+        kern<<<(unsigned)gvt_items.size(), 256, 0, h->s0>>>(h->chans, d_gvt_items, h->kcol,
+                                                           h->pp_pairs, md, h->v_t, h->v_tc,
+                                                           h->n_vtc);
       }
     } else {
-      tile_v_kernel<<<(unsigned)vrows.size(), 128, 0, h->s0>>>(h->chans, d_vrows, h->rowmap,
-                                                               h->kcol, d_vraw_off, vraw, h->v_t);
+      tile_v_kernel<<<(unsigned)vrows.size(), 128, 0, h->s0>>>(h->chans, d_vrows, h->kcol,
+                                                               d_vraw_off, vraw, h->v_t);
     }
     CK(cudaGetLastError());
     if (h->nt && !on_the_fly) {
       tile_v_tc_kernel<<<(unsigned)vrows.size(), 128, 0, h->s0>>>(
-          h->chans, d_vrows, h->rowmap, h->kcol, d_vraw_off, vraw, h->v_tc, h->n_vtc, h->nt);
+          h->chans, d_vrows, h->kcol, d_vraw_off, vraw, h->v_tc, h->n_vtc, h->nt);
       CK(cudaGetLastError());
     }
   }
@@ -1949,25 +1855,16 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   h->h_ctl = ctl_acquire();
   if (!h->h_ctl) return CCDGPU_ERR_OUT_OF_MEMORY;
 
-  h->ladder_smem = (size_t)kStages * (kMaxAS * kBK + kBK * kMaxBS) * 8 + 2 * kStages * 8;
-  h->ladder_smem_thin = (size_t)kStages * (kMaxAS * kBK + kBK * 8) * 8 + 2 * kStages * 8;
-  CK(cudaFuncSetAttribute(pp_ladder_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                          (int)h->ladder_smem_thin));
-  CK(cudaFuncSetAttribute(pp_ladder_kernel<0>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-  CK(cudaFuncSetAttribute(pp_ladder_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                          (int)h->ladder_smem));
-  CK(cudaFuncSetAttribute(pp_ladder_kernel<1>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-  CK(cudaFuncSetAttribute(pp_ladder_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                          (int)h->ladder_smem));
-  CK(cudaFuncSetAttribute(pp_ladder_kernel<2>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-  h->hh_smem = 0;  // static shared memory only
   // The attribute belongs to the kernel, not to this handle: set the device's opt-in maximum
   // (the same value for every handle), so that handles of different channel sizes coexist.
   int smem_optin = 0;
   CK(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->opt.device));
   if (ring16_smem(80) > (size_t)smem_optin) return CCDGPU_ERR_UNSUPPORTED;
-  CK(cudaFuncSetAttribute(hh_slice_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                          (int)hh_slice_smem(8 * kMaxCG)));
+  CK(cudaFuncSetAttribute(pp_ladder_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                          (int)kLadderSmem));
+  CK(cudaFuncSetAttribute(pp_ladder_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+  CK(cudaFuncSetAttribute(hh_ladder_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                          (int)kHHSmem));
   CK(cudaFuncSetAttribute(ring16_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                           (int)ring16_smem(32)));
   CK(cudaFuncSetAttribute(ring16_kernel<48>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2029,119 +1926,103 @@ cudaError_t launch_pdl(void (*kernel)(KArgs...), unsigned grid, unsigned block, 
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
-// gate: 0 = kernel of an FP64 iteration, 1 = of a mixed-precision iteration (which also writes
-// the bf16 operand images of the tensor-core ladder).
-// only: -1 everything, 0 units of hh <= 16, 1 the other units (2: neither); the reduction
-// runs when only < 0.
+// gate: 0 = kernel of an FP64 iteration, 1 = of a mixed-precision iteration.
+// only: -1 everything, 0 units of hk <= 8, 1 the other units, 2 the reduction.
 int launch_hh_ladder(ccdgpu_handle *h, cudaStream_t st, int gate, int only = -1) {
-  const int nt = gate ? h->nt : 0;
-  if (h->n_hh_small && only <= 0) {
+  const int n_cta = (only < 0 || only == 1) ? h->n_hh_cta : 0;
+  const int n_warp = only <= 0 ? h->n_hh_warp : 0;
+  if (n_cta + n_warp) {
     h->launches++;
-    CK(launch_pdl(hh_mma_kernel<2>, (int)ceil_div(h->n_hh_small, kHHWarps), kHHWarps * 32, 0, st,
-                  (const HHTile *)h->hh_tiles, h->n_hh_small, (const ChanInfo *)h->chans,
-                  (const double *)h->v_pphh, (const double *)h->t[0], (const double *)h->t[1],
-                  h->part, h->r, (const Control *)h->ctl, gate));
+    CK(launch_pdl(hh_ladder_kernel, n_cta + (int)ceil_div(n_warp, kHHThreads / 32), kHHThreads,
+                  n_cta ? kHHSmem : 0, st,
+                  (const HHTile *)(h->hh_tiles + (n_cta ? 0 : h->n_hh_cta)), n_cta, n_warp,
+                  (const ChanInfo *)h->chans, (const double *)h->vq, (const double *)h->tq[0],
+                  (const double *)h->tq[1], h->part, (const int64_t *)h->hh_part_off, h->r,
+                  (const Control *)h->ctl, gate));
   }
-  const int nbig = h->n_hh_tiles - h->n_hh_small;
-  if (nbig && (only < 0 || only == 1)) {
+  if (h->n_hh_out && (only < 0 || only == 2)) {
     h->launches++;
-    CK(launch_pdl(hh_slice_kernel, nbig, kHHSliceThreads, h->hh_slice_smem, st,
-                  (const HHTile *)(h->hh_tiles + h->n_hh_small), (const ChanInfo *)h->chans,
-                  (const double *)h->v_pphh, (const double *)h->t[0], (const double *)h->t[1],
-                  h->part, h->r, (const Control *)h->ctl, gate));
-  }
-  if (h->n_hh_red && (only < 0 || only == 2)) {
-    h->launches++;
-    CK(launch_pdl(hh_reduce_kernel, h->n_hh_red, 256, 0, st, (const HHRed *)h->hh_red,
-                  (const ChanInfo *)h->chans, (const double *)h->v_hhhh, (const double *)h->part,
-                  h->x, h->x_t, h->s, h->xt_tc, h->n_xttc, nt, (const Control *)h->ctl, gate));
+    CK(launch_pdl(hh_reduce_kernel, (int)ceil_div(h->n_hh_out, 128), 128, 0, st,
+                  (const HHOut *)h->hh_out, h->n_hh_out, (const double *)h->v_hhhh,
+                  (const double *)h->part, h->x, h->s, (const Control *)h->ctl, gate));
   }
   return CCDGPU_OK;
 }
 int launch_pp_ladder_tc(ccdgpu_handle *h, cudaStream_t st) {
   if (!h->n_tc_tiles) return CCDGPU_OK;
   h->launches++;
-  // Persistent: two CTAs per SM (shared memory and 2 x 128 tensor-memory columns each).
-  CK(launch_pdl(tc_kernel_of(h->nt, h->tc_gen), h->tc_grid, tc_threads(h->tc_gen), h->tc_smem,
-                st, (const LadderTile *)h->tc_tiles, h->n_tc_tiles, h->tc_sched,
-                (const __nv_bfloat16 *)h->v_tc, h->n_vtc, (const __nv_bfloat16 *)h->tkt_tc,
-                h->n_tkttc, (const __nv_bfloat16 *)h->tmt_tc, h->n_tmttc,
-                (const __nv_bfloat16 *)h->xt_tc, h->n_xttc, (const int32_t *)h->rowmap,
-                (const int32_t *)h->mirror, h->dmat, h->tc_part, (const Control *)h->ctl, h->err,
-                (const ChanInfo *)h->chans, (const VGenRow *)h->vg_rows,
-                (const uint32_t *)h->vg_cols, (const double *)h->vg_tab));
-  if (h->n_red_tc) {
-    CK(launch_pdl(ladder_reduce_kernel, h->n_red_tc, 256, 0, st, (const RedItem *)h->red_tc,
-                  (const LadderTile *)h->tc_tiles, (const int32_t *)h->rowmap,
-                  (const int32_t *)h->mirror, h->dmat, (const double *)h->tc_part,
-                  (const Control *)h->ctl, 1));
-    h->launches++;
-  }
-  return CCDGPU_OK;
+  return cuda_status(launch_pdl(
+      tc_kernel_of(h->nt, h->tc_gen), std::min(h->n_tc_tiles, kTcGrid), tc_threads(h->tc_gen),
+      h->tc_smem, st, (const LadderTile *)h->tc_tiles, h->n_tc_tiles, h->sched + 2,
+      (const __nv_bfloat16 *)h->v_tc, h->n_vtc, (const __nv_bfloat16 *)h->tkt_tc, h->n_tkttc,
+      h->tc_planes, (const Control *)h->ctl, h->err, (const ChanInfo *)h->chans,
+      (const VGenRow *)h->vg_rows, (const uint32_t *)h->vg_cols, (const double *)h->vg_tab));
 }
-// The three column classes run concurrently: mid and wide go to stream s2 (wide first, they
-// are the longest tiles), thin to `st`; s2 is joined back into `st` before returning.
-int launch_pp_ladder(ccdgpu_handle *h, cudaStream_t st) {
-  if (h->nt && h->n_ranges) {
-    // A mixed handle's FP64 ladder first refreshes its operand tiles if mixed iterations ran.
-    CK(launch_pdl(retile_kernel, h->n_ranges, 256, 0, st, (const ElemRange *)h->ranges,
-                  (const ChanInfo *)h->chans, (const int2 *)h->pk_idx, (const double *)h->t[0],
-                  (const double *)h->t[1], h->t_kt, h->t_mt, h->ctl, 0));
-    CK(launch_pdl(retile_done_kernel, 1, 32, 0, st, h->ctl));
-    h->launches += 2;
-  }
-  // The classes run one after another on `st`: each is persistent over every SM (its tiles
-  // balanced for CTAs that all start together), so concurrent classes only delay each other's
-  // CTAs.
-  cudaStream_t s2 = st;
-  if (h->n_cls[1] || h->n_cls[2]) {
-    if (h->n_cls[2]) {
-      pp_ladder_kernel<2><<<h->fp_grid[2], ladder_threads(2), h->ladder_smem, s2>>>(
-          h->tiles, h->fp_cta_off + h->fp_off_base[2], h->v_t, h->t_kt, h->t_mt, h->x_t,
-          h->rowmap, h->mirror, h->dmat, h->lpart, h->ctl, h->err, 0);
-      h->launches++;
-      CK(cudaGetLastError());
-    }
-    if (h->n_cls[1]) {
-      pp_ladder_kernel<1><<<h->fp_grid[1], ladder_threads(1), h->ladder_smem, s2>>>(
-          h->tiles, h->fp_cta_off + h->fp_off_base[1], h->v_t, h->t_kt, h->t_mt, h->x_t,
-          h->rowmap, h->mirror, h->dmat, h->lpart, h->ctl, h->err, 0);
-      h->launches++;
-      CK(cudaGetLastError());
-    }
-  }
-  if (h->n_cls[0]) {
-    CK(launch_pdl(pp_ladder_kernel<0>, h->fp_grid[0], kLadderThreads, h->ladder_smem_thin, st,
-                  (const LadderTile *)h->tiles, (const int32_t *)(h->fp_cta_off + h->fp_off_base[0]),
-                  (const double *)h->v_t, (const double *)h->t_kt, (const double *)h->t_mt,
-                  (const double *)h->x_t, (const int32_t *)h->rowmap, (const int32_t *)h->mirror,
-                  h->dmat, h->lpart, (const Control *)h->ctl, h->err, 0));
-    h->launches++;
-  }
-  if (h->n_red_fp) {
-    CK(launch_pdl(ladder_reduce_kernel, h->n_red_fp, 256, 0, st, (const RedItem *)h->red_fp,
-                  (const LadderTile *)h->tiles, (const int32_t *)h->rowmap,
-                  (const int32_t *)h->mirror, h->dmat, (const double *)h->lpart,
-                  (const Control *)h->ctl, 0));
-    h->launches++;
-  }
-  return CCDGPU_OK;
+// FP64 ladder; cls >= 0: the tiles of one column class alone (wide, mid, thin in list order).
+int launch_pp_ladder(ccdgpu_handle *h, cudaStream_t st, int cls = -1) {
+  const int first = cls < 0 || cls == 2 ? 0 : h->n_cls[2] + (cls == 0 ? h->n_cls[1] : 0);
+  const int n = cls < 0 ? h->n_tiles : h->n_cls[cls];
+  if (!n) return CCDGPU_OK;
+  h->launches++;
+  return cuda_status(launch_pdl(
+      pp_ladder_kernel, std::min(n, 148), kLadderThreads, kLadderSmem, st,
+      (const LadderTile *)(h->tiles + first), n, h->sched, (const double *)h->v_t,
+      (const double *)h->tq[0], (const double *)h->tq[1], h->d_planes, (const Control *)h->ctl,
+      h->err, 0));
+}
+// t2Diff_pphh from the ladder's planes (tc: the tensor-core ladder's) and the amplitudes of
+// buffer parity ^ flip.
+int launch_expand_d(ccdgpu_handle *h, bool tc, int flip) {
+  if (!h->n_quad_items) return CCDGPU_OK;
+  expand_d_kernel<<<h->n_quad_items, kAsmThreads, 0, h->s0>>>(
+      h->quad_items, h->chans, tc ? h->tc_lchans : h->lchans, h->quad_rows, h->quad_cols,
+      tc ? h->tc_planes : h->d_planes, h->x, h->tq[0], h->tq[1], flip, h->ctl, h->dmat);
+  h->launches++;
+  return cuda_status(cudaGetLastError());
+}
+// t2Diff_pphh of the last fused iteration into dmat, if that has not been done.
+int materialize_d(ccdgpu_handle *h) {
+  if (!h->d_from) return CCDGPU_OK;
+  const bool tc = h->d_from == 2;
+  h->d_from = 0;
+  return launch_expand_d(h, tc, 1);
+}
+// t[0] of the fused path: the current amplitudes in the reference order.
+int materialize_t(ccdgpu_handle *h) {
+  if (h->slab_current || h->opt.path != CCDGPU_PATH_FUSED) return CCDGPU_OK;
+  h->slab_current = true;
+  if (!h->n_ranges) return CCDGPU_OK;
+  expand_t_kernel<<<h->n_ranges, 256, 0, h->s0>>>(h->ranges, h->chans, h->prow, h->hcol, h->tq[0],
+                                                  h->tq[1], h->ctl, h->t[0]);
+  h->launches++;
+  return cuda_status(cudaGetLastError());
+}
+// The bf16 image of the current amplitudes, before a mixed iteration that does not follow a
+// mixed iteration.
+int refresh_tc_image(ccdgpu_handle *h) {
+  if (!h->nt || !h->tc_stale) return CCDGPU_OK;
+  h->tc_stale = false;
+  if (!h->n_quad_items) return CCDGPU_OK;
+  t_image_kernel<<<h->n_quad_items, kAsmThreads, 0, h->s0>>>(
+      h->quad_items, h->chans, h->tq[0], h->tq[1], h->ctl, h->tkt_tc, h->n_tkttc, h->nt);
+  h->launches++;
+  return cuda_status(cudaGetLastError());
 }
 
-// T' from the phhp slab in both paths.  fused: R scattered into pphh order for the fused
-// assembly; else the table path's t2Diff_phhp slab.
+// T' from the phhp slab in both paths.  fused: R into the quads' ring terms; else the table
+// path's t2Diff_phhp slab.
 // only: -1 every class, else 0 small, 1 mid, 2 large.
 int launch_phhp_gather(ccdgpu_handle *h, cudaStream_t st, int gate) {
   if (!h->n_m) return CCDGPU_OK;
   h->launches++;
   const unsigned blocks = (unsigned)ceil_div(h->n_m, (int64_t)256 * kGatherPer);
-  return cuda_status(launch_pdl(phhp_gather_kernel, blocks, 256, 0, st, (const int32_t *)h->inv4,
-                                h->n_m, (const double *)h->t[0], (const double *)h->t[1],
+  return cuda_status(launch_pdl(phhp_gather_kernel, blocks, 256, 0, st, (const int32_t *)h->ring_dst,
+                                h->n_m, (const double *)h->tq[0], (const double *)h->tq[1],
                                 h->old_phhp, (const Control *)h->ctl, gate));
 }
 int launch_ring(ccdgpu_handle *h, cudaStream_t st, int gate, bool fused, int only = -1) {
-  const int32_t *inv = fused ? h->inv4 : nullptr;
-  double *out = fused ? h->d_ring : h->r_phhp;
+  const int32_t *dst = fused ? h->ring_dst : nullptr;
+  double *out = fused ? h->r_quad : h->r_phhp;
   // Fused path: T' (the phhp slab) gathered from the current amplitudes first; the profile's
   // small class includes it.
   if (fused && (only < 0 || only == 0))
@@ -2150,7 +2031,7 @@ int launch_ring(ccdgpu_handle *h, cudaStream_t st, int gate, bool fused, int onl
     CK(launch_pdl(ring_small_kernel, (int)ceil_div(h->n_mod_small, kRingSmallWarps),
                   kRingSmallWarps * 32, 0, st, (const ModInfo *)h->mods, h->n_mod_small,
                   (const double *)h->v_hpph, (const double *)h->v_hphp,
-                  (const double *)h->old_phhp, inv, out, (const Control *)h->ctl, gate));
+                  (const double *)h->old_phhp, dst, out, (const Control *)h->ctl, gate));
     h->launches++;
   }
   // Groups by padded size; only = 1 launches the 32 group, only = 2 the wider ones.
@@ -2161,7 +2042,7 @@ int launch_ring(ccdgpu_handle *h, cudaStream_t st, int gate, bool fused, int onl
       auto go = [&](auto kern, int pad) {
         return launch_pdl(kern, n, 32 * ring16_warps(pad), ring16_smem(pad), st, mp,
                           (const double *)h->v_hpph, (const double *)h->v_hphp,
-                          (const double *)h->old_phhp, inv, out, (const Control *)h->ctl, gate);
+                          (const double *)h->old_phhp, dst, out, (const Control *)h->ctl, gate);
       };
       switch (k) {
         case 0: CK(go(ring16_kernel<32>, 32)); break;
@@ -2189,10 +2070,11 @@ int launch_assemble_fused(ccdgpu_handle *h, cudaStream_t st, int gate) {
   return cuda_status(launch_pdl(
       h->loop_capture ? assemble_fused_kernel<true> : assemble_fused_kernel<false>,
       h->n_asm_blocks, kAsmThreads, 0, st, (const QuadItem *)h->quad_items, h->n_quad_items,
-      (const ChanInfo *)h->chans, (const QuadRow *)h->quad_rows,
-      (const QuadCol *)h->quad_cols, (const double *)h->v_pphh, (const double *)h->dmat,
-      (const double *)h->d_ring, (const double *)h->xh, (const double *)h->yp, h->t[0], h->t[1], h->t_kt, h->t_mt, h->epart,
-      h->ticket, h->ctl, h->tkt_tc, h->n_tkttc, h->tmt_tc, h->n_tmttc, gate ? h->nt : 0,
+      (const ChanInfo *)h->chans, (const LadderChan *)(gate ? h->tc_lchans : h->lchans),
+      (const QuadRow *)h->quad_rows, (const QuadCol *)h->quad_cols, (const double *)h->vq,
+      (const double *)(gate ? h->tc_planes : h->d_planes), (const double *)h->x,
+      (const double *)h->r_quad, (const double *)h->xh, (const double *)h->yp, h->tq[0], h->tq[1],
+      h->epart, h->ticket, h->ctl, h->tkt_tc, h->n_tkttc, gate ? h->nt : 0,
       (cudaGraphConditionalHandle)(h->loop_capture ? h->loop_cond : 0), h->loop_capture, gate));
 }
 int launch_energy(ccdgpu_handle *h, cudaStream_t st, int flags) {
@@ -2200,19 +2082,22 @@ int launch_energy(ccdgpu_handle *h, cudaStream_t st, int flags) {
   h->launches++;
   return cuda_status(cudaGetLastError());
 }
-int launch_map_to(ccdgpu_handle *h, cudaStream_t st, const double *src, double *dst) {
+// mark: the pass over non-finite elements (map_to_kernel) instead of the scatters.
+int launch_map_to(ccdgpu_handle *h, cudaStream_t st, const double *src, double *dst,
+                  int mark = 0) {
   if (!h->n_ranges) return CCDGPU_OK;
-  map_to_kernel<<<h->n_ranges, 256, 0, st>>>(h->ranges, h->chans, h->pk_idx, h->flat, h->n_t, src, dst,
-                                               h->old_h2pp_h1, h->old_h1pp_h2, h->old_p1_p2hh,
-                                               h->old_p2_p1hh, h->old_phhp, h->t_kt, h->t_mt,
-                                               h->have_3body ? 1 : 0, h->tkt_tc, h->n_tkttc,
-                                               h->tmt_tc, h->n_tmttc, h->nt);
+  map_to_kernel<<<h->n_ranges, 256, 0, st>>>(h->ranges, h->chans, h->prow, h->hcol, h->flat,
+                                             h->n_t, src, dst, h->old_h2pp_h1, h->old_h1pp_h2,
+                                             h->old_p1_p2hh, h->old_p2_p1hh, h->old_phhp,
+                                             h->tq[0], h->tq[1], h->have_3body ? 1 : 0, h->ctl,
+                                             mark);
   h->launches++;
   return cuda_status(cudaGetLastError());
 }
 
-// One fused iteration: ring on s1 beside hh ladder, one-body sums and pp ladder on s0, then the
-// assembly.
+// One fused iteration: the pp ladder on s0, the ring on s1 and the hh ladder with the one-body
+// sums on s2 side by side (each needs only the amplitudes), then the assembly on s0.  The
+// ladder, bound by HBM on one CTA per SM, goes first; the others, bound by latency, run beside it.
 // mixed: the pp ladder runs on the tensor cores (split bf16) instead of the FP64 pipe.
 int enqueue_fused_iteration(ccdgpu_handle *h, bool mixed) {
   int rc;
@@ -2221,49 +2106,35 @@ int enqueue_fused_iteration(ccdgpu_handle *h, bool mixed) {
     return mixed ? launch_pp_ladder_tc(h, st) : launch_pp_ladder(h, st);
   };
   if (h->profiling) {
-    // ev: 0 start, 1 after hh ladder, 2 after one-body, 3 after pp ladder, 4/5 ring on s1,
-    // 6 after assembly, 7 after the energy reduction.
+    // One family after another: ev 0 start, 1 after hh ladder, 2 after one-body, 3 after pp
+    // ladder, 4/5 ring, 8 before and 6, 7 after the assembly.
     CK(cudaEventRecord(h->ev[0], h->s0));
-    CK(cudaStreamWaitEvent(h->s1, h->ev[0], 0));
-    CK(cudaEventRecord(h->ev[4], h->s1));
-    if ((rc = launch_ring(h, h->s1, gate, true))) return rc;
-    CK(cudaEventRecord(h->ev[5], h->s1));
     if ((rc = launch_hh_ladder(h, h->s0, gate))) return rc;
     CK(cudaEventRecord(h->ev[1], h->s0));
     if ((rc = launch_onebody_fused(h, h->s0, gate))) return rc;
     CK(cudaEventRecord(h->ev[2], h->s0));
     if ((rc = ladder(h->s0))) return rc;
     CK(cudaEventRecord(h->ev[3], h->s0));
-    CK(cudaStreamWaitEvent(h->s0, h->ev[5], 0));
+    CK(cudaEventRecord(h->ev[4], h->s0));
+    if ((rc = launch_ring(h, h->s0, gate, true))) return rc;
+    CK(cudaEventRecord(h->ev[5], h->s0));
     CK(cudaEventRecord(h->ev[8], h->s0));
     if ((rc = launch_assemble_fused(h, h->s0, gate))) return rc;
     CK(cudaEventRecord(h->ev[6], h->s0));
     CK(cudaEventRecord(h->ev[7], h->s0));
     return CCDGPU_OK;
   }
-  // The ring (s1) runs beside the hh ladder, the one-body sums and the pp ladder (s0); the
-  // latency-bound small ring channels fill SMs the hh ladder leaves idle.  The one-body sums
-  // stay on s0 ahead of the pp ladder: on a third stream their CTAs delayed the start of the
-  // persistent ladder's CTAs (device trace).
   CK(cudaEventRecord(h->ev_fork, h->s0));
   CK(cudaStreamWaitEvent(h->s1, h->ev_fork, 0));
+  CK(cudaStreamWaitEvent(h->s2, h->ev_fork, 0));
+  if ((rc = ladder(h->s0))) return rc;
   if ((rc = launch_ring(h, h->s1, gate, true))) return rc;
   CK(cudaEventRecord(h->ev_join, h->s1));
-  if ((rc = launch_hh_ladder(h, h->s0, gate))) return rc;
-  // FP64 iterations: the one-body sums (read only by the assembly) run on s3 beside the FP64
-  // ladder classes (FP64 iteration 2,836 -> 2,952 iter/s at EG N=54 |n|^2<=36).  Mixed
-  // iterations keep them on s0 ahead of the tensor-core ladder (3,925 against 3,900 iter/s
-  // beside it).
-  cudaStream_t ob = mixed ? h->s0 : h->s3;
-  if (!mixed) {
-    CK(cudaEventRecord(h->ev_fork3, h->s0));
-    CK(cudaStreamWaitEvent(h->s3, h->ev_fork3, 0));
-  }
-  if ((rc = launch_onebody_fused(h, ob, gate))) return rc;
-  if (!mixed) CK(cudaEventRecord(h->ev_join3, h->s3));
-  if ((rc = ladder(h->s0))) return rc;
-  if (!mixed) CK(cudaStreamWaitEvent(h->s0, h->ev_join3, 0));
+  if ((rc = launch_hh_ladder(h, h->s2, gate))) return rc;
+  if ((rc = launch_onebody_fused(h, h->s2, gate))) return rc;
+  CK(cudaEventRecord(h->ev_join2, h->s2));
   CK(cudaStreamWaitEvent(h->s0, h->ev_join, 0));
+  CK(cudaStreamWaitEvent(h->s0, h->ev_join2, 0));
   if ((rc = launch_assemble_fused(h, h->s0, gate))) return rc;  // + energy and stop rule
   if (h->loop_capture && !h->n_asm_blocks) {  // else the assembly set the loop condition
     h->launches++;
@@ -2314,11 +2185,10 @@ int check_errors(ccdgpu_handle *h) {
   CK(cudaMemcpy(&e, h->err, sizeof(int32_t), cudaMemcpyDeviceToHost));
   if (e & kErrTimeout) {
     // Reported once: the handle stays usable (the timed-out iteration's amplitudes are
-    // incomplete; ccdgpu_reset or ccdgpu_set_t2 starts over).  A tensor-core ladder CTA that
-    // gave up may have left the tile counter and exit ticket behind: zero them for the next
-    // launch.
+    // incomplete; ccdgpu_reset or ccdgpu_set_t2 starts over).  A ladder CTA that gave up may
+    // have left its tile counter and exit ticket behind: zero them for the next launch.
     CK(cudaMemset(h->err, 0, sizeof(int32_t)));
-    if (h->tc_sched) CK(cudaMemset(h->tc_sched, 0, 2 * sizeof(int32_t)));
+    if (h->sched) CK(cudaMemset(h->sched, 0, 4 * sizeof(int32_t)));
     return CCDGPU_ERR_TIMEOUT;
   }
   if (h->h_ctl->error & kErrNonFinite) return CCDGPU_ERR_NONFINITE;
@@ -2473,6 +2343,7 @@ int tables_iteration(ccdgpu_handle *h, double mixing, double *corr) {
   if ((rc = launch_ring(h, h->s0, 0, false))) return rc;   // calcT2Diff_phhp
   if ((rc = launch_hh_ladder(h, h->s0, 0))) return rc;     // calcT2Diff_pphh
   if ((rc = launch_pp_ladder(h, h->s0))) return rc;
+  if ((rc = launch_expand_d(h, false, 0))) return rc;
   if ((rc = stage_gather(h))) return rc;                   // 8 x mapFromDistributed
   if ((rc = stage_assemble_tables(h, mixing))) return rc;  // calcT2_pphh
   if ((rc = launch_energy(h, h->s0, 2))) return rc;
@@ -2571,28 +2442,31 @@ uint64_t ccdgpu_t2_size(const ccdgpu_handle *h) { return h ? (uint64_t)h->n_t : 
 int ccdgpu_reset(ccdgpu_handle *h) {
   if (!h) return CCDGPU_ERR_INVALID_ARGUMENT;
   CK(cudaSetDevice(h->opt.device));
+  // The fused path iterates on the packed amplitudes alone; the other buffer of the pair stays,
+  // since t2Diff_pphh of the last iteration may still be read from it.
+  const bool fused = h->opt.path == CCDGPU_PATH_FUSED;
   const std::pair<double *, int64_t> z[] = {
-      {h->t[0], h->n_t}, {h->t[1], h->n_t}, {h->old_phhp, h->n_m}, {h->t_kt, h->n_tkt},
-      {h->t_mt, h->n_tmt}, {h->old_h1pp_h2, h->n_h}, {h->old_h2pp_h1, h->n_h},
+      {h->tq[h->h_ctl->parity], h->n_q}, {h->old_phhp, h->n_m},
+      {fused ? nullptr : h->t[0], h->n_t}, {fused ? nullptr : h->t[1], h->n_t},
+      {h->old_h1pp_h2, h->n_h}, {h->old_h2pp_h1, h->n_h},
       {h->old_p1_p2hh, h->n_p}, {h->old_p2_p1hh, h->n_p}};
   for (const auto &b : z)
     if (b.first && b.second) CK(cudaMemsetAsync(b.first, 0, b.second * 8, h->s0));
-  if (h->nt) {
-    CK(cudaMemsetAsync(h->tkt_tc, 0, (size_t)h->nt * h->n_tkttc * 2, h->s0));
-    CK(cudaMemsetAsync(h->tmt_tc, 0, (size_t)h->nt * h->n_tmttc * 2, h->s0));
-  }
-  return set_ctl(h, 0, h->h_ctl->tol, h->h_ctl->max_iters, h->h_ctl->mixing, true, 0);
+  if (h->nt) CK(cudaMemsetAsync(h->tkt_tc, 0, (size_t)h->nt * h->n_tkttc * 2, h->s0));
+  h->slab_current = false;
+  h->tc_stale = false;
+  return set_ctl(h, 0, h->h_ctl->tol, h->h_ctl->max_iters, h->h_ctl->mixing, true);
 }
 
 int ccdgpu_set_t2(ccdgpu_handle *h, const double *t2, uint64_t n) {
   if (!h || !t2 || n != (uint64_t)h->n_t) return CCDGPU_ERR_INVALID_ARGUMENT;
   CK(cudaSetDevice(h->opt.device));
-  int rc = sync_ctl(h);
-  if (rc) return rc;
-  h->h_ctl->parity = 0;
-  CK(cudaMemcpyAsync(h->ctl, h->h_ctl, sizeof(Control), cudaMemcpyHostToDevice, h->s0));
+  int rc;
   CK(cudaMemcpyAsync(h->t[1], t2, n * 8, cudaMemcpyHostToDevice, h->s0));
   if ((rc = launch_map_to(h, h->s0, h->t[1], h->t[0]))) return rc;
+  if ((rc = launch_map_to(h, h->s0, h->t[1], h->t[0], 1))) return rc;
+  h->slab_current = true;
+  h->tc_stale = true;
   CK(cudaStreamSynchronize(h->s0));
   return CCDGPU_OK;
 }
@@ -2602,11 +2476,6 @@ int ccdgpu_mbpt2(ccdgpu_handle *h, int32_t init_t2, double *e_mbpt2) {
   CK(cudaSetDevice(h->opt.device));
   int rc = set_ctl(h, 0, h->h_ctl->tol, h->h_ctl->max_iters, h->h_ctl->mixing, false);
   if (rc) return rc;
-  if (init_t2) {
-    // The amplitudes become the current ones (parity 0, as after ccdgpu_set_t2).
-    h->h_ctl->parity = 0;
-    CK(cudaMemcpyAsync(h->ctl, h->h_ctl, sizeof(Control), cudaMemcpyHostToDevice, h->s0));
-  }
   if (h->n_ranges) {
     mbpt2_kernel<<<h->n_ranges, 256, 0, h->s0>>>(h->ranges, h->chans, h->pp_pairs, h->hh_pairs,
                                                   h->v_pphh, h->eps, init_t2 ? h->t[1] : nullptr,
@@ -2614,7 +2483,11 @@ int ccdgpu_mbpt2(ccdgpu_handle *h, int32_t init_t2, double *e_mbpt2) {
     CK(cudaGetLastError());
   }
   if ((rc = launch_energy(h, h->s0, 0))) return rc;
-  if (init_t2 && (rc = launch_map_to(h, h->s0, h->t[1], h->t[0]))) return rc;
+  if (init_t2) {  // the amplitudes become the current ones, as after ccdgpu_set_t2
+    if ((rc = launch_map_to(h, h->s0, h->t[1], h->t[0]))) return rc;
+    h->slab_current = true;
+    h->tc_stale = true;
+  }
   double e = 0.0;
   CK(cudaMemcpyAsync(&e, h->e_out, 8, cudaMemcpyDeviceToHost, h->s0));
   CK(cudaStreamSynchronize(h->s0));
@@ -2778,8 +2651,8 @@ int ccdgpu_get_t2(ccdgpu_handle *h, double *t2, uint64_t n) {
   CK(cudaSetDevice(h->opt.device));
   int rc = sync_ctl(h);
   if (rc) return rc;
-  const double *src = h->t[h->h_ctl->parity];
-  if (h->opt.path == CCDGPU_PATH_TABLES) src = h->t[1];
+  if ((rc = materialize_t(h))) return rc;
+  const double *src = h->opt.path == CCDGPU_PATH_TABLES ? h->t[1] : h->t[0];
   return copy_from_device(h, reinterpret_cast<char *>(t2), reinterpret_cast<const char *>(src),
                           n * 8);
 }
@@ -2795,8 +2668,13 @@ int ccdgpu_step(ccdgpu_handle *h, double mixing, double *e_corr) {
     const int32_t one = 1;
     CK(cudaMemcpyAsync(&h->ctl->inject, &one, sizeof(one), cudaMemcpyHostToDevice, h->s0));
   }
-  if (h->opt.path == CCDGPU_PATH_TABLES) rc = tables_iteration(h, mixing, nullptr);
-  else rc = enqueue_fused_iteration(h, h->nt > 0);
+  if (h->opt.path == CCDGPU_PATH_TABLES) {
+    rc = tables_iteration(h, mixing, nullptr);
+  } else if (!(rc = refresh_tc_image(h))) {
+    rc = enqueue_fused_iteration(h, h->nt > 0);
+    h->slab_current = false;
+    h->d_from = h->nt ? 2 : 1;
+  }
   if (inject) {  // the fault applies to this iteration only
     const int32_t zero = 0;
     CK(cudaMemcpyAsync(&h->ctl->inject, &zero, sizeof(zero), cudaMemcpyHostToDevice, h->s0));
@@ -2856,6 +2734,11 @@ int solve_begin(ccdgpu_handle *h, double tol, int64_t max_iters, double mixing, 
   st.device_loop = st.graph && h->opt.device_loop && h->loop_state == 1;
   if (st.graph && !st.device_loop && (rc = fused_ready_graph(h, false))) return rc;
   if (st.graph && !st.device_loop && st.mixed && (rc = fused_ready_graph(h, true))) return rc;
+  if (st.fused) {
+    if ((rc = refresh_tc_image(h))) return rc;
+    h->slab_current = false;
+    h->d_from = 0;  // until solve_finish
+  }
   st.t0 = std::chrono::steady_clock::now();
   if (st.device_loop) return loop_launch(h, st);
   return CCDGPU_OK;
@@ -2912,6 +2795,12 @@ int solve_finish(ccdgpu_handle *h, SolveState &st, double mixing, ccdgpu_result 
     if (h->h_ctl->done || launched >= st.cap) break;
   }
   auto t1 = std::chrono::steady_clock::now();
+  if (st.fused) {
+    // The last iteration was an FP64 one unless a mixed solve never left its mixed phase.
+    const bool last64 = !st.mixed || h->h_ctl->polish_iters > 0;
+    h->d_from = last64 ? 1 : 2;
+    if (st.mixed && last64) h->tc_stale = true;
+  }
   // The result reflects the control block also when the solve failed (for example non-finite
   // amplitudes of a diverging iteration); the status says so.
   const Control &c = *h->h_ctl;
@@ -2995,7 +2884,10 @@ int ccdgpu_calc_t2diff_phhp(ccdgpu_handle *h) {
 int ccdgpu_calc_t2diff_pphh(ccdgpu_handle *h) {
   if (!h) return CCDGPU_ERR_INVALID_ARGUMENT;
   int rc = set_ctl(h, 0, h->h_ctl->tol, h->h_ctl->max_iters, h->h_ctl->mixing, false);
-  if (rc || (rc = launch_hh_ladder(h, h->s0, 0)) || (rc = launch_pp_ladder(h, h->s0))) return rc;
+  if (rc || (rc = launch_hh_ladder(h, h->s0, 0)) || (rc = launch_pp_ladder(h, h->s0)) ||
+      (rc = launch_expand_d(h, false, 0)))
+    return rc;
+  h->d_from = 0;
   CK(cudaStreamSynchronize(h->s0));
   return check_errors(h);
 }
@@ -3031,10 +2923,10 @@ int ccdgpu_read_chain(ccdgpu_handle *h, int32_t chain, double *out, uint64_t n, 
   if (rc) return rc;
   const double *src = nullptr;
   uint64_t len = 0;
-  const int par = h->h_ctl->parity;
+  const bool tables = h->opt.path == CCDGPU_PATH_TABLES;
   switch (chain) {
-    case CCDGPU_CHAIN_T2: src = (h->opt.path == CCDGPU_PATH_TABLES) ? h->t[1] : h->t[par]; len = h->n_t; break;
-    case CCDGPU_CHAIN_T2_OLD: src = (h->opt.path == CCDGPU_PATH_TABLES) ? h->t[0] : h->t[par]; len = h->n_t; break;
+    case CCDGPU_CHAIN_T2: src = h->t[tables ? 1 : 0]; len = h->n_t; break;
+    case CCDGPU_CHAIN_T2_OLD: src = h->t[0]; len = h->n_t; break;
     case CCDGPU_CHAIN_DIFF_PPHH: src = h->dmat; len = h->n_t; break;
     case CCDGPU_CHAIN_DIFF_PHHP: src = h->r_phhp; len = h->n_m; break;
     case CCDGPU_CHAIN_OLD_PHHP: src = h->old_phhp; len = h->n_m; break;
@@ -3057,6 +2949,10 @@ int ccdgpu_read_chain(ccdgpu_handle *h, int32_t chain, double *out, uint64_t n, 
     if ((rc = launch_phhp_gather(h, h->s0, -1))) return rc;
     CK(cudaStreamSynchronize(h->s0));
   }
+  if (chain == CCDGPU_CHAIN_DIFF_PPHH && (rc = materialize_d(h))) return rc;
+  if ((chain == CCDGPU_CHAIN_T2 || chain == CCDGPU_CHAIN_T2_OLD) && (rc = materialize_t(h)))
+    return rc;
+  CK(cudaStreamSynchronize(h->s0));
   CK(cudaMemcpy(out, src, len * 8, cudaMemcpyDeviceToHost));
   return CCDGPU_OK;
 }
@@ -3092,9 +2988,10 @@ int ccdgpu_kernel_profile(ccdgpu_handle *h, int32_t reps, double *ms, double *fl
   CK(cudaSetDevice(h->opt.device));
   int rc = set_ctl(h, 0, h->h_ctl->tol, h->h_ctl->max_iters, h->h_ctl->mixing, false);
   if (rc) return rc;
+  if ((rc = materialize_d(h))) return rc;  // the kernels overwrite what it is expanded from
   for (int k = 0; k < 7; k++) ms[k] = flops[k] = bytes[k] = 0;
-  // Ring: Y = V_hphp + 0.5 V_hpph T' and R = T' Y; reads T', V_hpph, V_hphp and the inverse
-  // ai_jb table, writes R.
+  // Ring: Y = V_hphp + 0.5 V_hpph T' and R = T' Y; reads T', V_hpph, V_hphp and where R goes,
+  // writes R.
   for (const ModInfo &m : h->host_mods) {
     const int k = (m.ph <= kRingSmall && m.hp <= kRingSmall) ? 0
                   : (m.ph <= 32 && m.hp <= 32) ? 1 : 2;
@@ -3104,16 +3001,15 @@ int ccdgpu_kernel_profile(ccdgpu_handle *h, int32_t reps, double *ms, double *fl
   // The small class is launched with the phhp gather ahead of it (fused path): per slab
   // element an index, one read of t and the slab store.
   bytes[0] += 20.0 * (double)h->n_m;
-  // hh ladder: P = V_hhpp T over the pp rows and r = row dots; reads V_pphh and T, writes the
-  // slice partials of P and r.  Reduction: reads the partials and V_hhhh, writes X (reference
-  // layout and FP64 operand tiles) and s.
+  // hh ladder: P = V_hhpp T over the packed rows and r = row dots; reads packed V and T, writes
+  // the slice partials of P and r.  Reduction: reads the partials and V_hhhh, writes X and s.
   for (const ChanInfo &a : h->host_chans) {
-    const int k = a.hh <= 16 ? 3 : 4;
-    const double hh2 = (double)a.hh * a.hh;
-    flops[k] += 2.0 * a.pp * a.hh * (a.hh + 1.0);
-    bytes[k] += 16.0 * a.pp * a.hh + 8.0 * a.nhht * hh2 + 8.0 * a.pp;
-    flops[6] += (double)a.nhht * hh2;
-    bytes[6] += 8.0 * a.nhht * hh2 + 24.0 * hh2 + 8.0 * a.hh;
+    const int k = a.hk <= 8 ? 3 : 4;
+    const double hk2 = (double)a.hk * a.hk;
+    flops[k] += 2.0 * a.pk * a.hk * (a.hk + 1.0);
+    bytes[k] += a.hk ? 16.0 * a.pk * a.hk + 8.0 * a.nhht * hk2 + 8.0 * a.pk : 0.0;
+    flops[6] += (double)a.nhht * hk2;
+    bytes[6] += 8.0 * a.nhht * hk2 + 16.0 * hk2 + 8.0 * a.hk;
   }
   // One-body: segmented sums of s and r (one value per pair) into x_k and y_a.
   flops[5] = (double)h->n_t * 0;  // no arithmetic worth counting
@@ -3144,36 +3040,24 @@ int ccdgpu_ladder_profile(ccdgpu_handle *h, int32_t reps, double *ms, double *fl
   CK(cudaSetDevice(h->opt.device));
   int rc = set_ctl(h, 0, h->h_ctl->tol, h->h_ctl->max_iters, h->h_ctl->mixing, false);
   if (rc) return rc;
+  if ((rc = materialize_d(h))) return rc;  // the kernels overwrite what it is expanded from
   for (int k = 0; k < 4; k++) ms[k] = flops[k] = bytes[k] = 0;
   for (const ChanInfo &a : h->host_chans) {
-    const int k = a.nb <= 8 ? 0 : a.nb <= 32 ? 1 : 2;
-    const double f = 2.0 * a.pr * ((double)a.pk + a.hh) * a.hh;
-    const double b = (double)a.pr * a.pk + ((double)a.pk + a.pr) * a.hh + (double)a.hh * a.hh;
-    flops[k] += f;
-    bytes[k] += 8.0 * b + 8.0 * a.pp * a.hh;
+    if (!a.nmt) continue;
+    const int k = ladder_class(a.hs);
+    const double v = (double)a.pk * a.pk, q = (double)a.pk * a.hk;
+    flops[k] += 2.0 * v * a.hk;
+    bytes[k] += 8.0 * (v + 2.0 * q);
     if (h->nt) {
-      flops[3] += f;
-      bytes[3] += 2.0 * h->nt * (h->tc_gen ? b - (double)a.pr * a.pk : b) + 8.0 * a.pp * a.hh;
+      flops[3] += 2.0 * v * a.hk;
+      bytes[3] += 2.0 * h->nt * ((h->tc_gen ? 0.0 : v) + q) + 8.0 * q;
     }
   }
   for (int k = 0; k < 4; k++) {
     if (k < 3 && !h->n_cls[k]) continue;
     if (k == 3 && !h->n_tc_tiles) continue;
     auto launch = [&]() -> int {
-      if (k == 3) return launch_pp_ladder_tc(h, h->s0);
-      const size_t smem = k == 0 ? h->ladder_smem_thin : h->ladder_smem;
-      auto kern = k == 0 ? pp_ladder_kernel<0> : k == 1 ? pp_ladder_kernel<1> : pp_ladder_kernel<2>;
-      kern<<<h->fp_grid[k], ladder_threads(k), smem, h->s0>>>(
-          h->tiles, h->fp_cta_off + h->fp_off_base[k], h->v_t, h->t_kt, h->t_mt, h->x_t,
-          h->rowmap, h->mirror, h->dmat, h->lpart, h->ctl, h->err, 0);
-      CK(cudaGetLastError());
-      if (h->n_red_cls[k]) {
-        const int off = k == 0 ? 0 : k == 1 ? h->n_red_cls[0] : h->n_red_cls[0] + h->n_red_cls[1];
-        ladder_reduce_kernel<<<h->n_red_cls[k], 256, 0, h->s0>>>(
-            h->red_fp + off, h->tiles, h->rowmap, h->mirror, h->dmat, h->lpart, h->ctl, 0);
-        CK(cudaGetLastError());
-      }
-      return CCDGPU_OK;
+      return k == 3 ? launch_pp_ladder_tc(h, h->s0) : launch_pp_ladder(h, h->s0, k);
     };
     if ((rc = launch())) return rc;  // warm-up
     CK(cudaEventRecord(h->ev[0], h->s0));

@@ -142,8 +142,9 @@ enum ccdgpu_v_mode {
                                   memory; slower than streaming the images on B200) */
 };
 enum ccdgpu_path {
-  CCDGPU_PATH_FUSED = 0,       /* fused kernels: one-body terms from the ladder intermediates,
-                                  remaps folded into the assembly kernel */
+  CCDGPU_PATH_FUSED = 0,       /* fused kernels on one amplitude in four (a < b, i < j): one-body
+                                  terms from the ladder intermediates, remaps folded into the
+                                  assembly kernel */
   CCDGPU_PATH_TABLES = 1       /* stage by stage exactly as main.cpp:591-665: 8 gathers and
                                   5 scatters through the loadMaps tables */
 };
@@ -190,7 +191,9 @@ const char *ccdgpu_strerror(int status);
 /* Zero every amplitude chain (main.cpp:497-503). */
 int ccdgpu_reset(ccdgpu_handle *h);
 /* Load / read T2 in t2_pphh order (n = sum of pp*hh).  Loading also refreshes t2Old and
- * the scattered layouts, as main.cpp:660-665 would after an iteration. */
+ * the scattered layouts, as main.cpp:660-665 would after an iteration.  T2 is antisymmetric in
+ * (a, b) and in (i, j), as every T2 of the loop is: the ladder, the one-body sums and (fused path)
+ * the ring read its a < b, i < j elements. */
 int ccdgpu_set_t2(ccdgpu_handle *h, const double *t2_pphh, uint64_t n);
 int ccdgpu_get_t2(ccdgpu_handle *h, double *t2_pphh, uint64_t n);
 /* Second-order energy on the device, the reference's MBPT2 (MBPT2Corr.cpp:6-38):
@@ -320,12 +323,14 @@ int ccdgpu_work_per_iteration(const ccdgpu_handle *h, double *flops, double *lad
 
 /* pp-ladder schedule (no counterpart in the reference): how far the K dimension of each
  * channel block is split into deterministic partial sums, as a target of tiles per SM for the
- * FP64 thin class (hh <= 8), the FP64 mid/wide classes, and the tensor-core ladder. */
+ * FP64 thin class (at most 4 strict hole pairs i < j), the FP64 mid/wide classes, and the
+ * tensor-core ladder. */
 typedef struct ccdgpu_schedule {
   int32_t thin_split_mul;      /* default 1 */
-  int32_t wide_split_mul;      /* default 3: FP64 wide class (nb > 32; also mid when mid is 0) */
+  int32_t wide_split_mul;      /* default 3: FP64 wide class (also mid when mid is 0) */
   int32_t tc_split_mul;        /* default 2 */
-  int32_t mid_split_mul;       /* default 0 = as wide_split_mul: FP64 mid class (nb 16..32) */
+  int32_t mid_split_mul;       /* default 0 = as wide_split_mul: FP64 mid class (5 to 20
+                                  strict hole pairs) */
   int32_t reserved[4];
 } ccdgpu_schedule;
 int ccdgpu_set_schedule(ccdgpu_handle *h, const ccdgpu_schedule *sch);
@@ -337,9 +342,9 @@ int ccdgpu_autotune(ccdgpu_handle *h, int32_t reps, ccdgpu_schedule *chosen, dou
                     double *ms_tc);
 
 /* Each pp-ladder class launched alone, reps times (CUDA events): ms, executed flops (packed:
- * rows a<=b, K over c<d and hh) and algorithmic bytes per launch, indexed FP64 thin (hh <= 8),
- * FP64 mid (nb 16..32), FP64 wide (nb 40..72, the largest channels), tensor-core ladder
- * (mixed handles).  Amplitudes are not changed.  No counterpart in the reference. */
+ * rows a<b, columns i<j, K over c<d) and algorithmic bytes per launch, indexed FP64 thin (at
+ * most 4 strict hole pairs), FP64 mid (5 to 20), FP64 wide (21 to 36, the largest channels),
+ * tensor-core ladder (mixed handles).  An iteration runs the FP64 classes in one launch.  Amplitudes are not changed.  No counterpart in the reference. */
 int ccdgpu_ladder_profile(ccdgpu_handle *h, int32_t reps, double ms[4], double flops[4],
                           double bytes[4]);
 
@@ -347,7 +352,7 @@ int ccdgpu_ladder_profile(ccdgpu_handle *h, int32_t reps, double ms[4], double f
  * stream (after one warm-up launch): average ms per launch, FP64 flops and algorithmic bytes
  * per launch, indexed ring small (ph', hp' <= 16; with the phhp gather that precedes the ring
  * on the fused path), ring mid (<= 32), ring large, hh ladder
- * small (hh <= 16), hh ladder rest, one-body sums, hh-ladder slice reduction.  Amplitudes are
+ * small (at most 8 strict hole pairs), hh ladder rest, one-body sums, hh-ladder reduction.  Amplitudes are
  * not changed (the kernels write only intermediates).  No counterpart in the reference. */
 int ccdgpu_kernel_profile(ccdgpu_handle *h, int32_t reps, double ms[7], double flops[7],
                           double bytes[7]);
@@ -356,12 +361,12 @@ int ccdgpu_kernel_profile(ccdgpu_handle *h, int32_t reps, double ms[7], double f
  * of an iteration of the next solve (-1 disarms); every kernel of that iteration then records
  * the %globaltimer time (ns) at which its first and its last CTA started.  Kernel ids, in this
  * order: ring small, ring mid, ring large, hh ladder small, hh ladder tiled, one-body, pp
- * ladder thin, mid, wide, tensor-core pp ladder, assembly, loop control, energy, FP64 tile
- * refresh, split-K reduction, hh-ladder reduction, phhp gather (17). */
+ * ladder in FP64 (every class), two unused, tensor-core pp ladder, assembly, loop control,
+ * energy, two unused, hh-ladder reduction, phhp gather (17). */
 int ccdgpu_trace_arm(ccdgpu_handle *h, int64_t iteration);
 int ccdgpu_trace_read(ccdgpu_handle *h, uint64_t *first, uint64_t *last, int32_t n);
 /* The same trace: when the last CTA of each kernel finished (%globaltimer ns; 0 for kernels
- * that do not record it: the loop control, energy and FP64 tile refresh kernels). */
+ * that do not record it: the loop control and energy kernels). */
 int ccdgpu_trace_read_end(ccdgpu_handle *h, uint64_t *end, int32_t n);
 
 /* No counterpart in the reference.  The ladder term of one regular channel,
