@@ -233,7 +233,10 @@ __device__ __forceinline__ bool consume_mma(const StageInfo &ti, const double *A
 constexpr size_t kLadderSmem =
     (size_t)kStages * (kMaxAS * kBK + kBK * kMaxNB) * 8 + kStages * sizeof(StageInfo) +
     2 * kStages * 8 + kBK * 8;  // slack: the last B stage's fragment loads past hs
-__global__ void __launch_bounds__(kLadderThreads)
+// 80 registers: its nine warps then leave 8,704 registers of the fullest SM quarter (three ladder
+// warps), two warps of the ring's 64 group; at 94 no ring CTA of 8 warps fitted beside it and
+// the ring ran after the ladder.
+__global__ void __maxnreg__(80)
 pp_ladder_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *sched,
                  const double *__restrict__ v_t, const double *tq0, const double *tq1,
                  double *__restrict__ d, const Control *ctl, int32_t *err, int gate) {
@@ -382,7 +385,7 @@ __device__ __forceinline__ void cp_async_wait() {
 // where the ordered pairs' 47 MB and hh^2 outputs took 15 + 19 us.
 // ------------------------------------------------------------------------------------------
 constexpr int kHHRows = 32;       // packed rows of a warp's slice (hk <= 8)
-constexpr int kHHRowsL = 64;      // ... of a CTA's slice
+constexpr int kHHRowsL = 32;      // ... of a CTA's slice
 constexpr int kHHThreads = 256;
 constexpr int kHHNC = 2;
 __host__ __device__ inline int hh_rows(int hk) { return hk <= 8 ? kHHRows : kHHRowsL; }
@@ -532,18 +535,23 @@ hh_reduce_kernel(const HHOut *__restrict__ outs, int n, const double *__restrict
 
 // ------------------------------------------------------------------------------------------
 // Ring term: Y = V_hphp + 0.5 V_hpph T', R = T' Y per modified channel (calc.cpp:264-313).
-// T' is read from the phhp slab (t2Old_phhp); V_hpph is held transposed per channel
-// (Vt[k][i] = V_hpph[i][k], k < ph', i < hp').  Result layout: fused path (dst != null) stores
-// R[p] at out[dst[p]], the four terms of a quad side by side (dst < 0: a = b or i = j, in no
-// quad), so that the assembly reads them as one 32-byte word; table path (dst == null) writes
-// t2Diff_phhp, out[p] = R[p].
+// Table path (ring_small_kernel, ring16_kernel): T' read from the phhp slab (t2Old_phhp), V_hpph
+// held transposed per channel (Vt[k][i] = V_hpph[i][k], k < ph', i < hp'), R to t2Diff_phhp.
 // Channels with ph', hp' <= kRingSmall run one per warp; larger ones one per CTA, grouped by
-// padded size (ring16_kernel).
+// padded size.
+//
+// Fused path (ring_pair_*): the channel of (a, i) and that of (i, a) together.  T' of the second
+// is the transpose of the first's (t_ab,ij = t_ba,ji), and the assembly needs only the sums
+//   S[ai, jb] = R[ai, jb] + R[bj, ia] = T' (A + C T') + B T'
+// with A = V_hphp of the first channel, C = V_hpph (the same block for both, by the exchange of
+// both pairs) and B[ai, ck] = V_hphp[(k c), (i a)] of the second: three products instead of four
+// and half of the amplitudes, of V_hpph and of the results.  T' comes straight from the packed
+// amplitudes and S goes straight to the quad's two terms, both through dst.
 // ------------------------------------------------------------------------------------------
 constexpr int kRingSmall = 16;
 constexpr int kRingMax = 80;  // largest ph', hp'
 
-// dst[p] of the fused path: 4 * (packed position of the quad) + k, k = 0: (ab, ij), 1: (ab, ji),
+// Quad of a phhp slab position: 4 * (packed position) + k, k = 0: (ab, ij), 1: (ab, ji),
 // 2: (ba, ij), 3: (ba, ji); -1 outside every quad.  The amplitude there is +t, -t, -t, +t.
 __device__ __forceinline__ double ring_amplitude(const double *tq, int32_t dst) {
   if (dst < 0) return 0.0;
@@ -551,37 +559,15 @@ __device__ __forceinline__ double ring_amplitude(const double *tq, int32_t dst) 
   return ((dst & 3) == 1 || (dst & 3) == 2) ? -t : t;
 }
 
-// T' for the ring on the fused path: the phhp slab gathered from the packed amplitudes, at the
-// head of the ring stream: coalesced index loads and slab stores, scattered reads of an array a
-// quarter of the slab's size (which the previous assembly has just written, so mostly L2 hits).
-// Eight elements per thread, all their loads in flight together.  gate < 0: run outside the
-// iteration gating (a read of the slab after a solve).
-constexpr int kGatherPer = 8;
+// The phhp slab (t2Old_phhp) of a fused handle from its packed amplitudes, for readers of the
+// chain.
 __global__ void __launch_bounds__(256)
 phhp_gather_kernel(const int32_t *__restrict__ dst, int64_t n, const double *tq0,
-                   const double *tq1, double *__restrict__ phhp, const Control *ctl, int gate) {
-  if (gate >= 0) {
-    if (skip_iteration(ctl, gate, kTrGather)) return;
-  } else {
-    pdl_enter();
-  }
+                   const double *tq1, double *__restrict__ phhp, const Control *ctl) {
   const double *__restrict__ t = ctl->parity ? tq1 : tq0;
-  const int64_t p0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * kGatherPer;
-  if (p0 >= n) return;
-  double v[kGatherPer];
-  if (p0 + kGatherPer <= n) {
-    const int4 a = __ldg(reinterpret_cast<const int4 *>(dst + p0));
-    const int4 b = __ldg(reinterpret_cast<const int4 *>(dst + p0) + 1);
-    const int32_t idx[kGatherPer] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-    for (int k = 0; k < kGatherPer; ++k) v[k] = ring_amplitude(t, idx[k]);
-    double2 *o = reinterpret_cast<double2 *>(phhp + p0);
-#pragma unroll
-    for (int k = 0; k < kGatherPer / 2; ++k) o[k] = make_double2(v[2 * k], v[2 * k + 1]);
-  } else {
-    for (int64_t p = p0; p < n; ++p) phhp[p] = ring_amplitude(t, dst[p]);
-  }
-  if (gate >= 0) trace_end(ctl, kTrGather);
+  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n;
+       p += (int64_t)gridDim.x * blockDim.x)
+    phhp[p] = ring_amplitude(t, dst[p]);
 }
 
 // C (M8*8 x N8*8) = A B, K4*4 deep, on 8 x 8 tiles: warps warp, warp + nwarps, ... take items of
@@ -622,18 +608,15 @@ __host__ __device__ inline int ring_pad8(int n) { return (n + 7) & ~7; }
 
 // Channels with ph', hp' <= kRingSmall, one per warp (kRingSmallWarps per CTA), the same two
 // products on the FP64 MMA: the warp's stage is padded to P, H in {8, 16} with zeros and a row
-// stride of 20 doubles (4 mod 8: conflict-free fragment loads); R goes straight to global
-// memory (through dst on the fused path).
+// stride of 20 doubles (4 mod 8: conflict-free fragment loads).
 constexpr int kRingSmallWarps = 4;
 constexpr int kRingSmallLd = kRingSmall + 4;
 __global__ void __launch_bounds__(kRingSmallWarps * 32)
 ring_small_kernel(const ModInfo *__restrict__ mods, int n, const double *__restrict__ v_hpph,
                   const double *__restrict__ v_hphp, const double *__restrict__ t_phhp,
-                  const int32_t *__restrict__ dst, double *__restrict__ out, const Control *ctl,
-                  int gate) {
+                  double *__restrict__ out, const Control *ctl, int gate) {
   if (skip_iteration(ctl, gate, kTrRingSmall)) return;
   __shared__ __align__(16) double buf[kRingSmallWarps][3 * kRingSmall * kRingSmallLd];
-  __shared__ int32_t ibuf[kRingSmallWarps][kRingSmall * kRingSmall];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int mi = blockIdx.x * kRingSmallWarps + w;
   if (mi >= n) return;  // whole warps: the MMAs below are warp-collective
@@ -658,9 +641,6 @@ ring_small_kernel(const ModInfo *__restrict__ mods, int n, const double *__restr
     if (r < hp && c < hp) cp_async8(Ys + r * ld + c, v_hphp + m.y_off + r * hp + c);
     else Ys[r * ld + c] = 0.0;
   }
-  int32_t *Is = ibuf[w];  // scatter destinations (fused path), staged with the operands
-  if (dst)
-    for (int p = lane; p < ph * hp; p += 32) cp_async4(Is + p, dst + m.m_off + p);
   cp_async_commit();
   cp_async_wait<0>();
   __syncwarp();
@@ -669,11 +649,7 @@ ring_small_kernel(const ModInfo *__restrict__ mods, int n, const double *__restr
                    [&](int r, int c, double v) { Ys[r * ld + c] = 0.5 * v + Ys[r * ld + c]; });
   __syncwarp();
   warp_mma_gemm<2>(Ts, ld, 1, Ys, ld, P / 8, H / 8, H / 4, 0, 1, [&](int r, int c, double v) {
-    if (r < ph && c < hp) {
-      const int p = r * hp + c;
-      const int64_t o = dst ? (int64_t)Is[p] : m.m_off + p;
-      if (o >= 0) out[o] = v;
-    }
+    if (r < ph && c < hp) out[m.m_off + r * hp + c] = v;
   });
   trace_end(ctl, kTrRingSmall);
 }
@@ -753,8 +729,7 @@ template <int PAD>
 __global__ void __launch_bounds__(32 * ring16_warps(PAD), ring16_ctas(PAD))
 ring16_kernel(const ModInfo *__restrict__ mods, const double *__restrict__ v_hpph,
               const double *__restrict__ v_hphp, const double *__restrict__ t_phhp,
-              const int32_t *__restrict__ dst, double *__restrict__ out, const Control *ctl,
-              int gate) {
+              double *__restrict__ out, const Control *ctl, int gate) {
   if (skip_iteration(ctl, gate, PAD <= 32 ? kTrRingMid : kTrRingLarge)) return;
   extern __shared__ __align__(16) double r16[];
   constexpr int ld = PAD + 4, NT = 32 * ring16_warps(PAD), N8 = PAD / 8;
@@ -812,20 +787,306 @@ ring16_kernel(const ModInfo *__restrict__ mods, const double *__restrict__ v_hpp
         [&](int r, int c, double v, int) { Ys[r * ld + c] = 0.5 * v + Ys[r * ld + c]; });
   }
   __syncthreads();
-  // R = T' Y, stored for r < ph', c < hp' (through dst on the fused path);
-  // the destinations are loaded before the MMAs, so the stores do not wait on them.
-  int32_t to[4 * kRing16NC];
+  // R = T' Y, stored for r < ph', c < hp'.
   ring16_gemm<PAD, 1>(
-      Ts, Ys, warp,
-      [&](int slot, int r, int c) {
-        const int32_t p = (int32_t)(m.m_off + (int64_t)r * hp + c);
-        to[slot] = (r < ph && c < hp) ? (dst ? __ldg(dst + p) : p) : -1;
-        return 0.0;
-      },
-      [&](int, int, double v, int slot) {
-        if (to[slot] >= 0) out[to[slot]] = v;
+      Ts, Ys, warp, [](int, int, int) { return 0.0; },
+      [&](int r, int c, double v, int) {
+        if (r < ph && c < hp) out[m.m_off + (int64_t)r * hp + c] = v;
       });
   trace_end(ctl, PAD <= 32 ? kTrRingMid : kTrRingLarge);
+}
+
+// ---- Fused path: a channel and its transpose together ------------------------------------
+constexpr int32_t kRingNoStore = 1 << 30;  // ring_pair_dst: read only (the mirror stores)
+// The amplitude behind a destination in two steps, the load unconditional (position 0 for -1) and
+// the sign and the zeros afterwards: a load under a branch on d would leave one in flight.
+__device__ __forceinline__ double pair_load(const double *__restrict__ tq, int32_t d) {
+  return __ldcg(tq + (d < 0 ? 0 : (d & (kRingNoStore - 1)) >> 1));
+}
+__device__ __forceinline__ double pair_sign(double t, int32_t d) {
+  return d < 0 ? 0.0 : (d & 1) ? -t : t;
+}
+__device__ __forceinline__ void pair_store(double *out, int32_t d, double v) {
+  if (d >= 0 && !(d & kRingNoStore)) out[d] = v;
+}
+
+// ph', hp' <= kRingSmall: one pair per warp on m8n8k4, stages padded to 8 or 16 with zeros (row
+// stride 20 doubles), every load of the warp in flight at once.  Y replaces C once it is done
+// with.
+__global__ void __launch_bounds__(kRingSmallWarps * 32)
+ring_pair_small_kernel(const RingPair *__restrict__ pairs, int n,
+                       const double *__restrict__ v_hpph, const double *__restrict__ v_hphp,
+                       const double *__restrict__ img, const int32_t *__restrict__ dst,
+                       const double *tq0, const double *tq1, double *__restrict__ out,
+                       const Control *ctl, int gate) {
+  if (skip_iteration(ctl, gate, kTrRingSmall)) return;
+  constexpr int ld = kRingSmallLd, kPer = kRingSmall * kRingSmall / 32;
+  __shared__ __align__(16) double buf[kRingSmallWarps][3 * kRingSmall * ld];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int mi = blockIdx.x * kRingSmallWarps + w;
+  if (mi >= n) return;  // whole warps: the MMAs below are warp-collective
+  const RingPair m = pairs[mi];
+  const double *tq = ctl->parity ? tq1 : tq0;
+  const int ph = m.ph, hp = m.hp, P = ring_pad8(ph), H = ring_pad8(hp);
+  const int hs = H == 8 ? 3 : 4, ps = P == 8 ? 3 : 4;  // log2
+  double *Ts = buf[w], *Cs = Ts + kRingSmall * ld, *Bs = Cs + kRingSmall * ld;
+  const int32_t *dp = dst + m.dst_off;
+  int32_t idx[kPer];
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    const int e = lane + 32 * j, r = e >> hs, c = e & (H - 1);
+    idx[j] = e < P * H && r < ph && c < hp ? __ldg(dp + r * hp + c) : -1;
+  }
+  for (int e = lane; e < P * H; e += 32) {
+    const int r = e >> hs, c = e & (H - 1);
+    if (r < ph && c < hp) cp_async8(Cs + r * ld + c, v_hpph + m.m_off + r * hp + c);
+    else Cs[r * ld + c] = 0.0;
+  }
+  for (int e = lane; e < P * P; e += 32) {
+    const int r = e >> ps, c = e & (P - 1);
+    if (r < ph && c < ph) cp_async8(Bs + r * ld + c, img + m.b_img + r * ph + c);
+    else Bs[r * ld + c] = 0.0;
+  }
+  cp_async_commit();
+  double y[2][2][2];  // Y = A + C T', starting from A
+#pragma unroll
+  for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int r = 8 * mt + g, c = 8 * nt + 2 * t + q;
+        y[mt][nt][q] = r < hp && c < hp ? __ldg(v_hphp + m.a_off + r * hp + c) : 0.0;
+      }
+  double tv[kPer];
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) tv[j] = pair_load(tq, idx[j]);
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    const int e = lane + 32 * j;
+    if (e < P * H) Ts[(e >> hs) * ld + (e & (H - 1))] = pair_sign(tv[j], idx[j]);
+  }
+  cp_async_wait<0>();
+  __syncwarp();
+#pragma unroll 2
+  for (int k = 0; k < P; k += 4) {
+    double a[2], b[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      a[q] = 8 * q < H ? Cs[(k + t) * ld + 8 * q + g] : 0.0;
+      b[q] = 8 * q < H ? Ts[(k + t) * ld + 8 * q + g] : 0.0;
+    }
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt)
+        if (8 * mt < H && 8 * nt < H) dmma_884(y[mt][nt], a[mt], b[nt]);
+  }
+  __syncwarp();
+#pragma unroll
+  for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt)
+      if (8 * mt < H && 8 * nt < H)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) Cs[(8 * mt + g) * ld + 8 * nt + 2 * t + q] = y[mt][nt][q];
+  __syncwarp();
+  // S = T' Y + B T'.
+  double s[2][2][2] = {};
+  auto gemm = [&](const double *A, const double *B, int K) {
+#pragma unroll 2
+    for (int k = 0; k < K; k += 4) {
+      double a[2], b[2];
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        a[q] = 8 * q < P ? A[(8 * q + g) * ld + k + t] : 0.0;
+        b[q] = 8 * q < H ? B[(k + t) * ld + 8 * q + g] : 0.0;
+      }
+#pragma unroll
+      for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt)
+          if (8 * mt < P && 8 * nt < H) dmma_884(s[mt][nt], a[mt], b[nt]);
+    }
+  };
+  gemm(Ts, Cs, H);
+  gemm(Bs, Ts, P);
+#pragma unroll
+  for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int r = 8 * mt + g, c = 8 * nt + 2 * t + q;
+        if (r < ph && c < hp) pair_store(out, __ldg(dp + r * hp + c), s[mt][nt][q]);
+      }
+  trace_end(ctl, kTrRingSmall);
+}
+
+// Larger pairs on m16n8k16: units of one pair and a block of up to kPairNC 8-column tiles of S
+// (columns of Y and S depend on the same columns of T' alone, so blocks share no product), one
+// CTA each, warp w on the rows [16 w, 16 w + 16) of Y and S.  A, B, C and the destinations are
+// stored in the order in which the lanes of a fragment take them, so every load of them is a
+// 16-byte one, contiguous over the warp, straight into registers; shared memory holds T' (the B
+// operand of both first products and the A operand of the last) and Y.  S starts with B T', which
+// needs no Y, so Y's store and barrier hide behind it.
+// Why: a CTA per pair with staged operands kept its SM's L1 pipe 80 % busy (scalar operand loads,
+// staging, random reads and stores) in phases that did not overlap the MMAs, at two CTAs of 114
+// registers and 104 KB per SM, and one (or none, at 80 columns) beside the ladder.
+constexpr int kPairNC = 4;
+__host__ __device__ inline int pad16(int n) { return (n + 15) & ~15; }
+__host__ __device__ constexpr int pair_ldy() { return 8 * kPairNC + 4; }  // 4 mod 8 doubles
+__host__ __device__ constexpr size_t ring_pair_smem(int mt) {
+  return (size_t)16 * mt * (16 * mt + 4 + pair_ldy()) * sizeof(double);
+}
+// Fragment-ordered A operand: [16-row tile][16-deep step][4][lane][2].
+__device__ __forceinline__ void frag_load(double (&a)[8], const double *__restrict__ p) {
+  const double2 *q = reinterpret_cast<const double2 *>(p) + (threadIdx.x & 31);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const double2 v = __ldg(q + 32 * j);
+    a[2 * j] = v.x;
+    a[2 * j + 1] = v.y;
+  }
+}
+// acc += A B over K: A fragments from `frag`, two steps ahead of the products (f[0] and f[1] hold
+// the first two on entry), B[k][n] = Bs[k * ldb + n], nt column tiles.
+__device__ __forceinline__ void frag_start(double (&f)[2][8], const double *__restrict__ frag,
+                                           int K) {
+  frag_load(f[0], frag);
+  if (K > 16) frag_load(f[1], frag + 256);
+}
+__device__ __forceinline__ void frag_gemm(double (&acc)[kPairNC][4], double (&f)[2][8],
+                                          const double *__restrict__ frag, const double *Bs,
+                                          int ldb, int nt, int K) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  auto step = [&](double (&a)[8], int k0) {
+#pragma unroll
+    for (int n = 0; n < kPairNC; ++n) {
+      if (n >= nt) break;
+      double b[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) b[q] = Bs[(k0 + t + 4 * q) * ldb + 8 * n + g];
+      dmma_16816(acc[n], a, b);
+    }
+    if (k0 + 32 < K) frag_load(a, frag + (k0 + 32) * 16);
+  };
+  for (int k0 = 0; k0 < K; k0 += 32) {
+    step(f[0], k0);
+    if (k0 + 16 < K) step(f[1], k0 + 16);
+  }
+}
+template <int MT>
+__global__ void __launch_bounds__(32 * MT, 8 - MT)
+ring_pair_kernel(const RingUnit *__restrict__ units, const double *__restrict__ img,
+                 const int32_t *__restrict__ dst,
+                 const int32_t *__restrict__ to_img, const double *tq0, const double *tq1,
+                 double *__restrict__ out, const Control *ctl, int gate) {
+  constexpr int kTr = MT <= 2 ? kTrRingMid : kTrRingLarge;
+  if (skip_iteration(ctl, gate, kTr)) return;
+  extern __shared__ __align__(16) double rp_smem[];
+  const RingUnit m = units[blockIdx.x];
+  const double *tq = ctl->parity ? tq1 : tq0;
+  const int ph = m.ph, hp = m.hp, P = pad16(ph), H = pad16(hp), ldh = H + 4;
+  constexpr int ldy = pair_ldy();
+  double *Ts = rp_smem, *Ys = rp_smem + P * ldh;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int n8 = (hp + 7) >> 3, nt = m.nt;
+  const bool yrow = 16 * warp < H, srow = 16 * warp < P;
+  const double *c_frag = img + m.c_img + (int64_t)warp * P * 16;
+  const double *b_frag = img + m.b_img + (int64_t)warp * P * 16;
+  // T': rows warp, warp + MT, ..., lanes over the columns; index, then amplitude, eight rows'
+  // in flight together.  Behind the first indices: the loads that need nothing, C's first steps
+  // and A (where Y starts).
+  constexpr int COLS = (16 * MT + 31) / 32;
+  const int32_t *dp = dst + m.dst_off;
+  int32_t idx[2][8][COLS];
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < COLS; ++j) {
+        const int r = warp + MT * (8 * h + i), c = lane + 32 * j;
+        idx[h][i][j] = r < ph && c < hp ? __ldg(dp + r * hp + c) : -1;
+      }
+  double f[2][8], acc[kPairNC][4];
+  if (yrow) {
+    frag_start(f, c_frag, P);
+    const double2 *ap = reinterpret_cast<const double2 *>(img + m.a_img) +
+                        ((int64_t)warp * n8 + m.n0) * 64 + lane;
+#pragma unroll
+    for (int n = 0; n < kPairNC; ++n)
+      if (n < nt) {
+        const double2 lo = __ldg(ap + 64 * n), hi = __ldg(ap + 64 * n + 32);
+        acc[n][0] = lo.x; acc[n][1] = lo.y; acc[n][2] = hi.x; acc[n][3] = hi.y;
+      }
+  }
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    double tv[8][COLS];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < COLS; ++j) tv[i][j] = pair_load(tq, idx[h][i][j]);
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < COLS; ++j) {
+        const int r = warp + MT * (8 * h + i), c = lane + 32 * j;
+        if (r < P && c < H) Ts[r * ldh + c] = pair_sign(tv[i][j], idx[h][i][j]);
+      }
+  }
+  __syncthreads();
+  const double *Tj = Ts + 8 * m.n0;  // this unit's columns of T'
+  if (yrow) {  // Y = A + C T'
+    frag_gemm(acc, f, c_frag, Tj, ldh, nt, P);
+    if (srow) frag_start(f, b_frag, P);
+#pragma unroll
+    for (int n = 0; n < kPairNC; ++n)
+      if (n < nt)
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          Ys[(16 * warp + g + 8 * (q >> 1)) * ldy + 8 * n + 2 * t + (q & 1)] = acc[n][q];
+  }
+#pragma unroll
+  for (int n = 0; n < kPairNC; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.0;
+  int4 to[kPairNC];
+  if (srow) {  // S = B T' ...
+    if (!yrow) frag_start(f, b_frag, P);
+    frag_gemm(acc, f, b_frag, Tj, ldh, nt, P);
+    const int4 *tp = reinterpret_cast<const int4 *>(to_img + m.to_img) +
+                     ((int64_t)warp * n8 + m.n0) * 32 + lane;
+#pragma unroll
+    for (int n = 0; n < kPairNC; ++n)
+      if (n < nt) to[n] = __ldg(tp + 32 * n);
+  }
+  __syncthreads();
+  if (srow) {  // ... + T' Y, to the quads
+    double a[8];
+    for (int k0 = 0; k0 < H; k0 += 16) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        a[i] = Ts[(16 * warp + g + 8 * (i % 2)) * ldh + k0 + t + 4 * (i / 2)];
+#pragma unroll
+      for (int n = 0; n < kPairNC; ++n) {
+        if (n >= nt) break;
+        double b[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) b[q] = Ys[(k0 + t + 4 * q) * ldy + 8 * n + g];
+        dmma_16816(acc[n], a, b);
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < kPairNC; ++n)
+      if (n < nt) {
+        if (to[n].x >= 0) out[to[n].x] = acc[n][0];
+        if (to[n].y >= 0) out[to[n].y] = acc[n][1];
+        if (to[n].z >= 0) out[to[n].z] = acc[n][2];
+        if (to[n].w >= 0) out[to[n].w] = acc[n][3];
+      }
+  }
+  trace_end(ctl, kTr);
 }
 
 // Deterministic block reduction (fixed tree) of one double; result valid in thread 0.
@@ -934,7 +1195,7 @@ __device__ __forceinline__ void write_t_image(const ChanInfo &ch, int u, int w, 
 
 // ------------------------------------------------------------------------------------------
 // Fused assembly (calc.cpp:384-418 plus the remaps folded in):
-//   value = V + D + R_ai,jb - R_aj,ib - R_bi,ja + R_bj,ia          (4 ring terms, read side by side)
+//   value = V + D + R_ai,jb - R_aj,ib - R_bi,ja + R_bj,ia          (ring: the two sums S, side by side)
 //         + 0.5 x_i t_ab,ji - 0.5 x_j t_ab,ij                       (h2pp_h1 gathers, algebraically)
 //         + (-0.5 y_b) t_ab,ij - (-0.5 y_a) t_ba,ij                 (p2_p1hh gathers, algebraically)
 //   t_new = mixing value/(e_i+e_j-e_a-e_b) + (1-mixing) t_old;  E += V t_new
@@ -961,7 +1222,7 @@ __device__ __forceinline__ void loop_set_condition(const Control *ctl,
 // packed position and the four ring terms, and writes the new packed amplitude (and, in a mixed
 // iteration, its bf16 terms).  The energy gains 4 V t_new per quad.  Persistent CTAs stride over
 // work items of up to kQuadPerItem quads of one channel; a thread takes one quad of an item and
-// issues all its loads before the store.  EG N=54 |n|^2 <= 36: 64 bytes a quad against 136 when
+// issues all its loads before the store.  EG N=54 |n|^2 <= 36: 48 bytes a quad against 136 when
 // the ordered pairs were kept (four amplitudes written, D and R read in their layout).
 constexpr int kQuadPerItem = kAsmThreads;  // one quad per thread and item
 constexpr int kAsmCTAsPerSM = 3;
@@ -1013,17 +1274,15 @@ __device__ __forceinline__ double quad_d(const LadderChan &lc, const double *__r
 }
 
 // value of element (ab, ij) (calc.cpp:384-418) with t_ab,ji = -t and t_ba,ij = -t:
-//   V + D + R_ai,jb - R_aj,ib - R_bi,ja + R_bj,ia + 0.5 x_i t_ab,ji - 0.5 x_j t_ab,ij
+//   V + D + (R_ai,jb + R_bj,ia) - (R_aj,ib + R_bi,ja) + 0.5 x_i t_ab,ji - 0.5 x_j t_ab,ij
 //     + (-0.5 y_b) t_ab,ij - (-0.5 y_a) t_ba,ij
-__device__ __forceinline__ double quad_value(double v, double dm, double r1, double r2, double r3,
-                                             double r4, double t, double xi, double xj,
-                                             double ya, double yb, double den, double mixing) {
+__device__ __forceinline__ double quad_value(double v, double dm, double2 s, double t, double xi,
+                                             double xj, double ya, double yb, double den,
+                                             double mixing) {
   double value = v;
   value += dm;
-  value += r1;
-  value -= r2;
-  value -= r3;
-  value += r4;
+  value += s.x;
+  value -= s.y;
   value += (0.5 * xi) * (-t);
   value -= (0.5 * xj) * t;
   value += (-0.5 * yb) * t;
@@ -1066,14 +1325,12 @@ assemble_fused_kernel(const QuadItem *__restrict__ items, int n_items,
   for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
     const QuadRef cu = nx;
     double tv = 0.0, vv = 0.0, dv = 0.0, xs[2] = {0.0, 0.0}, ys[2] = {0.0, 0.0};
-    double2 r01 = make_double2(0.0, 0.0), r23 = r01;
+    double2 ring = make_double2(0.0, 0.0);
     const int64_t p = cu.q_off + (int64_t)cu.u * cu.hs + cu.w;
     if (cu.ok) {
       tv = t_old[p];
       vv = __ldg(vq + p);
-      const double2 *rp = reinterpret_cast<const double2 *>(r_quad + 4 * p);
-      r01 = __ldcg(rp);
-      r23 = __ldcg(rp + 1);
+      ring = __ldcg(reinterpret_cast<const double2 *>(r_quad + 2 * p));
       // The one-body sums are small arrays every quad reads: through L1 (an L2-only load
       // would send every warp to the same few L2 slices).
       xs[0] = xh[cu.i];
@@ -1084,8 +1341,8 @@ assemble_fused_kernel(const QuadItem *__restrict__ items, int n_items,
     }
     quad_fetch(items, n_items, qrows, qcols, it + gridDim.x, nx);
     if (!cu.ok) continue;
-    const double t1 = quad_value(vv, dv, r01.x, r01.y, r23.x, r23.y, tv, xs[0], xs[1], ys[0],
-                                 ys[1], cu.den, mixing);
+    const double t1 =
+        quad_value(vv, dv, ring, tv, xs[0], xs[1], ys[0], ys[1], cu.den, mixing);
     t_new[p] = t1;
     if (nt) write_t_image(chans[cu.ch], cu.u, cu.w, t1, nt, tkt_tc, tkt_tc_stride);
     corr += 4.0 * (vv * t1);

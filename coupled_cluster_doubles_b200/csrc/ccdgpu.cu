@@ -42,18 +42,19 @@ struct DevBuf {
 }  // namespace
 
 // A handle's streams and events (see the pool below).
+constexpr int kStreams = 6, kEvents = 18;
+constexpr int kJoin0 = 12;  // events kJoin0 + 1 .. kJoin0 + kStreams - 1: the branches' ends
 struct StreamSet {
   int dev = -1;
-  cudaStream_t s[4] = {nullptr, nullptr, nullptr, nullptr};
-  cudaEvent_t ev[16] = {};
+  cudaStream_t s[kStreams] = {};
+  cudaEvent_t ev[kEvents] = {};
 };
 
 struct ccdgpu_handle {
   ccdgpu_options opt{};
   StreamSet sset;  // the streams and events below, from the process-wide pool
   cudaStream_t s0 = nullptr, s1 = nullptr, s2 = nullptr, s3 = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_fork2 = nullptr, ev_join2 = nullptr;
-  cudaEvent_t ev_fork3 = nullptr, ev_join3 = nullptr;  // one-body sums beside the pp ladder
+  cudaEvent_t ev_fork = nullptr, ev_fork2 = nullptr;
   cudaEvent_t ev[10] = {};
   uint64_t nch = 0, nsp = 0, np = 0, npart = 0;
   int64_t n_t = 0, n_m = 0, n_h = 0, n_p = 0;
@@ -100,7 +101,15 @@ struct ccdgpu_handle {
   double *x = nullptr;
   double *s = nullptr, *r = nullptr, *xh = nullptr, *yp = nullptr, *epart = nullptr;
   int32_t *flat = nullptr;
-  int32_t *ring_dst = nullptr;  // fused path: phhp position -> 4 x packed position + term, -1
+  int32_t *ring_quads = nullptr;  // phhp position -> 4 x packed position + term, -1
+  // Fused-path ring: pairs of channels (one per warp first, then by padded size 32 .. 80), their
+  // operand images and destinations.
+  RingPair *ring_pairs = nullptr;
+  double *ring_img = nullptr;
+  RingUnit *ring_units = nullptr;
+  int32_t *ring_dst = nullptr, *ring_to = nullptr;
+  int n_pair_small = 0, n_unit[4] = {0, 0, 0, 0};  // units by row tiles 2 .. 5
+  std::vector<RingPair> host_pairs;
   double create_ms[5] = {};   // ccdgpu_profile::ms_create
   double loop_graph_ms = 0;   // ccdgpu_profile::ms_loop_graph
   int64_t *o_h = nullptr, *o_p = nullptr;
@@ -130,7 +139,6 @@ struct ccdgpu_handle {
   // pp-ladder work lists (make_ladder_tiles), in their own allocation so the autotuner can
   // rebuild them.
   std::vector<ChanInfo> host_chans;
-  std::vector<ModInfo> host_mods;
   int64_t n_list = 0;  // entries of the one-body segment lists
   ccdgpu_schedule schedule{};
   void *tile_mem = nullptr;
@@ -397,9 +405,9 @@ cudaError_t acquire_set(StreamSet &ss) {
       }
   }
   ss.dev = dev;
-  for (int k = 0; k < 4 && e == cudaSuccess; k++)
+  for (int k = 0; k < kStreams && e == cudaSuccess; k++)
     e = cudaStreamCreateWithFlags(&ss.s[k], cudaStreamNonBlocking);
-  for (int k = 0; k < 16 && e == cudaSuccess; k++)
+  for (int k = 0; k < kEvents && e == cudaSuccess; k++)
     e = k < 10 ? cudaEventCreate(&ss.ev[k]) : cudaEventCreateWithFlags(&ss.ev[k], cudaEventDisableTiming);
   if (e != cudaSuccess) {
     destroy_set(ss);
@@ -434,7 +442,7 @@ void release_stream_pool() {
 void release(ccdgpu_handle *h) {
   if (!h) return;
   // Cached blocks are handed to other handles: nothing of this one may still run on them.
-  for (cudaStream_t st : {h->s0, h->s1, h->s2, h->s3})
+  for (cudaStream_t st : h->sset.s)
     if (st) cudaStreamSynchronize(st);
   for (cudaGraphExec_t g : {h->graph, h->graph_tc, h->loop64, h->loop_tc})
     if (g) cudaGraphExecDestroy(g);
@@ -913,7 +921,7 @@ TcKernel tc_kernel_of(int nt, bool gen) {
 // on the largest bases), later creates only clear them.
 struct BuildScratch {
   std::vector<int32_t> rowmap, kcol, pp_swap, hh_swap, prow, hcol, qrow, list;
-  std::vector<int2> pp_pairs, hh_pairs, mod_ph, mod_hp, mod_dims;
+  std::vector<int2> pp_pairs, hh_pairs, mod_ph, mod_hp, mod_dims, mod_look;
   std::vector<int4> vrows;
   std::vector<QuadCol> quad_cols;
   std::vector<QuadItem> quad_items;
@@ -1222,12 +1230,13 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   int64_t y_tot = 0;
   std::vector<const double *> src_hpph, src_hphp;
   std::vector<int64_t> cnt_hpph, cnt_hphp;
-  std::vector<ModGen> mod_gen;        // generated V: modified channels in channel order
+  std::vector<ModGen> mod_gen;        // modified channels in channel order
   std::vector<int32_t> &mod_gen_chan = bs.mod_gen_chan;  // ... and their channel slots
   mod_gen_chan.clear();
   std::vector<int2> &mod_ph = bs.mod_ph, &mod_hp = bs.mod_hp;  // ... their ph' (b, j), hp' (i, a) pairs
   mod_ph.clear();
   mod_hp.clear();
+  bool mod_maps = true;  // the problem carries the ph' and hp' pair lists
   for (uint64_t c = 0; c < nch; c++) {
     const int64_t ph = MD[c].ph, hp = MD[c].hp;
     mod_dims[c] = make_int2((int)ph, (int)hp);
@@ -1235,14 +1244,16 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     if (ph > kRingMax || hp > kRingMax) return CCDGPU_ERR_UNSUPPORTED;  // ring tiles
     ModInfo m{};
     m.ph = (int)ph; m.hp = (int)hp; m.m_off = o_m[c]; m.y_off = y_tot;
-    if (gen_v) {
-      // The pairs themselves are copied in parallel after this loop.
-      if (!P->chan_mod_maps[c].ph || !P->chan_mod_maps[c].hp) return CCDGPU_ERR_INVALID_ARGUMENT;
-      const int64_t ph0 = mod_gen.empty() ? 0 : mod_gen.back().ph_off + mod_gen.back().ph;
-      const int64_t hp0 = mod_gen.empty() ? 0 : mod_gen.back().hp_off + mod_gen.back().hp;
-      mod_gen.push_back(ModGen{(int)ph, (int)hp, m.m_off, m.y_off, ph0, hp0});
-      mod_gen_chan.push_back((int32_t)c);
-    } else {
+    // The pairs themselves are copied in parallel after this loop.
+    if (!P->chan_mod_maps || !P->chan_mod_maps[c].ph || !P->chan_mod_maps[c].hp) {
+      if (derive_tables || gen_v) return CCDGPU_ERR_INVALID_ARGUMENT;
+      mod_maps = false;
+    }
+    const int64_t ph0 = mod_gen.empty() ? 0 : mod_gen.back().ph_off + mod_gen.back().ph;
+    const int64_t hp0 = mod_gen.empty() ? 0 : mod_gen.back().hp_off + mod_gen.back().hp;
+    mod_gen.push_back(ModGen{(int)ph, (int)hp, m.m_off, m.y_off, ph0, hp0});
+    mod_gen_chan.push_back((int32_t)c);
+    if (!gen_v) {
       if (!P->v_hpph_mod[c] || !P->v_hphp_mod[c]) return CCDGPU_ERR_INVALID_ARGUMENT;
       src_hpph.push_back(P->v_hpph_mod[c]); cnt_hpph.push_back(ph * hp);
       src_hphp.push_back(P->v_hphp_mod[c]); cnt_hphp.push_back(hp * hp);
@@ -1257,21 +1268,123 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     mod_hp.resize(mod_gen.back().hp_off + mod_gen.back().hp);
     const std::vector<int32_t> &mod_chan = mod_gen_chan;
     std::atomic<int> bad_mod{0};
+    if (mod_maps) {
 #pragma omp parallel for num_threads(host_threads) schedule(dynamic, 16)
-    for (int64_t g = 0; g < (int64_t)mod_gen.size(); g++) {
-      const ModGen &mg = mod_gen[g];
-      const ccdgpu_pair *phm = P->chan_mod_maps[mod_chan[g]].ph, *hpm = P->chan_mod_maps[mod_chan[g]].hp;
-      for (int64_t k = 0; k < mg.ph; k++) {
-        if (phm[k].p < np || phm[k].p >= nsp || phm[k].q >= np) bad_mod = 1;
-        mod_ph[mg.ph_off + k] = make_int2((int)phm[k].p, (int)phm[k].q);
+      for (int64_t g = 0; g < (int64_t)mod_gen.size(); g++) {
+        const ModGen &mg = mod_gen[g];
+        const ccdgpu_pair *phm = P->chan_mod_maps[mod_chan[g]].ph, *hpm = P->chan_mod_maps[mod_chan[g]].hp;
+        for (int64_t k = 0; k < mg.ph; k++) {
+          if (phm[k].p < np || phm[k].p >= nsp || phm[k].q >= np) bad_mod = 1;
+          mod_ph[mg.ph_off + k] = make_int2((int)phm[k].p, (int)phm[k].q);
+        }
+        for (int64_t k = 0; k < mg.hp; k++) {
+          if (hpm[k].p >= np || hpm[k].q < np || hpm[k].q >= nsp) bad_mod = 1;
+          mod_hp[mg.hp_off + k] = make_int2((int)hpm[k].p, (int)hpm[k].q);
+        }
       }
-      for (int64_t k = 0; k < mg.hp; k++) {
-        if (hpm[k].p >= np || hpm[k].q < np || hpm[k].q >= nsp) bad_mod = 1;
-        mod_hp[mg.hp_off + k] = make_int2((int)hpm[k].p, (int)hpm[k].q);
+    } else {
+      // A problem with tables and V blocks but without the pair lists: the ai_jb table names the
+      // (a, i) of every ph' row and the (j, b) of every hp' column.
+      std::fill(mod_ph.begin(), mod_ph.end(), make_int2(-1, -1));
+      std::fill(mod_hp.begin(), mod_hp.end(), make_int2(-1, -1));
+      std::vector<int64_t> gen_of(nch, -1);
+      for (size_t g = 0; g < mod_gen.size(); g++) gen_of[mod_chan[g]] = (int64_t)g;
+      for (int ai = 0; ai < n_act; ai++) {
+        const ccdgpu_chain_index *mp = P->maps[CCDGPU_MAP_AI_JB][act_chan[ai]];
+        if (!mp) return CCDGPU_ERR_INVALID_ARGUMENT;
+        const ChanInfo &a = chans[ai];
+        for (int64_t e = 0; e < (int64_t)a.pp * a.hh; e++) {
+          const int2 ab = pp_pairs[a.pp_off + e / a.hh], ij = hh_pairs[a.hh_off + e % a.hh];
+          const int64_t g = mp[e].channel < nch ? gen_of[mp[e].channel] : -1;
+          if (g < 0 || mp[e].row >= (uint64_t)mod_gen[g].ph || mp[e].column >= (uint64_t)mod_gen[g].hp)
+            return CCDGPU_ERR_BAD_TABLE;
+          mod_ph[mod_gen[g].ph_off + mp[e].row] = make_int2(ab.x, ij.x);
+          mod_hp[mod_gen[g].hp_off + mp[e].column] = make_int2(ij.y, ab.y);
+        }
       }
     }
     if (bad_mod) return CCDGPU_ERR_BAD_TABLE;
   }
+  // Fused-path ring: each channel with its transpose, the channel whose ph' pairs are this one's
+  // hp' pairs exchanged (the first of the two in channel order names the pair).
+  const bool paired = h->opt.path == CCDGPU_PATH_FUSED;
+  std::vector<RingPair> pairs, pairs_large;
+  std::vector<RingUnit> units;
+  std::vector<int32_t> ring_perm;
+  int64_t img_tot = 0, pair_dst_tot = 0, to_tot = 0;
+  if (paired) {
+    std::vector<int2> &look = bs.mod_look;  // (hole, particle) pair -> channel, hp' index
+    look.assign((size_t)np * h->npart, make_int2(-1, -1));
+    for (size_t g = 0; g < mod_gen.size(); g++)
+      for (int k = 0; k < mod_gen[g].hp; k++) {
+        const int2 ia = mod_hp[mod_gen[g].hp_off + k];
+        if (ia.x < 0) return CCDGPU_ERR_BAD_TABLE;
+        look[(size_t)ia.x * h->npart + (ia.y - np)] = make_int2((int)g, k);
+      }
+    for (size_t g = 0; g < mod_gen.size(); g++) {
+      const ModGen &m = mod_gen[g];
+      const int perm_off = (int)ring_perm.size();
+      int other = -2;
+      for (int k = 0; k < m.ph; k++) {
+        const int2 ai = mod_ph[m.ph_off + k];
+        if (ai.x < 0) return CCDGPU_ERR_BAD_TABLE;
+        const int2 l = look[(size_t)ai.y * h->npart + (ai.x - np)];
+        if (l.x < 0 || (other >= 0 && l.x != other)) return CCDGPU_ERR_BAD_TABLE;
+        other = l.x;
+        ring_perm.push_back(l.y);
+      }
+      if (mod_gen[other].hp != m.ph || mod_gen[other].ph != m.hp) return CCDGPU_ERR_BAD_TABLE;
+      if (other < (int)g) {  // named by its transpose
+        ring_perm.resize(perm_off);
+        continue;
+      }
+      RingPair r{};
+      r.ph = m.ph; r.hp = m.hp;
+      r.perm_off = perm_off;
+      r.self = other == (int)g;
+      r.m_off = m.m_off; r.a_off = m.y_off; r.b_src = mod_gen[other].y_off;
+      (std::max(m.ph, m.hp) <= kRingSmall ? pairs : pairs_large).push_back(r);
+    }
+    h->n_pair_small = (int)pairs.size();
+    // The largest first, so that the short ones fill in behind them.
+    std::stable_sort(pairs_large.begin(), pairs_large.end(),
+                     [](const RingPair &x, const RingPair &y) {
+                       return (int64_t)x.ph * x.hp > (int64_t)y.ph * y.hp;
+                     });
+    pairs.insert(pairs.end(), pairs_large.begin(), pairs_large.end());
+    for (RingPair &r : pairs) {
+      r.dst_off = pair_dst_tot;
+      pair_dst_tot += (int64_t)r.ph * r.hp;
+      r.b_img = img_tot;
+      if (std::max(r.ph, r.hp) <= kRingSmall) {
+        img_tot += (r.ph * r.ph + 1) & ~1;  // 16-byte aligned, as the vector loads need
+      } else {
+        const int64_t p = pad16(r.ph), q = pad16(r.hp), n8 = (r.hp + 7) / 8;
+        img_tot += p * p;
+        r.c_img = img_tot;
+        img_tot += q * p;
+        r.a_img = img_tot;
+        img_tot += q * 8 * n8;
+        r.to_img = to_tot;
+        to_tot += p * 8 * n8;
+      }
+    }
+    // Units by row tiles: the pair's column tiles in blocks of at most kPairNC, as equal as they
+    // come.
+    for (int k = 0; k < 4; k++) {
+      const size_t first = units.size();
+      for (size_t i = h->n_pair_small; i < pairs.size(); i++) {
+        if (pad16(std::max(pairs[i].ph, pairs[i].hp)) / 16 != k + 2) continue;
+        const int n8 = (pairs[i].hp + 7) / 8, blocks = (n8 + kPairNC - 1) / kPairNC;
+        for (int q = 0; q < blocks; q++)
+          units.push_back({pairs[i].ph, pairs[i].hp, n8 * q / blocks,
+                           n8 * (q + 1) / blocks - n8 * q / blocks, pairs[i].dst_off,
+                           pairs[i].a_img, pairs[i].b_img, pairs[i].c_img, pairs[i].to_img});
+      }
+      h->n_unit[k] = (int)(units.size() - first);
+    }
+  }
+  h->host_pairs = pairs;
   // Largest channels first within a group, so that the short ones fill in behind them.
   auto by_work = [](const ModInfo &x, const ModInfo &y) {
     return (int64_t)x.ph * x.hp * x.hp > (int64_t)y.ph * y.hp * y.hp;
@@ -1284,7 +1397,6 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   }
   h->n_mod_mid = h->n_mod_pad[0];
   h->n_mod = (int)mods.size();
-  h->host_mods = mods;
 
   std::vector<int64_t> o_h(np + 1, 0), o_p(h->npart + 1, 0);
   for (uint64_t k = 0; k < np; k++) o_h[k + 1] = o_h[k] + (int64_t)P->three_body_dims[k].hpp;
@@ -1433,7 +1545,10 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   if (on_the_fly) ar.add_unset(&h->v_t, vt);
   else ar.add(&h->v_t, vt);
   ar.add(&h->v_hpph, h->n_m); ar.add(&h->v_hphp, y_tot);
-  ar.add(&h->flat, (size_t)8 * n_t); ar.add(&h->ring_dst, n_t); ar.add(&h->r_quad, 4 * q_tot);
+  ar.add(&h->flat, (size_t)8 * n_t); ar.add(&h->ring_quads, n_t); ar.add(&h->r_quad, paired ? 2 * q_tot : 0);
+  ar.add(&h->ring_pairs, pairs.size()); ar.add(&h->ring_img, img_tot);
+  ar.add(&h->ring_dst, pair_dst_tot); ar.add(&h->ring_units, units.size());
+  ar.add(&h->ring_to, to_tot);
   ar.add(&h->o_h, o_h.size()); ar.add(&h->o_p, o_p.size());
   ar.add(&h->t[0], n_t); ar.add(&h->t[1], n_t); ar.add(&h->dmat, n_t);
   ar.add(&h->old_phhp, h->n_m); ar.add(&h->r_phhp, h->n_m);
@@ -1572,6 +1687,8 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     sc.add(&d_hblk, np * np);
     sc.add(&d_pblk, (nsp - np) * (nsp - np));
   }
+  int32_t *d_ring_perm = nullptr;
+  sc.add(&d_ring_perm, ring_perm.size());
   ModGen *d_mod_gen = nullptr;
   int2 *d_mod_ph = nullptr, *d_mod_hp = nullptr;
   int32_t *d_mod_chan = nullptr;
@@ -1662,6 +1779,8 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     return CCDGPU_OK;
   };
   TRY(put(h->chans, chans)); TRY(put(h->mods, mods));
+  TRY(put(h->ring_pairs, pairs)); TRY(put(h->ring_units, units));
+  TRY(put(d_ring_perm, ring_perm));
   TRY(put(h->hh_tiles, hh_tiles)); TRY(put(h->hh_out, hh_out)); TRY(put(h->hh_part_off, hh_part_off));
   TRY(put(h->ranges, ranges)); TRY(put(h->quad_items, quad_items));
   TRY(put(h->quad_cols, quad_cols));
@@ -1813,9 +1932,15 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     check_counts_kernel<<<std::max(nb, 1), 256, 0, h->s0>>>(counts, 5 * n_t, h->err);
     CK(cudaGetLastError());
     ring_maps_kernel<<<h->n_ranges, 256, 0, h->s0>>>(h->ranges, h->chans, h->pp_swap, h->hh_swap,
-                                                     h->prow, h->hcol, h->flat, n_t, h->ring_dst,
-                                                     h->err);
+                                                     h->prow, h->hcol, h->flat, n_t,
+                                                     h->ring_quads, h->err);
     CK(cudaGetLastError());
+    if (!pairs.empty()) {
+      ring_image_kernel<<<(unsigned)pairs.size(), 256, 0, h->s0>>>(
+          h->ring_pairs, d_ring_perm, h->v_hpph, h->v_hphp, h->ring_quads, h->ring_img,
+          h->ring_dst, h->ring_to);
+      CK(cudaGetLastError());
+    }
   }
   if (a_vrow_off[n_act] > 0) {
     if (on_the_fly) {
@@ -1860,6 +1985,14 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   int smem_optin = 0;
   CK(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->opt.device));
   if (ring16_smem(80) > (size_t)smem_optin) return CCDGPU_ERR_UNSUPPORTED;
+  auto pair_attr = [](auto kern, int mt) {
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)ring_pair_smem(mt));
+  };
+  CK(pair_attr(ring_pair_kernel<2>, 2));
+  CK(pair_attr(ring_pair_kernel<3>, 3));
+  CK(pair_attr(ring_pair_kernel<4>, 4));
+  CK(pair_attr(ring_pair_kernel<5>, 5));
   CK(cudaFuncSetAttribute(pp_ladder_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                           (int)kLadderSmem));
   CK(cudaFuncSetAttribute(pp_ladder_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
@@ -2009,40 +2142,32 @@ int refresh_tc_image(ccdgpu_handle *h) {
   return cuda_status(cudaGetLastError());
 }
 
-// T' from the phhp slab in both paths.  fused: R into the quads' ring terms; else the table
-// path's t2Diff_phhp slab.
-// only: -1 every class, else 0 small, 1 mid, 2 large.
-int launch_phhp_gather(ccdgpu_handle *h, cudaStream_t st, int gate) {
+// t2Old_phhp of a fused handle from its current amplitudes.
+int launch_phhp_gather(ccdgpu_handle *h, cudaStream_t st) {
   if (!h->n_m) return CCDGPU_OK;
   h->launches++;
-  const unsigned blocks = (unsigned)ceil_div(h->n_m, (int64_t)256 * kGatherPer);
-  return cuda_status(launch_pdl(phhp_gather_kernel, blocks, 256, 0, st, (const int32_t *)h->ring_dst,
-                                h->n_m, (const double *)h->tq[0], (const double *)h->tq[1],
-                                h->old_phhp, (const Control *)h->ctl, gate));
+  const unsigned blocks = (unsigned)std::min<int64_t>(ceil_div(h->n_m, 256), 148 * 16);
+  phhp_gather_kernel<<<blocks, 256, 0, st>>>(h->ring_quads, h->n_m, h->tq[0], h->tq[1],
+                                             h->old_phhp, h->ctl);
+  return cuda_status(cudaGetLastError());
 }
-int launch_ring(ccdgpu_handle *h, cudaStream_t st, int gate, bool fused, int only = -1) {
-  const int32_t *dst = fused ? h->ring_dst : nullptr;
-  double *out = fused ? h->r_quad : h->r_phhp;
-  // Fused path: T' (the phhp slab) gathered from the current amplitudes first; the profile's
-  // small class includes it.
-  if (fused && (only < 0 || only == 0))
-    if (int rc = launch_phhp_gather(h, st, gate)) return rc;
-  if (h->n_mod_small && (only < 0 || only == 0)) {
+// Table path: T' from the phhp slab, R to t2Diff_phhp.
+int launch_ring(ccdgpu_handle *h, cudaStream_t st, int gate) {
+  if (h->n_mod_small) {
     CK(launch_pdl(ring_small_kernel, (int)ceil_div(h->n_mod_small, kRingSmallWarps),
                   kRingSmallWarps * 32, 0, st, (const ModInfo *)h->mods, h->n_mod_small,
                   (const double *)h->v_hpph, (const double *)h->v_hphp,
-                  (const double *)h->old_phhp, dst, out, (const Control *)h->ctl, gate));
+                  (const double *)h->old_phhp, h->r_phhp, (const Control *)h->ctl, gate));
     h->launches++;
   }
-  // Groups by padded size; only = 1 launches the 32 group, only = 2 the wider ones.
-  const ModInfo *mp = h->mods + h->n_mod_small;
+  const ModInfo *mp = h->mods + h->n_mod_small;  // groups by padded size
   for (int k = 0; k < 4; k++) {
     const int n = h->n_mod_pad[k];
-    if (n && (only < 0 || only == (k == 0 ? 1 : 2))) {
+    if (n) {
       auto go = [&](auto kern, int pad) {
         return launch_pdl(kern, n, 32 * ring16_warps(pad), ring16_smem(pad), st, mp,
                           (const double *)h->v_hpph, (const double *)h->v_hphp,
-                          (const double *)h->old_phhp, dst, out, (const Control *)h->ctl, gate);
+                          (const double *)h->old_phhp, h->r_phhp, (const Control *)h->ctl, gate);
       };
       switch (k) {
         case 0: CK(go(ring16_kernel<32>, 32)); break;
@@ -2055,6 +2180,32 @@ int launch_ring(ccdgpu_handle *h, cudaStream_t st, int gate, bool fused, int onl
     mp += n;
   }
   return CCDGPU_OK;
+}
+// Fused path: pairs of channels.  group: 0 the pairs of the one-per-warp kernel, 1 .. 4 the units
+// of 2 .. 5 row tiles.
+int launch_ring_pairs(ccdgpu_handle *h, cudaStream_t st, int gate, int group) {
+  if (group == 0) {
+    if (!h->n_pair_small) return CCDGPU_OK;
+    h->launches++;
+    return cuda_status(launch_pdl(
+        ring_pair_small_kernel, (int)ceil_div(h->n_pair_small, kRingSmallWarps),
+        kRingSmallWarps * 32, 0, st, (const RingPair *)h->ring_pairs, h->n_pair_small,
+        (const double *)h->v_hpph, (const double *)h->v_hphp, (const double *)h->ring_img,
+        (const int32_t *)h->ring_dst, (const double *)h->tq[0], (const double *)h->tq[1],
+        h->r_quad, (const Control *)h->ctl, gate));
+  }
+  const int n = h->n_unit[group - 1], mt = group + 1;
+  if (!n) return CCDGPU_OK;
+  const RingUnit *units = h->ring_units;
+  for (int k = 0; k < group - 1; k++) units += h->n_unit[k];
+  auto kern = mt == 2 ? ring_pair_kernel<2> : mt == 3 ? ring_pair_kernel<3>
+              : mt == 4 ? ring_pair_kernel<4> : ring_pair_kernel<5>;
+  h->launches++;
+  return cuda_status(launch_pdl(kern, n, 32 * mt, ring_pair_smem(mt), st,
+                                units, (const double *)h->ring_img, (const int32_t *)h->ring_dst,
+                                (const int32_t *)h->ring_to, (const double *)h->tq[0],
+                                (const double *)h->tq[1], h->r_quad, (const Control *)h->ctl,
+                                gate));
 }
 int launch_onebody_fused(ccdgpu_handle *h, cudaStream_t st, int gate) {
   const int warps_per_block = 8;
@@ -2095,9 +2246,10 @@ int launch_map_to(ccdgpu_handle *h, cudaStream_t st, const double *src, double *
   return cuda_status(cudaGetLastError());
 }
 
-// One fused iteration: the pp ladder on s0, the ring on s1 and the hh ladder with the one-body
-// sums on s2 side by side (each needs only the amplitudes), then the assembly on s0.  The
-// ladder, bound by HBM on one CTA per SM, goes first; the others, bound by latency, run beside it.
+// One fused iteration: the pp ladder on s0, the groups of the ring and the hh ladder with the
+// one-body sums on streams of their own (each needs only the amplitudes), then the assembly on
+// s0.  The ladder, bound by HBM on one CTA per SM, goes first; the others, bound by latency, run
+// beside it, the longest first.
 // mixed: the pp ladder runs on the tensor cores (split bf16) instead of the FP64 pipe.
 int enqueue_fused_iteration(ccdgpu_handle *h, bool mixed) {
   int rc;
@@ -2116,7 +2268,8 @@ int enqueue_fused_iteration(ccdgpu_handle *h, bool mixed) {
     if ((rc = ladder(h->s0))) return rc;
     CK(cudaEventRecord(h->ev[3], h->s0));
     CK(cudaEventRecord(h->ev[4], h->s0));
-    if ((rc = launch_ring(h, h->s0, gate, true))) return rc;
+    for (int k = 4; k >= 0; k--)
+      if ((rc = launch_ring_pairs(h, h->s0, gate, k))) return rc;
     CK(cudaEventRecord(h->ev[5], h->s0));
     CK(cudaEventRecord(h->ev[8], h->s0));
     if ((rc = launch_assemble_fused(h, h->s0, gate))) return rc;
@@ -2124,17 +2277,22 @@ int enqueue_fused_iteration(ccdgpu_handle *h, bool mixed) {
     CK(cudaEventRecord(h->ev[7], h->s0));
     return CCDGPU_OK;
   }
+  // Branches in the reverse of the order in which their kernels should be placed: of the branches
+  // of a graph that become ready together, the one captured last is launched first.
   CK(cudaEventRecord(h->ev_fork, h->s0));
-  CK(cudaStreamWaitEvent(h->s1, h->ev_fork, 0));
-  CK(cudaStreamWaitEvent(h->s2, h->ev_fork, 0));
-  if ((rc = ladder(h->s0))) return rc;
-  if ((rc = launch_ring(h, h->s1, gate, true))) return rc;
-  CK(cudaEventRecord(h->ev_join, h->s1));
+  for (int k = 1; k < kStreams; k++) CK(cudaStreamWaitEvent(h->sset.s[k], h->ev_fork, 0));
   if ((rc = launch_hh_ladder(h, h->s2, gate))) return rc;
   if ((rc = launch_onebody_fused(h, h->s2, gate))) return rc;
-  CK(cudaEventRecord(h->ev_join2, h->s2));
-  CK(cudaStreamWaitEvent(h->s0, h->ev_join, 0));
-  CK(cudaStreamWaitEvent(h->s0, h->ev_join2, 0));
+  if ((rc = launch_ring_pairs(h, h->sset.s[5], gate, 0))) return rc;
+  if ((rc = launch_ring_pairs(h, h->sset.s[4], gate, 1))) return rc;
+  if ((rc = launch_ring_pairs(h, h->s3, gate, 2))) return rc;
+  for (int k = 4; k >= 3; k--)
+    if ((rc = launch_ring_pairs(h, h->s1, gate, k))) return rc;
+  if ((rc = ladder(h->s0))) return rc;
+  for (int k = 1; k < kStreams; k++) {
+    CK(cudaEventRecord(h->sset.ev[kJoin0 + k], h->sset.s[k]));
+    CK(cudaStreamWaitEvent(h->s0, h->sset.ev[kJoin0 + k], 0));
+  }
   if ((rc = launch_assemble_fused(h, h->s0, gate))) return rc;  // + energy and stop rule
   if (h->loop_capture && !h->n_asm_blocks) {  // else the assembly set the loop condition
     h->launches++;
@@ -2340,7 +2498,7 @@ int tables_iteration(ccdgpu_handle *h, double mixing, double *corr) {
   int rc;
   if ((rc = stage_onebody_tables(h, 0, 1))) return rc;     // calcT2Diff_p2_p1hh
   if ((rc = stage_onebody_tables(h, 1, 0))) return rc;     // calcT2Diff_h2pp_h1
-  if ((rc = launch_ring(h, h->s0, 0, false))) return rc;   // calcT2Diff_phhp
+  if ((rc = launch_ring(h, h->s0, 0))) return rc;   // calcT2Diff_phhp
   if ((rc = launch_hh_ladder(h, h->s0, 0))) return rc;     // calcT2Diff_pphh
   if ((rc = launch_pp_ladder(h, h->s0))) return rc;
   if ((rc = launch_expand_d(h, false, 0))) return rc;
@@ -2412,9 +2570,7 @@ int ccdgpu_create(const ccdgpu_problem *prob, const ccdgpu_options *opt, ccdgpu_
   if (!rc) {
     h->s0 = h->sset.s[0]; h->s1 = h->sset.s[1]; h->s2 = h->sset.s[2]; h->s3 = h->sset.s[3];
     for (int i = 0; i < 10; i++) h->ev[i] = h->sset.ev[i];
-    h->ev_fork = h->sset.ev[10]; h->ev_join = h->sset.ev[11];
-    h->ev_fork2 = h->sset.ev[12]; h->ev_join2 = h->sset.ev[13];
-    h->ev_fork3 = h->sset.ev[14]; h->ev_join3 = h->sset.ev[15];
+    h->ev_fork = h->sset.ev[10]; h->ev_fork2 = h->sset.ev[11];
   }
   if (!rc) rc = build(h, prob);
   if (!rc) rc = init_ctl(h);
@@ -2877,7 +3033,7 @@ int ccdgpu_calc_t2diff_h2pp_h1(ccdgpu_handle *h) {
 int ccdgpu_calc_t2diff_phhp(ccdgpu_handle *h) {
   if (!h) return CCDGPU_ERR_INVALID_ARGUMENT;
   int rc = set_ctl(h, 0, h->h_ctl->tol, h->h_ctl->max_iters, h->h_ctl->mixing, false);
-  if (rc || (rc = launch_ring(h, h->s0, 0, false))) return rc;
+  if (rc || (rc = launch_ring(h, h->s0, 0))) return rc;
   CK(cudaStreamSynchronize(h->s0));
   return CCDGPU_OK;
 }
@@ -2944,9 +3100,8 @@ int ccdgpu_read_chain(ccdgpu_handle *h, int32_t chain, double *out, uint64_t n, 
   if (!src) return CCDGPU_ERR_UNSUPPORTED;
   if (n < len) return CCDGPU_ERR_INVALID_ARGUMENT;
   if (chain == CCDGPU_CHAIN_OLD_PHHP && h->opt.path != CCDGPU_PATH_TABLES) {
-    // The fused path gathers the slab at the head of each iteration's ring: bring it up to
-    // the current amplitudes first.
-    if ((rc = launch_phhp_gather(h, h->s0, -1))) return rc;
+    // The fused path's iterations do not keep this slab.
+    if ((rc = launch_phhp_gather(h, h->s0))) return rc;
     CK(cudaStreamSynchronize(h->s0));
   }
   if (chain == CCDGPU_CHAIN_DIFF_PPHH && (rc = materialize_d(h))) return rc;
@@ -2990,17 +3145,14 @@ int ccdgpu_kernel_profile(ccdgpu_handle *h, int32_t reps, double *ms, double *fl
   if (rc) return rc;
   if ((rc = materialize_d(h))) return rc;  // the kernels overwrite what it is expanded from
   for (int k = 0; k < 7; k++) ms[k] = flops[k] = bytes[k] = 0;
-  // Ring: Y = V_hphp + 0.5 V_hpph T' and R = T' Y; reads T', V_hpph, V_hphp and where R goes,
-  // writes R.
-  for (const ModInfo &m : h->host_mods) {
-    const int k = (m.ph <= kRingSmall && m.hp <= kRingSmall) ? 0
-                  : (m.ph <= 32 && m.hp <= 32) ? 1 : 2;
-    flops[k] += 4.0 * m.ph * (double)m.hp * m.hp;
-    bytes[k] += 28.0 * m.ph * m.hp + 8.0 * m.hp * m.hp;
+  // Ring (fused path): S = T' (A + C T') + B T' per pair of channels; reads A, B, C, the
+  // destinations and the amplitudes they name, writes S.
+  for (const RingPair &m : h->host_pairs) {
+    const int w = std::max(m.ph, m.hp), k = w <= kRingSmall ? 0 : w <= 32 ? 1 : 2;
+    const double n = (double)m.ph * m.hp;
+    flops[k] += 2.0 * n * (2.0 * m.hp + m.ph);
+    bytes[k] += 28.0 * n + 8.0 * ((double)m.hp * m.hp + (double)m.ph * m.ph);
   }
-  // The small class is launched with the phhp gather ahead of it (fused path): per slab
-  // element an index, one read of t and the slab store.
-  bytes[0] += 20.0 * (double)h->n_m;
   // hh ladder: P = V_hhpp T over the packed rows and r = row dots; reads packed V and T, writes
   // the slice partials of P and r.  Reduction: reads the partials and V_hhhh, writes X and s.
   for (const ChanInfo &a : h->host_chans) {
@@ -3016,7 +3168,12 @@ int ccdgpu_kernel_profile(ccdgpu_handle *h, int32_t reps, double *ms, double *fl
   bytes[5] = 16.0 * (double)(h->nsp) + 12.0 * (double)h->n_list;
   for (int k = 0; k < 7; k++) {
     auto launch = [&]() -> int {
-      if (k <= 2) return launch_ring(h, h->s0, 0, true, k);
+      if (k <= 1) return launch_ring_pairs(h, h->s0, 0, k);
+      if (k == 2) {
+        for (int q = 4; q >= 2; q--)
+          if (const int r = launch_ring_pairs(h, h->s0, 0, q)) return r;
+        return CCDGPU_OK;
+      }
       if (k <= 4) return launch_hh_ladder(h, h->s0, 0, k - 3);
       if (k == 6) return launch_hh_ladder(h, h->s0, 0, 2);
       return launch_onebody_fused(h, h->s0, 0);
