@@ -26,7 +26,7 @@ namespace ccd {
 //     load fall on distinct banks.
 // The last row tile of a channel is stored compact (only its real rows, rounded up to 8).
 constexpr int kBK = 16;        // K depth of one pipeline stage
-constexpr int kStages = 4;     // bulk-copy pipeline depth (68-86 KB in flight per SM)
+constexpr int kStages = 5;     // bulk-copy pipeline depth (68-86 KB in flight per SM)
 constexpr int kMaxHH = 72;     // hole pairs of a channel (ordered)
 constexpr int kMaxCG = 5;      // column groups of 8 strict hole pairs (hk <= 36)
 constexpr int kLadderConsumers = 256;                  // 8 warps of 16 rows
@@ -214,22 +214,20 @@ struct ModInfo {
 };
 
 // Fused-path ring: a modified channel and its transpose (the channel of the exchanged pairs),
-// worked on in the layout of the first.
+// worked on in the layout of the first.  Set-up data of its operand images.
 struct RingPair {
   int32_t ph, hp;
-  int32_t perm_off, self;  // image set-up: hp' index in the transpose of each ph' pair; self: the
-                           // channel is its own transpose
+  int32_t perm_off, self;  // hp' index in the transpose of each ph' pair; self: the channel is its
+                           // own transpose
   int64_t m_off;   // phhp block of the channel (V_hpph, quads of its elements)
   int64_t a_off;   // A: V_hphp of the channel (hp' x hp')
   int64_t b_src;   // V_hphp of the transpose (ph' x ph' in its order), the source of B
-  int64_t dst_off; // ph' x hp' destinations (ring_pair_dst)
-  // Operand images (small pairs: B alone, ph' x ph') and destinations in fragment order.
-  int64_t a_img, b_img, c_img, to_img;
+  int64_t tp, a_img, b_img, c_img, to_img;  // T' image; operands and destinations
 };
-// A pair and column tiles [n0, n0 + nt) of its S, with what a CTA needs of the pair.
+// A pair and column tiles [n0, n0 + nt) of its S, with what its warps need of the pair.
 struct RingUnit {
   int32_t ph, hp, n0, nt;
-  int64_t dst_off, a_img, b_img, c_img, to_img;
+  int64_t tp, a_img, b_img, c_img, to_img;
 };
 
 // Contiguous element range [e0, e1) of one channel for the element-wise kernels.

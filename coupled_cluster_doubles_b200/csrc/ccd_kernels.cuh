@@ -3,10 +3,11 @@
 // Reference correspondence (calc.cpp / Chain.hpp of justinlietz/coupled_cluster_doubles):
 //   pp_ladder_kernel        V_pppp T part of D = 0.5 T X + 0.5 V T   calc.cpp:162-202
 //                           (antisymmetry-packed; the assembly adds T X)
-//   hh_ladder_kernel        X = V_hhhh + 0.5 V_hhpp T                calc.cpp:141-160
-//   ring_*_kernel           Y = V_hphp + 0.5 V_hpph T'; R = T' Y     calc.cpp:264-313
+//   hh_slice_kernel         X = V_hhhh + 0.5 V_hhpp T                calc.cpp:141-160
+//   ring_pair_kernel        the same as ring_* for the fused path
+//   hh_post_kernel          the same dot products, read from the ladder intermediates, and T X
+//   ring_small, ring16      Y = V_hphp + 0.5 V_hpph T'; R = T' Y     calc.cpp:264-313
 //   onebody_tables_kernel   calcChannelT2Diff_h2pp_h1 / _p2_p1hh     calc.cpp:9-25, 73-89
-//   onebody_fused_kernel    the same dot products, read from the ladder intermediates
 //   gather8_kernel          Chain::mapFromDistributed x 8            Chain.hpp:710-755
 //   assemble_*_kernel       calcChannelT2_pphh                       calc.cpp:368-421
 //   map_to_kernel           Chain::set + mapToDistributed x 5        Chain.hpp:503-527,757-802
@@ -234,8 +235,8 @@ constexpr size_t kLadderSmem =
     (size_t)kStages * (kMaxAS * kBK + kBK * kMaxNB) * 8 + kStages * sizeof(StageInfo) +
     2 * kStages * 8 + kBK * 8;  // slack: the last B stage's fragment loads past hs
 // 80 registers: its nine warps then leave 8,704 registers of the fullest SM quarter (three ladder
-// warps), two warps of the ring's 64 group; at 94 no ring CTA of 8 warps fitted beside it and
-// the ring ran after the ladder.
+// warps) to the kernels beside it; at 94 a CTA of 8 warps of the ring did not fit and ran after
+// the ladder.
 __global__ void __maxnreg__(80)
 pp_ladder_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *sched,
                  const double *__restrict__ v_t, const double *tq0, const double *tq1,
@@ -374,23 +375,20 @@ __device__ __forceinline__ void cp_async_wait() {
 //   s[ij] = P[ij][ij],  r[u] = sum_ij V[u, ij] T[u, ij],
 // a quarter of the reads and an eighth of the products of the ordered pairs.  V_hhpp is held in
 // the packed layout of T, so a K slice of either is one contiguous range.
-// hh_ladder_kernel: CTAs of two kinds in one launch.
+// hh_slice_kernel: units of two kinds in one launch.
 //   hk <= 8: a warp per slice of kHHRows rows, its m8n8k4 fragments loaded straight from global
 //   memory (8 consecutive columns of 4 rows a load, all loads of the slice in flight at once);
-//   wider: a CTA per slice of kHHRowsL rows, both ranges copied to shared memory (16-byte
-//   cp.async; the row stride hs is 4 mod 8 doubles, conflict-free for the fragments) and P on
-//   m16n8k16, warp w taking items of one 16-row tile by kHHNC 8-column tiles.
-// Both form the row dots r, and write the slice's partial P, which hh_reduce_kernel adds in
-// slice order (deterministic).  Bound by latency: 12 MB of operands at EG N=54 |n|^2 <= 36,
-// where the ordered pairs' 47 MB and hh^2 outputs took 15 + 19 us.
+//   wider: a CTA per slice, both ranges copied to shared memory (16-byte cp.async; the row stride
+//   hs is 4 mod 8 doubles, conflict-free for the fragments) and P on m16n8k16, warp w taking items
+//   of one 16-row tile by kHHNC 8-column tiles.
+// Both form the row dots r, and write the slice's partial P, which hh_reduce_kernel adds in slice order
+// (deterministic).
 // ------------------------------------------------------------------------------------------
-constexpr int kHHRows = 32;       // packed rows of a warp's slice (hk <= 8)
-constexpr int kHHRowsL = 32;      // ... of a CTA's slice
-constexpr int kHHThreads = 256;
+constexpr int kHHThreads = 128;
+constexpr int kHHRows = 32;  // packed rows of a slice
 constexpr int kHHNC = 2;
-__host__ __device__ inline int hh_rows(int hk) { return hk <= 8 ? kHHRows : kHHRowsL; }
 // Slack: fragment loads of the rows and columns past hk in the last row.
-constexpr size_t kHHSmem = (2 * (size_t)kHHRowsL * kMaxNB + 16) * sizeof(double);
+constexpr size_t kHHSmem = (2 * (size_t)kHHRows * kMaxNB + 16) * sizeof(double);
 
 __device__ __forceinline__ void hh_warp_unit(const HHTile &tt, const ChanInfo &ch,
                                              const double *__restrict__ vq, const double *tq,
@@ -477,16 +475,16 @@ __device__ __forceinline__ void hh_cta_unit(const HHTile &tt, const ChanInfo &ch
 }
 
 // Units [0, n_cta) one per CTA, then n_warp units, one per warp of the following CTAs.
-__global__ void __launch_bounds__(kHHThreads, 4)
-hh_ladder_kernel(const HHTile *__restrict__ tiles, int n_cta, int n_warp,
-                 const ChanInfo *__restrict__ chans, const double *__restrict__ vq,
-                 const double *tq0, const double *tq1, double *__restrict__ part,
-                 const int64_t *__restrict__ part_off, double *__restrict__ r_out,
-                 const Control *ctl, int gate) {
-  const int tr = (int)blockIdx.x < n_cta ? kTrHHTiled : kTrHHSmall;
+__global__ void __launch_bounds__(kHHThreads, 8)
+hh_slice_kernel(const HHTile *__restrict__ tiles, int n_cta, int n_warp,
+                const ChanInfo *__restrict__ chans, const double *__restrict__ vq,
+                const double *tq0, const double *tq1, double *__restrict__ part,
+                const int64_t *__restrict__ part_off, double *__restrict__ r_out,
+                const Control *ctl, int gate) {
+  const bool wide = (int)blockIdx.x < n_cta;
+  const int tr = wide ? kTrHHTiled : kTrHHSmall;
   if (skip_iteration(ctl, gate, tr)) return;
   extern __shared__ __align__(16) double hh_smem[];
-  const bool wide = (int)blockIdx.x < n_cta;
   const int w = ((int)blockIdx.x - n_cta) * (kHHThreads / 32) + (int)(threadIdx.x >> 5);
   if (!wide && w >= n_warp) return;
   const HHTile tt = tiles[wide ? (int)blockIdx.x : n_cta + w];
@@ -545,8 +543,7 @@ hh_reduce_kernel(const HHOut *__restrict__ outs, int n, const double *__restrict
 //   S[ai, jb] = R[ai, jb] + R[bj, ia] = T' (A + C T') + B T'
 // with A = V_hphp of the first channel, C = V_hpph (the same block for both, by the exchange of
 // both pairs) and B[ai, ck] = V_hphp[(k c), (i a)] of the second: three products instead of four
-// and half of the amplitudes, of V_hpph and of the results.  T' comes straight from the packed
-// amplitudes and S goes straight to the quad's two terms, both through dst.
+// and half of the amplitudes, of V_hpph and of the results (ring_unit, below).
 // ------------------------------------------------------------------------------------------
 constexpr int kRingSmall = 16;
 constexpr int kRingMax = 80;  // largest ph', hp'
@@ -797,147 +794,24 @@ ring16_kernel(const ModInfo *__restrict__ mods, const double *__restrict__ v_hpp
 }
 
 // ---- Fused path: a channel and its transpose together ------------------------------------
-constexpr int32_t kRingNoStore = 1 << 30;  // ring_pair_dst: read only (the mirror stores)
-// The amplitude behind a destination in two steps, the load unconditional (position 0 for -1) and
-// the sign and the zeros afterwards: a load under a branch on d would leave one in flight.
-__device__ __forceinline__ double pair_load(const double *__restrict__ tq, int32_t d) {
-  return __ldcg(tq + (d < 0 ? 0 : (d & (kRingNoStore - 1)) >> 1));
-}
-__device__ __forceinline__ double pair_sign(double t, int32_t d) {
-  return d < 0 ? 0.0 : (d & 1) ? -t : t;
-}
-__device__ __forceinline__ void pair_store(double *out, int32_t d, double v) {
-  if (d >= 0 && !(d & kRingNoStore)) out[d] = v;
-}
-
-// ph', hp' <= kRingSmall: one pair per warp on m8n8k4, stages padded to 8 or 16 with zeros (row
-// stride 20 doubles), every load of the warp in flight at once.  Y replaces C once it is done
-// with.
-__global__ void __launch_bounds__(kRingSmallWarps * 32)
-ring_pair_small_kernel(const RingPair *__restrict__ pairs, int n,
-                       const double *__restrict__ v_hpph, const double *__restrict__ v_hphp,
-                       const double *__restrict__ img, const int32_t *__restrict__ dst,
-                       const double *tq0, const double *tq1, double *__restrict__ out,
-                       const Control *ctl, int gate) {
-  if (skip_iteration(ctl, gate, kTrRingSmall)) return;
-  constexpr int ld = kRingSmallLd, kPer = kRingSmall * kRingSmall / 32;
-  __shared__ __align__(16) double buf[kRingSmallWarps][3 * kRingSmall * ld];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int mi = blockIdx.x * kRingSmallWarps + w;
-  if (mi >= n) return;  // whole warps: the MMAs below are warp-collective
-  const RingPair m = pairs[mi];
-  const double *tq = ctl->parity ? tq1 : tq0;
-  const int ph = m.ph, hp = m.hp, P = ring_pad8(ph), H = ring_pad8(hp);
-  const int hs = H == 8 ? 3 : 4, ps = P == 8 ? 3 : 4;  // log2
-  double *Ts = buf[w], *Cs = Ts + kRingSmall * ld, *Bs = Cs + kRingSmall * ld;
-  const int32_t *dp = dst + m.dst_off;
-  int32_t idx[kPer];
-#pragma unroll
-  for (int j = 0; j < kPer; ++j) {
-    const int e = lane + 32 * j, r = e >> hs, c = e & (H - 1);
-    idx[j] = e < P * H && r < ph && c < hp ? __ldg(dp + r * hp + c) : -1;
-  }
-  for (int e = lane; e < P * H; e += 32) {
-    const int r = e >> hs, c = e & (H - 1);
-    if (r < ph && c < hp) cp_async8(Cs + r * ld + c, v_hpph + m.m_off + r * hp + c);
-    else Cs[r * ld + c] = 0.0;
-  }
-  for (int e = lane; e < P * P; e += 32) {
-    const int r = e >> ps, c = e & (P - 1);
-    if (r < ph && c < ph) cp_async8(Bs + r * ld + c, img + m.b_img + r * ph + c);
-    else Bs[r * ld + c] = 0.0;
-  }
-  cp_async_commit();
-  double y[2][2][2];  // Y = A + C T', starting from A
-#pragma unroll
-  for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-    for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const int r = 8 * mt + g, c = 8 * nt + 2 * t + q;
-        y[mt][nt][q] = r < hp && c < hp ? __ldg(v_hphp + m.a_off + r * hp + c) : 0.0;
-      }
-  double tv[kPer];
-#pragma unroll
-  for (int j = 0; j < kPer; ++j) tv[j] = pair_load(tq, idx[j]);
-#pragma unroll
-  for (int j = 0; j < kPer; ++j) {
-    const int e = lane + 32 * j;
-    if (e < P * H) Ts[(e >> hs) * ld + (e & (H - 1))] = pair_sign(tv[j], idx[j]);
-  }
-  cp_async_wait<0>();
-  __syncwarp();
-#pragma unroll 2
-  for (int k = 0; k < P; k += 4) {
-    double a[2], b[2];
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      a[q] = 8 * q < H ? Cs[(k + t) * ld + 8 * q + g] : 0.0;
-      b[q] = 8 * q < H ? Ts[(k + t) * ld + 8 * q + g] : 0.0;
-    }
-#pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt)
-        if (8 * mt < H && 8 * nt < H) dmma_884(y[mt][nt], a[mt], b[nt]);
-  }
-  __syncwarp();
-#pragma unroll
-  for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-    for (int nt = 0; nt < 2; ++nt)
-      if (8 * mt < H && 8 * nt < H)
-#pragma unroll
-        for (int q = 0; q < 2; ++q) Cs[(8 * mt + g) * ld + 8 * nt + 2 * t + q] = y[mt][nt][q];
-  __syncwarp();
-  // S = T' Y + B T'.
-  double s[2][2][2] = {};
-  auto gemm = [&](const double *A, const double *B, int K) {
-#pragma unroll 2
-    for (int k = 0; k < K; k += 4) {
-      double a[2], b[2];
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        a[q] = 8 * q < P ? A[(8 * q + g) * ld + k + t] : 0.0;
-        b[q] = 8 * q < H ? B[(k + t) * ld + 8 * q + g] : 0.0;
-      }
-#pragma unroll
-      for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt)
-          if (8 * mt < P && 8 * nt < H) dmma_884(s[mt][nt], a[mt], b[nt]);
-    }
-  };
-  gemm(Ts, Cs, H);
-  gemm(Bs, Ts, P);
-#pragma unroll
-  for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-    for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const int r = 8 * mt + g, c = 8 * nt + 2 * t + q;
-        if (r < ph && c < hp) pair_store(out, __ldg(dp + r * hp + c), s[mt][nt][q]);
-      }
-  trace_end(ctl, kTrRingSmall);
-}
-
-// Larger pairs on m16n8k16: units of one pair and a block of up to kPairNC 8-column tiles of S
-// (columns of Y and S depend on the same columns of T' alone, so blocks share no product), one
-// CTA each, warp w on the rows [16 w, 16 w + 16) of Y and S.  A, B, C and the destinations are
-// stored in the order in which the lanes of a fragment take them, so every load of them is a
-// 16-byte one, contiguous over the warp, straight into registers; shared memory holds T' (the B
-// operand of both first products and the A operand of the last) and Y.  S starts with B T', which
-// needs no Y, so Y's store and barrier hide behind it.
-// Why: a CTA per pair with staged operands kept its SM's L1 pipe 80 % busy (scalar operand loads,
-// staging, random reads and stores) in phases that did not overlap the MMAs, at two CTAs of 114
-// registers and 104 KB per SM, and one (or none, at 80 columns) beside the ladder.
+// Units of one pair and a block of up to kPairNC 8-column tiles of S (columns of Y and S depend on
+// the same columns of T' alone, so blocks share no product), on m16n8k16, by G = 1, 2 or 4 warps
+// (ph', hp' <= 16, 32, 80), warp w on row tiles w, w + G, ...
+// A, B, C and the destinations are stored in the order in which the lanes of a fragment take them,
+// so every load of them is a 16-byte one, contiguous over the warp, straight into registers.  T'
+// arrives as a stored shared-memory image (16-row, 16-column padding, row stride H16 + 4) by one
+// bulk copy: a random 8-byte read of an amplitude costs the L2 a whole sector, and made by every
+// column block they were half of the ring's time (61 -> 36 us without them at EG N=54
+// |n|^2 <= 36), so tp_gather_kernel reads each amplitude once and writes the images.
 constexpr int kPairNC = 4;
 __host__ __device__ inline int pad16(int n) { return (n + 15) & ~15; }
-__host__ __device__ constexpr int pair_ldy() { return 8 * kPairNC + 4; }  // 4 mod 8 doubles
-__host__ __device__ constexpr size_t ring_pair_smem(int mt) {
-  return (size_t)16 * mt * (16 * mt + 4 + pair_ldy()) * sizeof(double);
+__host__ __device__ inline int ring_group(int ph, int hp) {
+  return (ph > hp ? ph : hp) <= 16 ? 1 : (ph > hp ? ph : hp) <= 32 ? 2 : 4;
+}
+// T' image and Y of a unit (doubles); Y's row stride is 4 mod 8 doubles too.
+__host__ __device__ constexpr int ring_ldy(int g) { return g == 1 ? 20 : 8 * kPairNC + 4; }
+__host__ __device__ constexpr int ring_unit_smem(int g, int p, int h) {
+  return p * (h + 4) + h * ring_ldy(g);
 }
 // Fragment-ordered A operand: [16-row tile][16-deep step][4][lane][2].
 __device__ __forceinline__ void frag_load(double (&a)[8], const double *__restrict__ p) {
@@ -956,129 +830,104 @@ __device__ __forceinline__ void frag_start(double (&f)[2][8], const double *__re
   frag_load(f[0], frag);
   if (K > 16) frag_load(f[1], frag + 256);
 }
-__device__ __forceinline__ void frag_gemm(double (&acc)[kPairNC][4], double (&f)[2][8],
-                                          const double *__restrict__ frag, const double *Bs,
-                                          int ldb, int nt, int K) {
+template <int NC>
+__device__ __forceinline__ void mma_row(double (&acc)[NC][4], const double (&a)[8],
+                                        const double *Bs, int ldb, int nt, int k0) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  auto step = [&](double (&a)[8], int k0) {
 #pragma unroll
-    for (int n = 0; n < kPairNC; ++n) {
-      if (n >= nt) break;
-      double b[4];
+  for (int n = 0; n < NC; ++n) {
+    if (n >= nt) break;
+    double b[4];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) b[q] = Bs[(k0 + t + 4 * q) * ldb + 8 * n + g];
-      dmma_16816(acc[n], a, b);
-    }
-    if (k0 + 32 < K) frag_load(a, frag + (k0 + 32) * 16);
-  };
-  for (int k0 = 0; k0 < K; k0 += 32) {
-    step(f[0], k0);
-    if (k0 + 16 < K) step(f[1], k0 + 16);
+    for (int q = 0; q < 4; ++q) b[q] = Bs[(k0 + t + 4 * q) * ldb + 8 * n + g];
+    dmma_16816(acc[n], a, b);
   }
 }
-template <int MT>
-__global__ void __launch_bounds__(32 * MT, 8 - MT)
-ring_pair_kernel(const RingUnit *__restrict__ units, const double *__restrict__ img,
-                 const int32_t *__restrict__ dst,
-                 const int32_t *__restrict__ to_img, const double *tq0, const double *tq1,
-                 double *__restrict__ out, const Control *ctl, int gate) {
-  constexpr int kTr = MT <= 2 ? kTrRingMid : kTrRingLarge;
-  if (skip_iteration(ctl, gate, kTr)) return;
-  extern __shared__ __align__(16) double rp_smem[];
-  const RingUnit m = units[blockIdx.x];
-  const double *tq = ctl->parity ? tq1 : tq0;
-  const int ph = m.ph, hp = m.hp, P = pad16(ph), H = pad16(hp), ldh = H + 4;
-  constexpr int ldy = pair_ldy();
-  double *Ts = rp_smem, *Ys = rp_smem + P * ldh;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int n8 = (hp + 7) >> 3, nt = m.nt;
-  const bool yrow = 16 * warp < H, srow = 16 * warp < P;
-  const double *c_frag = img + m.c_img + (int64_t)warp * P * 16;
-  const double *b_frag = img + m.b_img + (int64_t)warp * P * 16;
-  // T': rows warp, warp + MT, ..., lanes over the columns; index, then amplitude, eight rows'
-  // in flight together.  Behind the first indices: the loads that need nothing, C's first steps
-  // and A (where Y starts).
-  constexpr int COLS = (16 * MT + 31) / 32;
-  const int32_t *dp = dst + m.dst_off;
-  int32_t idx[2][8][COLS];
-#pragma unroll
-  for (int h = 0; h < 2; ++h)
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-      for (int j = 0; j < COLS; ++j) {
-        const int r = warp + MT * (8 * h + i), c = lane + 32 * j;
-        idx[h][i][j] = r < ph && c < hp ? __ldg(dp + r * hp + c) : -1;
-      }
-  double f[2][8], acc[kPairNC][4];
-  if (yrow) {
+template <int NC>
+__device__ __forceinline__ void frag_gemm(double (&acc)[NC][4], double (&f)[2][8],
+                                          const double *__restrict__ frag, const double *Bs,
+                                          int ldb, int nt, int K) {
+  for (int k0 = 0; k0 < K; k0 += 32) {
+    mma_row(acc, f[0], Bs, ldb, nt, k0);
+    if (k0 + 32 < K) frag_load(f[0], frag + (k0 + 32) * 16);
+    if (k0 + 16 < K) {
+      mma_row(acc, f[1], Bs, ldb, nt, k0 + 16);
+      if (k0 + 48 < K) frag_load(f[1], frag + (k0 + 48) * 16);
+    }
+  }
+}
+template <int G>
+__device__ __forceinline__ void group_sync() {
+  if constexpr (G == 1) __syncwarp();
+  else if constexpr (G == 2)
+    asm volatile("bar.sync %0, 64;" ::"r"(1 + (int)(threadIdx.x >> 6)) : "memory");
+  else __syncthreads();
+}
+template <int G>
+__device__ __forceinline__ void ring_unit(const RingUnit &m, const double *__restrict__ img,
+                                          const int32_t *__restrict__ to_img, const double *tp,
+                                          double *__restrict__ out, double *sm, uint32_t bar,
+                                          uint32_t parity, int32_t *err) {
+  constexpr int NC = G == 1 ? 2 : kPairNC, ldy = ring_ldy(G);
+  const int P = pad16(m.ph), H = pad16(m.hp), ldh = H + 4, n8 = (m.hp + 7) >> 3, nt = m.nt;
+  const int w = (threadIdx.x >> 5) % G, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  double *Ts = sm, *Ys = sm + P * ldh;
+  if (w == 0 && lane == 0) {
+    mbar_expect_tx(bar, P * ldh * 8);
+    bulk_g2s(smem_u32(Ts), tp + m.tp, P * ldh * 8, bar);
+  }
+  const double *Tj = Ts + 8 * m.n0;  // this unit's columns of T'
+  bool landed = false;
+  auto wait = [&]() {
+    if (!landed && !mbar_wait(bar, parity)) atomicOr(err, kErrTimeout);
+    landed = true;
+  };
+  double f[2][8], acc[NC][4];
+  for (int mt = w; 16 * mt < H; mt += G) {  // Y = A + C T'
+    const double *c_frag = img + m.c_img + (int64_t)mt * P * 16;
     frag_start(f, c_frag, P);
-    const double2 *ap = reinterpret_cast<const double2 *>(img + m.a_img) +
-                        ((int64_t)warp * n8 + m.n0) * 64 + lane;
+    const double2 *ap =
+        reinterpret_cast<const double2 *>(img + m.a_img) + ((int64_t)mt * n8 + m.n0) * 64 + lane;
 #pragma unroll
-    for (int n = 0; n < kPairNC; ++n)
+    for (int n = 0; n < NC; ++n)
       if (n < nt) {
         const double2 lo = __ldg(ap + 64 * n), hi = __ldg(ap + 64 * n + 32);
         acc[n][0] = lo.x; acc[n][1] = lo.y; acc[n][2] = hi.x; acc[n][3] = hi.y;
       }
-  }
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    double tv[8][COLS];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-      for (int j = 0; j < COLS; ++j) tv[i][j] = pair_load(tq, idx[h][i][j]);
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-      for (int j = 0; j < COLS; ++j) {
-        const int r = warp + MT * (8 * h + i), c = lane + 32 * j;
-        if (r < P && c < H) Ts[r * ldh + c] = pair_sign(tv[i][j], idx[h][i][j]);
-      }
-  }
-  __syncthreads();
-  const double *Tj = Ts + 8 * m.n0;  // this unit's columns of T'
-  if (yrow) {  // Y = A + C T'
+    wait();
     frag_gemm(acc, f, c_frag, Tj, ldh, nt, P);
-    if (srow) frag_start(f, b_frag, P);
 #pragma unroll
-    for (int n = 0; n < kPairNC; ++n)
+    for (int n = 0; n < NC; ++n)
       if (n < nt)
 #pragma unroll
         for (int q = 0; q < 4; ++q)
-          Ys[(16 * warp + g + 8 * (q >> 1)) * ldy + 8 * n + 2 * t + (q & 1)] = acc[n][q];
+          Ys[(16 * mt + g + 8 * (q >> 1)) * ldy + 8 * n + 2 * t + (q & 1)] = acc[n][q];
   }
+  const double *b_frag = img + m.b_img;
+  if (16 * w < P) frag_start(f, b_frag + (int64_t)w * P * 16, P);
+  wait();
+  group_sync<G>();
+  for (int mt = w; 16 * mt < P; mt += G) {  // S = B T' + T' Y, to the quads
+    const double *bf = b_frag + (int64_t)mt * P * 16;
+    if (mt != w) frag_start(f, bf, P);
 #pragma unroll
-  for (int n = 0; n < kPairNC; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.0;
-  int4 to[kPairNC];
-  if (srow) {  // S = B T' ...
-    if (!yrow) frag_start(f, b_frag, P);
-    frag_gemm(acc, f, b_frag, Tj, ldh, nt, P);
-    const int4 *tp = reinterpret_cast<const int4 *>(to_img + m.to_img) +
-                     ((int64_t)warp * n8 + m.n0) * 32 + lane;
+    for (int n = 0; n < NC; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.0;
+    frag_gemm(acc, f, bf, Tj, ldh, nt, P);
+    const int4 *qp =
+        reinterpret_cast<const int4 *>(to_img + m.to_img) + ((int64_t)mt * n8 + m.n0) * 32 + lane;
+    int4 to[NC];
 #pragma unroll
-    for (int n = 0; n < kPairNC; ++n)
-      if (n < nt) to[n] = __ldg(tp + 32 * n);
-  }
-  __syncthreads();
-  if (srow) {  // ... + T' Y, to the quads
-    double a[8];
+    for (int n = 0; n < NC; ++n)
+      if (n < nt) to[n] = __ldg(qp + 32 * n);
     for (int k0 = 0; k0 < H; k0 += 16) {
+      double a[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i)
-        a[i] = Ts[(16 * warp + g + 8 * (i % 2)) * ldh + k0 + t + 4 * (i / 2)];
-#pragma unroll
-      for (int n = 0; n < kPairNC; ++n) {
-        if (n >= nt) break;
-        double b[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) b[q] = Ys[(k0 + t + 4 * q) * ldy + 8 * n + g];
-        dmma_16816(acc[n], a, b);
-      }
+        a[i] = Ts[(16 * mt + g + 8 * (i % 2)) * ldh + k0 + t + 4 * (i / 2)];
+      mma_row(acc, a, Ys, ldy, nt, k0);
     }
 #pragma unroll
-    for (int n = 0; n < kPairNC; ++n)
+    for (int n = 0; n < NC; ++n)
       if (n < nt) {
         if (to[n].x >= 0) out[to[n].x] = acc[n][0];
         if (to[n].y >= 0) out[to[n].y] = acc[n][1];
@@ -1086,7 +935,74 @@ ring_pair_kernel(const RingUnit *__restrict__ units, const double *__restrict__ 
         if (to[n].w >= 0) out[to[n].w] = acc[n][3];
       }
   }
+}
+
+template <int G>
+__global__ void __launch_bounds__(G == 2 ? 64 : 128, G == 2 ? 8 : 4)
+ring_pair_kernel(const RingUnit *__restrict__ units, int n, const double *__restrict__ img,
+                 const int32_t *__restrict__ to_img, const double *tp, double *__restrict__ out,
+                 const Control *ctl, int32_t *err, int gate) {
+  constexpr int kTr = G == 1 ? kTrRingSmall : G == 2 ? kTrRingMid : kTrRingLarge;
+  if (skip_iteration(ctl, gate, kTr)) return;
+  extern __shared__ __align__(128) double rp_smem[];
+  __shared__ uint64_t bars[G == 1 ? 4 : 1];
+  constexpr int kPer = G == 1 ? 4 : 1;  // units per CTA
+  const int sub = G == 1 ? threadIdx.x >> 5 : 0, u = blockIdx.x * kPer + sub;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kPer; ++i) mbar_init(smem_u32(&bars[i]), 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  if (u < n)
+    ring_unit<G>(units[u], img, to_img, tp, out, rp_smem + sub * ring_unit_smem(1, 16, 16),
+                 smem_u32(&bars[sub]), 0, err);
   trace_end(ctl, kTr);
+}
+
+// T' images: kGatherPer elements a thread, all their loads in flight together.  src: 2 x the packed
+// position, + 1 where the amplitude is negated; -1 for the padding and outside every quad.
+constexpr int kGatherThreads = 256;
+constexpr int kGatherPer = 8;
+__global__ void __launch_bounds__(kGatherThreads)
+tp_gather_kernel(const int32_t *__restrict__ src, int64_t n, const double *tq0, const double *tq1,
+                 double *__restrict__ tp, const Control *ctl, int gate) {
+  if (skip_iteration(ctl, gate, kTrGather)) return;
+  const double *__restrict__ tq = ctl->parity ? tq1 : tq0;
+  const int64_t p0 = ((int64_t)blockIdx.x * kGatherThreads * (kGatherPer / 4) + threadIdx.x) * 4;
+  int4 d[kGatherPer / 4];
+  double v[kGatherPer];
+  // A predicated load: a branch would leave one load in flight, and a common address for the
+  // elements outside every quad would queue a request per warp at one L2 slice.
+  auto pick = [&](int32_t k) {
+    double t;
+    asm("{ .reg .pred p; setp.ge.s32 p, %2, 0; mov.f64 %0, 0d0000000000000000; "
+        "@p ld.global.cg.f64 %0, [%1]; }"
+        : "=d"(t)
+        : "l"(tq + (k >> 1)), "r"(k));
+    return t;
+  };
+#pragma unroll
+  for (int j = 0; j < kGatherPer / 4; ++j) {
+    const int64_t p = p0 + (int64_t)j * 4 * kGatherThreads;
+    d[j] = p < n ? __ldg(reinterpret_cast<const int4 *>(src + p)) : make_int4(-1, -1, -1, -1);
+  }
+#pragma unroll
+  for (int j = 0; j < kGatherPer / 4; ++j) {
+    v[4 * j] = pick(d[j].x);
+    v[4 * j + 1] = pick(d[j].y);
+    v[4 * j + 2] = pick(d[j].z);
+    v[4 * j + 3] = pick(d[j].w);
+  }
+  auto sign = [](double t, int32_t k) { return (k & 1) ? -t : t; };
+#pragma unroll
+  for (int j = 0; j < kGatherPer / 4; ++j) {
+    const int64_t p = p0 + (int64_t)j * 4 * kGatherThreads;
+    if (p >= n) continue;
+    double2 *o = reinterpret_cast<double2 *>(tp + p);
+    o[0] = make_double2(sign(v[4 * j], d[j].x), sign(v[4 * j + 1], d[j].y));
+    o[1] = make_double2(sign(v[4 * j + 2], d[j].z), sign(v[4 * j + 3], d[j].w));
+  }
+  trace_end(ctl, kTrGather);
 }
 
 // Deterministic block reduction (fixed tree) of one double; result valid in thread 0.
@@ -1140,14 +1056,42 @@ onebody_tables_kernel(int np, const int64_t *__restrict__ o_h, const int64_t *__
   }
 }
 
-// Fused path: x_k and y_a as segmented sums of the hh ladder's by-products s and r over the
-// strict pairs that hold the orbital; twice, for the two orders of the summed pair.
-// One warp per orbital, lane-strided partial sums and a fixed shuffle tree.
-__global__ void onebody_fused_kernel(int np, int nsp, const int64_t *__restrict__ list_off,
-                                     const int32_t *__restrict__ list, const double *__restrict__ s,
-                                     const double *__restrict__ r, double *__restrict__ xh,
-                                     double *__restrict__ yp, const Control *ctl, int gate) {
+// What follows X and s, in one launch:
+// - x_k and y_a as segmented sums of the hh ladder's by-products s and r over the strict pairs that
+//   hold the orbital (twice, for the two orders of the summed pair), one warp per orbital (the
+//   first n_ob CTAs), lane-strided partial sums and a fixed shuffle tree;
+// - tx[u, w] = 0.5 T X = sum_{k<l} T[u, kl] X[kl, w], one thread per quad (CTAs n_ob + item): hk
+//   multiply-adds on operands that L1 holds (T's row is one broadcast per k).  Here it runs beside
+//   the ladder and the ring; in the assembly, which nothing overlaps, it took 6 of 34 us at EG N=54
+//   |n|^2 <= 36 (12 of 47 at PNM N=66) and the registers of a third of the resident threads.
+__device__ __forceinline__ double quad_tx(const double *__restrict__ t_row,
+                                          const double *__restrict__ x, int hk, int hs, int w) {
+  double tx = 0.0;
+#pragma unroll 4
+  for (int k = 0; k < hk; ++k) tx = fma(t_row[k], x[k * hs + w], tx);
+  return tx;
+}
+constexpr int kPostThreads = 256;
+__global__ void __launch_bounds__(kPostThreads)
+hh_post_kernel(int n_ob, int np, int nsp, const int64_t *__restrict__ list_off,
+               const int32_t *__restrict__ list, const double *__restrict__ s,
+               const double *__restrict__ r, double *__restrict__ xh, double *__restrict__ yp,
+               const QuadItem *__restrict__ items, const double *__restrict__ x,
+               const double *tq0, const double *tq1, double *__restrict__ tx, const Control *ctl,
+               int gate) {
   if (skip_iteration(ctl, gate, kTrOneBody)) return;
+  if ((int)blockIdx.x >= n_ob) {
+    const QuadItem item = items[blockIdx.x - n_ob];
+    const int q = item.q0 + threadIdx.x;
+    if (q < item.q1) {
+      const int u = q / item.hk, w = q - u * item.hk;
+      const double *t_row = (ctl->parity ? tq1 : tq0) + item.q_off + (int64_t)u * item.hs;
+      tx[item.q_off + (int64_t)u * item.hs + w] =
+          quad_tx(t_row, x + item.x_off, item.hk, item.hs, w);
+    }
+    trace_end(ctl, kTrOneBody);
+    return;
+  }
   const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (w >= nsp) return;
   const bool hole = w < np;
@@ -1199,9 +1143,8 @@ __device__ __forceinline__ void write_t_image(const ChanInfo &ch, int u, int w, 
 //         + 0.5 x_i t_ab,ji - 0.5 x_j t_ab,ij                       (h2pp_h1 gathers, algebraically)
 //         + (-0.5 y_b) t_ab,ij - (-0.5 y_a) t_ba,ij                 (p2_p1hh gathers, algebraically)
 //   t_new = mixing value/(e_i+e_j-e_a-e_b) + (1-mixing) t_old;  E += V t_new
-// with D = V_pppp T from the ladder's planes plus 0.5 T X = sum_{k<l} T[u, kl] X[kl, w], formed
-// here: hk multiply-adds per quad on operands that L1 holds (T's row is one broadcast per k),
-// instead of a K extension of the ladder that made it wait for the hh ladder.
+// with D = V_pppp T from the ladder's planes plus 0.5 T X from hh_post_kernel (a K extension of the
+// ladder for T X would make it wait for the hh ladder).
 // ------------------------------------------------------------------------------------------
 constexpr int kAsmThreads = 256;
 constexpr int kAsmPerThread = 2;  // table path: elements per thread of an ElemRange
@@ -1219,58 +1162,23 @@ __device__ __forceinline__ void loop_set_condition(const Control *ctl,
 }
 
 // Work is organised over quads (u, w); one thread computes one quad from V, D and t at its
-// packed position and the four ring terms, and writes the new packed amplitude (and, in a mixed
+// packed position and the two ring sums, and writes the new packed amplitude (and, in a mixed
 // iteration, its bf16 terms).  The energy gains 4 V t_new per quad.  Persistent CTAs stride over
-// work items of up to kQuadPerItem quads of one channel; a thread takes one quad of an item and
-// issues all its loads before the store.  EG N=54 |n|^2 <= 36: 48 bytes a quad against 136 when
-// the ordered pairs were kept (four amplitudes written, D and R read in their layout).
+// work items of up to kQuadPerItem quads of one channel.  Bound by the latency of three dependent
+// loads (item, table rows, operands), so by how many threads are resident.
 constexpr int kQuadPerItem = kAsmThreads;  // one quad per thread and item
-constexpr int kAsmCTAsPerSM = 3;
+constexpr int kAsmCTAsPerSM = 5;
+static_assert(kQuadPerItem == kPostThreads, "hh_post_kernel works on the same items");
 
-// One thread's quad of a work item.  ok = false: no quad (past the item or past the last item).
-struct QuadRef {
-  int32_t u, w, hk, hs, pa, pb, i, j, ch;
-  bool ok;
-  int64_t q_off, x_off;
-  double den;
-};
-__device__ __forceinline__ void quad_fetch(const QuadItem *__restrict__ items, int n_items,
-                                           const QuadRow *__restrict__ qrows,
-                                           const QuadCol *__restrict__ qcols, int it,
-                                           QuadRef &r) {
-  r.ok = false;
-  if (it >= n_items) return;
-  const QuadItem item = items[it];
-  const int q = item.q0 + threadIdx.x;
-  if (q >= item.q1) return;
-  // q / hk as a multiply-high by ceil(2^32 / hk) (Granlund-Montgomery): exact for
-  // q < 2^32 / hk (q < 2^21, hk < 2^11 here); hk = 1 has no 32-bit multiplier.
-  const int hk = item.hk;
-  const uint32_t magic = hk > 1 ? 0xFFFFFFFFu / (uint32_t)hk + 1u : 0u;
-  const int u = hk > 1 ? (int)__umulhi((uint32_t)q, magic) : q, w = q - u * hk;
-  const QuadRow rw = qrows[item.pk_off + u];
-  const QuadCol cl = qcols[item.qcol_off + w];
-  r.u = u; r.w = w; r.hk = hk; r.hs = item.hs;
-  r.pa = rw.pa; r.pb = rw.pb; r.i = cl.i; r.j = cl.j;
-  r.den = cl.eij - rw.ea - rw.eb;
-  r.ch = item.ch;
-  r.q_off = item.q_off;
-  r.x_off = item.x_off;
-  r.ok = true;
-}
-
-// D of quad (u, w): the ladder's planes in order, then T X.
+// D of quad position p of a channel: the ladder's planes in order, then T X.
 __device__ __forceinline__ double quad_d(const LadderChan &lc, const double *__restrict__ dp,
-                                         const double *__restrict__ t_row,
-                                         const double *__restrict__ x, int hk, int hs, int u,
-                                         int w) {
-  const double *p = dp + lc.base + (int64_t)u * hs + w;
-  double d = __ldcg(p);
-  for (int s = 1; s < lc.nseg; ++s) d += __ldcg(p + (int64_t)s * lc.plane);
-  double tx = 0.0;
-#pragma unroll 4
-  for (int k = 0; k < hk; ++k) tx = fma(t_row[k], x[k * hs + w], tx);
-  return d + tx;
+                                         const double *__restrict__ tx, int64_t q_off,
+                                         int64_t p) {
+  const double *d = dp + lc.base + (p - q_off);
+  const double x = __ldcg(tx + p);
+  double v = __ldcg(d);
+  for (int s = 1; s < lc.nseg; ++s) v += __ldcg(d + (int64_t)s * lc.plane);
+  return v + x;
 }
 
 // value of element (ab, ij) (calc.cpp:384-418) with t_ab,ji = -t and t_ba,ij = -t:
@@ -1299,7 +1207,7 @@ assemble_fused_kernel(const QuadItem *__restrict__ items, int n_items,
                       const ChanInfo *__restrict__ chans, const LadderChan *__restrict__ lchans,
                       const QuadRow *__restrict__ qrows, const QuadCol *__restrict__ qcols,
                       const double *__restrict__ vq, const double *__restrict__ dp,
-                      const double *__restrict__ x, const double *__restrict__ r_quad,
+                      const double *__restrict__ tx, const double *__restrict__ r_quad,
                       const double *__restrict__ xh, const double *__restrict__ yp, double *tq0,
                       double *tq1, double *__restrict__ epart, int32_t *ticket, Control *ctl,
                       __nv_bfloat16 *__restrict__ tkt_tc, int64_t tkt_tc_stride, int nt,
@@ -1318,33 +1226,27 @@ assemble_fused_kernel(const QuadItem *__restrict__ items, int n_items,
   double *__restrict__ t_new = ctl->parity ? tq0 : tq1;
   const double mixing = ctl->mixing;
   double corr = 0.0;
-  // Two-stage pipeline over the CTA's items: the next item's header and this thread's row and
-  // column table entries are fetched while the current quad's operand loads are in flight.
-  QuadRef nx;
-  quad_fetch(items, n_items, qrows, qcols, blockIdx.x, nx);
   for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
-    const QuadRef cu = nx;
-    double tv = 0.0, vv = 0.0, dv = 0.0, xs[2] = {0.0, 0.0}, ys[2] = {0.0, 0.0};
-    double2 ring = make_double2(0.0, 0.0);
-    const int64_t p = cu.q_off + (int64_t)cu.u * cu.hs + cu.w;
-    if (cu.ok) {
-      tv = t_old[p];
-      vv = __ldg(vq + p);
-      ring = __ldcg(reinterpret_cast<const double2 *>(r_quad + 2 * p));
-      // The one-body sums are small arrays every quad reads: through L1 (an L2-only load
-      // would send every warp to the same few L2 slices).
-      xs[0] = xh[cu.i];
-      xs[1] = xh[cu.j];
-      ys[0] = yp[cu.pa];
-      ys[1] = yp[cu.pb];
-      dv = quad_d(lchans[cu.ch], dp, t_old + p - cu.w, x + cu.x_off, cu.hk, cu.hs, cu.u, cu.w);
-    }
-    quad_fetch(items, n_items, qrows, qcols, it + gridDim.x, nx);
-    if (!cu.ok) continue;
-    const double t1 =
-        quad_value(vv, dv, ring, tv, xs[0], xs[1], ys[0], ys[1], cu.den, mixing);
+    const QuadItem item = items[it];
+    const int q = item.q0 + threadIdx.x;
+    if (q >= item.q1) continue;
+    // q / hk as a multiply-high by ceil(2^32 / hk) (Granlund-Montgomery): exact for
+    // q < 2^32 / hk (q < 2^21, hk < 2^11 here); hk = 1 has no 32-bit multiplier.
+    const int hk = item.hk;
+    const uint32_t magic = hk > 1 ? 0xFFFFFFFFu / (uint32_t)hk + 1u : 0u;
+    const int u = hk > 1 ? (int)__umulhi((uint32_t)q, magic) : q, w = q - u * hk;
+    const int64_t p = item.q_off + (int64_t)u * item.hs + w;
+    const QuadRow rw = qrows[item.pk_off + u];
+    const QuadCol cl = qcols[item.qcol_off + w];
+    const double tv = t_old[p], vv = __ldg(vq + p);
+    const double2 ring = __ldcg(reinterpret_cast<const double2 *>(r_quad + 2 * p));
+    const double dv = quad_d(lchans[item.ch], dp, tx, item.q_off, p);
+    // The one-body sums are small arrays every quad reads: through L1 (an L2-only load
+    // would send every warp to the same few L2 slices).
+    const double t1 = quad_value(vv, dv, ring, tv, xh[cl.i], xh[cl.j], yp[rw.pa], yp[rw.pb],
+                                 cl.eij - rw.ea - rw.eb, mixing);
     t_new[p] = t1;
-    if (nt) write_t_image(chans[cu.ch], cu.u, cu.w, t1, nt, tkt_tc, tkt_tc_stride);
+    if (nt) write_t_image(chans[item.ch], u, w, t1, nt, tkt_tc, tkt_tc_stride);
     corr += 4.0 * (vv * t1);
   }
   const double sum = block_sum<kAsmThreads>(corr, scratch);
@@ -1367,22 +1269,19 @@ assemble_fused_kernel(const QuadItem *__restrict__ items, int n_items,
 
 // ---- Between the packed amplitudes and the reference's layout ----------------------------
 
-// D of the ladder in the reference layout (t2Diff_pphh), from the ladder's planes, X and the
-// amplitudes they were computed from (buffer parity ^ flip): a quad's four elements as
-// +D, -D, -D, +D; rows a = b and columns i = j stay zero.
+// D of the ladder in the reference layout (t2Diff_pphh), from the ladder's planes and T X: a quad's
+// four elements as +D, -D, -D, +D; rows a = b and columns i = j stay zero.
 __global__ void __launch_bounds__(kAsmThreads)
 expand_d_kernel(const QuadItem *__restrict__ items, const ChanInfo *__restrict__ chans,
                 const LadderChan *__restrict__ lchans, const QuadRow *__restrict__ qrows,
                 const QuadCol *__restrict__ qcols, const double *__restrict__ dp,
-                const double *__restrict__ x, const double *tq0, const double *tq1, int flip,
-                const Control *ctl, double *__restrict__ d) {
+                const double *__restrict__ tx, double *__restrict__ d) {
   const QuadItem item = items[blockIdx.x];
   const int q = item.q0 + threadIdx.x;
   if (q >= item.q1) return;
   const int u = q / item.hk, w = q - u * item.hk;
-  const double *t = (ctl->parity ^ flip) ? tq1 : tq0;
-  const double v = quad_d(lchans[item.ch], dp, t + item.q_off + (int64_t)u * item.hs,
-                          x + item.x_off, item.hk, item.hs, u, w);
+  const double v = quad_d(lchans[item.ch], dp, tx, item.q_off,
+                          item.q_off + (int64_t)u * item.hs + w);
   const QuadRow rw = qrows[item.pk_off + u];
   const QuadCol cl = qcols[item.qcol_off + w];
   double *o = d + chans[item.ch].t_off;

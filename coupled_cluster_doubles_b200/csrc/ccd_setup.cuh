@@ -651,33 +651,26 @@ __global__ void transpose_hpph_kernel(const ModInfo *__restrict__ mods,
 // A = V_hphp, B[r][r2] = V_hphp of the transpose at (perm[r2], perm[r]), zero padded, in the order
 // in which an m16n8k16 warp takes them: C and B as A operands ([row tile][K step][4][lane][2]), A
 // as accumulators ([row tile][column tile][2][lane][2]), and the destinations alike ([row tile]
-// [column tile][lane][4], -1 where nothing is stored).  Pairs of the one-per-warp kernel read A
-// and C from the blocks themselves and B as ph' x ph'.
-// dst: 2 * (packed position) + (0 for ab,ij / ba,ji, 1 for ab,ji / ba,ij, where the amplitude is
-// negated), kRingNoStore on the second of two elements of a quad's sum that lie in one channel,
-// -1 outside every quad.
+// [column tile][lane][4]).  A destination is 2 * (packed position) + (0 for ab,ij / ba,ji, 1 for
+// ab,ji / ba,ij); -1 outside every quad and on the second of two elements of a quad's sum that lie
+// in one channel.  tp_src: the same position of each element of the T' image (its amplitude is
+// negated where the last bit is set), -1 outside every quad and for the padding.
 __global__ void __launch_bounds__(256)
 ring_image_kernel(const RingPair *__restrict__ pairs, const int32_t *__restrict__ perm,
                   const double *__restrict__ v_hpph, const double *__restrict__ v_hphp,
                   const int32_t *__restrict__ quads, double *__restrict__ img,
-                  int32_t *__restrict__ dst, int32_t *__restrict__ to_img) {
+                  int32_t *__restrict__ tp_src, int32_t *__restrict__ to_img) {
   const RingPair m = pairs[blockIdx.x];
-  const int ph = m.ph, hp = m.hp;
-  auto dst_of = [&](int r, int c) {
-    const int32_t q = quads[m.m_off + (int64_t)r * hp + c];
-    const int k = q & 3;
-    return q < 0 ? -1
-                 : (2 * (q >> 2) + ((k == 1 || k == 2) ? 1 : 0)) |
-                       (m.self && k >= 2 ? kRingNoStore : 0);
+  const int ph = m.ph, hp = m.hp, P = pad16(ph), H = pad16(hp), n8 = (hp + 7) >> 3;
+  auto quad = [&](int r, int c) {
+    return r < ph && c < hp ? quads[m.m_off + (int64_t)r * hp + c] : -1;
   };
-  const int32_t *pm = perm + m.perm_off;
-  auto b_of = [&](int r, int c) { return v_hphp[m.b_src + (int64_t)pm[c] * ph + pm[r]]; };
-  for (int e = threadIdx.x; e < ph * hp; e += blockDim.x) dst[m.dst_off + e] = dst_of(e / hp, e % hp);
-  if (max(ph, hp) <= kRingSmall) {
-    for (int e = threadIdx.x; e < ph * ph; e += blockDim.x) img[m.b_img + e] = b_of(e / ph, e % ph);
-    return;
-  }
-  const int P = pad16(ph), H = pad16(hp), n8 = (hp + 7) >> 3;
+  auto place = [](int32_t q) {
+    const int k = q & 3;
+    return q < 0 ? -1 : 2 * (q >> 2) + ((k == 1 || k == 2) ? 1 : 0);
+  };
+  for (int e = threadIdx.x; e < P * (H + 4); e += blockDim.x)
+    tp_src[m.tp + e] = place(quad(e / (H + 4), e % (H + 4)));
   // Element e of an A-operand image of K steps: its row and k.
   auto a_elem = [](int e, int steps, int &row, int &k) {
     const int blk = e >> 8, lane = (e >> 1) & 31, i = 2 * ((e >> 6) & 3) + (e & 1);
@@ -689,10 +682,11 @@ ring_image_kernel(const RingPair *__restrict__ pairs, const int32_t *__restrict_
     a_elem(e, P / 16, i, k);
     img[m.c_img + e] = i < hp && k < ph ? v_hpph[m.m_off + (int64_t)k * hp + i] : 0.0;
   }
+  const int32_t *pm = perm + m.perm_off;
   for (int e = threadIdx.x; e < P * P; e += blockDim.x) {
     int r, k;
     a_elem(e, P / 16, r, k);
-    img[m.b_img + e] = r < ph && k < ph ? b_of(r, k) : 0.0;
+    img[m.b_img + e] = r < ph && k < ph ? v_hphp[m.b_src + (int64_t)pm[k] * ph + pm[r]] : 0.0;
   }
   // Accumulator q of a lane in a 16 x 8 tile.
   auto c_elem = [&](int blk, int lane, int q, int &row, int &col) {
@@ -707,8 +701,8 @@ ring_image_kernel(const RingPair *__restrict__ pairs, const int32_t *__restrict_
   for (int e = threadIdx.x; e < P * 8 * n8; e += blockDim.x) {
     int r, c;
     c_elem(e >> 7, (e >> 2) & 31, e & 3, r, c);
-    const int32_t d = r < ph && c < hp ? dst_of(r, c) : -1;
-    to_img[m.to_img + e] = d >= 0 && (d & kRingNoStore) ? -1 : d;
+    const int32_t q = quad(r, c);
+    to_img[m.to_img + e] = m.self && (q & 3) >= 2 ? -1 : place(q);
   }
 }
 

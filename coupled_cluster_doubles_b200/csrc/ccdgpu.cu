@@ -42,8 +42,7 @@ struct DevBuf {
 }  // namespace
 
 // A handle's streams and events (see the pool below).
-constexpr int kStreams = 6, kEvents = 18;
-constexpr int kJoin0 = 12;  // events kJoin0 + 1 .. kJoin0 + kStreams - 1: the branches' ends
+constexpr int kStreams = 5, kEvents = 17;
 struct StreamSet {
   int dev = -1;
   cudaStream_t s[kStreams] = {};
@@ -54,7 +53,8 @@ struct ccdgpu_handle {
   ccdgpu_options opt{};
   StreamSet sset;  // the streams and events below, from the process-wide pool
   cudaStream_t s0 = nullptr, s1 = nullptr, s2 = nullptr, s3 = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_fork2 = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_fork2 = nullptr, ev_fork3 = nullptr;
+  cudaEvent_t ev_join = nullptr, ev_join2 = nullptr, ev_join3 = nullptr;
   cudaEvent_t ev[10] = {};
   uint64_t nch = 0, nsp = 0, np = 0, npart = 0;
   int64_t n_t = 0, n_m = 0, n_h = 0, n_p = 0;
@@ -98,17 +98,18 @@ struct ccdgpu_handle {
   // the iteration kind (1 FP64, 2 mixed) whose ladder planes it is expanded from when read.
   bool slab_current = true;
   int d_from = 0;
-  double *x = nullptr;
+  double *x = nullptr, *tx = nullptr;  // hh-ladder X; 0.5 T X in the packed layout
   double *s = nullptr, *r = nullptr, *xh = nullptr, *yp = nullptr, *epart = nullptr;
   int32_t *flat = nullptr;
   int32_t *ring_quads = nullptr;  // phhp position -> 4 x packed position + term, -1
-  // Fused-path ring: pairs of channels (one per warp first, then by padded size 32 .. 80), their
-  // operand images and destinations.
-  RingPair *ring_pairs = nullptr;
-  double *ring_img = nullptr;
+  // Fused-path ring: units by group size (4, 2, 1 warps), operand images, destinations, and the
+  // T' images with where their elements come from.
   RingUnit *ring_units = nullptr;
-  int32_t *ring_dst = nullptr, *ring_to = nullptr;
-  int n_pair_small = 0, n_unit[4] = {0, 0, 0, 0};  // units by row tiles 2 .. 5
+  double *ring_img = nullptr, *ring_tp = nullptr;
+  int32_t *ring_to = nullptr, *ring_src = nullptr;
+  int n_ring[3] = {0, 0, 0};
+  int64_t n_tp = 0;
+  size_t ring_smem[3] = {0, 0, 0};  // dynamic shared memory of the groups' kernels
   std::vector<RingPair> host_pairs;
   double create_ms[5] = {};   // ccdgpu_profile::ms_create
   double loop_graph_ms = 0;   // ccdgpu_profile::ms_loop_graph
@@ -770,6 +771,7 @@ int upload_runs(ccdgpu_handle *h, T *dst, const std::vector<const T *> &src,
   return copy_runs_to_device(h, reinterpret_cast<char *>(dst), rs, rl);
 }
 
+constexpr int kSched = 4;
 int materialize_d(ccdgpu_handle *h);
 
 // pp-ladder work tiles for a schedule (split factors of K per column class), in their own
@@ -882,12 +884,12 @@ int make_ladder_tiles(ccdgpu_handle *h, const ccdgpu_schedule &sch) {
   Arena ar;
   ar.add(&h->tiles, tiles.size()); ar.add(&h->tc_tiles, tc_tiles.size());
   ar.add(&h->lchans, lchans.size()); ar.add(&h->tc_lchans, tc_lchans.size());
-  ar.add(&h->sched, 4);
+  ar.add(&h->sched, kSched);
   ar.add(&h->d_planes, planes); ar.add(&h->tc_planes, tc_planes);
   CK(dev_alloc(ar.used, &h->tile_mem, &h->tile_bytes));
   for (auto &r : ar.reqs) *r.first = static_cast<char *>(h->tile_mem) + r.second;
   // The planes are written in full (where the assembly reads them) by every ladder.
-  CK(cudaMemsetAsync(h->sched, 0, 4 * sizeof(int32_t), h->s3));
+  CK(cudaMemsetAsync(h->sched, 0, kSched * sizeof(int32_t), h->s3));
   auto up = [&](auto *dst, const auto &v) -> int {
     if (v.empty()) return CCDGPU_OK;
     return cuda_status(cudaMemcpyAsync(dst, v.data(), v.size() * sizeof(v[0]),
@@ -1117,7 +1119,7 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     if (pk && hk) {
       ci.nkc = (int)ceil_div(pk, kBK);
       ci.nmt = (int)ceil_div(pk, kMaxBM);
-      const int rows = hh_rows(hk);  // K slice of the hh ladder
+      const int rows = kHHRows;  // K slice of the hh ladder
       ci.nhht = (int)ceil_div(pk, rows);
       ci.nbt = tc_nb(hk);
       ci.nkct = (int)ceil_div(pk, kTcKC);
@@ -1308,10 +1310,10 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   // Fused-path ring: each channel with its transpose, the channel whose ph' pairs are this one's
   // hp' pairs exchanged (the first of the two in channel order names the pair).
   const bool paired = h->opt.path == CCDGPU_PATH_FUSED;
-  std::vector<RingPair> pairs, pairs_large;
+  std::vector<RingPair> pairs;
   std::vector<RingUnit> units;
   std::vector<int32_t> ring_perm;
-  int64_t img_tot = 0, pair_dst_tot = 0, to_tot = 0;
+  int64_t img_tot = 0, tp_tot = 0, to_tot = 0;
   if (paired) {
     std::vector<int2> &look = bs.mod_look;  // (hole, particle) pair -> channel, hp' index
     look.assign((size_t)np * h->npart, make_int2(-1, -1));
@@ -1343,47 +1345,40 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
       r.perm_off = perm_off;
       r.self = other == (int)g;
       r.m_off = m.m_off; r.a_off = m.y_off; r.b_src = mod_gen[other].y_off;
-      (std::max(m.ph, m.hp) <= kRingSmall ? pairs : pairs_large).push_back(r);
+      pairs.push_back(r);
     }
-    h->n_pair_small = (int)pairs.size();
     // The largest first, so that the short ones fill in behind them.
-    std::stable_sort(pairs_large.begin(), pairs_large.end(),
-                     [](const RingPair &x, const RingPair &y) {
-                       return (int64_t)x.ph * x.hp > (int64_t)y.ph * y.hp;
-                     });
-    pairs.insert(pairs.end(), pairs_large.begin(), pairs_large.end());
+    std::stable_sort(pairs.begin(), pairs.end(), [](const RingPair &x, const RingPair &y) {
+      return (int64_t)pad16(x.ph) * pad16(x.hp) > (int64_t)pad16(y.ph) * pad16(y.hp);
+    });
     for (RingPair &r : pairs) {
-      r.dst_off = pair_dst_tot;
-      pair_dst_tot += (int64_t)r.ph * r.hp;
+      const int64_t p = pad16(r.ph), q = pad16(r.hp), n8 = (r.hp + 7) / 8;
+      const int g = ring_group(r.ph, r.hp);
+      r.tp = tp_tot;
+      tp_tot += p * (q + 4);
       r.b_img = img_tot;
-      if (std::max(r.ph, r.hp) <= kRingSmall) {
-        img_tot += (r.ph * r.ph + 1) & ~1;  // 16-byte aligned, as the vector loads need
-      } else {
-        const int64_t p = pad16(r.ph), q = pad16(r.hp), n8 = (r.hp + 7) / 8;
-        img_tot += p * p;
-        r.c_img = img_tot;
-        img_tot += q * p;
-        r.a_img = img_tot;
-        img_tot += q * 8 * n8;
-        r.to_img = to_tot;
-        to_tot += p * 8 * n8;
-      }
+      r.c_img = r.b_img + p * p;
+      r.a_img = r.c_img + q * p;
+      img_tot = r.a_img + q * 8 * n8;
+      r.to_img = to_tot;
+      to_tot += p * 8 * n8;
+      size_t &smem = h->ring_smem[g == 4 ? 0 : g == 2 ? 1 : 2];
+      smem = std::max(smem, (g == 1 ? 4 : 1) * sizeof(double) * ring_unit_smem(g, (int)p, (int)q));
     }
-    // Units by row tiles: the pair's column tiles in blocks of at most kPairNC, as equal as they
-    // come.
-    for (int k = 0; k < 4; k++) {
+    // Units: the pair's column tiles in blocks of at most kPairNC, as equal as they come.
+    for (int k = 0; k < 3; k++) {
       const size_t first = units.size();
-      for (size_t i = h->n_pair_small; i < pairs.size(); i++) {
-        if (pad16(std::max(pairs[i].ph, pairs[i].hp)) / 16 != k + 2) continue;
-        const int n8 = (pairs[i].hp + 7) / 8, blocks = (n8 + kPairNC - 1) / kPairNC;
+      for (const RingPair &r : pairs) {
+        if (ring_group(r.ph, r.hp) != 4 >> k) continue;
+        const int n8 = (r.hp + 7) / 8, blocks = (n8 + kPairNC - 1) / kPairNC;
         for (int q = 0; q < blocks; q++)
-          units.push_back({pairs[i].ph, pairs[i].hp, n8 * q / blocks,
-                           n8 * (q + 1) / blocks - n8 * q / blocks, pairs[i].dst_off,
-                           pairs[i].a_img, pairs[i].b_img, pairs[i].c_img, pairs[i].to_img});
+          units.push_back({r.ph, r.hp, n8 * q / blocks, n8 * (q + 1) / blocks - n8 * q / blocks,
+                           r.tp, r.a_img, r.b_img, r.c_img, r.to_img});
       }
-      h->n_unit[k] = (int)(units.size() - first);
+      h->n_ring[k] = (int)(units.size() - first);
     }
   }
+  h->n_tp = tp_tot;
   h->host_pairs = pairs;
   // Largest channels first within a group, so that the short ones fill in behind them.
   auto by_work = [](const ModInfo &x, const ModInfo &y) {
@@ -1546,13 +1541,12 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   else ar.add(&h->v_t, vt);
   ar.add(&h->v_hpph, h->n_m); ar.add(&h->v_hphp, y_tot);
   ar.add(&h->flat, (size_t)8 * n_t); ar.add(&h->ring_quads, n_t); ar.add(&h->r_quad, paired ? 2 * q_tot : 0);
-  ar.add(&h->ring_pairs, pairs.size()); ar.add(&h->ring_img, img_tot);
-  ar.add(&h->ring_dst, pair_dst_tot); ar.add(&h->ring_units, units.size());
-  ar.add(&h->ring_to, to_tot);
+  ar.add(&h->ring_units, units.size()); ar.add(&h->ring_img, img_tot);
+  ar.add(&h->ring_tp, tp_tot); ar.add(&h->ring_src, tp_tot); ar.add(&h->ring_to, to_tot);
   ar.add(&h->o_h, o_h.size()); ar.add(&h->o_p, o_p.size());
   ar.add(&h->t[0], n_t); ar.add(&h->t[1], n_t); ar.add(&h->dmat, n_t);
   ar.add(&h->old_phhp, h->n_m); ar.add(&h->r_phhp, h->n_m);
-  ar.add(&h->x, x_tot);
+  ar.add(&h->x, x_tot); ar.add(&h->tx, q_tot);
   ar.add(&h->s, quad_cols.size()); ar.add(&h->r, h->n_quad_rows); ar.add(&h->xh, np); ar.add(&h->yp, h->npart);
   ar.add(&h->quad_items, quad_items.size());
   ar.add(&h->quad_rows, h->n_quad_rows); ar.add(&h->quad_cols, quad_cols.size());
@@ -1688,7 +1682,8 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     sc.add(&d_pblk, (nsp - np) * (nsp - np));
   }
   int32_t *d_ring_perm = nullptr;
-  sc.add(&d_ring_perm, ring_perm.size());
+  RingPair *d_pairs = nullptr;
+  sc.add(&d_ring_perm, ring_perm.size()); sc.add(&d_pairs, pairs.size());
   ModGen *d_mod_gen = nullptr;
   int2 *d_mod_ph = nullptr, *d_mod_hp = nullptr;
   int32_t *d_mod_chan = nullptr;
@@ -1779,7 +1774,7 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     return CCDGPU_OK;
   };
   TRY(put(h->chans, chans)); TRY(put(h->mods, mods));
-  TRY(put(h->ring_pairs, pairs)); TRY(put(h->ring_units, units));
+  TRY(put(d_pairs, pairs)); TRY(put(h->ring_units, units));
   TRY(put(d_ring_perm, ring_perm));
   TRY(put(h->hh_tiles, hh_tiles)); TRY(put(h->hh_out, hh_out)); TRY(put(h->hh_part_off, hh_part_off));
   TRY(put(h->ranges, ranges)); TRY(put(h->quad_items, quad_items));
@@ -1937,8 +1932,8 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     CK(cudaGetLastError());
     if (!pairs.empty()) {
       ring_image_kernel<<<(unsigned)pairs.size(), 256, 0, h->s0>>>(
-          h->ring_pairs, d_ring_perm, h->v_hpph, h->v_hphp, h->ring_quads, h->ring_img,
-          h->ring_dst, h->ring_to);
+          d_pairs, d_ring_perm, h->v_hpph, h->v_hphp, h->ring_quads, h->ring_img, h->ring_src,
+          h->ring_to);
       CK(cudaGetLastError());
     }
   }
@@ -1985,19 +1980,11 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   int smem_optin = 0;
   CK(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->opt.device));
   if (ring16_smem(80) > (size_t)smem_optin) return CCDGPU_ERR_UNSUPPORTED;
-  auto pair_attr = [](auto kern, int mt) {
-    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)ring_pair_smem(mt));
-  };
-  CK(pair_attr(ring_pair_kernel<2>, 2));
-  CK(pair_attr(ring_pair_kernel<3>, 3));
-  CK(pair_attr(ring_pair_kernel<4>, 4));
-  CK(pair_attr(ring_pair_kernel<5>, 5));
+  CK(cudaFuncSetAttribute(ring_pair_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                          ring_unit_smem(4, kRingMax, kRingMax) * (int)sizeof(double)));
   CK(cudaFuncSetAttribute(pp_ladder_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                           (int)kLadderSmem));
   CK(cudaFuncSetAttribute(pp_ladder_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-  CK(cudaFuncSetAttribute(hh_ladder_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                          (int)kHHSmem));
   CK(cudaFuncSetAttribute(ring16_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                           (int)ring16_smem(32)));
   CK(cudaFuncSetAttribute(ring16_kernel<48>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2066,7 +2053,7 @@ int launch_hh_ladder(ccdgpu_handle *h, cudaStream_t st, int gate, int only = -1)
   const int n_warp = only <= 0 ? h->n_hh_warp : 0;
   if (n_cta + n_warp) {
     h->launches++;
-    CK(launch_pdl(hh_ladder_kernel, n_cta + (int)ceil_div(n_warp, kHHThreads / 32), kHHThreads,
+    CK(launch_pdl(hh_slice_kernel, n_cta + (int)ceil_div(n_warp, kHHThreads / 32), kHHThreads,
                   n_cta ? kHHSmem : 0, st,
                   (const HHTile *)(h->hh_tiles + (n_cta ? 0 : h->n_hh_cta)), n_cta, n_warp,
                   (const ChanInfo *)h->chans, (const double *)h->vq, (const double *)h->tq[0],
@@ -2103,13 +2090,12 @@ int launch_pp_ladder(ccdgpu_handle *h, cudaStream_t st, int cls = -1) {
       (const double *)h->tq[0], (const double *)h->tq[1], h->d_planes, (const Control *)h->ctl,
       h->err, 0));
 }
-// t2Diff_pphh from the ladder's planes (tc: the tensor-core ladder's) and the amplitudes of
-// buffer parity ^ flip.
-int launch_expand_d(ccdgpu_handle *h, bool tc, int flip) {
+// t2Diff_pphh from the ladder's planes (tc: the tensor-core ladder's) and T X.
+int launch_expand_d(ccdgpu_handle *h, bool tc) {
   if (!h->n_quad_items) return CCDGPU_OK;
   expand_d_kernel<<<h->n_quad_items, kAsmThreads, 0, h->s0>>>(
       h->quad_items, h->chans, tc ? h->tc_lchans : h->lchans, h->quad_rows, h->quad_cols,
-      tc ? h->tc_planes : h->d_planes, h->x, h->tq[0], h->tq[1], flip, h->ctl, h->dmat);
+      tc ? h->tc_planes : h->d_planes, h->tx, h->dmat);
   h->launches++;
   return cuda_status(cudaGetLastError());
 }
@@ -2118,7 +2104,7 @@ int materialize_d(ccdgpu_handle *h) {
   if (!h->d_from) return CCDGPU_OK;
   const bool tc = h->d_from == 2;
   h->d_from = 0;
-  return launch_expand_d(h, tc, 1);
+  return launch_expand_d(h, tc);
 }
 // t[0] of the fused path: the current amplitudes in the reference order.
 int materialize_t(ccdgpu_handle *h) {
@@ -2181,39 +2167,37 @@ int launch_ring(ccdgpu_handle *h, cudaStream_t st, int gate) {
   }
   return CCDGPU_OK;
 }
-// Fused path: pairs of channels.  group: 0 the pairs of the one-per-warp kernel, 1 .. 4 the units
-// of 2 .. 5 row tiles.
-int launch_ring_pairs(ccdgpu_handle *h, cudaStream_t st, int gate, int group) {
-  if (group == 0) {
-    if (!h->n_pair_small) return CCDGPU_OK;
-    h->launches++;
-    return cuda_status(launch_pdl(
-        ring_pair_small_kernel, (int)ceil_div(h->n_pair_small, kRingSmallWarps),
-        kRingSmallWarps * 32, 0, st, (const RingPair *)h->ring_pairs, h->n_pair_small,
-        (const double *)h->v_hpph, (const double *)h->v_hphp, (const double *)h->ring_img,
-        (const int32_t *)h->ring_dst, (const double *)h->tq[0], (const double *)h->tq[1],
-        h->r_quad, (const Control *)h->ctl, gate));
-  }
-  const int n = h->n_unit[group - 1], mt = group + 1;
+// Fused-path ring: the T' images, and the units of group k (0: 4 warps, 1: 2, 2: 1).
+int launch_tp_gather(ccdgpu_handle *h, cudaStream_t st, int gate) {
+  if (!h->n_tp) return CCDGPU_OK;
+  h->launches++;
+  return cuda_status(launch_pdl(
+      tp_gather_kernel, (unsigned)ceil_div(h->n_tp, (int64_t)kGatherThreads * kGatherPer),
+      kGatherThreads, 0, st, (const int32_t *)h->ring_src, h->n_tp, (const double *)h->tq[0],
+      (const double *)h->tq[1], h->ring_tp, (const Control *)h->ctl, gate));
+}
+int launch_ring_units(ccdgpu_handle *h, cudaStream_t st, int gate, int k) {
+  const int n = h->n_ring[k];
   if (!n) return CCDGPU_OK;
   const RingUnit *units = h->ring_units;
-  for (int k = 0; k < group - 1; k++) units += h->n_unit[k];
-  auto kern = mt == 2 ? ring_pair_kernel<2> : mt == 3 ? ring_pair_kernel<3>
-              : mt == 4 ? ring_pair_kernel<4> : ring_pair_kernel<5>;
+  for (int j = 0; j < k; j++) units += h->n_ring[j];
+  auto kern = k == 0 ? ring_pair_kernel<4> : k == 1 ? ring_pair_kernel<2> : ring_pair_kernel<1>;
   h->launches++;
-  return cuda_status(launch_pdl(kern, n, 32 * mt, ring_pair_smem(mt), st,
-                                units, (const double *)h->ring_img, (const int32_t *)h->ring_dst,
-                                (const int32_t *)h->ring_to, (const double *)h->tq[0],
-                                (const double *)h->tq[1], h->r_quad, (const Control *)h->ctl,
-                                gate));
+  return cuda_status(launch_pdl(kern, k == 2 ? (int)ceil_div(n, 4) : n, k == 1 ? 64 : 128,
+                                h->ring_smem[k], st, units, n, (const double *)h->ring_img,
+                                (const int32_t *)h->ring_to, (const double *)h->ring_tp,
+                                h->r_quad, (const Control *)h->ctl, h->err, gate));
 }
-int launch_onebody_fused(ccdgpu_handle *h, cudaStream_t st, int gate) {
-  const int warps_per_block = 8;
-  const int blocks = (int)ceil_div((int64_t)h->nsp, warps_per_block);
+// One-body sums and T X.  only: -1 both, 0 the sums, 1 T X.
+int launch_hh_post(ccdgpu_handle *h, cudaStream_t st, int gate, int only = -1) {
+  const int n_ob = only != 1 ? (int)ceil_div((int64_t)h->nsp, kPostThreads / 32) : 0;
+  const int n_tx = only != 0 ? h->n_quad_items : 0;
+  if (!(n_ob + n_tx)) return CCDGPU_OK;
   h->launches++;
-  return cuda_status(launch_pdl(onebody_fused_kernel, blocks, warps_per_block * 32, 0, st,
-                                (int)h->np, (int)h->nsp, h->list_off, h->list, h->s, h->r, h->xh,
-                                h->yp, h->ctl, gate));
+  return cuda_status(launch_pdl(
+      hh_post_kernel, n_ob + n_tx, kPostThreads, 0, st, n_ob, (int)h->np, (int)h->nsp, h->list_off,
+      h->list, h->s, h->r, h->xh, h->yp, (const QuadItem *)h->quad_items, (const double *)h->x,
+      (const double *)h->tq[0], (const double *)h->tq[1], h->tx, (const Control *)h->ctl, gate));
 }
 int launch_assemble_fused(ccdgpu_handle *h, cudaStream_t st, int gate) {
   if (!h->n_asm_blocks) return CCDGPU_OK;
@@ -2223,7 +2207,7 @@ int launch_assemble_fused(ccdgpu_handle *h, cudaStream_t st, int gate) {
       h->n_asm_blocks, kAsmThreads, 0, st, (const QuadItem *)h->quad_items, h->n_quad_items,
       (const ChanInfo *)h->chans, (const LadderChan *)(gate ? h->tc_lchans : h->lchans),
       (const QuadRow *)h->quad_rows, (const QuadCol *)h->quad_cols, (const double *)h->vq,
-      (const double *)(gate ? h->tc_planes : h->d_planes), (const double *)h->x,
+      (const double *)(gate ? h->tc_planes : h->d_planes), (const double *)h->tx,
       (const double *)h->r_quad, (const double *)h->xh, (const double *)h->yp, h->tq[0], h->tq[1],
       h->epart, h->ticket, h->ctl, h->tkt_tc, h->n_tkttc, gate ? h->nt : 0,
       (cudaGraphConditionalHandle)(h->loop_capture ? h->loop_cond : 0), h->loop_capture, gate));
@@ -2246,10 +2230,9 @@ int launch_map_to(ccdgpu_handle *h, cudaStream_t st, const double *src, double *
   return cuda_status(cudaGetLastError());
 }
 
-// One fused iteration: the pp ladder on s0, the groups of the ring and the hh ladder with the
-// one-body sums on streams of their own (each needs only the amplitudes), then the assembly on
-// s0.  The ladder, bound by HBM on one CTA per SM, goes first; the others, bound by latency, run
-// beside it, the longest first.
+// One fused iteration: the pp ladder on s0, the ring on s1 and s3, and the hh ladder with the
+// one-body sums on s2 side by side (each needs only the amplitudes), then the assembly on s0.  The
+// ladder is bound by HBM on one CTA per SM, the others by latency and the L2.
 // mixed: the pp ladder runs on the tensor cores (split bf16) instead of the FP64 pipe.
 int enqueue_fused_iteration(ccdgpu_handle *h, bool mixed) {
   int rc;
@@ -2263,13 +2246,14 @@ int enqueue_fused_iteration(ccdgpu_handle *h, bool mixed) {
     CK(cudaEventRecord(h->ev[0], h->s0));
     if ((rc = launch_hh_ladder(h, h->s0, gate))) return rc;
     CK(cudaEventRecord(h->ev[1], h->s0));
-    if ((rc = launch_onebody_fused(h, h->s0, gate))) return rc;
+    if ((rc = launch_hh_post(h, h->s0, gate))) return rc;
     CK(cudaEventRecord(h->ev[2], h->s0));
     if ((rc = ladder(h->s0))) return rc;
     CK(cudaEventRecord(h->ev[3], h->s0));
     CK(cudaEventRecord(h->ev[4], h->s0));
-    for (int k = 4; k >= 0; k--)
-      if ((rc = launch_ring_pairs(h, h->s0, gate, k))) return rc;
+    if ((rc = launch_tp_gather(h, h->s0, gate))) return rc;
+    for (int k = 0; k < 3; k++)
+      if ((rc = launch_ring_units(h, h->s0, gate, k))) return rc;
     CK(cudaEventRecord(h->ev[5], h->s0));
     CK(cudaEventRecord(h->ev[8], h->s0));
     if ((rc = launch_assemble_fused(h, h->s0, gate))) return rc;
@@ -2277,22 +2261,32 @@ int enqueue_fused_iteration(ccdgpu_handle *h, bool mixed) {
     CK(cudaEventRecord(h->ev[7], h->s0));
     return CCDGPU_OK;
   }
-  // Branches in the reverse of the order in which their kernels should be placed: of the branches
-  // of a graph that become ready together, the one captured last is launched first.
+  // Kernels reach the GPU in the order in which they become ready, and the CTAs of one wait behind
+  // all CTAs of those before it; of branches that become ready together the one captured last comes
+  // first.  So: the ladder (it needs an SM's registers before smaller CTAs take them), the hh
+  // slices and the gather, then the short kernels that follow the hh slices, and the ring, which
+  // the gather holds back until then.
   CK(cudaEventRecord(h->ev_fork, h->s0));
-  for (int k = 1; k < kStreams; k++) CK(cudaStreamWaitEvent(h->sset.s[k], h->ev_fork, 0));
-  if ((rc = launch_hh_ladder(h, h->s2, gate))) return rc;
-  if ((rc = launch_onebody_fused(h, h->s2, gate))) return rc;
-  if ((rc = launch_ring_pairs(h, h->sset.s[5], gate, 0))) return rc;
-  if ((rc = launch_ring_pairs(h, h->sset.s[4], gate, 1))) return rc;
-  if ((rc = launch_ring_pairs(h, h->s3, gate, 2))) return rc;
-  for (int k = 4; k >= 3; k--)
-    if ((rc = launch_ring_pairs(h, h->s1, gate, k))) return rc;
-  if ((rc = ladder(h->s0))) return rc;
-  for (int k = 1; k < kStreams; k++) {
-    CK(cudaEventRecord(h->sset.ev[kJoin0 + k], h->sset.s[k]));
-    CK(cudaStreamWaitEvent(h->s0, h->sset.ev[kJoin0 + k], 0));
+  CK(cudaStreamWaitEvent(h->s1, h->ev_fork, 0));
+  CK(cudaStreamWaitEvent(h->s2, h->ev_fork, 0));
+  if ((rc = launch_tp_gather(h, h->s1, gate))) return rc;
+  // The groups of units side by side; the first that the system has stays on s1.
+  CK(cudaEventRecord(h->ev_fork3, h->s1));
+  const struct { cudaStream_t st; cudaEvent_t ev; } branch[3] = {
+      {h->s1, h->ev_join}, {h->s3, h->ev_join3}, {h->sset.s[4], h->sset.ev[16]}};
+  int used = 0;
+  for (int k = 0; k < 3; k++) {
+    if (!h->n_ring[k]) continue;
+    if (used) CK(cudaStreamWaitEvent(branch[used].st, h->ev_fork3, 0));
+    if ((rc = launch_ring_units(h, branch[used++].st, gate, k))) return rc;
   }
+  for (int k = 0; k < std::max(used, 1); k++) CK(cudaEventRecord(branch[k].ev, branch[k].st));
+  if ((rc = launch_hh_ladder(h, h->s2, gate))) return rc;
+  if ((rc = launch_hh_post(h, h->s2, gate))) return rc;
+  CK(cudaEventRecord(h->ev_join2, h->s2));
+  if ((rc = ladder(h->s0))) return rc;
+  for (int k = 0; k < std::max(used, 1); k++) CK(cudaStreamWaitEvent(h->s0, branch[k].ev, 0));
+  CK(cudaStreamWaitEvent(h->s0, h->ev_join2, 0));
   if ((rc = launch_assemble_fused(h, h->s0, gate))) return rc;  // + energy and stop rule
   if (h->loop_capture && !h->n_asm_blocks) {  // else the assembly set the loop condition
     h->launches++;
@@ -2346,7 +2340,7 @@ int check_errors(ccdgpu_handle *h) {
     // incomplete; ccdgpu_reset or ccdgpu_set_t2 starts over).  A ladder CTA that gave up may
     // have left its tile counter and exit ticket behind: zero them for the next launch.
     CK(cudaMemset(h->err, 0, sizeof(int32_t)));
-    if (h->sched) CK(cudaMemset(h->sched, 0, 4 * sizeof(int32_t)));
+    if (h->sched) CK(cudaMemset(h->sched, 0, kSched * sizeof(int32_t)));
     return CCDGPU_ERR_TIMEOUT;
   }
   if (h->h_ctl->error & kErrNonFinite) return CCDGPU_ERR_NONFINITE;
@@ -2500,8 +2494,9 @@ int tables_iteration(ccdgpu_handle *h, double mixing, double *corr) {
   if ((rc = stage_onebody_tables(h, 1, 0))) return rc;     // calcT2Diff_h2pp_h1
   if ((rc = launch_ring(h, h->s0, 0))) return rc;   // calcT2Diff_phhp
   if ((rc = launch_hh_ladder(h, h->s0, 0))) return rc;     // calcT2Diff_pphh
+  if ((rc = launch_hh_post(h, h->s0, 0, 1))) return rc;
   if ((rc = launch_pp_ladder(h, h->s0))) return rc;
-  if ((rc = launch_expand_d(h, false, 0))) return rc;
+  if ((rc = launch_expand_d(h, false))) return rc;
   if ((rc = stage_gather(h))) return rc;                   // 8 x mapFromDistributed
   if ((rc = stage_assemble_tables(h, mixing))) return rc;  // calcT2_pphh
   if ((rc = launch_energy(h, h->s0, 2))) return rc;
@@ -2570,7 +2565,8 @@ int ccdgpu_create(const ccdgpu_problem *prob, const ccdgpu_options *opt, ccdgpu_
   if (!rc) {
     h->s0 = h->sset.s[0]; h->s1 = h->sset.s[1]; h->s2 = h->sset.s[2]; h->s3 = h->sset.s[3];
     for (int i = 0; i < 10; i++) h->ev[i] = h->sset.ev[i];
-    h->ev_fork = h->sset.ev[10]; h->ev_fork2 = h->sset.ev[11];
+    h->ev_fork = h->sset.ev[10]; h->ev_fork2 = h->sset.ev[11]; h->ev_fork3 = h->sset.ev[12];
+    h->ev_join = h->sset.ev[13]; h->ev_join2 = h->sset.ev[14]; h->ev_join3 = h->sset.ev[15];
   }
   if (!rc) rc = build(h, prob);
   if (!rc) rc = init_ctl(h);
@@ -2598,8 +2594,7 @@ uint64_t ccdgpu_t2_size(const ccdgpu_handle *h) { return h ? (uint64_t)h->n_t : 
 int ccdgpu_reset(ccdgpu_handle *h) {
   if (!h) return CCDGPU_ERR_INVALID_ARGUMENT;
   CK(cudaSetDevice(h->opt.device));
-  // The fused path iterates on the packed amplitudes alone; the other buffer of the pair stays,
-  // since t2Diff_pphh of the last iteration may still be read from it.
+  // The fused path iterates on the packed amplitudes alone.
   const bool fused = h->opt.path == CCDGPU_PATH_FUSED;
   const std::pair<double *, int64_t> z[] = {
       {h->tq[h->h_ctl->parity], h->n_q}, {h->old_phhp, h->n_m},
@@ -3040,8 +3035,8 @@ int ccdgpu_calc_t2diff_phhp(ccdgpu_handle *h) {
 int ccdgpu_calc_t2diff_pphh(ccdgpu_handle *h) {
   if (!h) return CCDGPU_ERR_INVALID_ARGUMENT;
   int rc = set_ctl(h, 0, h->h_ctl->tol, h->h_ctl->max_iters, h->h_ctl->mixing, false);
-  if (rc || (rc = launch_hh_ladder(h, h->s0, 0)) || (rc = launch_pp_ladder(h, h->s0)) ||
-      (rc = launch_expand_d(h, false, 0)))
+  if (rc || (rc = launch_hh_ladder(h, h->s0, 0)) || (rc = launch_hh_post(h, h->s0, 0, 1)) ||
+      (rc = launch_pp_ladder(h, h->s0)) || (rc = launch_expand_d(h, false)))
     return rc;
   h->d_from = 0;
   CK(cudaStreamSynchronize(h->s0));
@@ -3145,10 +3140,10 @@ int ccdgpu_kernel_profile(ccdgpu_handle *h, int32_t reps, double *ms, double *fl
   if (rc) return rc;
   if ((rc = materialize_d(h))) return rc;  // the kernels overwrite what it is expanded from
   for (int k = 0; k < 7; k++) ms[k] = flops[k] = bytes[k] = 0;
-  // Ring (fused path): S = T' (A + C T') + B T' per pair of channels; reads A, B, C, the
-  // destinations and the amplitudes they name, writes S.
+  // Ring (fused path): S = T' (A + C T') + B T' per pair of channels; reads A, B, C, T' and the
+  // destinations, writes S.  The small class is launched with the gather of the T' images.
   for (const RingPair &m : h->host_pairs) {
-    const int w = std::max(m.ph, m.hp), k = w <= kRingSmall ? 0 : w <= 32 ? 1 : 2;
+    const int g = ring_group(m.ph, m.hp), k = g == 1 ? 0 : g == 2 ? 1 : 2;
     const double n = (double)m.ph * m.hp;
     flops[k] += 2.0 * n * (2.0 * m.hp + m.ph);
     bytes[k] += 28.0 * n + 8.0 * ((double)m.hp * m.hp + (double)m.ph * m.ph);
@@ -3168,15 +3163,12 @@ int ccdgpu_kernel_profile(ccdgpu_handle *h, int32_t reps, double *ms, double *fl
   bytes[5] = 16.0 * (double)(h->nsp) + 12.0 * (double)h->n_list;
   for (int k = 0; k < 7; k++) {
     auto launch = [&]() -> int {
-      if (k <= 1) return launch_ring_pairs(h, h->s0, 0, k);
-      if (k == 2) {
-        for (int q = 4; q >= 2; q--)
-          if (const int r = launch_ring_pairs(h, h->s0, 0, q)) return r;
-        return CCDGPU_OK;
-      }
+      if (k == 0)
+        if (const int r = launch_tp_gather(h, h->s0, 0)) return r;
+      if (k <= 2) return launch_ring_units(h, h->s0, 0, 2 - k);
       if (k <= 4) return launch_hh_ladder(h, h->s0, 0, k - 3);
       if (k == 6) return launch_hh_ladder(h, h->s0, 0, 2);
-      return launch_onebody_fused(h, h->s0, 0);
+      return launch_hh_post(h, h->s0, 0, 0);
     };
     if ((rc = launch())) return rc;  // warm-up
     CK(cudaEventRecord(h->ev[0], h->s0));
