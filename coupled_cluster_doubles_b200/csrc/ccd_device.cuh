@@ -16,39 +16,43 @@ namespace ccd {
 //
 // pp ladder.  D[ab,ij] = sum_{c<d} V[ab,cd] T[cd,ij] over the quads: V is the pk x pk packed
 // matrix (1/4 of V_pppp), T the packed amplitudes themselves (16 consecutive rows are one
-// contiguous B stage).  A stages are stored in HBM in their shared-memory image so that one bulk
-// copy (TMA) moves each:
-//   thin channels (hk <= 4, hs in {1, 2, 4}; two consumer threads per row):
-//     [rows][kBK] row-major, column XOR-swizzled by (row & 15): a warp reading two k of 16
-//     consecutive rows takes the minimum of two wavefronts;
-//   wider channels (FP64 MMA fragments): [kBK][as] k-major, as = rows rounded up to 8, plus 4,
-//     and hs = 4 mod 8: with strides of 4 mod 8 doubles the 4 k-rows of an m16n8k16 fragment
-//     load fall on distinct banks.
+// contiguous B stage).  V is symmetric (<ab|v|cd> = <cd|v|ab>), so a channel with at most kSymHK
+// strict hole pairs stores and streams only the blocks on and above the diagonal (blocks of
+// kMaxBM rows and columns): each block above it serves its rows and, transposed, its columns.
+// A stages are stored in HBM in their shared-memory image so that one bulk copy (TMA) moves each:
+// [kBK][as] k-major, as = rows rounded up to 8, plus 4.  hs is 4 mod 8 beyond 4 hole pairs: with
+// strides of 4 mod 8 doubles the 4 k-rows of an m16n8k16 fragment load fall on distinct banks.
 // The last row tile of a channel is stored compact (only its real rows, rounded up to 8).
-constexpr int kBK = 16;        // K depth of one pipeline stage
-constexpr int kStages = 5;     // bulk-copy pipeline depth (68-86 KB in flight per SM)
+constexpr int kBK = 16;        // K depth of one chunk
+constexpr int kStages = 3;     // bulk-copy pipeline depth, stages of two chunks (one if hs > 20)
 constexpr int kMaxHH = 72;     // hole pairs of a channel (ordered)
-constexpr int kMaxCG = 5;      // column groups of 8 strict hole pairs (hk <= 36)
 constexpr int kLadderConsumers = 256;                  // 8 warps of 16 rows
 constexpr int kLadderThreads = kLadderConsumers + 32;  // + 1 producer warp
 constexpr int kMaxBM = 128;    // rows per tile
+constexpr int kBlkChunks = kMaxBM / kBK;  // K chunks of a block of columns
 constexpr int kMaxNB = 36;     // largest row stride hs of the packed amplitudes
+constexpr int kSymHK = 20;     // hole pairs up to which V's symmetry is used ...
+constexpr int kSymHS = 20;     // ... and their largest hs
 constexpr int kMaxAS = kMaxBM + 4;  // A stage row stride bound (doubles)
 
-__host__ __device__ inline int swzA(int row, int k) { return row * kBK + (k ^ (row & 15)); }
 // Row stride of the packed layout for hk strict hole pairs.
 __host__ __device__ inline int quad_hs(int hk) {
   return hk <= 2 ? hk : hk <= 4 ? 4 : 8 * ((hk + 3) / 8) + 4;
 }
+// Chunks of a pipeline stage.
+__host__ __device__ inline int ladder_stage(int hs) { return hs <= 20 ? 2 : 1; }
+constexpr int kStageA = 2 * kBK * (kMaxBM + 4), kStageB = 2 * kBK * 20;  // doubles; 2 * 20 >= 36
 // Column classes: 0 thin, 1 mid (hs 12, 20), 2 wide (hs 28, 36).
 __host__ __device__ inline int ladder_class(int hs) { return hs <= 4 ? 0 : hs <= 20 ? 1 : 2; }
-__host__ __device__ inline bool ladder_kmajor(int hs) { return hs > 4; }
-// Doubles per k row of an A chunk (k-major) or rows of it (thin) for a tile of `rows` rows.
-__host__ __device__ inline int ladder_arows(int hs, int rows) {
-  return ladder_kmajor(hs) ? ((rows + 7) & ~7) + 4 : rows;
+// Doubles per k row of an A chunk for a tile of `rows` rows.
+__host__ __device__ inline int ladder_as(int rows) { return ((rows + 7) & ~7) + 4; }
+// First K chunk stored of row tile mt, and where K chunk kc of row tile mt (`rows` rows) starts in
+// the channel's A image of nkc chunks a row.
+__host__ __device__ inline int ladder_kc0(bool sym, int mt) { return sym ? kBlkChunks * mt : 0; }
+__host__ __device__ inline int64_t ladder_chunk(bool sym, int nkc, int mt, int kc, int rows) {
+  const int64_t before = (int64_t)mt * nkc - (sym ? kBlkChunks / 2 * mt * (mt - 1) : 0);
+  return (before * kMaxAS + (int64_t)(kc - ladder_kc0(sym, mt)) * ladder_as(rows)) * kBK;
 }
-// A image of row tile mt starts at mt * ladder_arows_full(hs) * nk * kBK (full tiles).
-__host__ __device__ inline int ladder_arows_full(int hs) { return ladder_arows(hs, kMaxBM); }
 
 // Mixed-precision pp-ladder images (tensor-core operands, ccd_tc.cuh).  A K chunk of a
 // 128-row tile holds kTcKC bf16 per row in 8 x 8 core matrices, K-major, no swizzle:
@@ -136,21 +140,30 @@ __device__ __forceinline__ void split_bf16_n(double x, __nv_bfloat16 (&out)[NT])
 }
 
 // One pp-ladder work tile: packed rows [128 mt, 128 mt + rows) of channel `ch`, K chunks
-// [kc0, kc0 + nks).  Tiles of one row block that split K write separate planes of the channel's
-// D partials (LadderChan), which the assembly adds in segment order.
+// [kc0, kc0 + nks).  Partial sums of D go to planes of one row tile each ([128][hs] doubles): the
+// planes of row tile J lie together (LadderRows), in a symmetric channel first those of the
+// transposed blocks of row tiles 0 .. J - 1, then one per K segment of its own.
 struct LadderTile {
   int32_t ch, mt, kc0, nks;
   int32_t rows, hk, hs, nb;  // nb: UMMA N (tensor-core tiles)
-  int64_t a_base;  // first A chunk: + c * ladder_arows(hs, rows) * kBK (tensor core: see there)
-  int64_t b_base;  // first B chunk: + c * kBK * hs
-  int64_t out;     // D of the tile's first row: + u_local * hs
+  int32_t sym, nseg;         // nseg: K segments the channel's row tiles have room for
+  int32_t pk, pad;
+  int64_t a_base;   // first A chunk: + c * ladder_as(rows) * kBK (tensor core: see there)
+  int64_t b_base;   // first B chunk: + c * kBK * hs
+  int64_t ti_base;  // T of the tile's own rows (symmetric channels)
+  int64_t out;      // D plane of the tile: + u_local * hs
+  int64_t planes;   // planes of the channel
 };
+// First plane of row tile mt of a channel.
+__host__ __device__ inline int ladder_plane(bool sym, int nseg, int mt) {
+  return mt * nseg + (sym ? mt * (mt - 1) / 2 : 0);
+}
 
-// Where the ladder leaves D of a channel: nseg planes of `plane` doubles from `base`, each in
-// the packed layout; D is their sum in plane order.
-struct LadderChan {
+// Where the ladder leaves D of a row tile: n planes of 128 * hs doubles from `base`; D is their sum
+// in plane order.
+struct LadderRows {
   int64_t base;
-  int32_t nseg, plane;
+  int32_t n, stride;
 };
 
 // Per active regular channel.  A channel without quads (pk or hk zero) has no ladder tile, hh
@@ -158,6 +171,7 @@ struct LadderChan {
 struct ChanInfo {
   int32_t pp, hh, pk, hk;
   int32_t hs, nkc, nmt, nhht;  // packed row stride, K chunks, row tiles, hh-ladder slices
+  int32_t sym, rt_off;  // V stored by its symmetry; first row tile among all channels'
   int64_t t_off;     // pphh block offset (reference t2 layout)
   int64_t pp_off;    // offset into pp_pairs / pp_swap / prow
   int64_t hh_off;    // offset into hh_pairs / hh_swap / hcol
@@ -202,7 +216,7 @@ struct QuadCol {
 // what its threads need of the channel (so their table reads depend on the item alone).
 struct QuadItem {
   int32_t ch, q0, q1, hk;
-  int32_t hs, pad;
+  int32_t hs, rt_off;
   int64_t q_off, x_off, pk_off, qcol_off;
 };
 

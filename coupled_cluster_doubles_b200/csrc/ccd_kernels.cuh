@@ -109,113 +109,144 @@ __device__ __forceinline__ bool skip_iteration(const Control *ctl, int gate, int
 }
 
 // ------------------------------------------------------------------------------------------
-// pp ladder in FP64 (FMA pipe for thin channels, FP64 MMA for the rest) over the packed quads:
+// pp ladder on the FP64 MMA over the packed quads:
 //   D[u, w] = sum_c V[u, c] T[c, w]        (u = a<b, c = c<d, w = i<j)
-// Half of the hole columns and none of the a = b rows of the full antisymmetry-packed product,
-// and no T X: the product needs only the amplitudes, so it starts at the head of an iteration
-// beside the hh ladder and the ring instead of behind the hh ladder (the assembly adds T X).
-// It streams V once and is bound by that: one CTA per SM leaves registers and shared memory
-// for the other streams' kernels, and its five 17-22 KB stages (85-108 KB in flight) still
-// cover HBM's latency.
+// It needs only the amplitudes (T X is added later), so it starts at the head of an iteration
+// beside the hh ladder and the ring.  Channels of up to kSymHK strict hole pairs stream the blocks
+// of V on and above the diagonal alone: a block of rows I and columns J > I gives D_I += V_IJ T_J
+// and D_J += V_IJ^T T_I.  EG N=54 |n|^2 <= 36: 559 MB of V become 351 (and 32 MB of D planes), in
+// the iteration the ladder's 145 us become 111; PNM N=66: 716 MB to 457, 190 us to 142.  V in full
+// is bound by HBM; halved, as much by each warp's chain of shared-memory loads, MMAs and barriers
+// (DRAM 50 % busy in the thin class, FP64 MMA 40 %).  Wider channels would need twice the FP64 MMA
+// they already wait for.
+// One CTA per SM, 80 registers, three 39 KB stages of two chunks: it leaves registers and shared
+// memory for the other streams' kernels (at 94 registers its nine warps kept the ring's CTAs
+// out; with a fourth stage the ladder alone is 5 % faster but the iteration slower, 64 for 56 us at
+// EG N=54 |n|^2 <= 19).  Stages of one chunk, five deep: 51 and 66 us for the thin and the mid
+// class alone at EG N=54 |n|^2 <= 36, 46 and 62 now.
 // One producer warp: a lane claims tiles from a launch-wide counter (list sorted by class, wide
 // first, then by decreasing work: longest-first list scheduling that adapts to CTAs starting
 // late behind another stream's kernels) and streams pre-tiled A/B stages with bulk copies (TMA,
 // no multicast) into a kStages-deep shared-memory ring guarded by mbarriers, across tile
-// boundaries; beside each stage it leaves the tile's description for the consumers.  The 8
-// consumer warps run DFMAs (thin: two threads a row, T as broadcasts) or m16n8k16 FP64 MMAs.
-// All classes share one launch (EG N=54 |n|^2 <= 36, 566 MB of V: the three launches of the
-// hh-wide columns took 181 us one after another).
+// boundaries; beside a tile's first stage it leaves the tile's description for the consumers.
+// T_I has a buffer of its own, filled once the previous tile's readers are done and needed only
+// after the diagonal block's chunks.
+// The 8 consumer warps: warp w owns rows [16w, 16w + 16) of the direct product; of the transposed
+// product of chunk kc (16 columns, all 128 rows) warp kc % 8 does the whole, so nothing is reduced
+// across warps.  (All warps sharing each chunk's transposed product, with a sum of eight parts
+// through shared memory, was no faster for one column tile and slower for two.)
 // ------------------------------------------------------------------------------------------
 
 // What the consumers need of the tile a stage belongs to.
 struct StageInfo {
-  int64_t out;
+  int64_t out, planes;
   int32_t rows, hk, hs, nks;  // nks: K chunks of the tile; 0: no more tiles
+  int32_t kc0, mt, nseg, pk;  // nseg < 0: no transposed product
 };
 
-// Thin tiles (hs = NB in {1, 2, 4}): two consumer threads per packed row, even and odd k.
-template <int NB>
-__device__ __forceinline__ void thin_chunk(const double *A, const double *B, int tid,
-                                           double (&acc)[NB]) {
-  const int row = tid >> 1, odd = tid & 1;
-#pragma unroll
-  for (int j = 0; j < kBK / 2; ++j) {
-    const int k = 2 * j + odd;
-    const double a = A[swzA(row, k)];
-    if constexpr (NB == 1) {
-      acc[0] = fma(a, B[k], acc[0]);
-    } else {
-      const double2 *bp = reinterpret_cast<const double2 *>(B + k * NB);
-#pragma unroll
-      for (int q = 0; q < NB / 2; ++q) {
-        const double2 b = bp[q];
-        acc[2 * q] = fma(a, b.x, acc[2 * q]);
-        acc[2 * q + 1] = fma(a, b.y, acc[2 * q + 1]);
-      }
+// The consumer side of one tile: its stages from the ring, then its D rows.  at: the next stage.
+// FULL: a tile of 128 rows, whose A stride is a constant; only those have a transposed product.  A
+// fragments (k-major, row stride ar) and B fragments (row stride hs) come from the stage
+// conflict-free.  A warp whose lower 8-row half has no rows feeds zeros there instead of reading
+// past the tile; columns past hk (the stage's next row, or stale) are not stored.  ti_bar,
+// ti_parity: T_I's barrier.  False: a wait ran out (rows stay unwritten).
+struct RingPos {  // a stage and the parity of its barriers
+  int s = 0;
+  uint32_t phase = 0;
+  __device__ __forceinline__ void next() {
+    if (++s == kStages) {
+      s = 0;
+      phase ^= 1;
     }
   }
-}
-
-// The consumer side of one tile: its chunks from the stage ring, then its D rows.  gc: chunks
-// this CTA has consumed so far.  False: a wait ran out (the tile's rows stay unwritten).
-template <int NB>
-__device__ __forceinline__ bool consume_thin(const StageInfo &ti, const double *As,
-                                             const double *Bs, uint64_t *bars, int tid, int gc,
-                                             double *__restrict__ d) {
-  double acc[NB];
-#pragma unroll
-  for (int j = 0; j < NB; ++j) acc[j] = 0.0;
-  for (int c = 0; c < ti.nks; ++c) {
-    const int g = gc + c, s = g % kStages;
-    if (!mbar_wait(smem_u32(&bars[s]), (g / kStages) & 1)) return false;
-    if ((tid >> 1) < ti.rows)
-      thin_chunk<NB>(As + s * (kMaxAS * kBK), Bs + s * (kBK * kMaxNB), tid, acc);
-    __syncwarp();
-    if ((tid & 31) == 0) mbar_arrive(smem_u32(&bars[kStages + s]));
-  }
-#pragma unroll
-  for (int j = 0; j < NB; ++j) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], 1);
-  if (!(tid & 1) && (tid >> 1) < ti.rows) {
-    double *o = d + ti.out + (int64_t)(tid >> 1) * NB;
-#pragma unroll
-    for (int j = 0; j < NB; ++j)
-      if (j < ti.hk) o[j] = acc[j];
-  }
-  return true;
-}
-
-// Wider tiles on the FP64 MMA: consumer warp w owns tile rows [16w, 16w + 16), one m16n8k16
-// per 8-column tile and stage (kBK = 16), 4 C accumulators per lane.  A (k-major, row stride
-// ar) and B (k-major, row stride hs) fragments come from the stage conflict-free: both strides
-// are 4 mod 8 doubles.  A warp whose lower 8-row half has no rows feeds zeros there instead of
-// reading past the tile; columns past hk (the stage's next row, or stale) are not stored.
-template <int C>
+};
+template <int C, bool FULL>
 __device__ __forceinline__ bool consume_mma(const StageInfo &ti, const double *As,
-                                            const double *Bs, uint64_t *bars, int tid, int gc,
-                                            double *__restrict__ d) {
-  static_assert(kBK == 16, "one m16n8k16 K step per stage");
+                                            const double *Bs, const double *Ti, uint64_t *bars,
+                                            uint32_t ti_bar, uint32_t ti_parity, int tid,
+                                            RingPos &at, double *__restrict__ d) {
+  static_assert(kBK == 16, "one m16n8k16 K step per chunk");
+  constexpr int kPer = C <= 3 ? 2 : 1;  // chunks of a stage
   const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  const int ar = ladder_arows(ti.hs, ti.rows), hs = ti.hs;
-  const int halves = min(2, max(0, ((ti.rows + 7) >> 3) - 2 * warp));  // 8-row halves with rows
+  const int rows = FULL ? kMaxBM : ti.rows;
+  const int ar = ladder_as(rows), hs = ti.hs;
+  const int halves = FULL ? 2 : min(2, max(0, ((rows + 7) >> 3) - 2 * warp));  // 8-row halves
+  // First chunk with a transposed product.
+  const int off = FULL && ti.nseg >= 0 ? kBlkChunks * (ti.mt + 1) - ti.kc0 : ti.nks;
+  bool have_ti = false;
   double acc[C][4];
 #pragma unroll
   for (int j = 0; j < C; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0;
-  for (int c = 0; c < ti.nks; ++c) {
-    const int gch = gc + c, s = gch % kStages;
-    if (!mbar_wait(smem_u32(&bars[s]), (gch / kStages) & 1)) return false;
-    if (halves > 0) {
-      const double *A = As + s * (kMaxAS * kBK) + t * ar + 16 * warp + g;
-      const double *B = Bs + s * (kBK * kMaxNB) + t * hs + g;
+  for (int c = 0; c < ti.nks; c += kPer) {
+    const int s = at.s;
+    if (!mbar_wait(smem_u32(&bars[s]), at.phase)) return false;
+    at.next();
+    const double *Ac = As + s * kStageA;
+    const double *A0 = Ac + t * ar + 16 * warp + g, *B0 = Bs + s * kStageB + t * hs + g;
+    auto direct = [&](const double *A, const double *B) {
       double a[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i)
-        a[i] = (i % 2 == 0 || halves > 1) ? A[4 * (i / 2) * ar + 8 * (i % 2)] : 0.0;
+        a[i] = (FULL || i % 2 == 0 || halves > 1) ? A[4 * (i / 2) * ar + 8 * (i % 2)] : 0.0;
 #pragma unroll
       for (int j = 0; j < C; ++j) {
         double b[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) b[q] = B[4 * q * hs + 8 * j];
         dmma_16816(acc[j], a, b);
+      }
+    };
+    if (FULL || halves > 0) {
+      if (kPer == 2 && c + 1 < ti.nks) {
+        direct(A0, B0);
+        direct(A0 + kBK * ar, B0 + kBK * hs);
+      } else {
+        direct(A0, B0);
+      }
+    }
+    if constexpr (FULL && C <= (kSymHK + 7) / 8) {
+      const int u = (warp - ti.kc0 - c) & (kBlkChunks - 1);  // this warp's chunk of the stage
+      if (c >= off && u < kPer && c + u < ti.nks) {
+        if (!have_ti && !mbar_wait(ti_bar, ti_parity)) return false;
+        have_ti = true;
+        // D_J[16 columns of the chunk] = sum over the 128 rows, two column tiles at a time (a
+        // lone one as two sums, of even and odd K steps: half the chain).
+        const int kc = ti.kc0 + c + u, J = kc / kBlkChunks;
+        const double *A = Ac + u * kBK * ar + g * ar + t;
+        double *o = d + ti.planes +
+                    (int64_t)(ladder_plane(true, ti.nseg, J) + ti.mt) * kMaxBM * hs +
+                    (kc % kBlkChunks) * kBK * hs;
+#pragma unroll
+        for (int j0 = 0; j0 < C; j0 += 2) {
+          constexpr int kHalf = C == 1 ? 2 : 1;
+          double e[2][4] = {};
+          const double *B = Ti + t * hs + g + 8 * j0;
+#pragma unroll 2
+          for (int k0 = 0; k0 < kMaxBM; k0 += 16 * kHalf) {
+#pragma unroll
+            for (int kk = 0; kk < kHalf; ++kk) {
+              double a[8];
+#pragma unroll
+              for (int i = 0; i < 8; ++i)
+                a[i] = A[8 * (i % 2) * ar + k0 + 16 * kk + 4 * (i / 2)];
+#pragma unroll
+              for (int j = 0; j < min(2, C - j0); ++j) {
+                double b[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) b[q] = B[(k0 + 16 * kk + 4 * q) * hs + 8 * j];
+                dmma_16816(e[j + kk], a, b);
+              }
+            }
+          }
+#pragma unroll
+          for (int j = 0; j < min(2, C - j0); ++j)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const int r = g + 8 * (q >> 1), col = 8 * (j0 + j) + 2 * t + (q & 1);
+              if (kc * kBK + r < ti.pk && col < ti.hk)
+                o[r * hs + col] = C == 1 ? e[0][q] + e[1][q] : e[j][q];
+            }
+        }
       }
     }
     __syncwarp();
@@ -226,17 +257,15 @@ __device__ __forceinline__ bool consume_mma(const StageInfo &ti, const double *A
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int r = 16 * warp + g + 8 * (q >> 1), col = 8 * j + 2 * t + (q & 1);
-      if (r < ti.rows && col < ti.hk) d[ti.out + (int64_t)r * hs + col] = acc[j][q];
+      if (r < rows && col < ti.hk) d[ti.out + (int64_t)r * hs + col] = acc[j][q];
     }
   return true;
 }
 
+// Slack: fragment loads past hs in the last B stage and the last row of T_I.
 constexpr size_t kLadderSmem =
-    (size_t)kStages * (kMaxAS * kBK + kBK * kMaxNB) * 8 + kStages * sizeof(StageInfo) +
-    2 * kStages * 8 + kBK * 8;  // slack: the last B stage's fragment loads past hs
-// 80 registers: its nine warps then leave 8,704 registers of the fullest SM quarter (three ladder
-// warps) to the kernels beside it; at 94 a CTA of 8 warps of the ring did not fit and ran after
-// the ladder.
+    ((size_t)kStages * (kStageA + kStageB) + kMaxBM * kSymHS + 2 * kBK) * 8 +
+    kStages * sizeof(StageInfo) + (2 * kStages + 2) * 8;
 __global__ void __maxnreg__(80)
 pp_ladder_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *sched,
                  const double *__restrict__ v_t, const double *tq0, const double *tq1,
@@ -244,9 +273,11 @@ pp_ladder_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *sch
   if (skip_iteration(ctl, gate, kTrLadderThin)) return;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   double *As = reinterpret_cast<double *>(smem_raw);
-  double *Bs = As + kStages * kMaxAS * kBK;
-  StageInfo *info = reinterpret_cast<StageInfo *>(Bs + kStages * kBK * kMaxNB + kBK);
+  double *Bs = As + kStages * kStageA;
+  double *Ti = Bs + kStages * kStageB + kBK;
+  StageInfo *info = reinterpret_cast<StageInfo *>(Ti + kMaxBM * kSymHS + kBK);
   uint64_t *bars = reinterpret_cast<uint64_t *>(info + kStages);  // full, then empty
+  uint64_t *ti_full = bars + 2 * kStages, *ti_free = ti_full + 1;
   constexpr int kConsumerWarps = kLadderConsumers / 32;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
@@ -254,6 +285,8 @@ pp_ladder_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *sch
       mbar_init(smem_u32(&bars[s]), 1);
       mbar_init(smem_u32(&bars[kStages + s]), kConsumerWarps);
     }
+    mbar_init(smem_u32(ti_full), 1);
+    mbar_init(smem_u32(ti_free), kConsumerWarps);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
@@ -261,12 +294,13 @@ pp_ladder_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *sch
   if (warp == kConsumerWarps) {
     if (lane == 0) {
       const double *t_q = ctl->parity ? tq1 : tq0;
-      int gc = 0;  // chunks issued by this CTA
+      int gc = 0;   // stages issued by this CTA
+      int nti = 0;  // tiles with a T_I so far
       bool stop = false;
       // Test-only fault (ccdgpu_inject_wait_timeout): CTA 0 never fills its first stage, so
       // its consumers' bounded waits run out, then this producer's wait for that stage does.
       const bool withhold = ctl->inject != 0 && blockIdx.x == 0;
-      auto free_stage = [&]() {  // the stage of chunk gc may be filled
+      auto free_stage = [&]() {  // stage gc may be filled
         if (gc < kStages ||
             mbar_wait(smem_u32(&bars[kStages + gc % kStages]), ((gc / kStages) - 1) & 1))
           return true;
@@ -278,22 +312,47 @@ pp_ladder_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *sch
         const LadderTile tile = tiles[ti];
         // The next claim's latency hides behind this tile.
         ti = (int)gridDim.x + atomicAdd(&sched[0], 1);
-        const uint32_t abytes = ladder_arows(tile.hs, tile.rows) * kBK * 8;
+        const uint32_t abytes = ladder_as(tile.rows) * kBK * 8;  // a chunk's
         const uint32_t bbytes = kBK * tile.hs * 8;
+        const int per = ladder_stage(tile.hs);
         const double *asrc = v_t + tile.a_base, *bsrc = t_q + tile.b_base;
-        for (int c = 0; c < tile.nks; ++c, ++gc) {
+        // Chunks from diag_end on have a transposed product, which reads T_I.
+        const int diag_end = kBlkChunks * (tile.mt + 1) - tile.kc0;
+        bool need_ti = tile.sym && diag_end < tile.nks;
+        const bool has_ti = need_ti;
+        for (int c = 0; c < tile.nks; c += per, ++gc) {
           const int s = gc % kStages;
+          if (need_ti) {
+            // Once the previous tile's readers of the buffer are done; waited for only when the
+            // next chunk needs it.
+            bool ok = nti == 0 || mbar_try_wait(smem_u32(ti_free), (nti - 1) & 1);
+            if (!ok && c + per > diag_end) ok = mbar_wait(smem_u32(ti_free), (nti - 1) & 1);
+            if (ok) {
+              const uint32_t bytes = kMaxBM * tile.hs * 8;
+              mbar_expect_tx(smem_u32(ti_full), bytes);
+              bulk_g2s(smem_u32(Ti), t_q + tile.ti_base, bytes, smem_u32(ti_full));
+              need_ti = false;
+            } else if (c + per > diag_end) {
+              atomicOr(err, kErrTimeout);
+              stop = true;
+              break;
+            }
+          }
           if (!free_stage()) {
             stop = true;
             break;
           }
           if (withhold && gc == 0) continue;
-          if (c == 0) info[s] = StageInfo{tile.out, tile.rows, tile.hk, tile.hs, tile.nks};
+          if (c == 0)
+            info[s] = StageInfo{tile.out,  tile.planes, tile.rows, tile.hk, tile.hs, tile.nks,
+                                tile.kc0, tile.mt, has_ti ? tile.nseg : -1, tile.pk};
           const uint32_t full = smem_u32(&bars[s]);
-          mbar_expect_tx(full, abytes + bbytes);
-          bulk_g2s(smem_u32(As + s * kMaxAS * kBK), asrc + c * (abytes / 8), abytes, full);
-          bulk_g2s(smem_u32(Bs + s * kBK * kMaxNB), bsrc + c * (bbytes / 8), bbytes, full);
+          const int n = min(per, tile.nks - c);
+          mbar_expect_tx(full, n * (abytes + bbytes));
+          bulk_g2s(smem_u32(As + s * kStageA), asrc + c * (abytes / 8), n * abytes, full);
+          bulk_g2s(smem_u32(Bs + s * kStageB), bsrc + c * (bbytes / 8), n * bbytes, full);
         }
+        nti += has_ti;
       }
       if (!stop && free_stage()) {  // the end marker
         info[gc % kStages].nks = 0;
@@ -311,37 +370,52 @@ pp_ladder_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *sch
     return;
   }
   const int tid = threadIdx.x;
-  int gc = 0;
+  RingPos at;
+  int nti = 0;
   for (;;) {
-    // The first chunk's stage describes the tile.
-    const int s = gc % kStages;
-    if (!mbar_wait(smem_u32(&bars[s]), (gc / kStages) & 1)) {
+    // The first stage describes the tile.
+    if (!mbar_wait(smem_u32(&bars[at.s]), at.phase)) {
       atomicOr(err, kErrTimeout);
       break;
     }
-    const StageInfo ti = info[s];
+    const StageInfo ti = info[at.s];
     if (ti.nks == 0) break;
     bool ok = true;
-    if (ti.hs <= 4) {
-      switch (ti.hs) {
-        case 1: ok = consume_thin<1>(ti, As, Bs, bars, tid, gc, d); break;
-        case 2: ok = consume_thin<2>(ti, As, Bs, bars, tid, gc, d); break;
-        default: ok = consume_thin<4>(ti, As, Bs, bars, tid, gc, d); break;
-      }
-    } else {
-      switch ((ti.hk + 7) / 8) {
-        case 1: ok = consume_mma<1>(ti, As, Bs, bars, tid, gc, d); break;
-        case 2: ok = consume_mma<2>(ti, As, Bs, bars, tid, gc, d); break;
-        case 3: ok = consume_mma<3>(ti, As, Bs, bars, tid, gc, d); break;
-        case 4: ok = consume_mma<4>(ti, As, Bs, bars, tid, gc, d); break;
-        default: ok = consume_mma<5>(ti, As, Bs, bars, tid, gc, d); break;
-      }
+    const uint32_t tb = smem_u32(ti_full), tp = nti & 1;
+    const bool full = ti.rows == kMaxBM;
+    switch ((ti.hk + 7) / 8) {
+      case 1:
+        ok = full ? consume_mma<1, true>(ti, As, Bs, Ti, bars, tb, tp, tid, at, d)
+                  : consume_mma<1, false>(ti, As, Bs, Ti, bars, tb, tp, tid, at, d);
+        break;
+      case 2:
+        ok = full ? consume_mma<2, true>(ti, As, Bs, Ti, bars, tb, tp, tid, at, d)
+                  : consume_mma<2, false>(ti, As, Bs, Ti, bars, tb, tp, tid, at, d);
+        break;
+      case 3:
+        if (ti.hs <= kSymHS)
+          ok = full ? consume_mma<3, true>(ti, As, Bs, Ti, bars, tb, tp, tid, at, d)
+                    : consume_mma<3, false>(ti, As, Bs, Ti, bars, tb, tp, tid, at, d);
+        else
+          ok = consume_mma<4, false>(ti, As, Bs, Ti, bars, tb, tp, tid, at, d);
+        break;
+      case 4: ok = consume_mma<4, false>(ti, As, Bs, Ti, bars, tb, tp, tid, at, d); break;
+      default: ok = consume_mma<5, false>(ti, As, Bs, Ti, bars, tb, tp, tid, at, d); break;
     }
     if (!ok) {  // a timed-out tile leaves its rows unfinished
       atomicOr(err, kErrTimeout);
       break;
     }
-    gc += ti.nks;
+    if (ti.nseg >= 0) {
+      // A warp that had no turn passes T_I's phase all the same before it frees the buffer.
+      if (!mbar_wait(tb, tp)) {
+        atomicOr(err, kErrTimeout);
+        break;
+      }
+      ++nti;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(ti_free));
+    }
   }
   trace_end(ctl, kTrLadderThin);
 }
@@ -1170,14 +1244,17 @@ constexpr int kQuadPerItem = kAsmThreads;  // one quad per thread and item
 constexpr int kAsmCTAsPerSM = 5;
 static_assert(kQuadPerItem == kPostThreads, "hh_post_kernel works on the same items");
 
-// D of quad position p of a channel: the ladder's planes in order, then T X.
-__device__ __forceinline__ double quad_d(const LadderChan &lc, const double *__restrict__ dp,
-                                         const double *__restrict__ tx, int64_t q_off,
+// D of quad (u, w) at packed position p: the planes of its row tile in order, then T X.
+__device__ __forceinline__ double quad_d(const LadderRows *__restrict__ lrows, int rt_off,
+                                         const double *__restrict__ dp,
+                                         const double *__restrict__ tx, int u, int w, int hs,
                                          int64_t p) {
-  const double *d = dp + lc.base + (p - q_off);
+  const LadderRows lr = lrows[rt_off + (u >> 7)];
+  const double *d = dp + lr.base + (u & 127) * hs + w;
   const double x = __ldcg(tx + p);
   double v = __ldcg(d);
-  for (int s = 1; s < lc.nseg; ++s) v += __ldcg(d + (int64_t)s * lc.plane);
+#pragma unroll 4
+  for (int s = 1; s < lr.n; ++s) v += __ldcg(d + (int64_t)s * lr.stride);
   return v + x;
 }
 
@@ -1204,7 +1281,7 @@ __device__ __forceinline__ double quad_value(double v, double dm, double2 s, dou
 template <bool LOOP>
 __global__ void __launch_bounds__(kAsmThreads, kAsmCTAsPerSM)
 assemble_fused_kernel(const QuadItem *__restrict__ items, int n_items,
-                      const ChanInfo *__restrict__ chans, const LadderChan *__restrict__ lchans,
+                      const ChanInfo *__restrict__ chans, const LadderRows *__restrict__ lrows,
                       const QuadRow *__restrict__ qrows, const QuadCol *__restrict__ qcols,
                       const double *__restrict__ vq, const double *__restrict__ dp,
                       const double *__restrict__ tx, const double *__restrict__ r_quad,
@@ -1240,7 +1317,7 @@ assemble_fused_kernel(const QuadItem *__restrict__ items, int n_items,
     const QuadCol cl = qcols[item.qcol_off + w];
     const double tv = t_old[p], vv = __ldg(vq + p);
     const double2 ring = __ldcg(reinterpret_cast<const double2 *>(r_quad + 2 * p));
-    const double dv = quad_d(lchans[item.ch], dp, tx, item.q_off, p);
+    const double dv = quad_d(lrows, item.rt_off, dp, tx, u, w, item.hs, p);
     // The one-body sums are small arrays every quad reads: through L1 (an L2-only load
     // would send every warp to the same few L2 slices).
     const double t1 = quad_value(vv, dv, ring, tv, xh[cl.i], xh[cl.j], yp[rw.pa], yp[rw.pb],
@@ -1273,14 +1350,14 @@ assemble_fused_kernel(const QuadItem *__restrict__ items, int n_items,
 // four elements as +D, -D, -D, +D; rows a = b and columns i = j stay zero.
 __global__ void __launch_bounds__(kAsmThreads)
 expand_d_kernel(const QuadItem *__restrict__ items, const ChanInfo *__restrict__ chans,
-                const LadderChan *__restrict__ lchans, const QuadRow *__restrict__ qrows,
+                const LadderRows *__restrict__ lrows, const QuadRow *__restrict__ qrows,
                 const QuadCol *__restrict__ qcols, const double *__restrict__ dp,
                 const double *__restrict__ tx, double *__restrict__ d) {
   const QuadItem item = items[blockIdx.x];
   const int q = item.q0 + threadIdx.x;
   if (q >= item.q1) return;
   const int u = q / item.hk, w = q - u * item.hk;
-  const double v = quad_d(lchans[item.ch], dp, tx, item.q_off,
+  const double v = quad_d(lrows, item.rt_off, dp, tx, u, w, item.hs,
                           item.q_off + (int64_t)u * item.hs + w);
   const QuadRow rw = qrows[item.pk_off + u];
   const QuadCol cl = qcols[item.qcol_off + w];

@@ -41,13 +41,30 @@ __global__ void tile_v_kernel(const ChanInfo *__restrict__ chans, const int4 *__
   const int u = it.y;
   const double *src = vraw + vraw_off[it.x] + (int64_t)it.z * ch.pp;
   const int mt = u / kMaxBM, r = u % kMaxBM, rows = min(kMaxBM, ch.pk - mt * kMaxBM);
-  const int ar = ladder_arows(ch.hs, rows);
-  const int64_t tb = ch.vkt_base + (int64_t)mt * ladder_arows_full(ch.hs) * ch.nkc * kBK;
-  for (int w = threadIdx.x; w < ch.pk; w += blockDim.x) {
-    const int k = w % kBK;
-    v_t[tb + (int64_t)(w / kBK) * ar * kBK + (ladder_kmajor(ch.hs) ? k * ar + r : swzA(r, k))] =
+  const int ar = ladder_as(rows);
+  for (int w = ladder_kc0(ch.sym, mt) * kBK + threadIdx.x; w < ch.pk; w += blockDim.x)
+    v_t[ch.vkt_base + ladder_chunk(ch.sym, ch.nkc, mt, w / kBK, rows) + (w % kBK) * ar + r] =
         src[kcol[ch.pk_off + w]];
+}
+
+// Whether each channel's packed V is symmetric, element for element (the ladder then streams half
+// of it): one CTA per packed row, against the column above the diagonal.
+__global__ void v_symmetry_kernel(const ChanInfo *__restrict__ chans, const int4 *__restrict__ items,
+                                  const int32_t *__restrict__ kcol,
+                                  const int32_t *__restrict__ prow_raw,
+                                  const int64_t *__restrict__ vraw_off,
+                                  const double *__restrict__ vraw, int32_t *asym) {
+  const int4 it = items[blockIdx.x];
+  const ChanInfo ch = chans[it.x];
+  const double *src = vraw + vraw_off[it.x] + (int64_t)it.z * ch.pp;
+  const int col = kcol[ch.pk_off + it.y];
+  bool differs = false;
+  for (int w = it.y + 1 + threadIdx.x; w < ch.pk; w += blockDim.x) {
+    const double a = src[kcol[ch.pk_off + w]];
+    const double b = vraw[vraw_off[it.x] + (int64_t)prow_raw[ch.pk_off + w] * ch.pp + col];
+    differs |= !(a == b);
   }
+  if (differs) asym[it.x] = 1;
 }
 
 // Packed V_pppp as nt bf16 terms in the tensor-core chunk images of the mixed-precision
@@ -298,7 +315,7 @@ __global__ void normal_order_kernel(ModelDev m, const double *__restrict__ bare,
 // V_pppp generated straight into the ladders' operand images, one CTA per image chunk, so that
 // each CTA writes one contiguous block (the chunk's elements in image order; padding rows and
 // K columns past pk get zeros).  FP64 ladder: items (channel, row tile, 16-deep K chunk), block
-// of ar x kBK doubles, k-major (wider channels) or XOR-swizzled rows (thin class).  The
+// of ar x kBK doubles, k-major.  The
 // tensor-core images of mixed handles come with the FP64 tiles from gen_v_both_chunks_kernel.
 template <bool EG>  // EG: the electron gas's orbital-code path only (fewer registers)
 __global__ void __launch_bounds__(256)
@@ -310,10 +327,8 @@ gen_v_chunks_kernel(const ChanInfo *__restrict__ chans, const int4 *__restrict__
   const int4 it = items[blockIdx.x];
   const ChanInfo ch = chans[it.x];
   const int mt = it.y, kc = it.z;
-  const int rows = min(kMaxBM, ch.pk - mt * kMaxBM), ar = ladder_arows(ch.hs, rows);
-  const bool kmajor = ladder_kmajor(ch.hs);
-  double *out = v_t + ch.vkt_base + (int64_t)mt * ladder_arows_full(ch.hs) * ch.nkc * kBK +
-                (int64_t)kc * ar * kBK;
+  const int rows = min(kMaxBM, ch.pk - mt * kMaxBM), ar = ladder_as(rows);
+  double *out = v_t + ch.vkt_base + ladder_chunk(ch.sym, ch.nkc, mt, kc, rows);
   if (EG) {  // the codes once per chunk, not once per element
     for (int r = threadIdx.x; r < rows; r += blockDim.x) {
       const int2 ab = pp_pairs[ch.pp_off + kcol[ch.pk_off + mt * kMaxBM + r]];
@@ -329,14 +344,7 @@ gen_v_chunks_kernel(const ChanInfo *__restrict__ chans, const int4 *__restrict__
     __syncthreads();
   }
   for (int e = threadIdx.x; e < ar * kBK; e += blockDim.x) {
-    int r, k;
-    if (kmajor) {
-      k = e / ar;
-      r = e - k * ar;
-    } else {
-      r = e >> 4;
-      k = (e & 15) ^ (r & 15);  // swzA(r, k) = 16 r + (k ^ (r & 15))
-    }
+    const int k = e / ar, r = e - k * ar;
     const int u = mt * kMaxBM + r, w = kc * kBK + k;
     double v = 0.0;
     if (r < rows && w < ch.pk) {
@@ -428,22 +436,14 @@ gen_v_both_chunks_kernel(const ChanInfo *__restrict__ chans, const int4 *__restr
     for (int p = 0; p < NT; ++p) v_tc[p * tc_stride + base + e] = hv[p];
   }
   // FP64 chunks 2 kc and 2 kc + 1, as gen_v_chunks_kernel (rows past `rows` are zero).
-  const int ar = ladder_arows(ch.hs, rows);
-  const bool kmajor = ladder_kmajor(ch.hs);
+  const int ar = ladder_as(rows);
   for (int h = 0; h < 2; ++h) {
     const int kc64 = 2 * kc + h;
     if (kc64 >= ch.nkc) break;
-    double *out = v_t + ch.vkt_base + (int64_t)mt * ladder_arows_full(ch.hs) * ch.nkc * kBK +
-                  (int64_t)kc64 * ar * kBK;
+    if (kc64 < ladder_kc0(ch.sym, mt)) continue;  // below the diagonal
+    double *out = v_t + ch.vkt_base + ladder_chunk(ch.sym, ch.nkc, mt, kc64, rows);
     for (int e = threadIdx.x; e < ar * kBK; e += blockDim.x) {
-      int r, k;
-      if (kmajor) {
-        k = e / ar;
-        r = e - k * ar;
-      } else {
-        r = e >> 4;
-        k = (e & 15) ^ (r & 15);  // swzA(r, k) = 16 r + (k ^ (r & 15))
-      }
+      const int k = e / ar, r = e - k * ar;
       out[e] = r < rows ? tile[(h * kBK + k) * kGenLd + r] : 0.0;
     }
   }

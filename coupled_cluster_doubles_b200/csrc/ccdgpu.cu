@@ -60,6 +60,7 @@ struct ccdgpu_handle {
   int64_t n_t = 0, n_m = 0, n_h = 0, n_p = 0;
   int n_hh_cta = 0, n_hh_warp = 0;  // hh-ladder units: one per CTA (hk > 8) first, then per warp
   int n_hh_out = 0;    // hh-ladder reduction outputs
+  int n_row_tiles = 0;  // row tiles of all channels
   int n_act = 0, n_mod = 0, n_mod_small = 0, n_mod_mid = 0, n_tiles = 0;
   int n_ranges = 0;
   int n_asm_blocks = 0;  // fused assembly CTAs (persistent, striding over quad_items)
@@ -144,7 +145,7 @@ struct ccdgpu_handle {
   ccdgpu_schedule schedule{};
   void *tile_mem = nullptr;
   size_t tile_bytes = 0;
-  LadderChan *lchans = nullptr, *tc_lchans = nullptr;  // D planes per channel
+  LadderRows *lrows = nullptr, *tc_lrows = nullptr;  // D planes per row tile
   double *d_planes = nullptr, *tc_planes = nullptr;
   // Tile counter and exit ticket of the FP64 ladder, then of the tensor-core ladder (zero
   // between launches).
@@ -776,12 +777,12 @@ int materialize_d(ccdgpu_handle *h);
 
 // pp-ladder work tiles for a schedule (split factors of K per column class), in their own
 // device allocation with the D planes they write; drops captured graphs, which hold the old
-// lists.  Row blocks stream at full bandwidth on their own, so K is split (into segments of at
-// least four chunks) only until a class has about its split factor's number of tiles per SM:
-// thin ones when there are fewer blocks than SMs, up to thin_split_mul tiles per SM; mid and
-// wide ones, compute bound per CTA, to about wide_split_mul (mid_split_mul); the tensor-core
-// ladder to about tc_split_mul.  Each segment writes its own plane of the channel's D, which the
-// assembly adds in segment order (deterministic).
+// lists.  An FP64 class is cut into K segments of at most 1 / (148 mul) of all the classes' chunks
+// (mul: its split factor, three times that for the wide class, whose chunks take three times as
+// long): longer tiles would leave SMs idle at the end, shorter ones cost planes (EG N=54
+// |n|^2 <= 36: 171 us an iteration at mul = 1 to 4, 175 at 8, 180 at 16).  The tensor-core
+// ladder's row tiles are cut into about tc_split_mul tiles per SM of at least four chunks.  Each
+// segment writes its own plane, which the assembly adds in segment order (deterministic).
 // The persistent CTAs claim tiles in list order from a launch-wide counter: FP64 tiles by class,
 // wide first (the longest work per byte), then by decreasing cost, the tensor-core tiles by
 // decreasing cost.  Cost = bytes streamed per K chunk x chunks, plus two chunks' worth for the
@@ -791,45 +792,57 @@ int make_ladder_tiles(ccdgpu_handle *h, const ccdgpu_schedule &sch) {
   const std::vector<ChanInfo> &chans = h->host_chans;
   const int64_t kSMs = 148;
   const int mid_mul = sch.mid_split_mul > 0 ? sch.mid_split_mul : sch.wide_split_mul;
-  int64_t blocks[3] = {0, 0, 0}, tc_blocks = 0;
+  int64_t chunks = 0, tc_blocks = 0;
   for (const ChanInfo &a : chans) {
-    if (a.nmt) blocks[ladder_class(a.hs)] += a.nmt;
+    for (int mt = 0; mt < a.nmt; mt++) chunks += a.nkc - ladder_kc0(a.sym, mt);
     tc_blocks += a.nmt;
   }
   auto want_of = [&](int64_t mul, int64_t b, int64_t most) {
     return (int)std::min<int64_t>(most, std::max<int64_t>(1, ceil_div(mul * kSMs, std::max<int64_t>(b, 1))));
   };
-  const int want_cls[3] = {blocks[0] >= kSMs ? 1 : want_of(sch.thin_split_mul, blocks[0], 8),
-                           want_of(mid_mul, blocks[1], 64),
-                           want_of(sch.wide_split_mul, blocks[2], 64)};
+  // Longest K segment of a class, in chunks.
+  auto longest_of = [&](int64_t mul) { return (int)std::max<int64_t>(4, ceil_div(chunks, mul * kSMs)); };
+  const int longest[3] = {longest_of(sch.thin_split_mul), longest_of(mid_mul),
+                          longest_of(3 * sch.wide_split_mul)};
   const int want_tc = want_of(sch.tc_split_mul, tc_blocks, 32);
   struct Key {
     int64_t cost;
     int32_t cls, pos;
   };
-  auto make = [&](bool tc, std::vector<LadderTile> &out, std::vector<LadderChan> &lchans,
+  auto make = [&](bool tc, std::vector<LadderTile> &out, std::vector<LadderRows> &lrows,
                   int64_t &planes) {
     std::vector<LadderTile> tiles;
     std::vector<Key> keys;
-    lchans.assign(h->n_act, LadderChan{0, 1, 0});
+    lrows.assign(h->n_row_tiles, LadderRows{0, 1, 0});
     planes = 0;
     for (int ai = 0; ai < h->n_act; ai++) {
       const ChanInfo &a = chans[ai];
       if (!a.nmt) continue;
       const int nk = tc ? a.nkct : a.nkc;
-      const int want = tc ? want_tc : want_cls[ladder_class(a.hs)];
-      const int nseg = std::max(1, std::min(want, nk / 4));
-      const int64_t plane = (int64_t)a.nkc * kBK * a.hs;
-      lchans[ai] = LadderChan{planes, nseg, (int32_t)plane};
+      auto segs = [&](int len) {
+        return tc ? std::max(1, std::min(want_tc, len / 4))
+                  : (int)ceil_div(len, longest[ladder_class(a.hs)]);
+      };
+      const int room = segs(nk);  // segments of the longest row tile
+      const bool sym = !tc && a.sym;
+      const int64_t plane = (int64_t)kMaxBM * a.hs;
       for (int mt = 0; mt < a.nmt; mt++) {
-        const int rows = std::min(kMaxBM, a.pk - mt * kMaxBM);
+        const int rows = std::min(kMaxBM, a.pk - mt * kMaxBM), first = ladder_kc0(sym, mt);
+        const int len = nk - first, nseg = segs(len);
+        const int64_t base = planes + ladder_plane(sym, room, mt) * plane;
+        const int direct = sym ? mt : 0;  // planes of the transposed blocks come first
+        lrows[a.rt_off + mt] = LadderRows{base, direct + nseg, (int32_t)plane};
         for (int sg = 0; sg < nseg; sg++) {
           LadderTile t{};
           t.ch = ai; t.mt = mt; t.rows = rows;
-          t.kc0 = (int)((int64_t)nk * sg / nseg);
-          t.nks = (int)((int64_t)nk * (sg + 1) / nseg) - t.kc0;
+          // Whole stages of two chunks.
+          auto cut = [&](int k) { return k == nseg ? nk : first + 2 * (int)((int64_t)(len / 2) * k / nseg); };
+          t.kc0 = cut(sg);
+          t.nks = cut(sg + 1) - t.kc0;
           t.hk = a.hk; t.hs = a.hs; t.nb = a.nbt;
-          t.out = planes + sg * plane + (int64_t)mt * kMaxBM * a.hs;
+          t.sym = sym; t.nseg = room; t.pk = a.pk;
+          t.out = base + (direct + sg) * plane;
+          t.planes = planes;
           int64_t cost;
           if (tc) {
             const int rg = (rows + 7) / 8, ng = a.nbt / 8;
@@ -837,16 +850,16 @@ int make_ladder_tiles(ccdgpu_handle *h, const ccdgpu_schedule &sch) {
             t.b_base = a.tkt_tc_base + (int64_t)t.kc0 * ng * kTcGroup;
             cost = (int64_t)(t.nks + 2) * (8 * rg + a.nbt);
           } else {
-            const int ar = ladder_arows(a.hs, rows);
-            t.a_base = a.vkt_base + ((int64_t)mt * ladder_arows_full(a.hs) * nk + (int64_t)t.kc0 * ar) * kBK;
+            t.a_base = a.vkt_base + ladder_chunk(sym, nk, mt, t.kc0, rows);
             t.b_base = a.q_off + (int64_t)t.kc0 * kBK * a.hs;
-            cost = (int64_t)(t.nks + 2) * (ar + a.hs);
+            t.ti_base = a.q_off + (int64_t)mt * kMaxBM * a.hs;
+            cost = (int64_t)(t.nks + 2) * (ladder_as(rows) + a.hs);
           }
           keys.push_back(Key{cost, tc ? 0 : 2 - ladder_class(a.hs), (int32_t)tiles.size()});
           tiles.push_back(t);
         }
       }
-      planes += nseg * plane;
+      planes += ladder_plane(sym, room, a.nmt) * plane;
     }
     std::sort(keys.begin(), keys.end(), [](const Key &x, const Key &y) {
       return x.cls != y.cls ? x.cls < y.cls : x.cost != y.cost ? x.cost > y.cost : x.pos < y.pos;
@@ -855,10 +868,10 @@ int make_ladder_tiles(ccdgpu_handle *h, const ccdgpu_schedule &sch) {
     for (size_t i = 0; i < keys.size(); i++) out[i] = tiles[keys[i].pos];
   };
   std::vector<LadderTile> tiles, tc_tiles;
-  std::vector<LadderChan> lchans, tc_lchans;
+  std::vector<LadderRows> lrows, tc_lrows;
   int64_t planes = 0, tc_planes = 0;
-  make(false, tiles, lchans, planes);
-  if (h->nt) make(true, tc_tiles, tc_lchans, tc_planes);
+  make(false, tiles, lrows, planes);
+  if (h->nt) make(true, tc_tiles, tc_lrows, tc_planes);
   // Device copies: one allocation, written on s3, which s0 then waits for.  A schedule that
   // replaces another first waits for the handle's work in flight (the old lists may be in use);
   // the first one, made in create while the set-up kernels run on s0, has nothing to wait for,
@@ -877,13 +890,13 @@ int make_ladder_tiles(ccdgpu_handle *h, const ccdgpu_schedule &sch) {
   h->tile_mem = nullptr;
   h->tile_bytes = 0;
   h->tiles = h->tc_tiles = nullptr;
-  h->lchans = h->tc_lchans = nullptr;
+  h->lrows = h->tc_lrows = nullptr;
   h->d_planes = h->tc_planes = nullptr;
   h->sched = nullptr;
   h->n_tiles = h->n_tc_tiles = 0;
   Arena ar;
   ar.add(&h->tiles, tiles.size()); ar.add(&h->tc_tiles, tc_tiles.size());
-  ar.add(&h->lchans, lchans.size()); ar.add(&h->tc_lchans, tc_lchans.size());
+  ar.add(&h->lrows, lrows.size()); ar.add(&h->tc_lrows, tc_lrows.size());
   ar.add(&h->sched, kSched);
   ar.add(&h->d_planes, planes); ar.add(&h->tc_planes, tc_planes);
   CK(dev_alloc(ar.used, &h->tile_mem, &h->tile_bytes));
@@ -897,8 +910,8 @@ int make_ladder_tiles(ccdgpu_handle *h, const ccdgpu_schedule &sch) {
   };
   if (int rc = up(h->tiles, tiles)) return rc;
   if (int rc = up(h->tc_tiles, tc_tiles)) return rc;
-  if (int rc = up(h->lchans, lchans)) return rc;
-  if (int rc = up(h->tc_lchans, tc_lchans)) return rc;
+  if (int rc = up(h->lrows, lrows)) return rc;
+  if (int rc = up(h->tc_lrows, tc_lrows)) return rc;
   CK(cudaEventRecord(h->ev_fork2, h->s3));
   CK(cudaStreamWaitEvent(h->s0, h->ev_fork2, 0));
   if (!first) CK(cudaStreamSynchronize(h->s0));
@@ -1119,6 +1132,9 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     if (pk && hk) {
       ci.nkc = (int)ceil_div(pk, kBK);
       ci.nmt = (int)ceil_div(pk, kMaxBM);
+      ci.sym = hk <= kSymHK;  // stored V: unless it turns out not to be symmetric
+      ci.rt_off = h->n_row_tiles;
+      h->n_row_tiles += ci.nmt;
       const int rows = kHHRows;  // K slice of the hh ladder
       ci.nhht = (int)ceil_div(pk, rows);
       ci.nbt = tc_nb(hk);
@@ -1127,10 +1143,8 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
       tkttc += (int64_t)ci.nkct * (ci.nbt / 8) * kTcGroup;
       x_tot += hk * ci.hs;
       q_tot += (int64_t)ci.nkc * kBK * ci.hs;
-      // Full row tiles at their A stride, then the compact last one.
-      const int64_t arows_tot = (int64_t)(ci.nmt - 1) * ladder_arows_full(ci.hs) +
-                                ladder_arows(ci.hs, pk - (ci.nmt - 1) * kMaxBM);
-      vt += (int64_t)ci.nkc * arows_tot * kBK;
+      // Stored V: room for the whole of it, should it not be symmetric.
+      vt += ladder_chunk(on_the_fly && ci.sym, ci.nkc, ci.nmt - 1, ci.nkc, pk - (ci.nmt - 1) * kMaxBM);
       part_tot += (int64_t)ci.nhht * hk * hk;
       for (int t = 0; t < ci.nhht; t++)
         hh_tiles.push_back({ai, t * rows, t, std::min(rows, pk - t * rows)});
@@ -1440,7 +1454,7 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     if (nq >= ((int64_t)1 << 31) / 2) return CCDGPU_ERR_UNSUPPORTED;
     for (int64_t q = 0; q < nq; q += kQuadPerItem)
       quad_items.push_back({ai, (int32_t)q, (int32_t)std::min<int64_t>(nq, q + kQuadPerItem),
-                            a.hk, a.hs, 0, a.q_off, a.x_off, a.pk_off, a.qcol_off});
+                            a.hk, a.hs, a.rt_off, a.q_off, a.x_off, a.pk_off, a.qcol_off});
     const QuadCol *qc = quad_cols.data() + a.qcol_off;
     for (int kl = 0; nq && kl < a.hk; kl++)
       for (int ij = 0; ij < a.hk; ij++)
@@ -1468,9 +1482,11 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   }
   for (const ModInfo &m : mods) fl += 4.0 * m.ph * (double)m.hp * m.hp;
   h->flops = fl; h->ladder_flops = lf; h->v_bytes = vb; h->v_packed_bytes = vbp;
-  // Bytes one pp-ladder launch must move: packed V, the packed amplitudes in and D out.
+  // Bytes one pp-ladder launch must move: packed V (of a symmetric channel one triangle), the
+  // packed amplitudes in and D out.
   double lb = vbp;
-  for (const ChanInfo &a : chans) lb += 16.0 * (double)a.pk * a.hk;
+  for (const ChanInfo &a : chans)
+    lb += 16.0 * (double)a.pk * a.hk - (a.sym ? 4.0 * a.pk * (a.pk - 1.0) : 0.0);
   h->ladder_bytes = lb;
   double lbt = 0;
   for (const ChanInfo &a : chans)
@@ -1583,6 +1599,7 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   int32_t *counts = nullptr;
   int2 *d_mod_dims = nullptr;
   int4 *d_vrows = nullptr;
+  int32_t *d_prow_raw = nullptr, *d_asym = nullptr;
   int4 *d_gv_items = nullptr, *d_gvt_items = nullptr;
   // Generated V_pppp: one item per operand-image chunk (channel, row tile, K chunk).
   // Counted per channel, then filled in parallel, each channel at its offset.
@@ -1595,7 +1612,9 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     std::vector<int64_t> go(h->n_act + 1, 0), gto(h->n_act + 1, 0);
     for (int ai = 0; ai < h->n_act; ai++) {
       const ChanInfo &a = chans[ai];
-      go[ai + 1] = go[ai] + (tc_images ? 0 : (int64_t)a.nmt * a.nkc);
+      int64_t chunks = 0;
+      for (int mt = 0; mt < a.nmt; mt++) chunks += a.nkc - ladder_kc0(a.sym, mt);
+      go[ai + 1] = go[ai] + (tc_images ? 0 : chunks);
       gto[ai + 1] = gto[ai] + (tc_images ? (int64_t)a.nmt * a.nkct : 0);
     }
     gv_items.resize(go[h->n_act]);
@@ -1606,7 +1625,7 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
       int4 *g = gv_items.data() + go[ai];
       if (!tc_images)
         for (int mt = 0; mt < a.nmt; mt++)
-          for (int kc = 0; kc < a.nkc; kc++) *g++ = make_int4(ai, mt, kc, 0);
+          for (int kc = ladder_kc0(a.sym, mt); kc < a.nkc; kc++) *g++ = make_int4(ai, mt, kc, 0);
       int4 *gt = gvt_items.data() + gto[ai];
       if (tc_images)
         for (int mt = 0; mt < a.nmt; mt++)
@@ -1694,6 +1713,10 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   sc.add(&vraw, vraw_tot); sc.add(&hhpp_raw, gen_v ? 0 : n_t);
   sc.add(&hpph_raw, gen_v ? 0 : h->n_m);
   sc.add(&counts, (size_t)5 * n_t); sc.add(&d_vrows, vrows.size());
+  // Row of V_pppp's uploaded rows (a <= b) of each packed row, and a mark per channel.
+  std::vector<int32_t> prow_raw(on_the_fly ? 0 : kcol.size());
+  for (const int4 &v : vrows) prow_raw[chans[v.x].pk_off + v.y] = v.z;
+  sc.add(&d_prow_raw, prow_raw.size()); sc.add(&d_asym, n_act);
   sc.add(&d_gv_items, gv_items.size()); sc.add(&d_gvt_items, gvt_items.size());
   sc.add(&d_vraw_off, vraw_off.size()); sc.add(&d_mod_dims, mod_dims.size()); sc.add(&d_o_m, o_m.size());
   // The model on the device (on-the-fly V, E_ref and normal ordering): quantum numbers and
@@ -1789,7 +1812,7 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   TRY(put(h->list_off, list_off)); TRY(put(h->list, list));
   TRY(put(h->prow, prow)); TRY(put(h->hcol, hcol));
   TRY(put(h->o_h, o_h)); TRY(put(h->o_p, o_p));
-  TRY(put(d_vrows, vrows)); TRY(put(d_vraw_off, vraw_off));
+  TRY(put(d_vrows, vrows)); TRY(put(d_vraw_off, vraw_off)); TRY(put(d_prow_raw, prow_raw));
   TRY(put(d_gv_items, gv_items)); TRY(put(d_gvt_items, gvt_items));
   TRY(put(d_mod_dims, mod_dims)); TRY(put(d_o_m, o_m));
   batch.push_back(UploadPiece{reinterpret_cast<char *>(h->eps),
@@ -1957,6 +1980,25 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
                                                            h->n_vtc);
       }
     } else {
+      // Channels whose V is not symmetric are stored and streamed in full.
+      v_symmetry_kernel<<<(unsigned)vrows.size(), 128, 0, h->s0>>>(
+          h->chans, d_vrows, h->kcol, d_prow_raw, d_vraw_off, vraw, d_asym);
+      CK(cudaGetLastError());
+      std::vector<int32_t> asym(n_act);
+      CK(cudaMemcpyAsync(asym.data(), d_asym, n_act * sizeof(int32_t), cudaMemcpyDeviceToHost,
+                         h->s0));
+      CK(cudaStreamSynchronize(h->s0));
+      bool any = false;
+      for (int ai = 0; ai < n_act; ai++)
+        if (asym[ai] && h->host_chans[ai].sym) {
+          ChanInfo &a = h->host_chans[ai];
+          a.sym = 0;
+          h->ladder_bytes += 4.0 * a.pk * (a.pk - 1.0);
+          any = true;
+        }
+      if (any)
+        CK(cudaMemcpy(h->chans, h->host_chans.data(), n_act * sizeof(ChanInfo),
+                      cudaMemcpyHostToDevice));
       tile_v_kernel<<<(unsigned)vrows.size(), 128, 0, h->s0>>>(h->chans, d_vrows, h->kcol,
                                                                d_vraw_off, vraw, h->v_t);
     }
@@ -2094,7 +2136,7 @@ int launch_pp_ladder(ccdgpu_handle *h, cudaStream_t st, int cls = -1) {
 int launch_expand_d(ccdgpu_handle *h, bool tc) {
   if (!h->n_quad_items) return CCDGPU_OK;
   expand_d_kernel<<<h->n_quad_items, kAsmThreads, 0, h->s0>>>(
-      h->quad_items, h->chans, tc ? h->tc_lchans : h->lchans, h->quad_rows, h->quad_cols,
+      h->quad_items, h->chans, tc ? h->tc_lrows : h->lrows, h->quad_rows, h->quad_cols,
       tc ? h->tc_planes : h->d_planes, h->tx, h->dmat);
   h->launches++;
   return cuda_status(cudaGetLastError());
@@ -2205,7 +2247,7 @@ int launch_assemble_fused(ccdgpu_handle *h, cudaStream_t st, int gate) {
   return cuda_status(launch_pdl(
       h->loop_capture ? assemble_fused_kernel<true> : assemble_fused_kernel<false>,
       h->n_asm_blocks, kAsmThreads, 0, st, (const QuadItem *)h->quad_items, h->n_quad_items,
-      (const ChanInfo *)h->chans, (const LadderChan *)(gate ? h->tc_lchans : h->lchans),
+      (const ChanInfo *)h->chans, (const LadderRows *)(gate ? h->tc_lrows : h->lrows),
       (const QuadRow *)h->quad_rows, (const QuadCol *)h->quad_cols, (const double *)h->vq,
       (const double *)(gate ? h->tc_planes : h->d_planes), (const double *)h->tx,
       (const double *)h->r_quad, (const double *)h->xh, (const double *)h->yp, h->tq[0], h->tq[1],
@@ -3194,9 +3236,10 @@ int ccdgpu_ladder_profile(ccdgpu_handle *h, int32_t reps, double *ms, double *fl
   for (const ChanInfo &a : h->host_chans) {
     if (!a.nmt) continue;
     const int k = ladder_class(a.hs);
+    // Algorithmic traffic: a symmetric channel's V once on and above the diagonal.
     const double v = (double)a.pk * a.pk, q = (double)a.pk * a.hk;
     flops[k] += 2.0 * v * a.hk;
-    bytes[k] += 8.0 * (v + 2.0 * q);
+    bytes[k] += 8.0 * ((a.sym ? 0.5 * (v + a.pk) : v) + 2.0 * q);
     if (h->nt) {
       flops[3] += 2.0 * v * a.hk;
       bytes[3] += 2.0 * h->nt * ((h->tc_gen ? 0.0 : v) + q) + 8.0 * q;

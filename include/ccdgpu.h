@@ -322,9 +322,10 @@ int ccdgpu_work_per_iteration(const ccdgpu_handle *h, double *flops, double *lad
                               double *ladder_flops);
 
 /* pp-ladder schedule (no counterpart in the reference): how far the K dimension of each
- * channel block is split into deterministic partial sums, as a target of tiles per SM for the
- * FP64 thin class (at most 4 strict hole pairs i < j), the FP64 mid/wide classes, and the
- * tensor-core ladder. */
+ * channel block is split into deterministic partial sums: for the FP64 thin class (at most 4 strict
+ * hole pairs i < j) and the FP64 mid and wide classes into segments of at most 1 / (148 x the
+ * value) of the ladder's K chunks (wide: a third of that), for the tensor-core ladder into about
+ * that many tiles per SM. */
 typedef struct ccdgpu_schedule {
   int32_t thin_split_mul;      /* default 1 */
   int32_t wide_split_mul;      /* default 3: FP64 wide class (also mid when mid is 0) */
