@@ -187,15 +187,24 @@ struct ChanInfo {
   int64_t vtc_base, tkt_tc_base;
 };
 
-// hh-ladder unit: rows [k0, k0+rows) of channel ch (slice idx).
-struct HHTile {
-  int32_t ch, k0, idx, rows;
+// hh-ladder unit: `rows` packed rows of channel ch from row r0 of all channels', V and T at `base`,
+// the partial of P at `part`.
+struct __align__(16) HHTile {
+  int32_t hk, hs, rows, ch;
+  int64_t base, part;
+  int32_t r0, pad[3];
 };
 // One element of X = V_hhhh + P: P's partials part[k * stride], k < nslices, the V_hhhh element
 // and where X (and, on the diagonal, s) goes (s < 0: off the diagonal).
-struct HHOut {
+struct __align__(16) HHOut {
   int64_t part;
   int32_t nslices, stride, v, x, s, pad;
+};
+
+// A warp's part of T X: `rows` rows, T and T X at `at`, X at `x`.
+struct __align__(16) TXTile {
+  int32_t hk, hs, rows, pad;
+  int64_t at, x;
 };
 
 // Fused assembly, static data of strict packed row u (a < b) of a channel (index pk_off + u):

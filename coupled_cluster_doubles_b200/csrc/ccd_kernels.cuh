@@ -464,12 +464,11 @@ constexpr int kHHNC = 2;
 // Slack: fragment loads of the rows and columns past hk in the last row.
 constexpr size_t kHHSmem = (2 * (size_t)kHHRows * kMaxNB + 16) * sizeof(double);
 
-__device__ __forceinline__ void hh_warp_unit(const HHTile &tt, const ChanInfo &ch,
-                                             const double *__restrict__ vq, const double *tq,
-                                             double *__restrict__ part,
+__device__ __forceinline__ void hh_warp_unit(const HHTile &tt, const double *__restrict__ vq,
+                                             const double *tq, double *__restrict__ part,
                                              double *__restrict__ r_out) {
-  const int hk = ch.hk, hs = ch.hs, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int64_t base = ch.q_off + (int64_t)tt.k0 * hs + g;
+  const int hk = tt.hk, hs = tt.hs, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int64_t base = tt.base + g;
   constexpr int kSteps = kHHRows / 4;
   double a[kSteps], b[kSteps], acc[2] = {0.0, 0.0};
 #pragma unroll
@@ -486,21 +485,20 @@ __device__ __forceinline__ void hh_warp_unit(const HHTile &tt, const ChanInfo &c
     d += __shfl_xor_sync(0xffffffffu, d, 4);
     d += __shfl_xor_sync(0xffffffffu, d, 8);
     d += __shfl_xor_sync(0xffffffffu, d, 16);
-    if (g == 0 && 4 * k4 + t < tt.rows) r_out[ch.pk_off + tt.k0 + 4 * k4 + t] = d;
+    if (g == 0 && 4 * k4 + t < tt.rows) r_out[tt.r0 + 4 * k4 + t] = d;
   }
 #pragma unroll
   for (int q = 0; q < 2; ++q)
     if (g < hk && 2 * t + q < hk) part[g * hk + 2 * t + q] = acc[q];
 }
 
-__device__ __forceinline__ void hh_cta_unit(const HHTile &tt, const ChanInfo &ch,
-                                            const double *__restrict__ vq, const double *tq,
-                                            double *__restrict__ part,
+__device__ __forceinline__ void hh_cta_unit(const HHTile &tt, const double *__restrict__ vq,
+                                            const double *tq, double *__restrict__ part,
                                             double *__restrict__ r_out, double *sm) {
-  const int hk = ch.hk, hs = ch.hs, rows = tt.rows, rows16 = (rows + 15) & ~15;
+  const int hk = tt.hk, hs = tt.hs, rows = tt.rows, rows16 = (rows + 15) & ~15;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   double *Vs = sm, *Ts = sm + rows16 * hs;
-  const int64_t base = ch.q_off + (int64_t)tt.k0 * hs;
+  const int64_t base = tt.base;
   // Rows up to the next multiple of 16 are the block's zero padding, which is copied too.
   for (int e = 2 * threadIdx.x; e < rows16 * hs; e += 2 * kHHThreads) {
     cp_async16(Vs + e, vq + base + e);
@@ -544,64 +542,59 @@ __device__ __forceinline__ void hh_cta_unit(const HHTile &tt, const ChanInfo &ch
     for (int c = lane; c < hk; c += 32) d = fma(Vs[k * hs + c], Ts[k * hs + c], d);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-    if (lane == 0) r_out[ch.pk_off + tt.k0 + k] = d;
+    if (lane == 0) r_out[tt.r0 + k] = d;
   }
 }
 
 // Units [0, n_cta) one per CTA, then n_warp units, one per warp of the following CTAs.
 __global__ void __launch_bounds__(kHHThreads, 8)
 hh_slice_kernel(const HHTile *__restrict__ tiles, int n_cta, int n_warp,
-                const ChanInfo *__restrict__ chans, const double *__restrict__ vq,
-                const double *tq0, const double *tq1, double *__restrict__ part,
-                const int64_t *__restrict__ part_off, double *__restrict__ r_out,
-                const Control *ctl, int gate) {
+                const double *__restrict__ vq, const double *tq0, const double *tq1,
+                double *__restrict__ part, double *__restrict__ r_out, const Control *ctl,
+                int gate) {
   const bool wide = (int)blockIdx.x < n_cta;
   const int tr = wide ? kTrHHTiled : kTrHHSmall;
+  const int w = ((int)blockIdx.x - n_cta) * (kHHThreads / 32) + (int)(threadIdx.x >> 5);
+  // Static data, loaded beside the control block.
+  const HHTile tt = tiles[wide ? (int)blockIdx.x : n_cta + min(w, n_warp - 1)];
   if (skip_iteration(ctl, gate, tr)) return;
   extern __shared__ __align__(16) double hh_smem[];
-  const int w = ((int)blockIdx.x - n_cta) * (kHHThreads / 32) + (int)(threadIdx.x >> 5);
   if (!wide && w >= n_warp) return;
-  const HHTile tt = tiles[wide ? (int)blockIdx.x : n_cta + w];
-  const ChanInfo &ch = chans[tt.ch];
   const double *tq = ctl->parity ? tq1 : tq0;
-  double *pb = part + part_off[tt.ch] + (int64_t)tt.idx * ch.hk * ch.hk;
-  if (wide) hh_cta_unit(tt, ch, vq, tq, pb, r_out, hh_smem);
-  else hh_warp_unit(tt, ch, vq, tq, pb, r_out);
+  if (wide) hh_cta_unit(tt, vq, tq, part + tt.part, r_out, hh_smem);
+  else hh_warp_unit(tt, vq, tq, part + tt.part, r_out);
   trace_end(ctl, tr);
 }
 
-// X and s: one thread per element of every channel's P (a flat list, so that channels of one
-// hole pair do not take a CTA each), the slices' partials added in slice order with a block of
-// loads in flight ahead of the additions.
+// X and s: kHHLanes lanes per element of every channel's P (a flat list, so that channels of one
+// hole pair do not take a CTA each), each adding every kHHLanes-th slice's partial with eight loads
+// in flight, then a fixed shuffle tree.
+constexpr int kHHLanes = 4;
 __global__ void __launch_bounds__(128)
 hh_reduce_kernel(const HHOut *__restrict__ outs, int n, const double *__restrict__ v_hhhh,
                  const double *__restrict__ part, double *__restrict__ x,
                  double *__restrict__ s_out, const Control *ctl, int gate) {
-  if (skip_iteration(ctl, gate, kTrHHReduce)) return;
-  const int i = blockIdx.x * 128 + threadIdx.x;
-  if (i >= n) return;
-  const HHOut o = outs[i];
-  const double *pb = part + o.part;
+  const int i = (blockIdx.x * 128 + threadIdx.x) / kHHLanes, sub = threadIdx.x % kHHLanes;
+  const HHOut o = outs[min(i, n - 1)];  // static data, loaded beside the control block
   const double vh = __ldg(v_hhhh + o.v);
+  if (skip_iteration(ctl, gate, kTrHHReduce)) return;
+  const double *pb = part + o.part;
   double p = 0.0;
-  int sl = 0;
-  for (; sl + 8 <= o.nslices; sl += 8) {
-    double y[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) y[k] = __ldcg(pb + (int64_t)(sl + k) * o.stride);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) p += y[k];
-  }
-  {
+  for (int sl = sub; sl < o.nslices; sl += 8 * kHHLanes) {
     double y[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k)
-      y[k] = sl + k < o.nslices ? __ldcg(pb + (int64_t)(sl + k) * o.stride) : 0.0;
+      y[k] = sl + k * kHHLanes < o.nslices ? __ldcg(pb + (int64_t)(sl + k * kHHLanes) * o.stride)
+                                           : 0.0;
 #pragma unroll
     for (int k = 0; k < 8; ++k) p += y[k];
   }
-  x[o.x] = vh + p;
-  if (o.s >= 0) s_out[o.s] = p;
+#pragma unroll
+  for (int m = kHHLanes / 2; m > 0; m >>= 1) p += __shfl_xor_sync(0xffffffffu, p, m);
+  if (sub == 0 && i < n) {
+    x[o.x] = vh + p;
+    if (o.s >= 0) s_out[o.s] = p;
+  }
   trace_end(ctl, kTrHHReduce);
 }
 
@@ -1134,38 +1127,96 @@ onebody_tables_kernel(int np, const int64_t *__restrict__ o_h, const int64_t *__
 // - x_k and y_a as segmented sums of the hh ladder's by-products s and r over the strict pairs that
 //   hold the orbital (twice, for the two orders of the summed pair), one warp per orbital (the
 //   first n_ob CTAs), lane-strided partial sums and a fixed shuffle tree;
-// - tx[u, w] = 0.5 T X = sum_{k<l} T[u, kl] X[kl, w], one thread per quad (CTAs n_ob + item): hk
-//   multiply-adds on operands that L1 holds (T's row is one broadcast per k).  Here it runs beside
-//   the ladder and the ring; in the assembly, which nothing overlaps, it took 6 of 34 us at EG N=54
-//   |n|^2 <= 36 (12 of 47 at PNM N=66) and the registers of a third of the resident threads.
-__device__ __forceinline__ double quad_tx(const double *__restrict__ t_row,
-                                          const double *__restrict__ x, int hk, int hs, int w) {
-  double tx = 0.0;
-#pragma unroll 4
-  for (int k = 0; k < hk; ++k) tx = fma(t_row[k], x[k * hs + w], tx);
-  return tx;
+// - tx[u, w] = 0.5 T X = sum_{k<l} T[u, kl] X[kl, w] on the FP64 MMA (m8n8k4): a warp per unit of
+//   tx_rows(hk) rows of a channel, T and X straight from global memory (X mostly from L1).  Here it
+//   runs beside the ladder and the ring; in the assembly, which nothing overlaps, it took 6 of 34 us
+//   at EG N=54 |n|^2 <= 36 (12 of 47 at PNM N=66).  Its CTAs queue before the ring's, and beside the
+//   ladder an SM holds few, each for several times its time alone (dependent loads): one thread per
+//   quad, 3051 CTAs of 256 threads, took from 51 to 81 us of the iteration, these 42 to 55.  (X's sum
+//   over the slices done again by a CTA per row tile, without hh_reduce_kernel: 42 to 67.)
+constexpr int kPostThreads = 128;
+__host__ __device__ inline int tx_rows(int hk) { return hk <= 4 ? 128 : hk <= 8 ? 64 : 16; }
+
+// Up to 8 hole pairs: X's fragments stay in registers (KS K steps of 4), rows by 8.
+template <int KS>
+__device__ __forceinline__ void tx_thin(const TXTile &tt, const double *__restrict__ tq,
+                                        const double *__restrict__ x, double *__restrict__ tx) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3, hk = tt.hk, hs = tt.hs;
+  double b[KS];
+#pragma unroll
+  for (int k = 0; k < KS; ++k)
+    b[k] = q + 4 * k < hk && g < hk ? __ldcg(x + tt.x + (q + 4 * k) * hs + g) : 0.0;
+  constexpr int kRows = 8 / KS;  // groups of 8 rows in flight
+  for (int u0 = g; u0 - g < tt.rows; u0 += 8 * kRows) {
+    double a[kRows][KS];
+#pragma unroll
+    for (int i = 0; i < kRows; ++i)
+#pragma unroll
+      for (int k = 0; k < KS; ++k)
+        a[i][k] = u0 + 8 * i < tt.rows && q + 4 * k < hk
+                      ? tq[tt.at + (u0 + 8 * i) * hs + q + 4 * k] : 0.0;
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) {
+      double c[2] = {0.0, 0.0};
+#pragma unroll
+      for (int k = 0; k < KS; ++k) dmma_884(c, a[i][k], b[k]);
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        if (u0 + 8 * i < tt.rows && 2 * q + e < hk)
+          tx[tt.at + (u0 + 8 * i) * hs + 2 * q + e] = c[e];
+    }
+  }
 }
-constexpr int kPostThreads = 256;
-__global__ void __launch_bounds__(kPostThreads)
+// More: 16 rows, two 8-column tiles at a time.
+__device__ __forceinline__ void tx_wide(const TXTile &tt, const double *__restrict__ tq,
+                                        const double *__restrict__ x, double *__restrict__ tx) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3, hk = tt.hk, hs = tt.hs;
+  const bool in0 = g < tt.rows, in1 = g + 8 < tt.rows;
+  const double *t0 = tq + tt.at + g * hs, *t1 = t0 + 8 * hs;
+  for (int j = 0; j < hk; j += 16) {
+    const bool j0 = j + g < hk, j1 = j + 8 + g < hk;
+    double c[4][2] = {};
+#pragma unroll 3
+    for (int k = q; k < hk + q; k += 4) {
+      const bool in = k < hk;
+      const double a0 = in0 && in ? t0[k] : 0.0, a1 = in1 && in ? t1[k] : 0.0;
+      const double b0 = in && j0 ? x[tt.x + k * hs + j + g] : 0.0;
+      const double b1 = in && j1 ? x[tt.x + k * hs + j + 8 + g] : 0.0;
+      dmma_884(c[0], a0, b0);
+      dmma_884(c[1], a1, b0);
+      dmma_884(c[2], a0, b1);
+      dmma_884(c[3], a1, b1);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int u = g + 8 * (i & 1), w = j + 8 * (i >> 1) + 2 * q + e;
+        if (u < tt.rows && w < hk) tx[tt.at + (int64_t)u * hs + w] = c[i][e];
+      }
+  }
+}
+
+__global__ void __launch_bounds__(kPostThreads, 8)
 hh_post_kernel(int n_ob, int np, int nsp, const int64_t *__restrict__ list_off,
                const int32_t *__restrict__ list, const double *__restrict__ s,
                const double *__restrict__ r, double *__restrict__ xh, double *__restrict__ yp,
-               const QuadItem *__restrict__ items, const double *__restrict__ x,
-               const double *tq0, const double *tq1, double *__restrict__ tx, const Control *ctl,
-               int gate) {
-  if (skip_iteration(ctl, gate, kTrOneBody)) return;
+               const TXTile *__restrict__ tiles, int n_tx, const double *x, const double *tq0,
+               const double *tq1, double *__restrict__ tx, const Control *ctl, int gate) {
   if ((int)blockIdx.x >= n_ob) {
-    const QuadItem item = items[blockIdx.x - n_ob];
-    const int q = item.q0 + threadIdx.x;
-    if (q < item.q1) {
-      const int u = q / item.hk, w = q - u * item.hk;
-      const double *t_row = (ctl->parity ? tq1 : tq0) + item.q_off + (int64_t)u * item.hs;
-      tx[item.q_off + (int64_t)u * item.hs + w] =
-          quad_tx(t_row, x + item.x_off, item.hk, item.hs, w);
+    const int i = ((int)blockIdx.x - n_ob) * (kPostThreads / 32) + (int)(threadIdx.x >> 5);
+    const TXTile tt = tiles[min(i, n_tx - 1)];  // static data, loaded beside the control block
+    if (skip_iteration(ctl, gate, kTrOneBody)) return;
+    if (i < n_tx) {
+      const double *tq = ctl->parity ? tq1 : tq0;
+      if (tt.hk <= 4) tx_thin<1>(tt, tq, x, tx);
+      else if (tt.hk <= 8) tx_thin<2>(tt, tq, x, tx);
+      else tx_wide(tt, tq, x, tx);
     }
     trace_end(ctl, kTrOneBody);
     return;
   }
+  if (skip_iteration(ctl, gate, kTrOneBody)) return;
   const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (w >= nsp) return;
   const bool hole = w < np;
@@ -1242,7 +1293,6 @@ __device__ __forceinline__ void loop_set_condition(const Control *ctl,
 // loads (item, table rows, operands), so by how many threads are resident.
 constexpr int kQuadPerItem = kAsmThreads;  // one quad per thread and item
 constexpr int kAsmCTAsPerSM = 5;
-static_assert(kQuadPerItem == kPostThreads, "hh_post_kernel works on the same items");
 
 // D of quad (u, w) at packed position p: the planes of its row tile in order, then T X.
 __device__ __forceinline__ double quad_d(const LadderRows *__restrict__ lrows, int rt_off,

@@ -74,7 +74,8 @@ struct ccdgpu_handle {
   LadderTile *tiles = nullptr;
   HHTile *hh_tiles = nullptr;
   HHOut *hh_out = nullptr;
-  int64_t *hh_part_off = nullptr;  // per channel: its hh-ladder partials (nhht * hk * hk)
+  TXTile *tx_tiles = nullptr;
+  int n_tx = 0;
   int32_t *prow = nullptr, *hcol = nullptr;  // pp / hh pair -> 2 u (+ 1 when a > b), -1
   double *part = nullptr;
   ElemRange *ranges = nullptr;
@@ -1145,9 +1146,11 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
       q_tot += (int64_t)ci.nkc * kBK * ci.hs;
       // Stored V: room for the whole of it, should it not be symmetric.
       vt += ladder_chunk(on_the_fly && ci.sym, ci.nkc, ci.nmt - 1, ci.nkc, pk - (ci.nmt - 1) * kMaxBM);
-      part_tot += (int64_t)ci.nhht * hk * hk;
       for (int t = 0; t < ci.nhht; t++)
-        hh_tiles.push_back({ai, t * rows, t, std::min(rows, pk - t * rows)});
+        hh_tiles.push_back({hk, ci.hs, std::min(rows, pk - t * rows), ai,
+                            ci.q_off + (int64_t)t * rows * ci.hs,
+                            part_tot + (int64_t)t * hk * hk, (int32_t)(ci.pk_off + t * rows), {}});
+      part_tot += (int64_t)ci.nhht * hk * hk;
     }
     vraw_off.push_back(vraw_tot);
     if (!on_the_fly) vraw_tot += (int64_t)a_pr[ai] * pp;  // rows a <= b only
@@ -1440,6 +1443,7 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   // Rows: the packed rows with a < b (pk of them per channel), filled in parallel below;
   // columns (i < j) and work items here.
   std::vector<HHOut> hh_out;
+  std::vector<TXTile> tx_tiles;
   for (int ai = 0; ai < h->n_act; ai++) {
     const ChanInfo &a = chans[ai];
     for (int j = 0; j < a.hh; j++) {
@@ -1463,6 +1467,14 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
                           (int32_t)(a.x_off + kl * a.hs + ij),
                           kl == ij ? (int32_t)(a.qcol_off + ij) : -1, 0});
   }
+  // T X: the widest channels first, the short units fill in behind them.
+  for (const int rows : {16, 64, 128})
+    for (const ChanInfo &a : chans)
+      if (a.nmt && tx_rows(a.hk) == rows)
+        for (int u = 0; u < a.pk; u += rows)
+          tx_tiles.push_back({a.hk, a.hs, std::min(rows, a.pk - u), 0,
+                              a.q_off + (int64_t)u * a.hs, a.x_off});
+  h->n_tx = (int)tx_tiles.size();
   h->n_hh_out = (int)hh_out.size();
   h->n_quad_rows = a_pk_off[n_act];  // built on the device (quad_rows_kernel)
 
@@ -1541,7 +1553,7 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   Arena ar;
   ar.add(&h->chans, chans.size()); ar.add(&h->mods, mods.size());
   ar.add(&h->hh_tiles, hh_tiles.size()); ar.add(&h->hh_out, hh_out.size());
-  ar.add(&h->hh_part_off, hh_part_off.size());
+  ar.add(&h->tx_tiles, tx_tiles.size());
   ar.add(&h->ranges, ranges.size());
   ar.add(&h->pp_pairs, pp_pairs.size()); ar.add(&h->hh_pairs, hh_pairs.size());
   ar.add(&h->pp_swap, pp_swap.size()); ar.add(&h->hh_swap, hh_swap.size());
@@ -1799,7 +1811,7 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   TRY(put(h->chans, chans)); TRY(put(h->mods, mods));
   TRY(put(d_pairs, pairs)); TRY(put(h->ring_units, units));
   TRY(put(d_ring_perm, ring_perm));
-  TRY(put(h->hh_tiles, hh_tiles)); TRY(put(h->hh_out, hh_out)); TRY(put(h->hh_part_off, hh_part_off));
+  TRY(put(h->hh_tiles, hh_tiles)); TRY(put(h->hh_out, hh_out)); TRY(put(h->tx_tiles, tx_tiles));
   TRY(put(h->ranges, ranges)); TRY(put(h->quad_items, quad_items));
   TRY(put(h->quad_cols, quad_cols));
 
@@ -2098,13 +2110,12 @@ int launch_hh_ladder(ccdgpu_handle *h, cudaStream_t st, int gate, int only = -1)
     CK(launch_pdl(hh_slice_kernel, n_cta + (int)ceil_div(n_warp, kHHThreads / 32), kHHThreads,
                   n_cta ? kHHSmem : 0, st,
                   (const HHTile *)(h->hh_tiles + (n_cta ? 0 : h->n_hh_cta)), n_cta, n_warp,
-                  (const ChanInfo *)h->chans, (const double *)h->vq, (const double *)h->tq[0],
-                  (const double *)h->tq[1], h->part, (const int64_t *)h->hh_part_off, h->r,
+                  (const double *)h->vq, (const double *)h->tq[0], (const double *)h->tq[1], h->part, h->r,
                   (const Control *)h->ctl, gate));
   }
   if (h->n_hh_out && (only < 0 || only == 2)) {
     h->launches++;
-    CK(launch_pdl(hh_reduce_kernel, (int)ceil_div(h->n_hh_out, 128), 128, 0, st,
+    CK(launch_pdl(hh_reduce_kernel, (int)ceil_div((int64_t)h->n_hh_out * kHHLanes, 128), 128, 0, st,
                   (const HHOut *)h->hh_out, h->n_hh_out, (const double *)h->v_hhhh,
                   (const double *)h->part, h->x, h->s, (const Control *)h->ctl, gate));
   }
@@ -2233,12 +2244,12 @@ int launch_ring_units(ccdgpu_handle *h, cudaStream_t st, int gate, int k) {
 // One-body sums and T X.  only: -1 both, 0 the sums, 1 T X.
 int launch_hh_post(ccdgpu_handle *h, cudaStream_t st, int gate, int only = -1) {
   const int n_ob = only != 1 ? (int)ceil_div((int64_t)h->nsp, kPostThreads / 32) : 0;
-  const int n_tx = only != 0 ? h->n_quad_items : 0;
+  const int n_tx = only != 0 ? (int)ceil_div(h->n_tx, kPostThreads / 32) : 0;
   if (!(n_ob + n_tx)) return CCDGPU_OK;
   h->launches++;
   return cuda_status(launch_pdl(
       hh_post_kernel, n_ob + n_tx, kPostThreads, 0, st, n_ob, (int)h->np, (int)h->nsp, h->list_off,
-      h->list, h->s, h->r, h->xh, h->yp, (const QuadItem *)h->quad_items, (const double *)h->x,
+      h->list, h->s, h->r, h->xh, h->yp, (const TXTile *)h->tx_tiles, h->n_tx, (const double *)h->x,
       (const double *)h->tq[0], (const double *)h->tq[1], h->tx, (const Control *)h->ctl, gate));
 }
 int launch_assemble_fused(ccdgpu_handle *h, cudaStream_t st, int gate) {
@@ -2306,12 +2317,20 @@ int enqueue_fused_iteration(ccdgpu_handle *h, bool mixed) {
   // Kernels reach the GPU in the order in which they become ready, and the CTAs of one wait behind
   // all CTAs of those before it; of branches that become ready together the one captured last comes
   // first.  So: the ladder (it needs an SM's registers before smaller CTAs take them), the hh
-  // slices and the gather, then the short kernels that follow the hh slices, and the ring, which
-  // the gather holds back until then.
+  // slices and the gather, then the short kernels that follow the hh slices, then the ring.  Where
+  // the ring is more than about a wave of CTAs it waits for X as well as for the gather, which end
+  // together: ahead of T X it would hold that back to the end of the iteration (EG N=54
+  // |n|^2 <= 36: 167 us an iteration, 160 so; a smaller ring leaves room, and would only start
+  // later).
   CK(cudaEventRecord(h->ev_fork, h->s0));
   CK(cudaStreamWaitEvent(h->s1, h->ev_fork, 0));
   CK(cudaStreamWaitEvent(h->s2, h->ev_fork, 0));
   if ((rc = launch_tp_gather(h, h->s1, gate))) return rc;
+  if ((rc = launch_hh_ladder(h, h->s2, gate))) return rc;
+  if (h->n_ring[0] + h->n_ring[1] > 2 * 148) {
+    CK(cudaEventRecord(h->ev_join2, h->s2));
+    CK(cudaStreamWaitEvent(h->s1, h->ev_join2, 0));
+  }
   // The groups of units side by side; the first that the system has stays on s1.
   CK(cudaEventRecord(h->ev_fork3, h->s1));
   const struct { cudaStream_t st; cudaEvent_t ev; } branch[3] = {
@@ -2323,7 +2342,6 @@ int enqueue_fused_iteration(ccdgpu_handle *h, bool mixed) {
     if ((rc = launch_ring_units(h, branch[used++].st, gate, k))) return rc;
   }
   for (int k = 0; k < std::max(used, 1); k++) CK(cudaEventRecord(branch[k].ev, branch[k].st));
-  if ((rc = launch_hh_ladder(h, h->s2, gate))) return rc;
   if ((rc = launch_hh_post(h, h->s2, gate))) return rc;
   CK(cudaEventRecord(h->ev_join2, h->s2));
   if ((rc = ladder(h->s0))) return rc;
