@@ -201,9 +201,9 @@ struct __align__(16) HHOut {
   int32_t nslices, stride, v, x, s, pad;
 };
 
-// A warp's part of T X: `rows` rows, T and T X at `at`, X at `x`.
+// A warp's part of T X: `rows` rows, T and T X at `at`, X at `x`; from column j0 (hk > 8: 16 of them).
 struct __align__(16) TXTile {
-  int32_t hk, hs, rows, pad;
+  int32_t hk, hs, rows, j0;
   int64_t at, x;
 };
 

@@ -875,10 +875,19 @@ __host__ __device__ inline int pad16(int n) { return (n + 15) & ~15; }
 __host__ __device__ inline int ring_group(int ph, int hp) {
   return (ph > hp ? ph : hp) <= 16 ? 1 : (ph > hp ? ph : hp) <= 32 ? 2 : 4;
 }
-// T' image and Y of a unit (doubles); Y's row stride is 4 mod 8 doubles too.
-__host__ __device__ constexpr int ring_ldy(int g) { return g == 1 ? 20 : 8 * kPairNC + 4; }
-__host__ __device__ constexpr int ring_unit_smem(int g, int p, int h) {
-  return p * (h + 4) + h * ring_ldy(g);
+// T' and Y of a unit (doubles): all of T' (row stride h + 4), or (COLS) the unit's columns alone,
+// with Y's row stride 8 nt + 4.  Strides are 4 mod 8 doubles.  All of T' is 35 to 54 KB, which
+// leaves room for one CTA of four warps beside the ladder; the columns leave room for two, and T' as
+// the A operand then comes from L2.  Where those units are more than a CTA or two per SM the
+// columns are the better choice (EG N=54 |n|^2 <= 36, 732 units: 160 -> 153 us an iteration, PNM
+// N=66, 1300: 221 -> 210), else all of T' (EG N=54 |n|^2 <= 19, 238 units: 58.8 us an iteration,
+// 60.3 with the columns).
+__host__ __device__ inline bool ring_cols(int64_t units4) { return units4 > 2 * 148; }
+__host__ __device__ constexpr int ring_ldy(int g, bool cols, int nt) {
+  return g == 1 ? 20 : cols ? 8 * nt + 4 : 8 * kPairNC + 4;
+}
+__host__ __device__ constexpr int ring_unit_smem(int g, bool cols, int p, int h, int nt) {
+  return p * (cols ? ring_ldy(g, cols, nt) : h + 4) + h * ring_ldy(g, cols, nt);
 }
 // Fragment-ordered A operand: [16-row tile][16-deep step][4][lane][2].
 __device__ __forceinline__ void frag_load(double (&a)[8], const double *__restrict__ p) {
@@ -930,20 +939,28 @@ __device__ __forceinline__ void group_sync() {
     asm volatile("bar.sync %0, 64;" ::"r"(1 + (int)(threadIdx.x >> 6)) : "memory");
   else __syncthreads();
 }
-template <int G>
+template <int G, bool COLS>
 __device__ __forceinline__ void ring_unit(const RingUnit &m, const double *__restrict__ img,
                                           const int32_t *__restrict__ to_img, const double *tp,
                                           double *__restrict__ out, double *sm, uint32_t bar,
                                           uint32_t parity, int32_t *err) {
-  constexpr int NC = G == 1 ? 2 : kPairNC, ldy = ring_ldy(G);
+  constexpr int NC = G == 1 ? 2 : kPairNC;
   const int P = pad16(m.ph), H = pad16(m.hp), ldh = H + 4, n8 = (m.hp + 7) >> 3, nt = m.nt;
   const int w = (threadIdx.x >> 5) % G, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  double *Ts = sm, *Ys = sm + P * ldh;
-  if (w == 0 && lane == 0) {
+  const int ldy = ring_ldy(G, COLS, nt), ldt = COLS ? ldy : ldh;
+  double *Ts = sm, *Ys = sm + P * ldt;
+  if (COLS) {
+    if (w == 0) {
+      if (lane == 0) mbar_expect_tx(bar, P * nt * 64);
+      __syncwarp();
+      for (int r = lane; r < P; r += 32)
+        bulk_g2s(smem_u32(Ts + r * ldt), tp + m.tp + (int64_t)r * ldh + 8 * m.n0, nt * 64, bar);
+    }
+  } else if (w == 0 && lane == 0) {
     mbar_expect_tx(bar, P * ldh * 8);
     bulk_g2s(smem_u32(Ts), tp + m.tp, P * ldh * 8, bar);
   }
-  const double *Tj = Ts + 8 * m.n0;  // this unit's columns of T'
+  const double *Tj = COLS ? Ts : Ts + 8 * m.n0;  // this unit's columns of T'
   bool landed = false;
   auto wait = [&]() {
     if (!landed && !mbar_wait(bar, parity)) atomicOr(err, kErrTimeout);
@@ -962,7 +979,7 @@ __device__ __forceinline__ void ring_unit(const RingUnit &m, const double *__res
         acc[n][0] = lo.x; acc[n][1] = lo.y; acc[n][2] = hi.x; acc[n][3] = hi.y;
       }
     wait();
-    frag_gemm(acc, f, c_frag, Tj, ldh, nt, P);
+    frag_gemm(acc, f, c_frag, Tj, ldt, nt, P);
 #pragma unroll
     for (int n = 0; n < NC; ++n)
       if (n < nt)
@@ -973,25 +990,45 @@ __device__ __forceinline__ void ring_unit(const RingUnit &m, const double *__res
   const double *b_frag = img + m.b_img;
   if (16 * w < P) frag_start(f, b_frag + (int64_t)w * P * 16, P);
   wait();
-  group_sync<G>();
+  if (!COLS) group_sync<G>();
   for (int mt = w; 16 * mt < P; mt += G) {  // S = B T' + T' Y, to the quads
     const double *bf = b_frag + (int64_t)mt * P * 16;
     if (mt != w) frag_start(f, bf, P);
 #pragma unroll
     for (int n = 0; n < NC; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.0;
-    frag_gemm(acc, f, bf, Tj, ldh, nt, P);
+    frag_gemm(acc, f, bf, Tj, ldt, nt, P);
     const int4 *qp =
         reinterpret_cast<const int4 *>(to_img + m.to_img) + ((int64_t)mt * n8 + m.n0) * 32 + lane;
     int4 to[NC];
 #pragma unroll
     for (int n = 0; n < NC; ++n)
       if (n < nt) to[n] = __ldg(qp + 32 * n);
-    for (int k0 = 0; k0 < H; k0 += 16) {
-      double a[8];
+    // T' as the A operand: from its image in shared memory, or (COLS) in global memory, 8 sectors
+    // a load, all of them used, two steps ahead.
+    const double *ta = COLS ? tp + m.tp + (int64_t)(16 * mt + g) * ldh + t
+                             : Ts + (16 * mt + g) * ldh + t;
+    auto t_load = [&](double (&a)[8], int k0) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
-        a[i] = Ts[(16 * mt + g + 8 * (i % 2)) * ldh + k0 + t + 4 * (i / 2)];
-      mma_row(acc, a, Ys, ldy, nt, k0);
+      for (int i = 0; i < 8; ++i) a[i] = ta[8 * (i % 2) * ldh + k0 + 4 * (i / 2)];
+    };
+    if constexpr (COLS) {
+      t_load(f[0], 0);
+      if (H > 16) t_load(f[1], 16);
+      if (mt == w) group_sync<G>();  // Y is complete
+      for (int k0 = 0; k0 < H; k0 += 32) {
+        mma_row(acc, f[0], Ys, ldy, nt, k0);
+        if (k0 + 32 < H) t_load(f[0], k0 + 32);
+        if (k0 + 16 < H) {
+          mma_row(acc, f[1], Ys, ldy, nt, k0 + 16);
+          if (k0 + 48 < H) t_load(f[1], k0 + 48);
+        }
+      }
+    } else {
+      for (int k0 = 0; k0 < H; k0 += 16) {
+        double a[8];
+        t_load(a, k0);
+        mma_row(acc, a, Ys, ldy, nt, k0);
+      }
     }
 #pragma unroll
     for (int n = 0; n < NC; ++n)
@@ -1002,9 +1039,10 @@ __device__ __forceinline__ void ring_unit(const RingUnit &m, const double *__res
         if (to[n].w >= 0) out[to[n].w] = acc[n][3];
       }
   }
+  if (COLS && 16 * w >= P) group_sync<G>();  // a warp without rows of S
 }
 
-template <int G>
+template <int G, bool COLS = false>
 __global__ void __launch_bounds__(G == 2 ? 64 : 128, G == 2 ? 8 : 4)
 ring_pair_kernel(const RingUnit *__restrict__ units, int n, const double *__restrict__ img,
                  const int32_t *__restrict__ to_img, const double *tp, double *__restrict__ out,
@@ -1021,7 +1059,7 @@ ring_pair_kernel(const RingUnit *__restrict__ units, int n, const double *__rest
   }
   __syncthreads();
   if (u < n)
-    ring_unit<G>(units[u], img, to_img, tp, out, rp_smem + sub * ring_unit_smem(1, 16, 16),
+    ring_unit<G, COLS>(units[u], img, to_img, tp, out, rp_smem + sub * ring_unit_smem(1, false, 16, 16, 2),
                  smem_u32(&bars[sub]), 0, err);
   trace_end(ctl, kTr);
 }
@@ -1167,34 +1205,33 @@ __device__ __forceinline__ void tx_thin(const TXTile &tt, const double *__restri
     }
   }
 }
-// More: 16 rows, two 8-column tiles at a time.
+// More: 16 rows and two 8-column tiles.
 __device__ __forceinline__ void tx_wide(const TXTile &tt, const double *__restrict__ tq,
                                         const double *__restrict__ x, double *__restrict__ tx) {
   const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3, hk = tt.hk, hs = tt.hs;
   const bool in0 = g < tt.rows, in1 = g + 8 < tt.rows;
   const double *t0 = tq + tt.at + g * hs, *t1 = t0 + 8 * hs;
-  for (int j = 0; j < hk; j += 16) {
-    const bool j0 = j + g < hk, j1 = j + 8 + g < hk;
-    double c[4][2] = {};
-#pragma unroll 3
-    for (int k = q; k < hk + q; k += 4) {
-      const bool in = k < hk;
-      const double a0 = in0 && in ? t0[k] : 0.0, a1 = in1 && in ? t1[k] : 0.0;
-      const double b0 = in && j0 ? x[tt.x + k * hs + j + g] : 0.0;
-      const double b1 = in && j1 ? x[tt.x + k * hs + j + 8 + g] : 0.0;
-      dmma_884(c[0], a0, b0);
-      dmma_884(c[1], a1, b0);
-      dmma_884(c[2], a0, b1);
-      dmma_884(c[3], a1, b1);
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int u = g + 8 * (i & 1), w = j + 8 * (i >> 1) + 2 * q + e;
-        if (u < tt.rows && w < hk) tx[tt.at + (int64_t)u * hs + w] = c[i][e];
-      }
+  const int j = tt.j0;
+  const bool j0 = j + g < hk, j1 = j + 8 + g < hk;
+  double c[4][2] = {};
+#pragma unroll 4
+  for (int k = q; k < hk + q; k += 4) {
+    const bool in = k < hk;
+    const double a0 = in0 && in ? t0[k] : 0.0, a1 = in1 && in ? t1[k] : 0.0;
+    const double b0 = in && j0 ? x[tt.x + k * hs + j + g] : 0.0;
+    const double b1 = in && j1 ? x[tt.x + k * hs + j + 8 + g] : 0.0;
+    dmma_884(c[0], a0, b0);
+    dmma_884(c[1], a1, b0);
+    dmma_884(c[2], a0, b1);
+    dmma_884(c[3], a1, b1);
   }
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int u = g + 8 * (i & 1), w = j + 8 * (i >> 1) + 2 * q + e;
+      if (u < tt.rows && w < hk) tx[tt.at + (int64_t)u * hs + w] = c[i][e];
+    }
 }
 
 __global__ void __launch_bounds__(kPostThreads, 8)

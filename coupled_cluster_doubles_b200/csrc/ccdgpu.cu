@@ -111,6 +111,7 @@ struct ccdgpu_handle {
   int32_t *ring_to = nullptr, *ring_src = nullptr;
   int n_ring[3] = {0, 0, 0};
   int64_t n_tp = 0;
+  bool ring_cols = false;               // the four-warp units hold only their columns of T'
   size_t ring_smem[3] = {0, 0, 0};  // dynamic shared memory of the groups' kernels
   std::vector<RingPair> host_pairs;
   double create_ms[5] = {};   // ccdgpu_profile::ms_create
@@ -1379,8 +1380,6 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
       img_tot = r.a_img + q * 8 * n8;
       r.to_img = to_tot;
       to_tot += p * 8 * n8;
-      size_t &smem = h->ring_smem[g == 4 ? 0 : g == 2 ? 1 : 2];
-      smem = std::max(smem, (g == 1 ? 4 : 1) * sizeof(double) * ring_unit_smem(g, (int)p, (int)q));
     }
     // Units: the pair's column tiles in blocks of at most kPairNC, as equal as they come.
     for (int k = 0; k < 3; k++) {
@@ -1393,6 +1392,14 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
                            r.tp, r.a_img, r.b_img, r.c_img, r.to_img});
       }
       h->n_ring[k] = (int)(units.size() - first);
+    }
+    h->ring_cols = ring_cols(h->n_ring[0]);
+    for (const RingUnit &u : units) {
+      const int g = ring_group(u.ph, u.hp);
+      size_t &smem = h->ring_smem[g == 4 ? 0 : g == 2 ? 1 : 2];
+      smem = std::max(smem, (g == 1 ? 4 : 1) * sizeof(double) *
+                                ring_unit_smem(g, g == 4 && h->ring_cols, pad16(u.ph),
+                                               pad16(u.hp), u.nt));
     }
   }
   h->n_tp = tp_tot;
@@ -1472,8 +1479,9 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     for (const ChanInfo &a : chans)
       if (a.nmt && tx_rows(a.hk) == rows)
         for (int u = 0; u < a.pk; u += rows)
-          tx_tiles.push_back({a.hk, a.hs, std::min(rows, a.pk - u), 0,
-                              a.q_off + (int64_t)u * a.hs, a.x_off});
+          for (int j0 = 0; j0 < a.hk; j0 += 16)
+            tx_tiles.push_back({a.hk, a.hs, std::min(rows, a.pk - u), j0,
+                                a.q_off + (int64_t)u * a.hs, a.x_off});
   h->n_tx = (int)tx_tiles.size();
   h->n_hh_out = (int)hh_out.size();
   h->n_quad_rows = a_pk_off[n_act];  // built on the device (quad_rows_kernel)
@@ -2035,7 +2043,9 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   CK(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->opt.device));
   if (ring16_smem(80) > (size_t)smem_optin) return CCDGPU_ERR_UNSUPPORTED;
   CK(cudaFuncSetAttribute(ring_pair_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                          ring_unit_smem(4, kRingMax, kRingMax) * (int)sizeof(double)));
+                          ring_unit_smem(4, false, kRingMax, kRingMax, kPairNC) * (int)sizeof(double)));
+  CK(cudaFuncSetAttribute(ring_pair_kernel<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                          ring_unit_smem(4, true, kRingMax, kRingMax, kPairNC) * (int)sizeof(double)));
   CK(cudaFuncSetAttribute(pp_ladder_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                           (int)kLadderSmem));
   CK(cudaFuncSetAttribute(pp_ladder_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
@@ -2234,7 +2244,7 @@ int launch_ring_units(ccdgpu_handle *h, cudaStream_t st, int gate, int k) {
   if (!n) return CCDGPU_OK;
   const RingUnit *units = h->ring_units;
   for (int j = 0; j < k; j++) units += h->n_ring[j];
-  auto kern = k == 0 ? ring_pair_kernel<4> : k == 1 ? ring_pair_kernel<2> : ring_pair_kernel<1>;
+  auto kern = k == 0 ? (h->ring_cols ? ring_pair_kernel<4, true> : ring_pair_kernel<4>) : k == 1 ? ring_pair_kernel<2> : ring_pair_kernel<1>;
   h->launches++;
   return cuda_status(launch_pdl(kern, k == 2 ? (int)ceil_div(n, 4) : n, k == 1 ? 64 : 128,
                                 h->ring_smem[k], st, units, n, (const double *)h->ring_img,
