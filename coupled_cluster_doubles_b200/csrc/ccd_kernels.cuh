@@ -104,8 +104,9 @@ __device__ __forceinline__ void trace_end(const Control *ctl, int tr) {
 __device__ __forceinline__ bool skip_iteration(const Control *ctl, int gate, int tr) {
   pdl_enter();
   trace_start(ctl, tr);
-  if (!ctl->active) return false;
-  return ctl->done || ((gate == 1) != (ctl->phase == 1));
+  // One round trip (the fields share a line), whatever the outcome.
+  const int active = ctl->active, done = ctl->done, phase = ctl->phase;
+  return active && (done || ((gate == 1) != (phase == 1)));
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1310,16 +1311,20 @@ __device__ __forceinline__ void write_t_image(const ChanInfo &ch, int u, int w, 
 // ------------------------------------------------------------------------------------------
 constexpr int kAsmThreads = 256;
 constexpr int kAsmPerThread = 2;  // table path: elements per thread of an ElemRange
-__device__ __forceinline__ void energy_reduce(const double *epart, int n, Control *ctl, int flags,
-                                              double *e_out);
+struct StopState {  // what decides whether the device solve loop goes on
+  int64_t iterations, stop_at;
+  int32_t done, phase;
+};
+__device__ __forceinline__ StopState energy_reduce(const double *epart, int n, Control *ctl,
+                                                   int flags, double *e_out);
 // Condition of the device solve loop's WHILE node after an iteration: another iteration while
 // the stop rule has not fired, below the launch's iteration limit, and (body_mixed) in the
 // mixed phase or (FP64 body) past it.
-__device__ __forceinline__ void loop_set_condition(const Control *ctl,
+__device__ __forceinline__ void loop_set_condition(const StopState &st,
                                                    cudaGraphConditionalHandle cond,
                                                    bool body_mixed) {
-  const bool more = !ctl->done && ctl->iterations < ctl->stop_at;
-  const bool mixed_phase = ctl->phase == 1;
+  const bool more = !st.done && st.iterations < st.stop_at;
+  const bool mixed_phase = st.phase == 1;
   cudaGraphSetConditional(cond, (more && (body_mixed ? mixed_phase : !mixed_phase)) ? 1u : 0u);
 }
 
@@ -1424,10 +1429,10 @@ assemble_fused_kernel(const QuadItem *__restrict__ items, int n_items,
   __syncthreads();
   if (!last) return;
   __threadfence();
-  energy_reduce(epart, gridDim.x, ctl, 3, nullptr);
+  const StopState st = energy_reduce(epart, gridDim.x, ctl, 3, nullptr);
   if (threadIdx.x == 0) {
     *ticket = 0;
-    if constexpr (LOOP) loop_set_condition(ctl, cond, loop_body == 2);
+    if constexpr (LOOP) loop_set_condition(st, cond, loop_body == 2);
   }
 }
 
@@ -1611,58 +1616,87 @@ __global__ void map_to_kernel(const ElemRange *__restrict__ ranges, const ChanIn
 // Sum of the per-CTA energy partials (Neumaier-compensated, fixed order) by one block of
 // kEnergyThreads threads, then the reference's stop rule on the device.  flags: 1 = flip the
 // amplitude buffer parity, 2 = count this as an iteration of the solve loop.
+// Nothing overlaps it at the end of an iteration, so every memory round trip counts: the control
+// block's fields are read together, beside the partial sums.  The state is thread 0's.
 constexpr int kEnergyThreads = 256;
-__device__ __forceinline__ void energy_reduce(const double *epart, int n, Control *ctl, int flags,
-                                              double *e_out) {
-  __shared__ double ss[kEnergyThreads], cs[kEnergyThreads];
-  double s = 0.0, c = 0.0;
-  for (int i = threadIdx.x; i < n; i += kEnergyThreads) {
-    const double x = __ldcg(epart + i);
-    const double t = s + x;
-    c += fabs(s) >= fabs(x) ? (s - t) + x : (x - t) + s;
-    s = t;
-  }
-  ss[threadIdx.x] = s;
-  cs[threadIdx.x] = c;
-  __syncthreads();
-  for (int w = kEnergyThreads / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) {
-      const double a = ss[threadIdx.x], b = ss[threadIdx.x + w];
-      const double t = a + b;
-      const double e = fabs(a) >= fabs(b) ? (a - t) + b : (b - t) + a;
-      ss[threadIdx.x] = t;
-      cs[threadIdx.x] += cs[threadIdx.x + w] + e;
-    }
-    __syncthreads();
-  }
+__device__ __forceinline__ void neumaier_add(double &s, double &c, double x) {
+  const double t = s + x;
+  c += fabs(s) >= fabs(x) ? (s - t) + x : (x - t) + s;
+  s = t;
+}
+__device__ __forceinline__ StopState energy_reduce(const double *epart, int n, Control *ctl,
+                                                   int flags, double *e_out) {
+  constexpr int kWarps = kEnergyThreads / 32;
+  __shared__ double ss[kWarps], cs[kWarps];
+  Control c0;
   if (threadIdx.x == 0) {
-    const double corr = 0.25 * (ss[0] + cs[0]);
+    c0.e_prev = ctl->e_prev;
+    c0.e_diff = ctl->e_diff;
+    c0.tol = ctl->tol;
+    c0.polish_rel = ctl->polish_rel;
+    c0.iterations = ctl->iterations;
+    c0.max_iters = ctl->max_iters;
+    c0.polish_iters = ctl->polish_iters;
+    c0.stop_at = ctl->stop_at;
+    c0.active = ctl->active;
+    c0.phase = ctl->phase;
+    c0.done = ctl->done;
+    c0.error = ctl->error;
+    c0.parity = ctl->parity;
+  }
+  double s = 0.0, c = 0.0;
+  for (int i = threadIdx.x; i < n; i += kEnergyThreads) neumaier_add(s, c, __ldcg(epart + i));
+  // (s, c) pairs: within a warp by a fixed tree, then the warps' likewise.
+#pragma unroll
+  for (int w = 16; w > 0; w >>= 1) {
+    c += __shfl_down_sync(0xffffffffu, c, w);
+    neumaier_add(s, c, __shfl_down_sync(0xffffffffu, s, w));
+  }
+  if (threadIdx.x % 32 == 0) {
+    ss[threadIdx.x / 32] = s;
+    cs[threadIdx.x / 32] = c;
+  }
+  __syncthreads();
+  if (threadIdx.x >= 32) return StopState{};
+  s = threadIdx.x < kWarps ? ss[threadIdx.x] : 0.0;
+  c = threadIdx.x < kWarps ? cs[threadIdx.x] : 0.0;
+#pragma unroll
+  for (int w = kWarps / 2; w > 0; w >>= 1) {
+    c += __shfl_down_sync(0xffffffffu, c, w);
+    neumaier_add(s, c, __shfl_down_sync(0xffffffffu, s, w));
+  }
+  StopState st{};
+  if (threadIdx.x == 0) {
+    const double corr = 0.25 * (s + c);
     if (e_out) *e_out = corr;
     if (flags & 2) {
-      const double diff = corr - ctl->e_prev, prev_diff = ctl->e_diff;
+      const double diff = corr - c0.e_prev;
       ctl->e_prev = corr;
       ctl->e_corr = corr;
       ctl->e_diff = diff;
-      if (ctl->iterations < 128) ctl->energies[ctl->iterations] = corr;
-      ctl->iterations += 1;
-      if (ctl->active && ctl->phase == 2) ctl->polish_iters += 1;
+      if (c0.iterations < 128) ctl->energies[c0.iterations] = corr;
+      ctl->iterations = ++c0.iterations;
+      if (c0.active && c0.phase == 2) ctl->polish_iters = c0.polish_iters + 1;
       if (!isfinite(corr)) {
-        ctl->error |= kErrNonFinite;
-        ctl->done = 1;
+        ctl->error = c0.error | kErrNonFinite;
+        c0.done = 1;
       }
-      if (ctl->active && ctl->phase == 1) {
+      if (c0.active && c0.phase == 1) {
         // Mixed phase: hand over to FP64 iterations once the energy change reaches the
         // rounding floor of the split-bf16 ladder, or stops shrinking.
-        if (fabs(diff) <= fmax(ctl->tol, ctl->polish_rel * fabs(corr)) ||
-            (ctl->iterations > 2 && fabs(diff) >= fabs(prev_diff)))
-          ctl->phase = 2;
-        if (ctl->iterations > ctl->max_iters) ctl->done = 1;
-      } else if (fabs(diff) <= ctl->tol || ctl->iterations > ctl->max_iters) {
-        ctl->done = 1;
+        if (fabs(diff) <= fmax(c0.tol, c0.polish_rel * fabs(corr)) ||
+            (c0.iterations > 2 && fabs(diff) >= fabs(c0.e_diff)))
+          ctl->phase = c0.phase = 2;
+        if (c0.iterations > c0.max_iters) c0.done = 1;
+      } else if (fabs(diff) <= c0.tol || c0.iterations > c0.max_iters) {
+        c0.done = 1;
       }
+      if (c0.done) ctl->done = 1;
     }
-    if (flags & 1) ctl->parity ^= 1;
+    if (flags & 1) ctl->parity = c0.parity ^ 1;
+    st = StopState{c0.iterations, c0.stop_at, c0.done, c0.phase};
   }
+  return st;
 }
 
 // Last node of an iteration body of the device solve loop (a CUDA graph with WHILE conditional
@@ -1676,7 +1710,8 @@ __global__ void loop_ctl_kernel(const Control *ctl, cudaGraphConditionalHandle c
   pdl_enter();
   trace_start(ctl, kTrLoopCtl);
   if (threadIdx.x != 0) return;
-  loop_set_condition(ctl, cond, body_mixed != 0);
+  loop_set_condition(StopState{ctl->iterations, ctl->stop_at, ctl->done, ctl->phase}, cond,
+                     body_mixed != 0);
 }
 
 // MBPT2 (MBPT2Corr.cpp:6-38) over the elements of the active channels, one CTA per range:
