@@ -293,6 +293,7 @@ struct Control {
   uint64_t trace_last[kTraceKernels];
   uint64_t trace_end[kTraceKernels];    // %globaltimer when the last CTA finished
   double energies[128];  // corrCCD per iteration (first 128)
+  int32_t err;           // kErrTimeout, kErrBadIndex, ... raised by kernels (never uploaded)
 };
 
 constexpr int32_t kErrNonFinite = 1;

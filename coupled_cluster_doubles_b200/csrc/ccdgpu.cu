@@ -123,6 +123,7 @@ struct ccdgpu_handle {
   double *gath = nullptr;
   Control *ctl = nullptr;
   Control *h_ctl = nullptr;  // pinned mirror
+  bool ctl_current = false;  // the mirror is what the device holds (but for err and the trace)
   int32_t *ticket = nullptr;  // assembly's last-CTA ticket
   double *e_out = nullptr;
   int32_t *err = nullptr;
@@ -1587,7 +1588,7 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   ar.add(&h->quad_items, quad_items.size());
   ar.add(&h->quad_rows, h->n_quad_rows); ar.add(&h->quad_cols, quad_cols.size());
   ar.add(&h->kcol, kcol.size());  // V tiling at create
-  ar.add(&h->epart, std::max(h->n_ranges, h->n_asm_blocks)); ar.add(&h->ctl, 1); ar.add(&h->e_out, 1); ar.add(&h->err, 1);
+  ar.add(&h->epart, std::max(h->n_ranges, h->n_asm_blocks)); ar.add(&h->ctl, 1); ar.add(&h->e_out, 1);
   ar.add(&h->ticket, 1);
   if (h->nt) {
     auto round_up = [](int64_t n) { return std::max<int64_t>(256, (n + 255) / 256 * 256); };
@@ -1612,6 +1613,7 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   int rc;
 #define TRY(x) do { rc = (x); if (rc) return rc; } while (0)
   TRY(ar.commit(h));
+  h->err = &h->ctl->err;
   // Scratch for the raw inputs, released at the end of create.
   Arena sc;
   double *vraw = nullptr, *hhpp_raw = nullptr, *hpph_raw = nullptr;
@@ -2263,6 +2265,7 @@ int launch_hh_post(ccdgpu_handle *h, cudaStream_t st, int gate, int only = -1) {
       (const double *)h->tq[0], (const double *)h->tq[1], h->tx, (const Control *)h->ctl, gate));
 }
 int launch_assemble_fused(ccdgpu_handle *h, cudaStream_t st, int gate) {
+  h->ctl_current = false;
   if (!h->n_asm_blocks) return CCDGPU_OK;
   h->launches++;
   return cuda_status(launch_pdl(
@@ -2276,6 +2279,7 @@ int launch_assemble_fused(ccdgpu_handle *h, cudaStream_t st, int gate) {
       (cudaGraphConditionalHandle)(h->loop_capture ? h->loop_cond : 0), h->loop_capture, gate));
 }
 int launch_energy(ccdgpu_handle *h, cudaStream_t st, int flags) {
+  if (flags) h->ctl_current = false;
   energy_kernel<<<1, kEnergyThreads, 0, st>>>(h->epart, h->n_ranges, h->ctl, flags, h->e_out, 0);
   h->launches++;
   return cuda_status(cudaGetLastError());
@@ -2396,20 +2400,32 @@ int stage_assemble_tables(ccdgpu_handle *h, double mixing) {
   return CCDGPU_OK;
 }
 
+constexpr size_t kCtlUpload = offsetof(Control, err);  // what the host writes of it
+
 int sync_ctl(ccdgpu_handle *h) {
   CK(cudaMemcpyAsync(h->h_ctl, h->ctl, sizeof(Control), cudaMemcpyDeviceToHost, h->s0));
   CK(cudaStreamSynchronize(h->s0));
+  h->ctl_current = true;
   return CCDGPU_OK;
 }
+// The same where no kernel that writes the block has been launched since: nothing to read (a call
+// that only launches one stage spent 20 of its 20 to 50 us on reading and writing it).
+int fresh_ctl(ccdgpu_handle *h) {
+  return h->ctl_current && h->h_ctl->trace_iter < 0 ? CCDGPU_OK : sync_ctl(h);
+}
 
-int check_errors(ccdgpu_handle *h) {
-  int32_t e = 0;
-  CK(cudaMemcpy(&e, h->err, sizeof(int32_t), cudaMemcpyDeviceToHost));
-  if (e & kErrTimeout) {
+// read: fetch the error word first (otherwise sync_ctl just has).
+int check_errors(ccdgpu_handle *h, bool read = true) {
+  if (read) {
+    CK(cudaMemcpyAsync(&h->h_ctl->err, h->err, sizeof(int32_t), cudaMemcpyDeviceToHost, h->s0));
+    CK(cudaStreamSynchronize(h->s0));
+  }
+  if (h->h_ctl->err & kErrTimeout) {
     // Reported once: the handle stays usable (the timed-out iteration's amplitudes are
     // incomplete; ccdgpu_reset or ccdgpu_set_t2 starts over).  A ladder CTA that gave up may
     // have left its tile counter and exit ticket behind: zero them for the next launch.
     CK(cudaMemset(h->err, 0, sizeof(int32_t)));
+    h->h_ctl->err = 0;
     if (h->sched) CK(cudaMemset(h->sched, 0, kSched * sizeof(int32_t)));
     return CCDGPU_ERR_TIMEOUT;
   }
@@ -2419,9 +2435,11 @@ int check_errors(ccdgpu_handle *h) {
 
 int set_ctl(ccdgpu_handle *h, int active, double tol, int64_t max_iters, double mixing,
             bool reset_loop, int parity = -1, int phase = 0) {
-  int rc = sync_ctl(h);
+  int rc = fresh_ctl(h);
   if (rc) return rc;
   Control &c = *h->h_ctl;
+  unsigned char was[kCtlUpload];
+  std::memcpy(was, &c, kCtlUpload);
   if (parity >= 0) c.parity = parity;
   if (reset_loop) {
     c.e_prev = 100.0;
@@ -2438,8 +2456,10 @@ int set_ctl(ccdgpu_handle *h, int active, double tol, int64_t max_iters, double 
   c.tol = tol;
   c.max_iters = max_iters;
   c.mixing = mixing;
-  CK(cudaMemcpyAsync(h->ctl, h->h_ctl, sizeof(Control), cudaMemcpyHostToDevice, h->s0));
-  CK(cudaStreamSynchronize(h->s0));
+  // In stream order before what is launched next; the next host change of the mirror is either
+  // after a synchronisation or followed by its own upload.
+  if (std::memcmp(was, &c, kCtlUpload) != 0)
+    CK(cudaMemcpyAsync(h->ctl, h->h_ctl, kCtlUpload, cudaMemcpyHostToDevice, h->s0));
   return CCDGPU_OK;
 }
 
@@ -2455,8 +2475,9 @@ int init_ctl(ccdgpu_handle *h) {
   c.mixing = 0.5;
   c.trace_iter = -1;
   for (int k = 0; k < kTraceKernels; k++) c.trace_first[k] = ~0ull;
-  CK(cudaMemcpyAsync(h->ctl, h->h_ctl, sizeof(Control), cudaMemcpyHostToDevice, h->s0));
+  CK(cudaMemcpyAsync(h->ctl, h->h_ctl, kCtlUpload, cudaMemcpyHostToDevice, h->s0));
   CK(cudaStreamSynchronize(h->s0));
+  h->ctl_current = true;
   return CCDGPU_OK;
 }
 
@@ -2676,7 +2697,9 @@ int ccdgpu_reset(ccdgpu_handle *h) {
   if (h->nt) CK(cudaMemsetAsync(h->tkt_tc, 0, (size_t)h->nt * h->n_tkttc * 2, h->s0));
   h->slab_current = false;
   h->tc_stale = false;
-  return set_ctl(h, 0, h->h_ctl->tol, h->h_ctl->max_iters, h->h_ctl->mixing, true);
+  if (int rc = set_ctl(h, 0, h->h_ctl->tol, h->h_ctl->max_iters, h->h_ctl->mixing, true)) return rc;
+  CK(cudaStreamSynchronize(h->s0));
+  return CCDGPU_OK;
 }
 
 int ccdgpu_set_t2(ccdgpu_handle *h, const double *t2, uint64_t n) {
@@ -2711,9 +2734,9 @@ int ccdgpu_mbpt2(ccdgpu_handle *h, int32_t init_t2, double *e_mbpt2) {
   }
   double e = 0.0;
   CK(cudaMemcpyAsync(&e, h->e_out, 8, cudaMemcpyDeviceToHost, h->s0));
-  CK(cudaStreamSynchronize(h->s0));
+  rc = check_errors(h);
   if (e_mbpt2) *e_mbpt2 = h->n_ranges ? e : 0.0;
-  return check_errors(h);
+  return rc;
 }
 
 int ccdgpu_reference_energy(ccdgpu_handle *h, const double *sp_energy_bare, double *e_ref,
@@ -2870,7 +2893,7 @@ int ccdgpu_build_channels(const ccdgpu_channel_rule *rule, ccdgpu_channel_dims *
 int ccdgpu_get_t2(ccdgpu_handle *h, double *t2, uint64_t n) {
   if (!h || !t2 || n != (uint64_t)h->n_t) return CCDGPU_ERR_INVALID_ARGUMENT;
   CK(cudaSetDevice(h->opt.device));
-  int rc = sync_ctl(h);
+  int rc = fresh_ctl(h);
   if (rc) return rc;
   if ((rc = materialize_t(h))) return rc;
   const double *src = h->opt.path == CCDGPU_PATH_TABLES ? h->t[1] : h->t[0];
@@ -2902,7 +2925,7 @@ int ccdgpu_step(ccdgpu_handle *h, double mixing, double *e_corr) {
   }
   if (rc) return rc;
   if ((rc = sync_ctl(h))) return rc;
-  if ((rc = check_errors(h))) return rc;
+  if ((rc = check_errors(h, false))) return rc;
   if (e_corr) *e_corr = h->h_ctl->e_corr;
   return std::isfinite(h->h_ctl->e_corr) ? CCDGPU_OK : CCDGPU_ERR_NONFINITE;
 }
@@ -2936,6 +2959,7 @@ int loop_launch(ccdgpu_handle *h, SolveState &st) {
     t_pdl = true;
     if (rc) return rc;
   }
+  h->ctl_current = false;
   CK(cudaGraphLaunch(g, h->s0));
   return CCDGPU_OK;
 }
@@ -2994,6 +3018,7 @@ int solve_finish(ccdgpu_handle *h, SolveState &st, double mixing, ccdgpu_result 
       }
     }
     launched += batch;
+    h->ctl_current = false;
     if (st.graph)
       h->launches += batch * (mphase ? h->kernels_per_graph_tc : h->kernels_per_graph);
     if ((rc = sync_ctl(h))) return rc;
@@ -3033,7 +3058,7 @@ int solve_finish(ccdgpu_handle *h, SolveState &st, double mixing, ccdgpu_result 
     res->polish_iterations = (int32_t)c.polish_iters;
     res->seconds = std::chrono::duration<double>(t1 - st.t0).count();
   }
-  return check_errors(h);
+  return check_errors(h, false);
 }
 
 }  // namespace
@@ -3073,7 +3098,7 @@ int ccdgpu_solve_batch(ccdgpu_handle *const *hs, int32_t n, double tol, int64_t 
 int ccdgpu_energy_history(ccdgpu_handle *h, double *out, int64_t cap, int64_t *n_out) {
   if (!h || cap < 0) return CCDGPU_ERR_INVALID_ARGUMENT;
   CK(cudaSetDevice(h->opt.device));
-  int rc = sync_ctl(h);
+  int rc = fresh_ctl(h);
   if (rc) return rc;
   const int64_t n = std::min<int64_t>(h->h_ctl->iterations, 128);
   if (n_out) *n_out = n;
@@ -3109,7 +3134,6 @@ int ccdgpu_calc_t2diff_pphh(ccdgpu_handle *h) {
       (rc = launch_pp_ladder(h, h->s0)) || (rc = launch_expand_d(h, false)))
     return rc;
   h->d_from = 0;
-  CK(cudaStreamSynchronize(h->s0));
   return check_errors(h);
 }
 int ccdgpu_map_from_distributed(ccdgpu_handle *h) {
@@ -3140,7 +3164,7 @@ int ccdgpu_map_to_distributed(ccdgpu_handle *h) {
 int ccdgpu_read_chain(ccdgpu_handle *h, int32_t chain, double *out, uint64_t n, uint64_t *n_out) {
   if (!h) return CCDGPU_ERR_INVALID_ARGUMENT;
   CK(cudaSetDevice(h->opt.device));
-  int rc = sync_ctl(h);
+  int rc = fresh_ctl(h);
   if (rc) return rc;
   const double *src = nullptr;
   uint64_t len = 0;
@@ -3386,7 +3410,7 @@ int ccdgpu_trace_arm(ccdgpu_handle *h, int64_t iteration) {
     c.trace_last[k] = 0;
     c.trace_end[k] = 0;
   }
-  CK(cudaMemcpyAsync(h->ctl, h->h_ctl, sizeof(Control), cudaMemcpyHostToDevice, h->s0));
+  CK(cudaMemcpyAsync(h->ctl, h->h_ctl, kCtlUpload, cudaMemcpyHostToDevice, h->s0));
   CK(cudaStreamSynchronize(h->s0));
   return CCDGPU_OK;
 }
