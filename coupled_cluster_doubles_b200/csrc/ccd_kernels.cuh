@@ -1133,33 +1133,37 @@ __device__ __forceinline__ double block_sum(double v, double *scratch) {
 // One-body terms through the 3-body chains (table path), one CTA per orbital:
 //   hole k:     x = sum v_h_hpp * t2Old_h2pp_h1;  diff_h2pp_h1 = 0.5 x t2Old_h1pp_h2
 //   particle a: y = sum t2Old_p1_p2hh * v_phh_p;  diff_p2_p1hh = -0.5 y t2Old_p2_p1hh
-// (argument order of main.cpp:591-607).
+// (argument order of main.cpp:591-607).  Bound by latency: the few holes' blocks are long (18000
+// elements at EG N=54 |n|^2 <= 19), so those CTAs have 1024 threads, the particles' 256, four
+// elements each in flight: the call for the holes at EG N=38 |n|^2 <= 15 30 -> 17 us.
 // ------------------------------------------------------------------------------------------
-constexpr int kOBThreads = 256;
-__global__ void __launch_bounds__(kOBThreads)
-onebody_tables_kernel(int np, const int64_t *__restrict__ o_h, const int64_t *__restrict__ o_p,
-                      const double *__restrict__ v_h_hpp, const double *__restrict__ old_h2pp_h1,
-                      const double *__restrict__ old_h1pp_h2, double *__restrict__ diff_h2pp_h1,
-                      const double *__restrict__ v_phh_p, const double *__restrict__ old_p1_p2hh,
-                      const double *__restrict__ old_p2_p1hh, double *__restrict__ diff_p2_p1hh,
-                      int do_holes, int do_particles) {
+constexpr int kOBHoles = 1024, kOBParticles = 256, kOBPer = 4;
+template <int NT>
+__global__ void __launch_bounds__(NT)
+onebody_tables_kernel(const int64_t *__restrict__ off, const double *__restrict__ va,
+                      const double *__restrict__ vb, const double *__restrict__ t,
+                      double *__restrict__ diff, double sign) {
   __shared__ double scratch[32];
   __shared__ double total;
-  const int b = blockIdx.x;
-  const bool hole = b < np;
-  if ((hole && !do_holes) || (!hole && !do_particles)) return;
-  const int64_t lo = hole ? o_h[b] : o_p[b - np], hi = hole ? o_h[b + 1] : o_p[b - np + 1];
+  const int64_t lo = off[blockIdx.x], hi = off[blockIdx.x + 1];
   double part = 0.0;
-  for (int64_t e = lo + threadIdx.x; e < hi; e += kOBThreads)
-    part += hole ? v_h_hpp[e] * old_h2pp_h1[e] : old_p1_p2hh[e] * v_phh_p[e];
-  const double sum = block_sum<kOBThreads>(part, scratch);
+  for (int64_t e0 = lo + threadIdx.x; e0 < hi; e0 += kOBPer * NT) {
+    double a[kOBPer], b[kOBPer];
+#pragma unroll
+    for (int k = 0; k < kOBPer; ++k) {
+      const int64_t e = e0 + k * NT;
+      a[k] = e < hi ? va[e] : 0.0;
+      b[k] = e < hi ? vb[e] : 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < kOBPer; ++k) part += a[k] * b[k];
+  }
+  const double sum = block_sum<NT>(part, scratch);
   if (threadIdx.x == 0) total = sum;
   __syncthreads();
-  const double f = hole ? 0.5 * total : -0.5 * total;
-  for (int64_t e = lo + threadIdx.x; e < hi; e += kOBThreads) {
-    if (hole) diff_h2pp_h1[e] = f * old_h1pp_h2[e];
-    else diff_p2_p1hh[e] = f * old_p2_p1hh[e];
-  }
+  const double f = sign * total;
+#pragma unroll 4
+  for (int64_t e = lo + threadIdx.x; e < hi; e += NT) diff[e] = f * t[e];
 }
 
 // What follows X and s, in one launch:

@@ -2373,11 +2373,16 @@ int enqueue_fused_iteration(ccdgpu_handle *h, bool mixed) {
 // Table path stages (mirrors main.cpp:591-665).
 int stage_onebody_tables(ccdgpu_handle *h, int holes, int particles) {
   if (!h->have_3body) return CCDGPU_ERR_UNSUPPORTED;
-  const int nb = (int)h->nsp;
-  onebody_tables_kernel<<<nb, kOBThreads, 0, h->s0>>>(
-      (int)h->np, h->o_h, h->o_p, h->v_h_hpp, h->old_h2pp_h1, h->old_h1pp_h2, h->diff_h2pp_h1,
-      h->v_phh_p, h->old_p1_p2hh, h->old_p2_p1hh, h->diff_p2_p1hh, holes, particles);
-  h->launches++;
+  if (holes) {
+    onebody_tables_kernel<kOBHoles><<<(unsigned)h->np, kOBHoles, 0, h->s0>>>(
+        h->o_h, h->v_h_hpp, h->old_h2pp_h1, h->old_h1pp_h2, h->diff_h2pp_h1, 0.5);
+    h->launches++;
+  }
+  if (particles) {
+    onebody_tables_kernel<kOBParticles><<<(unsigned)h->npart, kOBParticles, 0, h->s0>>>(
+        h->o_p, h->old_p1_p2hh, h->v_phh_p, h->old_p2_p1hh, h->diff_p2_p1hh, -0.5);
+    h->launches++;
+  }
   return cuda_status(cudaGetLastError());
 }
 int stage_gather(ccdgpu_handle *h) {
