@@ -268,6 +268,7 @@ pp_ladder_tc_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *
     if (lane == 0) {
       int gc = 0;  // chunks issued by this CTA (all its tiles)
       bool stop = false;
+      const uint64_t v_policy = l2_evict_first();
       for (int k = 0; !stop; ++k) {
         // Claim the next tile of the launch (tiles are sorted by decreasing work, so this is
         // longest-first list scheduling: a CTA that starts late simply takes fewer tiles) and
@@ -302,7 +303,7 @@ pp_ladder_tc_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *
           mbar_expect_tx(fb, NT * ((GEN ? 0u : abytes) + bbytes));  // GEN: V is generated
 #pragma unroll
           for (int p = 0; p < NT; ++p) {
-            if (!GEN) bulk_g2s(sa + p * kTcAPlane * 2, asrc + p * v_stride, abytes, fb);
+            if (!GEN) bulk_g2s(sa + p * kTcAPlane * 2, asrc + p * v_stride, abytes, fb, v_policy);
             bulk_g2s(sb + p * kTcBPlane * 2, bsrc + p * tkt_stride, bbytes, fb);
           }
         }
