@@ -147,7 +147,8 @@ struct LadderTile {
   int32_t ch, mt, kc0, nks;
   int32_t rows, hk, hs, nb;  // nb: UMMA N (tensor-core tiles)
   int32_t sym, nseg;         // nseg: K segments the channel's row tiles have room for
-  int32_t pk, pad;
+  int32_t pk, nkx;  // nkx: chunks of T X after the tile's own (tensor-core tiles)
+  int64_t tmt_base, xt_base;
   int64_t a_base;   // first A chunk: + c * ladder_as(rows) * kBK (tensor core: see there)
   int64_t b_base;   // first B chunk: + c * kBK * hs
   int64_t ti_base;  // T of the tile's own rows (symmetric channels)
@@ -171,6 +172,10 @@ struct LadderRows {
 struct ChanInfo {
   int32_t pp, hh, pk, hk;
   int32_t hs, nkc, nmt, nhht;  // packed row stride, K chunks, row tiles, hh-ladder slices
+  // T X in the tensor-core ladder (small systems): its 32-deep K chunks (all hh columns), and where
+  // its operands T (A, rows u) and X / 2 (B) are in the T image.
+  int32_t nkx, pad_x;
+  int64_t tmt_base, xt_base;
   int32_t sym, rt_off;  // V stored by its symmetry; first row tile among all channels'
   int64_t t_off;     // pphh block offset (reference t2 layout)
   int64_t pp_off;    // offset into pp_pairs / pp_swap / prow
@@ -198,7 +203,9 @@ struct __align__(16) HHTile {
 // and where X (and, on the diagonal, s) goes (s < 0: off the diagonal).
 struct __align__(16) HHOut {
   int64_t part;
-  int32_t nslices, stride, v, x, s, pad;
+  int32_t nslices, stride, v, x, s;
+  int32_t xt[2];  // X / 2 in the T image, rows kl and (negated) lk; -1: not there
+  int32_t pad[3];
 };
 
 // A warp's part of T X: `rows` rows, T and T X at `at`, X at `x`; from column j0 (hk > 8: 16 of them).

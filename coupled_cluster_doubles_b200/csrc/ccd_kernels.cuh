@@ -590,10 +590,13 @@ hh_slice_kernel(const HHTile *__restrict__ tiles, int n_cta, int n_warp,
 // hole pair do not take a CTA each), each adding every kHHLanes-th slice's partial with eight loads
 // in flight, then a fixed shuffle tree.
 constexpr int kHHLanes = 4;
+// NT > 0: X / 2 also as NT bf16 terms, for the tensor-core ladder of a small system.
+template <int NT>
 __global__ void __launch_bounds__(128)
 hh_reduce_kernel(const HHOut *__restrict__ outs, int n, const double *__restrict__ v_hhhh,
                  const double *__restrict__ part, double *__restrict__ x,
-                 double *__restrict__ s_out, const Control *ctl, int gate) {
+                 double *__restrict__ s_out, __nv_bfloat16 *img, int64_t img_stride,
+                 const Control *ctl, int gate) {
   const int i = (blockIdx.x * 128 + threadIdx.x) / kHHLanes, sub = threadIdx.x % kHHLanes;
   const HHOut o = outs[min(i, n - 1)];  // static data, loaded beside the control block
   const double vh = __ldg(v_hhhh + o.v);
@@ -614,6 +617,18 @@ hh_reduce_kernel(const HHOut *__restrict__ outs, int n, const double *__restrict
   if (sub == 0 && i < n) {
     x[o.x] = vh + p;
     if (o.s >= 0) s_out[o.s] = p;
+    if constexpr (NT > 0) {
+      if (o.xt[0] >= 0) {
+        __nv_bfloat16 a[NT], b[NT];
+        split_bf16_n<NT>(0.5 * (vh + p), a);
+        split_bf16_n<NT>(-0.5 * (vh + p), b);
+#pragma unroll
+        for (int q = 0; q < NT; ++q) {
+          img[q * img_stride + o.xt[0]] = a[q];
+          img[q * img_stride + o.xt[1]] = b[q];
+        }
+      }
+    }
   }
   trace_end(ctl, kTrHHReduce);
 }
@@ -1308,19 +1323,33 @@ hh_post_kernel(int n_ob, int np, int nsp, const int64_t *__restrict__ list_off,
 // One packed amplitude t of quad (u, w) into the mixed-precision operand image: nt bf16 terms
 // of T as the B operand of V T in the tensor-core chunk layout (K = u).
 template <int NT>
-__device__ __forceinline__ void write_t_image_n(const ChanInfo &ch, int u, int w, double t,
-                                                __nv_bfloat16 *img, int64_t stride) {
+__device__ __forceinline__ void write_t_image_n(const ChanInfo &ch, int u, int w,
+                                                const QuadCol &cl, double t, __nv_bfloat16 *img,
+                                                int64_t stride) {
   __nv_bfloat16 hv[NT];
   split_bf16_n<NT>(t, hv);
   const int64_t o =
       ch.tkt_tc_base + (int64_t)(u >> 5) * (ch.nbt >> 3) * kTcGroup + tc_off_mn(w, u & 31);
 #pragma unroll
   for (int p = 0; p < NT; ++p) img[p * stride + o] = hv[p];
+  if (ch.nkx) {  // rows of T as the A operand of T X: columns ij and, negated, ji
+    __nv_bfloat16 mv[NT];
+    split_bf16_n<NT>(-t, mv);
+    const int rg = (ch.pk + 7) >> 3;
+    const int64_t oi = ch.tmt_base + (int64_t)(cl.c_ij >> 5) * rg * kTcGroup + tc_off(u, cl.c_ij & 31);
+    const int64_t oj = ch.tmt_base + (int64_t)(cl.c_ji >> 5) * rg * kTcGroup + tc_off(u, cl.c_ji & 31);
+#pragma unroll
+    for (int p = 0; p < NT; ++p) {
+      img[p * stride + oi] = hv[p];
+      img[p * stride + oj] = mv[p];
+    }
+  }
 }
-__device__ __forceinline__ void write_t_image(const ChanInfo &ch, int u, int w, double t, int nt,
-                                              __nv_bfloat16 *img, int64_t stride) {
-  if (nt == 3) write_t_image_n<3>(ch, u, w, t, img, stride);
-  else write_t_image_n<2>(ch, u, w, t, img, stride);
+__device__ __forceinline__ void write_t_image(const ChanInfo &ch, int u, int w, const QuadCol &cl,
+                                              double t, int nt, __nv_bfloat16 *img,
+                                              int64_t stride) {
+  if (nt == 3) write_t_image_n<3>(ch, u, w, cl, t, img, stride);
+  else write_t_image_n<2>(ch, u, w, cl, t, img, stride);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1438,7 +1467,7 @@ assemble_fused_kernel(const QuadItem *__restrict__ items, int n_items,
     const double t1 = quad_value(vv, dv, ring, tv, xh[cl.i], xh[cl.j], yp[rw.pa], yp[rw.pb],
                                  cl.eij - rw.ea - rw.eb, mixing);
     t_new[p] = t1;
-    if (nt) write_t_image(chans[item.ch], u, w, t1, nt, tkt_tc, tkt_tc_stride);
+    if (nt) write_t_image(chans[item.ch], u, w, cl, t1, nt, tkt_tc, tkt_tc_stride);
     corr += 4.0 * (vv * t1);
   }
   const double sum = block_sum<kAsmThreads>(corr, scratch);
@@ -1535,14 +1564,15 @@ pack_quads_kernel(const QuadItem *__restrict__ items, const ChanInfo *__restrict
 // before a mixed iteration that follows something other than a mixed iteration.
 __global__ void __launch_bounds__(kAsmThreads)
 t_image_kernel(const QuadItem *__restrict__ items, const ChanInfo *__restrict__ chans,
-               const double *tq0, const double *tq1, const Control *ctl,
+               const QuadCol *__restrict__ qcols, const double *tq0, const double *tq1, const Control *ctl,
                __nv_bfloat16 *__restrict__ img, int64_t stride, int nt) {
   const QuadItem item = items[blockIdx.x];
   const int q = item.q0 + threadIdx.x;
   if (q >= item.q1) return;
   const int u = q / item.hk, w = q - u * item.hk;
   const double *t = ctl->parity ? tq1 : tq0;
-  write_t_image(chans[item.ch], u, w, t[item.q_off + (int64_t)u * item.hs + w], nt, img, stride);
+  write_t_image(chans[item.ch], u, w, qcols[item.qcol_off + w],
+                t[item.q_off + (int64_t)u * item.hs + w], nt, img, stride);
 }
 
 // Table path assembly: exactly calcChannelT2_pphh over the eight gathered chains.

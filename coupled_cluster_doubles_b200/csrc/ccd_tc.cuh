@@ -190,6 +190,9 @@ constexpr int kTcGrid = 148;          // persistent grid: one CTA on each SM
 // operand planes of every V T chunk into the stage (fence.proxy.async, then one arrival per
 // warp on the stage's full barrier, for every chunk); the producer copies only the B planes of
 // those chunks.  No V image is read from HBM.
+// Tiles with nkx > 0 go on with T X from the T image's own operands (small systems, where the
+// ladder is too short to be worth starting before X: their mixed iterations then round D as one
+// sum, and a solve with few FP64 iterations after them depends on that at 1e-8).
 template <int NT, bool GEN>
 __global__ void __launch_bounds__(tc_threads(GEN), GEN ? 2 : 1)
 pp_ladder_tc_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *sched,
@@ -284,7 +287,7 @@ pp_ladder_tc_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *
         mbar_arrive(smem_u32(&tq_full[slot]));
         if (ti < 0) break;
         const LadderTile tile = tiles[ti];
-        const int nchunks = tile.nks;
+        const int nchunks = tile.nks + tile.nkx;
         const int rg = (tile.rows + 7) >> 3;  // stored row groups of the A chunks
         const int ng = tile.nb >> 3;          // row groups of a B chunk
         const uint32_t abytes = (uint32_t)rg * kTcGroup * 2, bbytes = (uint32_t)ng * kTcGroup * 2;
@@ -296,14 +299,20 @@ pp_ladder_tc_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *
             stop = true;
             break;
           }
-          const __nv_bfloat16 *asrc = v_tc + tile.a_base + (int64_t)c * rg * kTcGroup;
-          const __nv_bfloat16 *bsrc = tkt_tc + tile.b_base + (int64_t)c * ng * kTcGroup;
+          const bool vt = c < tile.nks;  // V T; then T X
+          const int cx = c - tile.nks;
+          const __nv_bfloat16 *asrc = vt ? v_tc + tile.a_base + (int64_t)c * rg * kTcGroup
+                                         : tkt_tc + tile.tmt_base + (int64_t)cx * rg * kTcGroup;
+          const __nv_bfloat16 *bsrc = vt ? tkt_tc + tile.b_base + (int64_t)c * ng * kTcGroup
+                                         : tkt_tc + tile.xt_base + (int64_t)cx * ng * kTcGroup;
+          const int64_t a_stride = vt ? v_stride : tkt_stride;
+          const bool copy_a = !GEN || !vt;  // GEN: the generator warps write V
           const uint32_t fb = smem_u32(&full[s]);
           const uint32_t sa = base + s * kStageBytes, sb = sa + NT * kTcAPlane * 2;
-          mbar_expect_tx(fb, NT * ((GEN ? 0u : abytes) + bbytes));  // GEN: V is generated
+          mbar_expect_tx(fb, NT * ((copy_a ? abytes : 0u) + bbytes));
 #pragma unroll
           for (int p = 0; p < NT; ++p) {
-            if (!GEN) bulk_g2s(sa + p * kTcAPlane * 2, asrc + p * v_stride, abytes, fb, v_policy);
+            if (copy_a) bulk_g2s(sa + p * kTcAPlane * 2, asrc + p * a_stride, abytes, fb, v_policy);
             bulk_g2s(sb + p * kTcBPlane * 2, bsrc + p * tkt_stride, bbytes, fb);
           }
         }
@@ -332,7 +341,7 @@ pp_ladder_tc_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *
         tc_fence_after();
         const uint32_t acc = tmem + buf * kTcAccCols;
         const uint32_t idesc = tc_idesc(tile.nb);
-        const int nchunks = tile.nks;
+        const int nchunks = tile.nks + tile.nkx;
         bool ok = true;
         for (int c = 0; c < nchunks; ++c, ++gc) {
           const int s = gc % S;
@@ -380,7 +389,7 @@ pp_ladder_tc_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *
       }
       if (ti < 0) break;
       const LadderTile tile = tiles[ti];
-      const int nchunks = tile.nks;
+      const int nchunks = tile.nks + tile.nkx;
       const int64_t pk_off = chans[tile.ch].pk_off;
       const int pk = chans[tile.ch].pk;
       VGenRow rw[RG];
@@ -415,7 +424,7 @@ pp_ladder_tc_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *
           stop = true;
           break;
         }
-        {
+        if (c < tile.nks) {
           unsigned char *sa = stage0 + s * kStageBytes;
 #pragma unroll
           for (int i = 0; i < RG; ++i) {

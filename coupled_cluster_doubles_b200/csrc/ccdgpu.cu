@@ -160,6 +160,8 @@ struct ccdgpu_handle {
   LadderTile *tc_tiles = nullptr;
   int32_t *kcol = nullptr;  // pp index of the w-th c<d pair of each channel (pk_off + w)
   __nv_bfloat16 *v_tc = nullptr, *tkt_tc = nullptr;
+  bool tc_tx = false;     // the tensor-core ladder does T X too
+  double *tx_zero = nullptr;  // ... and the assembly then adds this in place of tx
   bool tc_stale = false;  // tkt_tc is not the image of the current amplitudes
   // Electron gas with V generated on the device: the tensor-core ladder generates its V
   // planes itself (no v_tc images) from these per-row / per-K-column codes and the q^2 table.
@@ -851,6 +853,7 @@ int make_ladder_tiles(ccdgpu_handle *h, const ccdgpu_schedule &sch) {
             const int rg = (rows + 7) / 8, ng = a.nbt / 8;
             t.a_base = a.vtc_base + (int64_t)mt * kTcBM * nk * kTcKC + (int64_t)t.kc0 * rg * kTcGroup;
             t.b_base = a.tkt_tc_base + (int64_t)t.kc0 * ng * kTcGroup;
+            t.nkx = a.nkx; t.tmt_base = a.tmt_base; t.xt_base = a.xt_base;
             cost = (int64_t)(t.nks + 2) * (8 * rg + a.nbt);
           } else {
             t.a_base = a.vkt_base + ladder_chunk(sym, nk, mt, t.kc0, rows);
@@ -1110,6 +1113,10 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
       if (hh_pairs[hoff + k].x > hh_pairs[hoff + k].y)
         hcol[hoff + k] = hcol[hoff + hh_swap[hoff + k]] + 1;
   }
+  // Small systems: every channel one row tile of the tensor-core ladder.
+  h->tc_tx = h->nt > 0;
+  for (int ai = 0; ai < n_act; ai++)
+    if (a_hk[ai] && a_pk[ai] > kTcBM) h->tc_tx = false;
   std::vector<HHTile> hh_tiles;
   int64_t vhh_tot = 0, x_tot = 0, q_tot = 0, vt = 0, part_tot = 0, qcol_tot = 0;
   int64_t vraw_tot = 0;
@@ -1144,6 +1151,13 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
       ci.nkct = (int)ceil_div(pk, kTcKC);
       vtc += (int64_t)ci.nkct * kTcGroup * ceil_div(pk, 8);
       tkttc += (int64_t)ci.nkct * (ci.nbt / 8) * kTcGroup;
+      if (h->tc_tx) {
+        ci.nkx = (int)ceil_div(hh, kTcKC);
+        ci.tmt_base = tkttc;
+        tkttc += (int64_t)ci.nkx * ceil_div(pk, 8) * kTcGroup;
+        ci.xt_base = tkttc;
+        tkttc += (int64_t)ci.nkx * (ci.nbt / 8) * kTcGroup;
+      }
       x_tot += hk * ci.hs;
       q_tot += (int64_t)ci.nkc * kBK * ci.hs;
       // Stored V: room for the whole of it, should it not be symmetric.
@@ -1468,12 +1482,18 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
       quad_items.push_back({ai, (int32_t)q, (int32_t)std::min<int64_t>(nq, q + kQuadPerItem),
                             a.hk, a.hs, a.rt_off, a.q_off, a.x_off, a.pk_off, a.qcol_off});
     const QuadCol *qc = quad_cols.data() + a.qcol_off;
+    auto xt_at = [&](int row, int col) {
+      return a.nkx ? (int32_t)(a.xt_base + (int64_t)(row >> 5) * (a.nbt >> 3) * kTcGroup +
+                               tc_off_mn(col, row & 31))
+                   : -1;
+    };
     for (int kl = 0; nq && kl < a.hk; kl++)
       for (int ij = 0; ij < a.hk; ij++)
         hh_out.push_back({hh_part_off[ai] + kl * a.hk + ij, a.nhht, a.hk * a.hk,
                           (int32_t)(a.vhh_off + (int64_t)qc[kl].c_ij * a.hh + qc[ij].c_ij),
                           (int32_t)(a.x_off + kl * a.hs + ij),
-                          kl == ij ? (int32_t)(a.qcol_off + ij) : -1, 0});
+                          kl == ij ? (int32_t)(a.qcol_off + ij) : -1,
+                          {xt_at(qc[kl].c_ij, ij), xt_at(qc[kl].c_ji, ij)}, {}});
   }
   // T X: the widest channels first, the short units fill in behind them.
   for (const int rows : {16, 64, 128})
@@ -1583,7 +1603,7 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   ar.add(&h->o_h, o_h.size()); ar.add(&h->o_p, o_p.size());
   ar.add(&h->t[0], n_t); ar.add(&h->t[1], n_t); ar.add(&h->dmat, n_t);
   ar.add(&h->old_phhp, h->n_m); ar.add(&h->r_phhp, h->n_m);
-  ar.add(&h->x, x_tot); ar.add(&h->tx, q_tot);
+  ar.add(&h->x, x_tot); ar.add(&h->tx, q_tot); ar.add(&h->tx_zero, h->tc_tx ? q_tot : 0);
   ar.add(&h->s, quad_cols.size()); ar.add(&h->r, h->n_quad_rows); ar.add(&h->xh, np); ar.add(&h->yp, h->npart);
   ar.add(&h->quad_items, quad_items.size());
   ar.add(&h->quad_rows, h->n_quad_rows); ar.add(&h->quad_cols, quad_cols.size());
@@ -2127,9 +2147,12 @@ int launch_hh_ladder(ccdgpu_handle *h, cudaStream_t st, int gate, int only = -1)
   }
   if (h->n_hh_out && (only < 0 || only == 2)) {
     h->launches++;
-    CK(launch_pdl(hh_reduce_kernel, (int)ceil_div((int64_t)h->n_hh_out * kHHLanes, 128), 128, 0, st,
+    const int nt = h->tc_tx && gate ? h->nt : 0;
+    CK(launch_pdl(nt == 3 ? hh_reduce_kernel<3> : nt ? hh_reduce_kernel<2> : hh_reduce_kernel<0>,
+                  (int)ceil_div((int64_t)h->n_hh_out * kHHLanes, 128), 128, 0, st,
                   (const HHOut *)h->hh_out, h->n_hh_out, (const double *)h->v_hhhh,
-                  (const double *)h->part, h->x, h->s, (const Control *)h->ctl, gate));
+                  (const double *)h->part, h->x, h->s, h->tkt_tc, h->n_tkttc,
+                  (const Control *)h->ctl, gate));
   }
   return CCDGPU_OK;
 }
@@ -2160,7 +2183,7 @@ int launch_expand_d(ccdgpu_handle *h, bool tc) {
   if (!h->n_quad_items) return CCDGPU_OK;
   expand_d_kernel<<<h->n_quad_items, kAsmThreads, 0, h->s0>>>(
       h->quad_items, h->chans, tc ? h->tc_lrows : h->lrows, h->quad_rows, h->quad_cols,
-      tc ? h->tc_planes : h->d_planes, h->tx, h->dmat);
+      tc ? h->tc_planes : h->d_planes, tc && h->tc_tx ? h->tx_zero : h->tx, h->dmat);
   h->launches++;
   return cuda_status(cudaGetLastError());
 }
@@ -2188,7 +2211,7 @@ int refresh_tc_image(ccdgpu_handle *h) {
   h->tc_stale = false;
   if (!h->n_quad_items) return CCDGPU_OK;
   t_image_kernel<<<h->n_quad_items, kAsmThreads, 0, h->s0>>>(
-      h->quad_items, h->chans, h->tq[0], h->tq[1], h->ctl, h->tkt_tc, h->n_tkttc, h->nt);
+      h->quad_items, h->chans, h->quad_cols, h->tq[0], h->tq[1], h->ctl, h->tkt_tc, h->n_tkttc, h->nt);
   h->launches++;
   return cuda_status(cudaGetLastError());
 }
@@ -2273,7 +2296,8 @@ int launch_assemble_fused(ccdgpu_handle *h, cudaStream_t st, int gate) {
       h->n_asm_blocks, kAsmThreads, 0, st, (const QuadItem *)h->quad_items, h->n_quad_items,
       (const ChanInfo *)h->chans, (const LadderRows *)(gate ? h->tc_lrows : h->lrows),
       (const QuadRow *)h->quad_rows, (const QuadCol *)h->quad_cols, (const double *)h->vq,
-      (const double *)(gate ? h->tc_planes : h->d_planes), (const double *)h->tx,
+      (const double *)(gate ? h->tc_planes : h->d_planes),
+      (const double *)(gate && h->tc_tx ? h->tx_zero : h->tx),
       (const double *)h->r_quad, (const double *)h->xh, (const double *)h->yp, h->tq[0], h->tq[1],
       h->epart, h->ticket, h->ctl, h->tkt_tc, h->n_tkttc, gate ? h->nt : 0,
       (cudaGraphConditionalHandle)(h->loop_capture ? h->loop_cond : 0), h->loop_capture, gate));
@@ -2313,7 +2337,7 @@ int enqueue_fused_iteration(ccdgpu_handle *h, bool mixed) {
     CK(cudaEventRecord(h->ev[0], h->s0));
     if ((rc = launch_hh_ladder(h, h->s0, gate))) return rc;
     CK(cudaEventRecord(h->ev[1], h->s0));
-    if ((rc = launch_hh_post(h, h->s0, gate))) return rc;
+    if ((rc = launch_hh_post(h, h->s0, gate, mixed && h->tc_tx ? 0 : -1))) return rc;
     CK(cudaEventRecord(h->ev[2], h->s0));
     if ((rc = ladder(h->s0))) return rc;
     CK(cudaEventRecord(h->ev[3], h->s0));
@@ -2356,7 +2380,11 @@ int enqueue_fused_iteration(ccdgpu_handle *h, bool mixed) {
     if ((rc = launch_ring_units(h, branch[used++].st, gate, k))) return rc;
   }
   for (int k = 0; k < std::max(used, 1); k++) CK(cudaEventRecord(branch[k].ev, branch[k].st));
-  if ((rc = launch_hh_post(h, h->s2, gate))) return rc;
+  if (mixed && h->tc_tx) {  // the ladder reads X
+    CK(cudaEventRecord(h->ev_fork2, h->s2));
+    CK(cudaStreamWaitEvent(h->s0, h->ev_fork2, 0));
+  }
+  if ((rc = launch_hh_post(h, h->s2, gate, mixed && h->tc_tx ? 0 : -1))) return rc;
   CK(cudaEventRecord(h->ev_join2, h->s2));
   if ((rc = ladder(h->s0))) return rc;
   for (int k = 0; k < std::max(used, 1); k++) CK(cudaStreamWaitEvent(h->s0, branch[k].ev, 0));
