@@ -253,6 +253,7 @@ struct RingPair {
   int64_t a_off;   // A: V_hphp of the channel (hp' x hp')
   int64_t b_src;   // V_hphp of the transpose (ph' x ph' in its order), the source of B
   int64_t tp, a_img, b_img, c_img, to_img;  // T' image; operands and destinations
+  int32_t g, pad;  // warps of its units
 };
 // A pair and column tiles [n0, n0 + nt) of its S, with what its warps need of the pair.
 struct RingUnit {
@@ -306,6 +307,7 @@ struct Control {
 constexpr int32_t kErrNonFinite = 1;
 constexpr int32_t kErrTimeout = 2;
 constexpr int32_t kErrBadIndex = 4;
+constexpr int32_t kErrAsym = 16;     // set-up: a channel's stored V is not symmetric
 constexpr int32_t kErrRingMaps = 8;  // aj_ib / bi_ja / bj_ia are not ai_jb under the swaps
 
 }  // namespace ccd

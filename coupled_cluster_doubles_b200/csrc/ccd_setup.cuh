@@ -53,9 +53,10 @@ __global__ void v_symmetry_kernel(const ChanInfo *__restrict__ chans, const int4
                                   const int32_t *__restrict__ kcol,
                                   const int32_t *__restrict__ prow_raw,
                                   const int64_t *__restrict__ vraw_off,
-                                  const double *__restrict__ vraw, int32_t *asym) {
+                                  const double *__restrict__ vraw, int32_t *asym, int32_t *err) {
   const int4 it = items[blockIdx.x];
   const ChanInfo ch = chans[it.x];
+  if (!ch.sym) return;
   const double *src = vraw + vraw_off[it.x] + (int64_t)it.z * ch.pp;
   const int col = kcol[ch.pk_off + it.y];
   bool differs = false;
@@ -64,7 +65,10 @@ __global__ void v_symmetry_kernel(const ChanInfo *__restrict__ chans, const int4
     const double b = vraw[vraw_off[it.x] + (int64_t)prow_raw[ch.pk_off + w] * ch.pp + col];
     differs |= !(a == b);
   }
-  if (differs) asym[it.x] = 1;
+  if (differs) {
+    asym[it.x] = 1;
+    atomicOr(err, kErrAsym);
+  }
 }
 
 // Packed V_pppp as nt bf16 terms in the tensor-core chunk images of the mixed-precision
