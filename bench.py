@@ -290,12 +290,11 @@ def quad_count(system):
 
 
 def assemble_bytes(n_quads, nt):
-    """Algorithmic bytes of one fused assembly launch, per quad (four amplitudes (ab,ij),
-    (ab,ji), (ba,ij), (ba,ji)): read t, V and D at (ab,ij), R and the int32 phhp index at the
-    four positions (72 B); write the four amplitudes and their phhp copies (64 B) and the next
-    iteration's operand-image entries of row ab, columns ij and ji, in both images: nt bf16
-    terms each (mixed) or one FP64 value."""
-    return n_quads * (136.0 + (8.0 * nt if nt else 32.0))
+    """Algorithmic bytes of one fused assembly launch, per quad (one amplitude of the four (ab,ij),
+    (ab,ji), (ba,ij), (ba,ji)): read t, V, T X, D and the two ring sums, write the new
+    amplitude (56 B; D is one plane here, row tiles with several read 8 B more each), and in a
+    mixed iteration its nt bf16 terms."""
+    return n_quads * (56.0 + 2.0 * nt)
 
 
 def main():
@@ -510,17 +509,17 @@ def main():
         # average device time in the profiled solve (events around each family on its stream).
         def kernel_rooflines(a):
             nt = nt_of[a]
-            lad = "pp_ladder_tc_kernel<2>" if a == "mixed" else "pp_ladder_kernel<0,1,2>"
+            lad = "pp_ladder_tc_kernel<2>" if a == "mixed" else "pp_ladder_kernel"
             fams = [
                 ("pp_ladder", lad, work[a]["ladder_bytes"], work[a]["ladder_flops"]),
                 ("assemble_energy", "assemble_fused_kernel", assemble_bytes(n_quads, nt), 0.0),
-                ("ring", "phhp_gather_kernel + ring_small_kernel + ring16_kernel<32/48/64>",
+                ("ring", "tp_gather_kernel + ring_pair_kernel<1/2/4>",
                  cls_bytes("ring_small", "ring_mid", "ring_large"),
                  cls_flops("ring_small", "ring_mid", "ring_large")),
-                ("hh_ladder", "hh_mma_kernel<2> + hh_slice_kernel + hh_reduce_kernel",
+                ("hh_ladder", "hh_slice_kernel + hh_reduce_kernel",
                  cls_bytes("hh_small", "hh_large", "hh_reduce"),
                  cls_flops("hh_small", "hh_large")),
-                ("onebody", "onebody_fused_kernel", cls_bytes("onebody"), 0.0),
+                ("onebody", "hh_post_kernel", cls_bytes("onebody"), 0.0),
             ]
             out = {}
             for fam, kname, by, fl in fams:
