@@ -475,7 +475,7 @@ __device__ __forceinline__ void cp_async_wait() {
 //   wider: a CTA per slice, both ranges copied to shared memory (16-byte cp.async; the row stride
 //   hs is 4 mod 8 doubles, conflict-free for the fragments) and P on m16n8k16, warp w taking items
 //   of one 16-row tile by kHHNC 8-column tiles.
-// Both form the row dots r, and write the slice's partial P, which hh_reduce_kernel adds in slice order
+// Both form the row dots r, and write the slice's partial P, which hh_reduce_kernel adds in a fixed order
 // (deterministic).
 // ------------------------------------------------------------------------------------------
 constexpr int kHHThreads = 128;

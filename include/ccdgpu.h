@@ -280,10 +280,10 @@ int ccdgpu_read_chain(ccdgpu_handle *h, int32_t chain, double *out, uint64_t n, 
 /* Device timing of the last ccdgpu_solve / ccdgpu_step, per kernel family, in
  * milliseconds summed over the iterations, and launch counts. */
 typedef struct ccdgpu_profile {
-  double ms_ladder;      /* pp ladder + T X GEMM (calc.cpp:162-202) */
+  double ms_ladder;      /* pp ladder (calc.cpp:162-202) */
   double ms_hh_ladder;   /* hh ladder intermediate X (calc.cpp:141-160) */
-  double ms_ring;        /* ring GEMMs (calc.cpp:264-313), on the second stream */
-  double ms_onebody;     /* one-body terms (calc.cpp:9-25, 73-89) */
+  double ms_ring;        /* ring GEMMs (calc.cpp:264-313), on side streams */
+  double ms_onebody;     /* one-body terms (calc.cpp:9-25, 73-89) and T X */
   double ms_assemble;    /* assembly + remaps + energy (calc.cpp:368-421, Chain.hpp:710-802) */
   double ms_total;       /* whole iterations */
   int64_t launches;      /* kernels launched by this library since create */
@@ -352,7 +352,8 @@ int ccdgpu_ladder_profile(ccdgpu_handle *h, int32_t reps, double ms[4], double f
 /* The other kernels of an iteration, each class launched alone `reps` times on the handle's
  * stream (after one warm-up launch): average ms per launch, FP64 flops and algorithmic bytes
  * per launch, indexed ring small (ph', hp' <= 16; with the phhp gather that precedes the ring
- * on the fused path), ring mid (<= 32), ring large, hh ladder
+ * on the fused path), ring mid (<= 32), ring large (a class with fewer units than SMs joins the
+ * next), hh ladder
  * small (at most 8 strict hole pairs), hh ladder rest, one-body sums, hh-ladder reduction.  Amplitudes are
  * not changed (the kernels write only intermediates).  No counterpart in the reference. */
 int ccdgpu_kernel_profile(ccdgpu_handle *h, int32_t reps, double ms[7], double flops[7],
