@@ -99,6 +99,10 @@ struct ccdgpu_handle {
   // (it is expanded when they are read); dmat likewise holds t2Diff_pphh unless d_from names
   // the iteration kind (1 FP64, 2 mixed) whose ladder planes it is expanded from when read.
   bool slab_current = true;
+  // Fused path, for the stage calls: whether old_phhp and the three-body chains hold the current
+  // amplitudes too, and whether t[1] holds the T2 that ccdgpu_map_to_distributed scatters (the
+  // last one loaded or assembled by a stage; else it is the current amplitudes).
+  bool chains_current = true, t2_staged = false;
   int d_from = 0;
   double *x = nullptr, *tx = nullptr;  // hh-ladder X; 0.5 T X in the packed layout
   double *s = nullptr, *r = nullptr, *xh = nullptr, *yp = nullptr, *epart = nullptr;
@@ -2223,6 +2227,22 @@ int materialize_t(ccdgpu_handle *h) {
   h->launches++;
   return cuda_status(cudaGetLastError());
 }
+// The state that the stage calls read, on a handle of the fused path, whose iterations keep the
+// packed amplitudes alone: t2Old_pphh, t2Old_phhp and the three-body chains.
+int launch_map_to(ccdgpu_handle *h, cudaStream_t st, const double *src, double *dst, int mark = 0);
+int ready_slabs(ccdgpu_handle *h) {
+  if (h->opt.path != CCDGPU_PATH_FUSED) return CCDGPU_OK;
+  if (int rc = materialize_t(h)) return rc;
+  if (h->chains_current) return CCDGPU_OK;
+  h->chains_current = true;
+  return launch_map_to(h, h->s0, h->t[0], h->t[0]);
+}
+// A fused iteration leaves the packed amplitudes ahead of everything in the reference's layouts.
+void slabs_behind(ccdgpu_handle *h) { h->slab_current = h->chains_current = h->t2_staged = false; }
+// The amplitudes in t[1] have been scattered: everything but the bf16 image is current.
+void slabs_loaded(ccdgpu_handle *h) {
+  h->slab_current = h->chains_current = h->t2_staged = h->tc_stale = true;
+}
 // The bf16 image of the current amplitudes, before a mixed iteration that does not follow a
 // mixed iteration.
 int refresh_tc_image(ccdgpu_handle *h) {
@@ -2328,8 +2348,7 @@ int launch_energy(ccdgpu_handle *h, cudaStream_t st, int flags) {
   return cuda_status(cudaGetLastError());
 }
 // mark: the pass over non-finite elements (map_to_kernel) instead of the scatters.
-int launch_map_to(ccdgpu_handle *h, cudaStream_t st, const double *src, double *dst,
-                  int mark = 0) {
+int launch_map_to(ccdgpu_handle *h, cudaStream_t st, const double *src, double *dst, int mark) {
   if (!h->n_ranges) return CCDGPU_OK;
   map_to_kernel<<<h->n_ranges, 256, 0, st>>>(h->ranges, h->chans, h->prow, h->hcol, h->flat,
                                              h->n_t, src, dst, h->old_h2pp_h1, h->old_h1pp_h2,
@@ -2737,7 +2756,8 @@ uint64_t ccdgpu_t2_size(const ccdgpu_handle *h) { return h ? (uint64_t)h->n_t : 
 int ccdgpu_reset(ccdgpu_handle *h) {
   if (!h) return CCDGPU_ERR_INVALID_ARGUMENT;
   CK(cudaSetDevice(h->opt.device));
-  // The fused path iterates on the packed amplitudes alone.
+  if (int rc = fresh_ctl(h)) return rc;
+  // The fused path iterates on the packed amplitudes alone; its slabs follow when they are read.
   const bool fused = h->opt.path == CCDGPU_PATH_FUSED;
   const std::pair<double *, int64_t> z[] = {
       {h->tq[h->h_ctl->parity], h->n_q}, {h->old_phhp, h->n_m},
@@ -2747,7 +2767,8 @@ int ccdgpu_reset(ccdgpu_handle *h) {
   for (const auto &b : z)
     if (b.first && b.second) CK(cudaMemsetAsync(b.first, 0, b.second * 8, h->s0));
   if (h->nt) CK(cudaMemsetAsync(h->tkt_tc, 0, (size_t)h->nt * h->n_tkttc * 2, h->s0));
-  h->slab_current = false;
+  slabs_behind(h);
+  h->chains_current = true;  // zeroed above
   h->tc_stale = false;
   if (int rc = set_ctl(h, 0, h->h_ctl->tol, h->h_ctl->max_iters, h->h_ctl->mixing, true)) return rc;
   CK(cudaStreamSynchronize(h->s0));
@@ -2761,8 +2782,7 @@ int ccdgpu_set_t2(ccdgpu_handle *h, const double *t2, uint64_t n) {
   CK(cudaMemcpyAsync(h->t[1], t2, n * 8, cudaMemcpyHostToDevice, h->s0));
   if ((rc = launch_map_to(h, h->s0, h->t[1], h->t[0]))) return rc;
   if ((rc = launch_map_to(h, h->s0, h->t[1], h->t[0], 1))) return rc;
-  h->slab_current = true;
-  h->tc_stale = true;
+  slabs_loaded(h);
   CK(cudaStreamSynchronize(h->s0));
   return CCDGPU_OK;
 }
@@ -2781,8 +2801,7 @@ int ccdgpu_mbpt2(ccdgpu_handle *h, int32_t init_t2, double *e_mbpt2) {
   if ((rc = launch_energy(h, h->s0, 0))) return rc;
   if (init_t2) {  // the amplitudes become the current ones, as after ccdgpu_set_t2
     if ((rc = launch_map_to(h, h->s0, h->t[1], h->t[0]))) return rc;
-    h->slab_current = true;
-    h->tc_stale = true;
+    slabs_loaded(h);
   }
   double e = 0.0;
   CK(cudaMemcpyAsync(&e, h->e_out, 8, cudaMemcpyDeviceToHost, h->s0));
@@ -2968,7 +2987,7 @@ int ccdgpu_step(ccdgpu_handle *h, double mixing, double *e_corr) {
     rc = tables_iteration(h, mixing, nullptr);
   } else if (!(rc = refresh_tc_image(h))) {
     rc = enqueue_fused_iteration(h, h->nt > 0);
-    h->slab_current = false;
+    slabs_behind(h);
     h->d_from = h->nt ? 2 : 1;
   }
   if (inject) {  // the fault applies to this iteration only
@@ -3033,7 +3052,7 @@ int solve_begin(ccdgpu_handle *h, double tol, int64_t max_iters, double mixing, 
   if (st.graph && !st.device_loop && st.mixed && (rc = fused_ready_graph(h, true))) return rc;
   if (st.fused) {
     if ((rc = refresh_tc_image(h))) return rc;
-    h->slab_current = false;
+    slabs_behind(h);
     h->d_from = 0;  // until solve_finish
   }
   st.t0 = std::chrono::steady_clock::now();
@@ -3161,21 +3180,21 @@ int ccdgpu_energy_history(ccdgpu_handle *h, double *out, int64_t cap, int64_t *n
 int ccdgpu_calc_t2diff_p2_p1hh(ccdgpu_handle *h) {
   if (!h) return CCDGPU_ERR_INVALID_ARGUMENT;
   int rc = set_ctl(h, 0, h->h_ctl->tol, h->h_ctl->max_iters, h->h_ctl->mixing, false);
-  if (rc || (rc = stage_onebody_tables(h, 0, 1))) return rc;
+  if (rc || (rc = ready_slabs(h)) || (rc = stage_onebody_tables(h, 0, 1))) return rc;
   CK(cudaStreamSynchronize(h->s0));
   return CCDGPU_OK;
 }
 int ccdgpu_calc_t2diff_h2pp_h1(ccdgpu_handle *h) {
   if (!h) return CCDGPU_ERR_INVALID_ARGUMENT;
   int rc = set_ctl(h, 0, h->h_ctl->tol, h->h_ctl->max_iters, h->h_ctl->mixing, false);
-  if (rc || (rc = stage_onebody_tables(h, 1, 0))) return rc;
+  if (rc || (rc = ready_slabs(h)) || (rc = stage_onebody_tables(h, 1, 0))) return rc;
   CK(cudaStreamSynchronize(h->s0));
   return CCDGPU_OK;
 }
 int ccdgpu_calc_t2diff_phhp(ccdgpu_handle *h) {
   if (!h) return CCDGPU_ERR_INVALID_ARGUMENT;
   int rc = set_ctl(h, 0, h->h_ctl->tol, h->h_ctl->max_iters, h->h_ctl->mixing, false);
-  if (rc || (rc = launch_ring(h, h->s0, 0))) return rc;
+  if (rc || (rc = ready_slabs(h)) || (rc = launch_ring(h, h->s0, 0))) return rc;
   CK(cudaStreamSynchronize(h->s0));
   return CCDGPU_OK;
 }
@@ -3197,8 +3216,9 @@ int ccdgpu_map_from_distributed(ccdgpu_handle *h) {
 }
 int ccdgpu_calc_t2_pphh(ccdgpu_handle *h, double mixing, double *corr) {
   if (!h) return CCDGPU_ERR_INVALID_ARGUMENT;
-  int rc = stage_assemble_tables(h, mixing);
-  if (rc || (rc = launch_energy(h, h->s0, 0))) return rc;
+  int rc = ready_slabs(h);
+  if (rc || (rc = stage_assemble_tables(h, mixing)) || (rc = launch_energy(h, h->s0, 0))) return rc;
+  h->t2_staged = true;
   double e = 0;
   CK(cudaMemcpyAsync(&e, h->e_out, 8, cudaMemcpyDeviceToHost, h->s0));
   CK(cudaStreamSynchronize(h->s0));
@@ -3207,8 +3227,10 @@ int ccdgpu_calc_t2_pphh(ccdgpu_handle *h, double mixing, double *corr) {
 }
 int ccdgpu_map_to_distributed(ccdgpu_handle *h) {
   if (!h) return CCDGPU_ERR_INVALID_ARGUMENT;
-  int rc = launch_map_to(h, h->s0, h->t[1], h->t[0]);
-  if (rc) return rc;
+  int rc = ready_slabs(h);
+  const bool staged = h->t2_staged || h->opt.path == CCDGPU_PATH_TABLES;
+  if (rc || (rc = launch_map_to(h, h->s0, h->t[staged ? 1 : 0], h->t[0]))) return rc;
+  slabs_loaded(h);
   CK(cudaStreamSynchronize(h->s0));
   return CCDGPU_OK;
 }
@@ -3240,7 +3262,7 @@ int ccdgpu_read_chain(ccdgpu_handle *h, int32_t chain, double *out, uint64_t n, 
   if (!out) return CCDGPU_OK;
   if (!src) return CCDGPU_ERR_UNSUPPORTED;
   if (n < len) return CCDGPU_ERR_INVALID_ARGUMENT;
-  if (chain == CCDGPU_CHAIN_OLD_PHHP && h->opt.path != CCDGPU_PATH_TABLES) {
+  if (chain == CCDGPU_CHAIN_OLD_PHHP && !h->chains_current) {
     // The fused path's iterations do not keep this slab.
     if ((rc = launch_phhp_gather(h, h->s0))) return rc;
     CK(cudaStreamSynchronize(h->s0));
