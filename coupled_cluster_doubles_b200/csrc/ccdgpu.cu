@@ -2105,21 +2105,23 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   if (e & kErrAsym) {  // those channels are stored and streamed in full
     e &= ~kErrAsym;
     std::vector<int32_t> asym(n_act);
-    CK(cudaMemcpy(asym.data(), d_asym, n_act * sizeof(int32_t), cudaMemcpyDeviceToHost));
+    CK(cudaMemcpyAsync(asym.data(), d_asym, n_act * sizeof(int32_t), cudaMemcpyDeviceToHost, h->s0));
+    CK(cudaStreamSynchronize(h->s0));
     for (int ai = 0; ai < n_act; ai++)
       if (asym[ai]) {
         ChanInfo &a = h->host_chans[ai];
         a.sym = 0;
         h->ladder_bytes += 4.0 * a.pk * (a.pk - 1.0);
       }
-    CK(cudaMemcpy(h->chans, h->host_chans.data(), n_act * sizeof(ChanInfo), cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(h->chans, h->host_chans.data(), n_act * sizeof(ChanInfo),
+                       cudaMemcpyHostToDevice, h->s0));
     CK(cudaMemsetAsync(h->v_t, 0, vt * sizeof(double), h->s0));
     tile_v_kernel<<<(unsigned)vrows.size(), 128, 0, h->s0>>>(h->chans, d_vrows, h->kcol,
                                                              d_vraw_off, vraw, h->v_t);
     CK(cudaGetLastError());
+    CK(cudaMemsetAsync(h->err, 0, sizeof(int32_t), h->s0));
     if (int rc2 = make_ladder_tiles(h, sch)) return rc2;
     CK(cudaStreamSynchronize(h->s0));
-    CK(cudaMemset(h->err, 0, sizeof(int32_t)));
   }
   // Release the scratch allocation.
   for (size_t i = n_allocs; i < h->allocs.size(); i++) dev_free(h->allocs[i].p, h->allocs[i].bytes);
@@ -2495,9 +2497,9 @@ int check_errors(ccdgpu_handle *h, bool read = true) {
     // Reported once: the handle stays usable (the timed-out iteration's amplitudes are
     // incomplete; ccdgpu_reset or ccdgpu_set_t2 starts over).  A ladder CTA that gave up may
     // have left its tile counter and exit ticket behind: zero them for the next launch.
-    CK(cudaMemset(h->err, 0, sizeof(int32_t)));
+    CK(cudaMemsetAsync(h->err, 0, sizeof(int32_t), h->s0));
     h->h_ctl->err = 0;
-    if (h->sched) CK(cudaMemset(h->sched, 0, kSched * sizeof(int32_t)));
+    if (h->sched) CK(cudaMemsetAsync(h->sched, 0, kSched * sizeof(int32_t), h->s0));
     return CCDGPU_ERR_TIMEOUT;
   }
   if (h->h_ctl->error & kErrNonFinite) return CCDGPU_ERR_NONFINITE;
@@ -3270,8 +3272,8 @@ int ccdgpu_read_chain(ccdgpu_handle *h, int32_t chain, double *out, uint64_t n, 
   if (chain == CCDGPU_CHAIN_DIFF_PPHH && (rc = materialize_d(h))) return rc;
   if ((chain == CCDGPU_CHAIN_T2 || chain == CCDGPU_CHAIN_T2_OLD) && (rc = materialize_t(h)))
     return rc;
+  CK(cudaMemcpyAsync(out, src, len * 8, cudaMemcpyDeviceToHost, h->s0));
   CK(cudaStreamSynchronize(h->s0));
-  CK(cudaMemcpy(out, src, len * 8, cudaMemcpyDeviceToHost));
   return CCDGPU_OK;
 }
 
