@@ -199,13 +199,12 @@ struct __align__(16) HHTile {
   int64_t base, part;
   int32_t r0, pad[3];
 };
-// One element of X = V_hhhh + P: P's partials part[k * stride], k < nslices, the V_hhhh element
-// and where X (and, on the diagonal, s) goes (s < 0: off the diagonal).
+// One element of X = V_hhhh + P: P's partials part[k * stride], k < nslices, where X goes (and the
+// packed V_hhhh comes from) and, on the diagonal, s (s < 0: off the diagonal).
 struct __align__(16) HHOut {
   int64_t part;
-  int32_t nslices, stride, v, x, s;
+  int32_t nslices, stride, x, s;
   int32_t xt[2];  // X / 2 in the T image, rows kl and (negated) lk; -1: not there
-  int32_t pad[3];
 };
 
 // A warp's part of T X: `rows` rows, T and T X at `at`, X at `x`; from column j0 (hk > 8: 16 of them).
@@ -247,11 +246,12 @@ struct ModInfo {
 // worked on in the layout of the first.  Set-up data of its operand images.
 struct RingPair {
   int32_t ph, hp;
-  int32_t perm_off, self;  // hp' index in the transpose of each ph' pair; self: the channel is its
-                           // own transpose
+  int32_t perm_off, self;  // hp' index in the transpose of each ph' pair, then (c_src >= 0) the ph'
+                           // index of each hp' pair; self: the channel is its own transpose
   int64_t m_off;   // phhp block of the channel (V_hpph, quads of its elements)
   int64_t a_off;   // A: V_hphp of the channel (hp' x hp')
   int64_t b_src;   // V_hphp of the transpose (ph' x ph' in its order), the source of B
+  int64_t c_src;   // V_hpph of the transpose, averaged with the channel's; -1: the same by the model
   int64_t tp, a_img, b_img, c_img, to_img;  // T' image; operands and destinations
   int32_t g, pad;  // warps of its units
 };

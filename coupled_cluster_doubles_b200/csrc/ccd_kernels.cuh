@@ -593,13 +593,13 @@ constexpr int kHHLanes = 4;
 // NT > 0: X / 2 also as NT bf16 terms, for the tensor-core ladder of a small system.
 template <int NT>
 __global__ void __launch_bounds__(128)
-hh_reduce_kernel(const HHOut *__restrict__ outs, int n, const double *__restrict__ v_hhhh,
+hh_reduce_kernel(const HHOut *__restrict__ outs, int n, const double *__restrict__ v_x,
                  const double *__restrict__ part, double *__restrict__ x,
                  double *__restrict__ s_out, __nv_bfloat16 *img, int64_t img_stride,
                  const Control *ctl, int gate) {
   const int i = (blockIdx.x * 128 + threadIdx.x) / kHHLanes, sub = threadIdx.x % kHHLanes;
   const HHOut o = outs[min(i, n - 1)];  // static data, loaded beside the control block
-  const double vh = __ldg(v_hhhh + o.v);
+  const double vh = __ldg(v_x + o.x);
   if (skip_iteration(ctl, gate, kTrHHReduce)) return;
   const double *pb = part + o.part;
   double p = 0.0;
@@ -644,7 +644,7 @@ hh_reduce_kernel(const HHOut *__restrict__ outs, int n, const double *__restrict
 // is the transpose of the first's (t_ab,ij = t_ba,ji), and the assembly needs only the sums
 //   S[ai, jb] = R[ai, jb] + R[bj, ia] = T' (A + C T') + B T'
 // with A = V_hphp of the first channel, C = V_hpph (the same block for both, by the exchange of
-// both pairs) and B[ai, ck] = V_hphp[(k c), (i a)] of the second: three products instead of four
+// both pairs; of blocks that come from the host, their mean, which is exact for any) and B[ai, ck] = V_hphp[(k c), (i a)] of the second: three products instead of four
 // and half of the amplitudes, of V_hpph and of the results (ring_unit, below).
 // ------------------------------------------------------------------------------------------
 constexpr int kRingSmall = 16;
@@ -1544,6 +1544,21 @@ expand_t_kernel(const ElemRange *__restrict__ ranges, const ChanInfo *__restrict
       if (neg) v = -v;
     }
     t2[e] = v;
+  }
+}
+
+// V_hhhh of the strict pairs in the layout of X.  T is antisymmetric in (k, l), so T X takes the
+// antisymmetric part of X's rows alone: of blocks from the host, whatever they hold, exactly.
+__global__ void __launch_bounds__(256)
+pack_hhhh_kernel(const ChanInfo *__restrict__ chans, const QuadCol *__restrict__ qcols,
+                 const double *__restrict__ v_hhhh, double *__restrict__ v_x) {
+  const ChanInfo ch = chans[blockIdx.x];
+  if (!ch.pk) return;  // no X
+  const double *v = v_hhhh + ch.vhh_off;
+  for (int e = threadIdx.x; e < ch.hk * ch.hk; e += blockDim.x) {
+    const int kl = e / ch.hk, ij = e - kl * ch.hk, col = qcols[ch.qcol_off + ij].c_ij;
+    const QuadCol c = qcols[ch.qcol_off + kl];
+    v_x[ch.x_off + kl * ch.hs + ij] = 0.5 * (v[c.c_ij * ch.hh + col] - v[c.c_ji * ch.hh + col]);
   }
 }
 

@@ -651,7 +651,8 @@ __global__ void transpose_hpph_kernel(const ModInfo *__restrict__ mods,
 }
 
 // Operand images and destinations of the fused path's ring (one CTA per pair), from the blocks
-// and the quads of all modified channels.  C[i][k] = V_hpph (held transposed, ph' rows),
+// and the quads of all modified channels.  C[i][k] = V_hpph (held transposed, ph' rows; c_src >= 0:
+// the mean of it and the transpose's at the exchanged pairs),
 // A = V_hphp, B[r][r2] = V_hphp of the transpose at (perm[r2], perm[r]), zero padded, in the order
 // in which an m16n8k16 warp takes them: C and B as A operands ([row tile][K step][4][lane][2]), A
 // as accumulators ([row tile][column tile][2][lane][2]), and the destinations alike ([row tile]
@@ -681,12 +682,17 @@ ring_image_kernel(const RingPair *__restrict__ pairs, const int32_t *__restrict_
     row = 16 * (blk / steps) + (lane >> 2) + 8 * (i & 1);
     k = 16 * (blk % steps) + (lane & 3) + 4 * (i >> 1);
   };
+  const int32_t *pm = perm + m.perm_off;
   for (int e = threadIdx.x; e < H * P; e += blockDim.x) {
     int i, k;
     a_elem(e, P / 16, i, k);
-    img[m.c_img + e] = i < hp && k < ph ? v_hpph[m.m_off + (int64_t)k * hp + i] : 0.0;
+    double v = 0.0;
+    if (i < hp && k < ph) {
+      v = v_hpph[m.m_off + (int64_t)k * hp + i];
+      if (m.c_src >= 0) v = 0.5 * (v + v_hpph[m.c_src + (int64_t)pm[ph + i] * ph + pm[k]]);
+    }
+    img[m.c_img + e] = v;
   }
-  const int32_t *pm = perm + m.perm_off;
   for (int e = threadIdx.x; e < P * P; e += blockDim.x) {
     int r, k;
     a_elem(e, P / 16, r, k);

@@ -105,6 +105,7 @@ struct ccdgpu_handle {
   bool chains_current = true, t2_staged = false;
   int d_from = 0;
   double *x = nullptr, *tx = nullptr;  // hh-ladder X; 0.5 T X in the packed layout
+  double *v_x = nullptr;               // V_hhhh in the layout of X
   double *s = nullptr, *r = nullptr, *xh = nullptr, *yp = nullptr, *epart = nullptr;
   int32_t *flat = nullptr;
   int32_t *ring_quads = nullptr;  // phhp position -> 4 x packed position + term, -1
@@ -1360,6 +1361,14 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
         if (ia.x < 0) return CCDGPU_ERR_BAD_TABLE;
         look[(size_t)ia.x * h->npart + (ia.y - np)] = make_int2((int)g, k);
       }
+    // ... and -> channel, ph' index, for V_hpph of the transpose (V from the host).
+    std::vector<int2> look_ph(gen_v ? 0 : look.size(), make_int2(-1, -1));
+    for (size_t g = 0; g < mod_gen.size() && !gen_v; g++)
+      for (int k = 0; k < mod_gen[g].ph; k++) {
+        const int2 ai = mod_ph[mod_gen[g].ph_off + k];
+        if (ai.x < 0) return CCDGPU_ERR_BAD_TABLE;
+        look_ph[(size_t)ai.y * h->npart + (ai.x - np)] = make_int2((int)g, k);
+      }
     for (size_t g = 0; g < mod_gen.size(); g++) {
       const ModGen &m = mod_gen[g];
       const int perm_off = (int)ring_perm.size();
@@ -1382,6 +1391,16 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
       r.perm_off = perm_off;
       r.self = other == (int)g;
       r.m_off = m.m_off; r.a_off = m.y_off; r.b_src = mod_gen[other].y_off;
+      r.c_src = -1;
+      if (!gen_v) {
+        r.c_src = mod_gen[other].m_off;
+        for (int k = 0; k < m.hp; k++) {
+          const int2 ia = mod_hp[m.hp_off + k];
+          const int2 l = look_ph[(size_t)ia.x * h->npart + (ia.y - np)];
+          if (l.x != other) return CCDGPU_ERR_BAD_TABLE;
+          ring_perm.push_back(l.y);
+        }
+      }
       pairs.push_back(r);
     }
     // The largest first, so that the short ones fill in behind them.
@@ -1509,10 +1528,9 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     for (int kl = 0; nq && kl < a.hk; kl++)
       for (int ij = 0; ij < a.hk; ij++)
         hh_out.push_back({hh_part_off[ai] + kl * a.hk + ij, a.nhht, a.hk * a.hk,
-                          (int32_t)(a.vhh_off + (int64_t)qc[kl].c_ij * a.hh + qc[ij].c_ij),
                           (int32_t)(a.x_off + kl * a.hs + ij),
                           kl == ij ? (int32_t)(a.qcol_off + ij) : -1,
-                          {xt_at(qc[kl].c_ij, ij), xt_at(qc[kl].c_ji, ij)}, {}});
+                          {xt_at(qc[kl].c_ij, ij), xt_at(qc[kl].c_ji, ij)}});
   }
   // T X: the widest channels first, the short units fill in behind them.
   for (const int rows : {16, 64, 128})
@@ -1622,7 +1640,7 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   ar.add(&h->o_h, o_h.size()); ar.add(&h->o_p, o_p.size());
   ar.add(&h->t[0], n_t); ar.add(&h->t[1], n_t); ar.add(&h->dmat, n_t);
   ar.add(&h->old_phhp, h->n_m); ar.add(&h->r_phhp, h->n_m);
-  ar.add(&h->x, x_tot); ar.add(&h->tx, q_tot); ar.add(&h->tx_zero, h->tc_tx ? q_tot : 0);
+  ar.add(&h->x, x_tot); ar.add(&h->v_x, x_tot); ar.add(&h->tx, q_tot); ar.add(&h->tx_zero, h->tc_tx ? q_tot : 0);
   ar.add(&h->s, quad_cols.size()); ar.add(&h->r, h->n_quad_rows); ar.add(&h->xh, np); ar.add(&h->yp, h->npart);
   ar.add(&h->quad_items, quad_items.size());
   ar.add(&h->quad_rows, h->n_quad_rows); ar.add(&h->quad_cols, quad_cols.size());
@@ -1971,6 +1989,9 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
       pack_quads_kernel<<<h->n_quad_items, kAsmThreads, 0, h->s0>>>(
           h->quad_items, h->chans, h->quad_rows, h->quad_cols, h->v_pphh, h->vq);
       CK(cudaGetLastError());
+      pack_hhhh_kernel<<<(unsigned)h->n_act, 256, 0, h->s0>>>(h->chans, h->quad_cols, h->v_hhhh,
+                                                              h->v_x);
+      CK(cudaGetLastError());
     }
     if (derive_tables || gen_v3) {
       pair_sizes_kernel<<<(unsigned)chans.size(), 256, 0, h->s0>>>(
@@ -2175,7 +2196,7 @@ int launch_hh_ladder(ccdgpu_handle *h, cudaStream_t st, int gate, int only = -1)
     const int nt = h->tc_tx && gate ? h->nt : 0;
     CK(launch_pdl(nt == 3 ? hh_reduce_kernel<3> : nt ? hh_reduce_kernel<2> : hh_reduce_kernel<0>,
                   (int)ceil_div((int64_t)h->n_hh_out * kHHLanes, 128), 128, 0, st,
-                  (const HHOut *)h->hh_out, h->n_hh_out, (const double *)h->v_hhhh,
+                  (const HHOut *)h->hh_out, h->n_hh_out, (const double *)h->v_x,
                   (const double *)h->part, h->x, h->s, h->tkt_tc, h->n_tkttc,
                   (const Control *)h->ctl, gate));
   }
