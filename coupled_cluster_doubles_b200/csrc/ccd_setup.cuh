@@ -40,6 +40,11 @@ __global__ void tile_v_kernel(const ChanInfo *__restrict__ chans, const int4 *__
   const ChanInfo ch = chans[it.x];
   const int u = it.y;
   const double *src = vraw + vraw_off[it.x] + (int64_t)it.z * ch.pp;
+  if (!ch.hk) {  // no ladder tiles
+    for (int w = threadIdx.x; w < ch.pk; w += blockDim.x)
+      v_t[ch.vkt_base + (int64_t)u * ch.pk + w] = src[kcol[ch.pk_off + w]];
+    return;
+  }
   const int mt = u / kMaxBM, r = u % kMaxBM, rows = min(kMaxBM, ch.pk - mt * kMaxBM);
   const int ar = ladder_as(rows);
   for (int w = ladder_kc0(ch.sym, mt) * kBK + threadIdx.x; w < ch.pk; w += blockDim.x)
@@ -79,6 +84,7 @@ __global__ void tile_v_tc_kernel(const ChanInfo *__restrict__ chans, const int4 
                                  __nv_bfloat16 *__restrict__ v_tc, int64_t stride, int nt) {
   const int4 it = items[blockIdx.x];
   const ChanInfo ch = chans[it.x];
+  if (!ch.hk) return;
   const int u = it.y;
   const double *src = vraw + vraw_off[it.x] + (int64_t)it.z * ch.pp;
   const int mt = u >> 7, r = u & 127;
@@ -721,7 +727,8 @@ ring_image_kernel(const RingPair *__restrict__ pairs, const int32_t *__restrict_
 // destinations come from it (ring_image_kernel).  The other three ring maps of loadMaps
 // are ai_jb composed with the swaps i<->j and a<->b (load.cpp:469-526 builds all four from the
 // same (a,i),(j,b) pairing); this is checked here, since the fused ring and assembly
-// take R_aj,ib, R_bi,ja and R_bj,ia from the exchanged elements.
+// take R_aj,ib, R_bi,ja and R_bj,ia from the exchanged elements.  irregular (tables from the host):
+// marks three-body tables that are not each other's under those swaps.
 __global__ void ring_maps_kernel(const ElemRange *__restrict__ ranges,
                                  const ChanInfo *__restrict__ chans,
                                  const int32_t *__restrict__ pp_swap,
@@ -729,7 +736,8 @@ __global__ void ring_maps_kernel(const ElemRange *__restrict__ ranges,
                                  const int32_t *__restrict__ prow,
                                  const int32_t *__restrict__ hcol,
                                  const int32_t *__restrict__ flat, int64_t n_t,
-                                 int32_t *__restrict__ dst, int32_t *err) {
+                                 int32_t *__restrict__ dst, unsigned long long *irregular,
+                                 int32_t *err) {
   const ElemRange rg = ranges[blockIdx.x];
   const ChanInfo ch = chans[rg.ch];
   for (int64_t e = rg.e0 + threadIdx.x; e < rg.e1; e += blockDim.x) {
@@ -747,6 +755,8 @@ __global__ void ring_maps_kernel(const ElemRange *__restrict__ ranges,
     if (flat[5 * n_t + e] != flat[4 * n_t + e_ji] || flat[6 * n_t + e] != flat[4 * n_t + e_ba] ||
         flat[7 * n_t + e] != flat[4 * n_t + e_baji])
       atomicOr(err, kErrRingMaps);
+    if (irregular && (flat[n_t + e_ji] != flat[e] || flat[3 * n_t + e_ba] != flat[2 * n_t + e]))
+      *irregular = 1;
   }
 }
 

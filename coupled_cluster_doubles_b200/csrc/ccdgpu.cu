@@ -24,6 +24,7 @@
 
 #include "ccd_channels.cuh"
 #include "ccd_device.cuh"
+#include "ccd_general.cuh"
 #include "ccd_kernels.cuh"
 #include "ccd_setup.cuh"
 #include "ccd_tc.cuh"
@@ -137,6 +138,13 @@ struct ccdgpu_handle {
   ModelDev md{};
   bool has_model = false;
   double *eps_io = nullptr;
+  // Inputs that lack the antisymmetry in (a, b) or (i, j) that the packed kernels rely on: host V
+  // blocks or tables, and the amplitudes last loaded.  The table path and the stage calls then form
+  // t2Diff_pphh element by element (ccd_general.cuh); dmat_full: it has elements outside the quads.
+  unsigned long long *irr = nullptr;  // largest element, and the check's mark
+  bool irregular = false, irregular_t = false, dmat_full = false, v_generated = false;
+  int64_t n_vhh = 0;         // hh x hh elements of all channels
+  double *x_full = nullptr;  // X, hh x hh (allocated when first needed)
 
   cudaGraphExec_t graph = nullptr;
   int64_t kernels_per_graph = 0;
@@ -964,6 +972,7 @@ double ms_since(std::chrono::steady_clock::time_point t0) {
 }
 
 void ready_loop_graphs(ccdgpu_handle *h);
+int launch_antisymmetry(ccdgpu_handle *h, const double *src);
 
 int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   const auto t_build = std::chrono::steady_clock::now();
@@ -1083,7 +1092,7 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   for (int ai = 0; ai < n_act; ai++) {
     a_row_off[ai + 1] = a_row_off[ai] + a_pr[ai];
     a_pk_off[ai + 1] = a_pk_off[ai] + a_pk[ai];
-    a_vrow_off[ai + 1] = a_vrow_off[ai] + (a_hk[ai] ? a_pk[ai] : 0);
+    a_vrow_off[ai + 1] = a_vrow_off[ai] + a_pk[ai];
   }
   rowmap.resize(on_the_fly ? 0 : a_row_off[n_act]);  // rows a <= b, as V_pppp is uploaded
   // Row items of the stored-V tiling kernels (not needed when V_pppp is generated).
@@ -1094,7 +1103,7 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     const int64_t pp = D[act_chan[ai]].pp, off = a_pp_off[ai];
     const int64_t hh = D[act_chan[ai]].hh, hoff = a_hh_off[ai];
     int32_t *rm = on_the_fly ? nullptr : rowmap.data() + a_row_off[ai];
-    int4 *vr = on_the_fly || !a_hk[ai] ? nullptr : vrows.data() + a_vrow_off[ai];
+    int4 *vr = on_the_fly ? nullptr : vrows.data() + a_vrow_off[ai];
     int32_t *kc = kcol.data() + a_pk_off[ai];
     int pr = 0, pk = 0;
     for (int64_t k = 0; k < pp; k++) {
@@ -1172,6 +1181,8 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
                             ci.q_off + (int64_t)t * rows * ci.hs,
                             part_tot + (int64_t)t * hk * hk, (int32_t)(ci.pk_off + t * rows), {}});
       part_tot += (int64_t)ci.nhht * hk * hk;
+    } else if (!on_the_fly) {
+      vt += (int64_t)pk * pk;  // row-major, for ccd_general.cuh alone
     }
     vraw_off.push_back(vraw_tot);
     if (!on_the_fly) vraw_tot += (int64_t)a_pr[ai] * pp;  // rows a <= b only
@@ -1179,6 +1190,8 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   }
   if (q_tot * 4 >= INT32_MAX) return CCDGPU_ERR_UNSUPPORTED;  // ring_dst is 32-bit
   h->n_q = q_tot;
+  h->n_vhh = vhh_tot;
+  h->v_generated = on_the_fly;
   const int64_t pp_tot = a_pp_off[n_act], hh_tot = a_hh_off[n_act];
   h->n_act = n_act;
   // hh-ladder units: one per CTA (hk > 8) first, then one per warp; within each the largest
@@ -1646,7 +1659,7 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   ar.add(&h->quad_rows, h->n_quad_rows); ar.add(&h->quad_cols, quad_cols.size());
   ar.add(&h->kcol, kcol.size());  // V tiling at create
   ar.add(&h->epart, std::max(h->n_ranges, h->n_asm_blocks)); ar.add(&h->ctl, 1); ar.add(&h->e_out, 1);
-  ar.add(&h->ticket, 1);
+  ar.add(&h->ticket, 1); ar.add(&h->irr, 2);
   if (h->nt) {
     auto round_up = [](int64_t n) { return std::max<int64_t>(256, (n + 255) / 256 * 256); };
     h->n_vtc = round_up(vtc); h->n_tkttc = round_up(tkttc);
@@ -2033,8 +2046,15 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     CK(cudaGetLastError());
     ring_maps_kernel<<<h->n_ranges, 256, 0, h->s0>>>(h->ranges, h->chans, h->pp_swap, h->hh_swap,
                                                      h->prow, h->hcol, h->flat, n_t,
-                                                     h->ring_quads, h->err);
+                                                     h->ring_quads,
+                                                     derive_tables ? nullptr : h->irr + 1, h->err);
     CK(cudaGetLastError());
+    if (!gen_v) {
+      TRY(launch_antisymmetry(h, h->v_pphh));
+      antisymmetry_hhhh_kernel<<<(unsigned)h->n_act, 256, 0, h->s0>>>(h->chans, h->hh_swap,
+                                                                      h->v_hhhh, h->irr + 1);
+      CK(cudaGetLastError());
+    }
     if (!pairs.empty()) {
       ring_image_kernel<<<(unsigned)pairs.size(), 256, 0, h->s0>>>(
           d_pairs, d_ring_perm, h->v_hpph, h->v_hphp, h->ring_quads, h->ring_img, h->ring_src,
@@ -2120,9 +2140,12 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   }
   h->create_ms[3] = ms_since(t_sched);
   int32_t e = 0;
+  unsigned long long irr = 0;
   CK(cudaMemcpyAsync(&e, h->err, sizeof(e), cudaMemcpyDeviceToHost, h->s0));
+  CK(cudaMemcpyAsync(&irr, h->irr + 1, sizeof(irr), cudaMemcpyDeviceToHost, h->s0));
   CK(cudaStreamSynchronize(h->s0));
   h->create_ms[2] = ms_since(t_build) - h->create_ms[0] - h->create_ms[1];
+  h->irregular = irr != 0 || (e & kErrRingMaps);
   if (e & kErrAsym) {  // those channels are stored and streamed in full
     e &= ~kErrAsym;
     std::vector<int32_t> asym(n_act);
@@ -2226,6 +2249,8 @@ int launch_pp_ladder(ccdgpu_handle *h, cudaStream_t st, int cls = -1) {
 }
 // t2Diff_pphh from the ladder's planes (tc: the tensor-core ladder's) and T X.
 int launch_expand_d(ccdgpu_handle *h, bool tc) {
+  if (h->dmat_full) CK(cudaMemsetAsync(h->dmat, 0, h->n_t * sizeof(double), h->s0));
+  h->dmat_full = false;
   if (!h->n_quad_items) return CCDGPU_OK;
   expand_d_kernel<<<h->n_quad_items, kAsmThreads, 0, h->s0>>>(
       h->quad_items, h->chans, tc ? h->tc_lrows : h->lrows, h->quad_rows, h->quad_cols,
@@ -2250,6 +2275,18 @@ int materialize_t(ccdgpu_handle *h) {
   h->launches++;
   return cuda_status(cudaGetLastError());
 }
+// Marks in h->irr whether src (t2_pphh layout) lacks the antisymmetry of the packed layout.
+int launch_antisymmetry(ccdgpu_handle *h, const double *src) {
+  if (!h->n_ranges) return CCDGPU_OK;
+  CK(cudaMemsetAsync(h->irr, 0, sizeof(*h->irr), h->s0));
+  max_abs_kernel<<<(unsigned)std::min<int64_t>(ceil_div(h->n_t, 1024), 148 * 8), 256, 0, h->s0>>>(
+      src, h->n_t, h->irr);
+  CK(cudaGetLastError());
+  antisymmetry_kernel<<<h->n_ranges, 256, 0, h->s0>>>(h->ranges, h->chans, h->pp_swap, h->hh_swap,
+                                                      src, h->irr, h->irr + 1);
+  h->launches += 2;
+  return cuda_status(cudaGetLastError());
+}
 // The state that the stage calls read, on a handle of the fused path, whose iterations keep the
 // packed amplitudes alone: t2Old_pphh, t2Old_phhp and the three-body chains.
 int launch_map_to(ccdgpu_handle *h, cudaStream_t st, const double *src, double *dst, int mark = 0);
@@ -2261,7 +2298,9 @@ int ready_slabs(ccdgpu_handle *h) {
   return launch_map_to(h, h->s0, h->t[0], h->t[0]);
 }
 // A fused iteration leaves the packed amplitudes ahead of everything in the reference's layouts.
-void slabs_behind(ccdgpu_handle *h) { h->slab_current = h->chains_current = h->t2_staged = false; }
+void slabs_behind(ccdgpu_handle *h) {
+  h->slab_current = h->chains_current = h->t2_staged = h->irregular_t = false;
+}
 // The amplitudes in t[1] have been scattered: everything but the bf16 image is current.
 void slabs_loaded(ccdgpu_handle *h) {
   h->slab_current = h->chains_current = h->t2_staged = h->tc_stale = true;
@@ -2379,6 +2418,34 @@ int launch_map_to(ccdgpu_handle *h, cudaStream_t st, const double *src, double *
                                              h->tq[0], h->tq[1], h->have_3body ? 1 : 0, h->ctl,
                                              mark);
   h->launches++;
+  return cuda_status(cudaGetLastError());
+}
+
+// t2Diff_pphh of the table path and the stage calls into dmat, from t2Old_pphh (t[0]).
+int launch_pphh(ccdgpu_handle *h) {
+  int rc;
+  if (!h->irregular && !h->irregular_t) {
+    if ((rc = launch_hh_ladder(h, h->s0, 0)) || (rc = launch_hh_post(h, h->s0, 0, 1)) ||
+        (rc = launch_pp_ladder(h, h->s0)))
+      return rc;
+    return launch_expand_d(h, false);
+  }
+  if (!h->n_ranges) return CCDGPU_OK;
+  if (!h->x_full) {
+    void *p = nullptr;
+    size_t got = 0;
+    CK(dev_alloc(std::max<int64_t>(h->n_vhh, 1) * sizeof(double), &p, &got));
+    h->allocs.push_back({p, got});
+    h->x_full = static_cast<double *>(p);
+  }
+  h->dmat_full = true;
+  general_x_kernel<<<dim3((unsigned)h->n_act, 8), 256, 0, h->s0>>>(h->chans, h->v_pphh, h->v_hhhh,
+                                                                   h->t[0], h->x_full);
+  CK(cudaGetLastError());
+  general_d_kernel<<<h->n_ranges, 256, 0, h->s0>>>(h->ranges, h->chans, h->prow, h->kcol, h->pp_swap,
+                                                   h->pp_pairs, h->v_t, h->md, h->v_generated,
+                                                   h->x_full, h->t[0], h->dmat);
+  h->launches += 2;
   return cuda_status(cudaGetLastError());
 }
 
@@ -2678,10 +2745,7 @@ int tables_iteration(ccdgpu_handle *h, double mixing, double *corr) {
   if ((rc = stage_onebody_tables(h, 0, 1))) return rc;     // calcT2Diff_p2_p1hh
   if ((rc = stage_onebody_tables(h, 1, 0))) return rc;     // calcT2Diff_h2pp_h1
   if ((rc = launch_ring(h, h->s0, 0))) return rc;   // calcT2Diff_phhp
-  if ((rc = launch_hh_ladder(h, h->s0, 0))) return rc;     // calcT2Diff_pphh
-  if ((rc = launch_hh_post(h, h->s0, 0, 1))) return rc;
-  if ((rc = launch_pp_ladder(h, h->s0))) return rc;
-  if ((rc = launch_expand_d(h, false))) return rc;
+  if ((rc = launch_pphh(h))) return rc;                    // calcT2Diff_pphh
   if ((rc = stage_gather(h))) return rc;                   // 8 x mapFromDistributed
   if ((rc = stage_assemble_tables(h, mixing))) return rc;  // calcT2_pphh
   if ((rc = launch_energy(h, h->s0, 2))) return rc;
@@ -2806,7 +2870,12 @@ int ccdgpu_set_t2(ccdgpu_handle *h, const double *t2, uint64_t n) {
   if ((rc = launch_map_to(h, h->s0, h->t[1], h->t[0]))) return rc;
   if ((rc = launch_map_to(h, h->s0, h->t[1], h->t[0], 1))) return rc;
   slabs_loaded(h);
+  unsigned long long irr = 0;
+  CK(cudaMemsetAsync(h->irr + 1, 0, sizeof(irr), h->s0));
+  if ((rc = launch_antisymmetry(h, h->t[1]))) return rc;
+  CK(cudaMemcpyAsync(&irr, h->irr + 1, sizeof(irr), cudaMemcpyDeviceToHost, h->s0));
   CK(cudaStreamSynchronize(h->s0));
+  h->irregular_t = irr != 0;
   return CCDGPU_OK;
 }
 
@@ -2825,6 +2894,7 @@ int ccdgpu_mbpt2(ccdgpu_handle *h, int32_t init_t2, double *e_mbpt2) {
   if (init_t2) {  // the amplitudes become the current ones, as after ccdgpu_set_t2
     if ((rc = launch_map_to(h, h->s0, h->t[1], h->t[0]))) return rc;
     slabs_loaded(h);
+    h->irregular_t = false;  // V / D: as V_hhpp
   }
   double e = 0.0;
   CK(cudaMemcpyAsync(&e, h->e_out, 8, cudaMemcpyDeviceToHost, h->s0));
@@ -3224,9 +3294,7 @@ int ccdgpu_calc_t2diff_phhp(ccdgpu_handle *h) {
 int ccdgpu_calc_t2diff_pphh(ccdgpu_handle *h) {
   if (!h) return CCDGPU_ERR_INVALID_ARGUMENT;
   int rc = set_ctl(h, 0, h->h_ctl->tol, h->h_ctl->max_iters, h->h_ctl->mixing, false);
-  if (rc || (rc = launch_hh_ladder(h, h->s0, 0)) || (rc = launch_hh_post(h, h->s0, 0, 1)) ||
-      (rc = launch_pp_ladder(h, h->s0)) || (rc = launch_expand_d(h, false)))
-    return rc;
+  if (rc || (rc = ready_slabs(h)) || (rc = launch_pphh(h))) return rc;
   h->d_from = 0;
   return check_errors(h);
 }

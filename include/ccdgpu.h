@@ -191,9 +191,10 @@ const char *ccdgpu_strerror(int status);
 /* Zero every amplitude chain (main.cpp:497-503). */
 int ccdgpu_reset(ccdgpu_handle *h);
 /* Load / read T2 in t2_pphh order (n = sum of pp*hh).  Loading also refreshes t2Old and
- * the scattered layouts, as main.cpp:660-665 would after an iteration.  T2 is antisymmetric in
- * (a, b) and in (i, j), as every T2 of the loop is: the ladder, the one-body sums and (fused path)
- * the ring read its a < b, i < j elements. */
+ * the scattered layouts, as main.cpp:660-665 would after an iteration.  The
+ * iterations of the fused path take a < b, i < j elements alone (T2 is antisymmetric in (a, b) and
+ * in (i, j), as every T2 of the loop is); those of the table path and the stage calls take any T2
+ * as it is. */
 int ccdgpu_set_t2(ccdgpu_handle *h, const double *t2_pphh, uint64_t n);
 int ccdgpu_get_t2(ccdgpu_handle *h, double *t2_pphh, uint64_t n);
 /* Second-order energy on the device, the reference's MBPT2 (MBPT2Corr.cpp:6-38):
