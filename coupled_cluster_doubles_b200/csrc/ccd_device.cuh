@@ -308,6 +308,7 @@ constexpr int32_t kErrNonFinite = 1;
 constexpr int32_t kErrTimeout = 2;
 constexpr int32_t kErrBadIndex = 4;
 constexpr int32_t kErrAsym = 16;     // set-up: a channel's stored V is not symmetric
+constexpr int32_t kErrRingLists = 32;  // ai_jb's rows and columns are not the ph' and hp' lists'
 constexpr int32_t kErrRingMaps = 8;  // aj_ib / bi_ja / bj_ia are not ai_jb under the swaps
 
 }  // namespace ccd

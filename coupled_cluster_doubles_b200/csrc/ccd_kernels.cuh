@@ -651,9 +651,10 @@ constexpr int kRingSmall = 16;
 constexpr int kRingMax = 80;  // largest ph', hp'
 
 // Quad of a phhp slab position: 4 * (packed position) + k, k = 0: (ab, ij), 1: (ab, ji),
-// 2: (ba, ij), 3: (ba, ji); -1 outside every quad.  The amplitude there is +t, -t, -t, +t.
-__device__ __forceinline__ double ring_amplitude(const double *tq, int32_t dst) {
-  if (dst < 0) return 0.0;
+// 2: (ba, ij), 3: (ba, ji); kNoQuad outside every quad.  The amplitude there is +t, -t, -t, +t.
+constexpr uint32_t kNoQuad = ~0u;
+__device__ __forceinline__ double ring_amplitude(const double *tq, uint32_t dst) {
+  if (dst == kNoQuad) return 0.0;
   const double t = __ldcg(tq + (dst >> 2));
   return ((dst & 3) == 1 || (dst & 3) == 2) ? -t : t;
 }
@@ -661,7 +662,7 @@ __device__ __forceinline__ double ring_amplitude(const double *tq, int32_t dst) 
 // The phhp slab (t2Old_phhp) of a fused handle from its packed amplitudes, for readers of the
 // chain.
 __global__ void __launch_bounds__(256)
-phhp_gather_kernel(const int32_t *__restrict__ dst, int64_t n, const double *tq0,
+phhp_gather_kernel(const uint32_t *__restrict__ dst, int64_t n, const double *tq0,
                    const double *tq1, double *__restrict__ phhp, const Control *ctl) {
   const double *__restrict__ t = ctl->parity ? tq1 : tq0;
   for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n;
@@ -1145,6 +1146,26 @@ tp_gather_kernel(const int32_t *__restrict__ src, int64_t n, const double *tq0, 
   trace_end(ctl, kTrGather);
 }
 
+// The two ring sums of every quad from R in the phhp slab, of a fused handle whose channels do not
+// pair up (at: ai_jb, the phhp position of an amplitude).
+constexpr int kAsmThreads = 256;
+__global__ void __launch_bounds__(kAsmThreads)
+ring_sums_kernel(const QuadItem *__restrict__ items, const ChanInfo *__restrict__ chans,
+                 const QuadRow *__restrict__ qrows, const QuadCol *__restrict__ qcols,
+                 const int32_t *__restrict__ at, const double *__restrict__ r,
+                 double *__restrict__ r_quad) {
+  const QuadItem item = items[blockIdx.x];
+  const int q = item.q0 + threadIdx.x;
+  if (q >= item.q1) return;
+  const int u = q / item.hk, w = q - u * item.hk;
+  const QuadRow rw = qrows[item.pk_off + u];
+  const QuadCol cl = qcols[item.qcol_off + w];
+  at += chans[item.ch].t_off;
+  double *o = r_quad + 2 * (item.q_off + (int64_t)u * item.hs + w);
+  o[0] = r[at[rw.o_ab + cl.c_ij]] + r[at[rw.o_ba + cl.c_ji]];
+  o[1] = r[at[rw.o_ab + cl.c_ji]] + r[at[rw.o_ba + cl.c_ij]];
+}
+
 // Deterministic block reduction (fixed tree) of one double; result valid in thread 0.
 template <int NT>
 __device__ __forceinline__ double block_sum(double v, double *scratch) {
@@ -1361,7 +1382,6 @@ __device__ __forceinline__ void write_t_image(const ChanInfo &ch, int u, int w, 
 // with D = V_pppp T from the ladder's planes plus 0.5 T X from hh_post_kernel (a K extension of the
 // ladder for T X would make it wait for the hh ladder).
 // ------------------------------------------------------------------------------------------
-constexpr int kAsmThreads = 256;
 constexpr int kAsmPerThread = 2;  // table path: elements per thread of an ElemRange
 struct StopState {  // what decides whether the device solve loop goes on
   int64_t iterations, stop_at;

@@ -523,6 +523,34 @@ __global__ void convert_tables_kernel(const ElemRange *__restrict__ ranges, cons
   }
 }
 
+// Whether the ai_jb table puts every amplitude where the ph' and hp' pair lists do (mod_at: each
+// channel's first entry in them).
+__global__ void check_lists_kernel(const ElemRange *__restrict__ ranges,
+                                   const ChanInfo *__restrict__ chans,
+                                   const int2 *__restrict__ pp_pairs,
+                                   const int2 *__restrict__ hh_pairs,
+                                   const RawIndex *__restrict__ ai_jb, uint64_t nch,
+                                   const int2 *__restrict__ mod_dims,
+                                   const int2 *__restrict__ mod_at,
+                                   const int2 *__restrict__ ph_pairs,
+                                   const int2 *__restrict__ hp_pairs, int32_t *err) {
+  const ElemRange rg = ranges[blockIdx.x];
+  const ChanInfo ch = chans[rg.ch];
+  bool differs = false;
+  for (int64_t e = rg.e0 + threadIdx.x; e < rg.e1; e += blockDim.x) {
+    const int64_t loc = e - ch.t_off;
+    const int ab = (int)(loc / ch.hh), ij = (int)(loc - (int64_t)ab * ch.hh);
+    const int2 pab = pp_pairs[ch.pp_off + ab], pij = hh_pairs[ch.hh_off + ij];
+    const RawIndex x = ai_jb[e];
+    if (x.channel >= nch) continue;  // reported by convert_tables_kernel
+    const int2 md = mod_dims[x.channel], at = mod_at[x.channel];
+    if (x.row >= (uint64_t)md.x || x.column >= (uint64_t)md.y) continue;
+    const int2 ai = ph_pairs[at.x + x.row], jb = hp_pairs[at.y + x.column];
+    differs |= ai.x != pab.x || ai.y != pij.x || jb.x != pij.y || jb.y != pab.y;
+  }
+  if (differs) atomicOr(err, kErrRingLists);
+}
+
 // ---- Remap tables derived on the device (problem without loadMaps tables) ----------------
 // loadMaps (load.cpp:389-532) builds the eight tables from the channel maps alone; the same
 // derivation here needs only the pair lists the solver already holds.  Block sizes first:
@@ -669,16 +697,16 @@ __global__ void transpose_hpph_kernel(const ModInfo *__restrict__ mods,
 __global__ void __launch_bounds__(256)
 ring_image_kernel(const RingPair *__restrict__ pairs, const int32_t *__restrict__ perm,
                   const double *__restrict__ v_hpph, const double *__restrict__ v_hphp,
-                  const int32_t *__restrict__ quads, double *__restrict__ img,
+                  const uint32_t *__restrict__ quads, double *__restrict__ img,
                   int32_t *__restrict__ tp_src, int32_t *__restrict__ to_img) {
   const RingPair m = pairs[blockIdx.x];
   const int ph = m.ph, hp = m.hp, P = pad16(ph), H = pad16(hp), n8 = (hp + 7) >> 3;
   auto quad = [&](int r, int c) {
-    return r < ph && c < hp ? quads[m.m_off + (int64_t)r * hp + c] : -1;
+    return r < ph && c < hp ? quads[m.m_off + (int64_t)r * hp + c] : kNoQuad;
   };
-  auto place = [](int32_t q) {
-    const int k = q & 3;
-    return q < 0 ? -1 : 2 * (q >> 2) + ((k == 1 || k == 2) ? 1 : 0);
+  auto place = [](uint32_t q) {
+    const uint32_t k = q & 3;
+    return q == kNoQuad ? -1 : (int32_t)(2 * (q >> 2) + ((k == 1 || k == 2) ? 1 : 0));
   };
   for (int e = threadIdx.x; e < P * (H + 4); e += blockDim.x)
     tp_src[m.tp + e] = place(quad(e / (H + 4), e % (H + 4)));
@@ -717,13 +745,13 @@ ring_image_kernel(const RingPair *__restrict__ pairs, const int32_t *__restrict_
   for (int e = threadIdx.x; e < P * 8 * n8; e += blockDim.x) {
     int r, c;
     c_elem(e >> 7, (e >> 2) & 31, e & 3, r, c);
-    const int32_t q = quad(r, c);
+    const uint32_t q = quad(r, c);
     to_img[m.to_img + e] = m.self && (q & 3) >= 2 ? -1 : place(q);
   }
 }
 
 // Quads of the phhp slab.  dst[ai_jb(e)] of amplitude e: 4 x the packed position of its quad
-// plus 0 (ab, ij), 1 (ab, ji), 2 (ba, ij) or 3 (ba, ji); -1 for a = b or i = j.  The ring's
+// plus 0 (ab, ij), 1 (ab, ji), 2 (ba, ij) or 3 (ba, ji); kNoQuad for a = b or i = j.  The ring's
 // destinations come from it (ring_image_kernel).  The other three ring maps of loadMaps
 // are ai_jb composed with the swaps i<->j and a<->b (load.cpp:469-526 builds all four from the
 // same (a,i),(j,b) pairing); this is checked here, since the fused ring and assembly
@@ -736,7 +764,7 @@ __global__ void ring_maps_kernel(const ElemRange *__restrict__ ranges,
                                  const int32_t *__restrict__ prow,
                                  const int32_t *__restrict__ hcol,
                                  const int32_t *__restrict__ flat, int64_t n_t,
-                                 int32_t *__restrict__ dst, unsigned long long *irregular,
+                                 uint32_t *__restrict__ dst, unsigned long long *irregular,
                                  int32_t *err) {
   const ElemRange rg = ranges[blockIdx.x];
   const ChanInfo ch = chans[rg.ch];
@@ -749,8 +777,8 @@ __global__ void ring_maps_kernel(const ElemRange *__restrict__ ranges,
     const int64_t e_baji = ch.t_off + (int64_t)ps * ch.hh + hs;
     const int32_t f = flat[4 * n_t + e];
     const int r = prow[ch.pp_off + ab], c = hcol[ch.hh_off + ij];
-    dst[f] = r < 0 || c < 0 ? -1
-                            : (int32_t)(4 * (ch.q_off + (int64_t)(r >> 1) * ch.hs + (c >> 1)) +
+    dst[f] = r < 0 || c < 0 ? kNoQuad
+                            : (uint32_t)(4 * (ch.q_off + (int64_t)(r >> 1) * ch.hs + (c >> 1)) +
                                         2 * (r & 1) + (c & 1));
     if (flat[5 * n_t + e] != flat[4 * n_t + e_ji] || flat[6 * n_t + e] != flat[4 * n_t + e_ba] ||
         flat[7 * n_t + e] != flat[4 * n_t + e_baji])

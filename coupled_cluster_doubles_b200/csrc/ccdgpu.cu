@@ -109,7 +109,7 @@ struct ccdgpu_handle {
   double *v_x = nullptr;               // V_hhhh in the layout of X
   double *s = nullptr, *r = nullptr, *xh = nullptr, *yp = nullptr, *epart = nullptr;
   int32_t *flat = nullptr;
-  int32_t *ring_quads = nullptr;  // phhp position -> 4 x packed position + term, -1
+  uint32_t *ring_quads = nullptr;  // phhp position -> 4 x packed position + term (kNoQuad: none)
   // Fused-path ring: units by group size (4, 2, 1 warps), operand images, destinations, and the
   // T' images with where their elements come from.
   RingUnit *ring_units = nullptr;
@@ -120,6 +120,7 @@ struct ccdgpu_handle {
   bool ring_cols = false;               // the four-warp units hold only their columns of T'
   size_t ring_smem[3] = {0, 0, 0};  // dynamic shared memory of the groups' kernels
   std::vector<RingPair> host_pairs;
+  bool ring_paired = false;  // else the fused ring runs channel by channel
   double create_ms[5] = {};   // ccdgpu_profile::ms_create
   double loop_graph_ms = 0;   // ccdgpu_profile::ms_loop_graph
   int64_t *o_h = nullptr, *o_p = nullptr;
@@ -1188,7 +1189,9 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     if (!on_the_fly) vraw_tot += (int64_t)a_pr[ai] * pp;  // rows a <= b only
     chans.push_back(ci);
   }
-  if (q_tot * 4 >= INT32_MAX) return CCDGPU_ERR_UNSUPPORTED;  // ring_dst is 32-bit
+  // 2 x a packed position is 31-bit, 4 x one 32-bit (the ring's tables).  Amplitudes below the limit
+  // above reach this only if their padding (rows to 16, 5 hole pairs to 12) quadruples them.
+  if (q_tot * 2 >= INT32_MAX) return CCDGPU_ERR_UNSUPPORTED;
   h->n_q = q_tot;
   h->n_vhh = vhh_tot;
   h->v_generated = on_the_fly;
@@ -1289,7 +1292,9 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   std::vector<int2> &mod_ph = bs.mod_ph, &mod_hp = bs.mod_hp;  // ... their ph' (b, j), hp' (i, a) pairs
   mod_ph.clear();
   mod_hp.clear();
+  const bool fused = h->opt.path == CCDGPU_PATH_FUSED;
   bool mod_maps = true;  // the problem carries the ph' and hp' pair lists
+  const bool lists_needed = derive_tables || gen_v;
   for (uint64_t c = 0; c < nch; c++) {
     const int64_t ph = MD[c].ph, hp = MD[c].hp;
     mod_dims[c] = make_int2((int)ph, (int)hp);
@@ -1299,7 +1304,7 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     m.ph = (int)ph; m.hp = (int)hp; m.m_off = o_m[c]; m.y_off = y_tot;
     // The pairs themselves are copied in parallel after this loop.
     if (!P->chan_mod_maps || !P->chan_mod_maps[c].ph || !P->chan_mod_maps[c].hp) {
-      if (derive_tables || gen_v) return CCDGPU_ERR_INVALID_ARGUMENT;
+      if (lists_needed) return CCDGPU_ERR_INVALID_ARGUMENT;
       mod_maps = false;
     }
     const int64_t ph0 = mod_gen.empty() ? 0 : mod_gen.back().ph_off + mod_gen.back().ph;
@@ -1335,66 +1340,83 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
           mod_hp[mg.hp_off + k] = make_int2((int)hpm[k].p, (int)hpm[k].q);
         }
       }
-    } else {
-      // A problem with tables and V blocks but without the pair lists: the ai_jb table names the
+      if (bad_mod && lists_needed) return CCDGPU_ERR_BAD_TABLE;
+    }
+    if (fused && (!mod_maps || bad_mod)) {
+      // A problem with tables and V blocks but without usable pair lists: the ai_jb table names the
       // (a, i) of every ph' row and the (j, b) of every hp' column.
       std::fill(mod_ph.begin(), mod_ph.end(), make_int2(-1, -1));
       std::fill(mod_hp.begin(), mod_hp.end(), make_int2(-1, -1));
       std::vector<int64_t> gen_of(nch, -1);
       for (size_t g = 0; g < mod_gen.size(); g++) gen_of[mod_chan[g]] = (int64_t)g;
+      auto put = [](int2 &at, int x, int y) {  // rows and columns recur in other channels
+        const int2 v = make_int2(x, y);
+        int64_t bits;
+        std::memcpy(&bits, &v, sizeof(bits));
+        __atomic_store_n(reinterpret_cast<int64_t *>(&at), bits, __ATOMIC_RELAXED);
+      };
+      std::atomic<int> rc_maps{0};
+#pragma omp parallel for num_threads(host_threads) schedule(dynamic, 4)
       for (int ai = 0; ai < n_act; ai++) {
         const ccdgpu_chain_index *mp = P->maps[CCDGPU_MAP_AI_JB][act_chan[ai]];
-        if (!mp) return CCDGPU_ERR_INVALID_ARGUMENT;
         const ChanInfo &a = chans[ai];
-        for (int64_t e = 0; e < (int64_t)a.pp * a.hh; e++) {
+        if (!mp) rc_maps = CCDGPU_ERR_INVALID_ARGUMENT;
+        for (int64_t e = 0; mp && e < (int64_t)a.pp * a.hh; e++) {
           const int2 ab = pp_pairs[a.pp_off + e / a.hh], ij = hh_pairs[a.hh_off + e % a.hh];
           const int64_t g = mp[e].channel < nch ? gen_of[mp[e].channel] : -1;
-          if (g < 0 || mp[e].row >= (uint64_t)mod_gen[g].ph || mp[e].column >= (uint64_t)mod_gen[g].hp)
-            return CCDGPU_ERR_BAD_TABLE;
-          mod_ph[mod_gen[g].ph_off + mp[e].row] = make_int2(ab.x, ij.x);
-          mod_hp[mod_gen[g].hp_off + mp[e].column] = make_int2(ij.y, ab.y);
+          if (g < 0 || mp[e].row >= (uint64_t)mod_gen[g].ph ||
+              mp[e].column >= (uint64_t)mod_gen[g].hp) {
+            rc_maps = CCDGPU_ERR_BAD_TABLE;
+            break;
+          }
+          put(mod_ph[mod_gen[g].ph_off + mp[e].row], ab.x, ij.x);
+          put(mod_hp[mod_gen[g].hp_off + mp[e].column], ij.y, ab.y);
         }
       }
+      if (rc_maps) return rc_maps;
     }
-    if (bad_mod) return CCDGPU_ERR_BAD_TABLE;
   }
   // Fused-path ring: each channel with its transpose, the channel whose ph' pairs are this one's
   // hp' pairs exchanged (the first of the two in channel order names the pair).
-  const bool paired = h->opt.path == CCDGPU_PATH_FUSED;
+  // Tables from the host may describe blocks that do not pair up; then (and if their rows and columns
+  // turn out not to be those of the lists) the ring runs channel by channel, as on the table path.
   std::vector<RingPair> pairs;
   std::vector<RingUnit> units;
   std::vector<int32_t> ring_perm;
   int64_t img_tot = 0, tp_tot = 0, to_tot = 0;
-  if (paired) {
-    std::vector<int2> &look = bs.mod_look;  // (hole, particle) pair -> channel, hp' index
+  auto pair_up = [&]() {
+    // (hole, particle) pair -> channel, hp' index; and (V_hpph of the transpose, V from the host)
+    // -> channel, ph' index.
+    std::vector<int2> &look = bs.mod_look;
     look.assign((size_t)np * h->npart, make_int2(-1, -1));
-    for (size_t g = 0; g < mod_gen.size(); g++)
+    std::vector<int2> look_ph(gen_v ? 0 : look.size(), make_int2(-1, -1));
+    for (size_t g = 0; g < mod_gen.size(); g++) {
       for (int k = 0; k < mod_gen[g].hp; k++) {
         const int2 ia = mod_hp[mod_gen[g].hp_off + k];
-        if (ia.x < 0) return CCDGPU_ERR_BAD_TABLE;
-        look[(size_t)ia.x * h->npart + (ia.y - np)] = make_int2((int)g, k);
+        if (ia.x < 0) return false;
+        int2 &l = look[(size_t)ia.x * h->npart + (ia.y - np)];
+        if (l.x >= 0) return false;  // in two channels
+        l = make_int2((int)g, k);
       }
-    // ... and -> channel, ph' index, for V_hpph of the transpose (V from the host).
-    std::vector<int2> look_ph(gen_v ? 0 : look.size(), make_int2(-1, -1));
-    for (size_t g = 0; g < mod_gen.size() && !gen_v; g++)
-      for (int k = 0; k < mod_gen[g].ph; k++) {
+      for (int k = 0; k < mod_gen[g].ph && !gen_v; k++) {
         const int2 ai = mod_ph[mod_gen[g].ph_off + k];
-        if (ai.x < 0) return CCDGPU_ERR_BAD_TABLE;
+        if (ai.x < 0) return false;
         look_ph[(size_t)ai.y * h->npart + (ai.x - np)] = make_int2((int)g, k);
       }
+    }
     for (size_t g = 0; g < mod_gen.size(); g++) {
       const ModGen &m = mod_gen[g];
       const int perm_off = (int)ring_perm.size();
       int other = -2;
       for (int k = 0; k < m.ph; k++) {
         const int2 ai = mod_ph[m.ph_off + k];
-        if (ai.x < 0) return CCDGPU_ERR_BAD_TABLE;
+        if (ai.x < 0) return false;
         const int2 l = look[(size_t)ai.y * h->npart + (ai.x - np)];
-        if (l.x < 0 || (other >= 0 && l.x != other)) return CCDGPU_ERR_BAD_TABLE;
+        if (l.x < 0 || (other >= 0 && l.x != other)) return false;
         other = l.x;
         ring_perm.push_back(l.y);
       }
-      if (mod_gen[other].hp != m.ph || mod_gen[other].ph != m.hp) return CCDGPU_ERR_BAD_TABLE;
+      if (mod_gen[other].hp != m.ph || mod_gen[other].ph != m.hp) return false;
       if (other < (int)g) {  // named by its transpose
         ring_perm.resize(perm_off);
         continue;
@@ -1410,12 +1432,20 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
         for (int k = 0; k < m.hp; k++) {
           const int2 ia = mod_hp[m.hp_off + k];
           const int2 l = look_ph[(size_t)ia.x * h->npart + (ia.y - np)];
-          if (l.x != other) return CCDGPU_ERR_BAD_TABLE;
+          if (l.x != other) return false;
           ring_perm.push_back(l.y);
         }
       }
       pairs.push_back(r);
     }
+    return true;
+  };
+  h->ring_paired = fused && pair_up();
+  if (!h->ring_paired) {
+    pairs.clear();
+    ring_perm.clear();
+    if (fused && derive_tables) return CCDGPU_ERR_BAD_TABLE;  // no tables could fit such lists
+  } else {
     // The largest first, so that the short ones fill in behind them.
     std::stable_sort(pairs.begin(), pairs.end(), [](const RingPair &x, const RingPair &y) {
       return (int64_t)pad16(x.ph) * pad16(x.hp) > (int64_t)pad16(y.ph) * pad16(y.hp);
@@ -1647,7 +1677,7 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   if (on_the_fly) ar.add_unset(&h->v_t, vt);
   else ar.add(&h->v_t, vt);
   ar.add(&h->v_hpph, h->n_m); ar.add(&h->v_hphp, y_tot);
-  ar.add(&h->flat, (size_t)8 * n_t); ar.add(&h->ring_quads, n_t); ar.add(&h->r_quad, paired ? 2 * q_tot : 0);
+  ar.add(&h->flat, (size_t)8 * n_t); ar.add(&h->ring_quads, n_t); ar.add(&h->r_quad, fused ? 2 * q_tot : 0);
   ar.add(&h->ring_units, units.size()); ar.add(&h->ring_img, img_tot);
   ar.add(&h->ring_tp, tp_tot); ar.add(&h->ring_src, tp_tot); ar.add(&h->ring_to, to_tot);
   ar.add(&h->o_h, o_h.size()); ar.add(&h->o_p, o_p.size());
@@ -1798,9 +1828,19 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   ModGen *d_mod_gen = nullptr;
   int2 *d_mod_ph = nullptr, *d_mod_hp = nullptr;
   int32_t *d_mod_chan = nullptr;
+  // With tables from the host, the lists that the ring's pairs rest on are checked against them.
+  const bool check_lists = h->ring_paired && !derive_tables;
+  const bool lists_on_device = gen_v || check_lists;
+  std::vector<int2> mod_at(check_lists ? nch : 0, make_int2(0, 0));
+  for (size_t g = 0; g < mod_gen.size() && check_lists; g++)
+    mod_at[mod_gen_chan[g]] = make_int2((int)mod_gen[g].ph_off, (int)mod_gen[g].hp_off);
+  int2 *d_mod_at = nullptr;
+  sc.add(&d_mod_at, mod_at.size());
+  if (lists_on_device) {
+    sc.add(&d_mod_ph, mod_ph.size()); sc.add(&d_mod_hp, mod_hp.size());
+  }
   if (gen_v) {
-    sc.add(&d_mod_gen, mod_gen.size()); sc.add(&d_mod_ph, mod_ph.size());
-    sc.add(&d_mod_hp, mod_hp.size()); sc.add(&d_mod_chan, mod_gen_chan.size());
+    sc.add(&d_mod_gen, mod_gen.size()); sc.add(&d_mod_chan, mod_gen_chan.size());
   }
   sc.add(&vraw, vraw_tot); sc.add(&hhpp_raw, gen_v ? 0 : n_t);
   sc.add(&hpph_raw, gen_v ? 0 : h->n_m);
@@ -1943,10 +1983,13 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     for (int k = 0; k < 8 && !derive_tables; k++)
       TRY(upload_runs(h, reinterpret_cast<ccdgpu_chain_index *>(raw_idx) + (size_t)k * n_t, sm[k], nm));
     if (derive_tables && !mlook_dev) TRY(put(d_mlook, mlook));
-    if (gen_v) {
-      TRY(put(d_mod_gen, mod_gen));
+    TRY(put(d_mod_at, mod_at));
+    if (lists_on_device) {
       TRY(put(d_mod_ph, mod_ph));
       TRY(put(d_mod_hp, mod_hp));
+    }
+    if (gen_v) {
+      TRY(put(d_mod_gen, mod_gen));
       TRY(put(d_mod_chan, mod_gen_chan));
     }
     TRY(upload_runs(h, hpph_raw, src_hpph, cnt_hpph));
@@ -2039,6 +2082,11 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
       TableGeometry geo{h->o_h, h->o_p, d_o_m, d_mod_dims, nch, np, h->npart};
       convert_tables_kernel<<<h->n_ranges, 256, 0, h->s0>>>(h->ranges, raw_idx, n_t, geo,
                                                             h->flat, counts, h->err);
+      CK(cudaGetLastError());
+      if (check_lists)
+        check_lists_kernel<<<h->n_ranges, 256, 0, h->s0>>>(
+            h->ranges, h->chans, h->pp_pairs, h->hh_pairs, raw_idx + CCDGPU_MAP_AI_JB * n_t, nch,
+            d_mod_dims, d_mod_at, d_mod_ph, d_mod_hp, h->err);
     }
     CK(cudaGetLastError());
     const int nb = (int)std::min<int64_t>(ceil_div(5 * n_t, 256), 148 * 32);
@@ -2166,6 +2214,17 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     CK(cudaMemsetAsync(h->err, 0, sizeof(int32_t), h->s0));
     if (int rc2 = make_ladder_tiles(h, sch)) return rc2;
     CK(cudaStreamSynchronize(h->s0));
+  }
+  if (e & kErrRingLists) {  // the tables' blocks are not those that the lists name
+    e &= ~kErrRingLists;
+    h->ring_paired = false;
+    h->host_pairs.clear();
+    h->n_tp = h->n_ring[0] = h->n_ring[1] = h->n_ring[2] = 0;
+    if (h->loop64) cudaGraphExecDestroy(h->loop64);
+    if (h->loop_tc) cudaGraphExecDestroy(h->loop_tc);
+    h->loop64 = h->loop_tc = nullptr;
+    h->loop_state = 0;
+    CK(cudaMemsetAsync(h->err, 0, sizeof(int32_t), h->s0));
   }
   // Release the scratch allocation.
   for (size_t i = n_allocs; i < h->allocs.size(); i++) dev_free(h->allocs[i].p, h->allocs[i].bytes);
@@ -2356,8 +2415,19 @@ int launch_ring(ccdgpu_handle *h, cudaStream_t st, int gate) {
   }
   return CCDGPU_OK;
 }
-// Fused-path ring: the T' images, and the units of group k (0: 4 warps, 1: 2, 2: 1).
+// Fused-path ring: the T' images, and the units of group k (0: 4 warps, 1: 2, 2: 1).  Without pairs
+// the whole of it: the phhp slab, the table path's kernels, the quads' two sums.
 int launch_tp_gather(ccdgpu_handle *h, cudaStream_t st, int gate) {
+  if (!h->ring_paired) {
+    if (!h->n_quad_items) return CCDGPU_OK;
+    int rc;
+    if ((rc = launch_phhp_gather(h, st)) || (rc = launch_ring(h, st, gate))) return rc;
+    ring_sums_kernel<<<h->n_quad_items, kAsmThreads, 0, st>>>(
+        h->quad_items, h->chans, h->quad_rows, h->quad_cols, h->flat + CCDGPU_MAP_AI_JB * h->n_t,
+        h->r_phhp, h->r_quad);
+    h->launches++;
+    return cuda_status(cudaGetLastError());
+  }
   if (!h->n_tp) return CCDGPU_OK;
   h->launches++;
   return cuda_status(launch_pdl(
