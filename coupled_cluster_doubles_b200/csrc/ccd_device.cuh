@@ -183,6 +183,8 @@ struct ChanInfo {
   int64_t vhh_off;   // hh x hh block offset (V_hhhh)
   int64_t q_off;     // packed block: 16 nkc x hs doubles (T, V_hhpp)
   int64_t x_off;     // X: hk x hs
+  int64_t part_off;  // partials of the hh ladder
+  int32_t hh_first, tx_first;  // first of the channel's HHOut and TXTile records
   int64_t vkt_base;  // A tiles of V
   int64_t pk_off;    // strict particle pairs: offset into kcol / quad rows / r (pk entries)
   int64_t qcol_off;  // strict hole pairs: offset into quad columns / s (hk entries)
@@ -246,8 +248,8 @@ struct ModInfo {
 // worked on in the layout of the first.  Set-up data of its operand images.
 struct RingPair {
   int32_t ph, hp;
-  int32_t perm_off, self;  // hp' index in the transpose of each ph' pair, then (c_src >= 0) the ph'
-                           // index of each hp' pair; self: the channel is its own transpose
+  int32_t ph_off, hp_off;  // the channel's ph' and hp' pairs
+  int32_t other, self;     // channel slot of the transpose; self: it is the channel itself
   int64_t m_off;   // phhp block of the channel (V_hpph, quads of its elements)
   int64_t a_off;   // A: V_hphp of the channel (hp' x hp')
   int64_t b_src;   // V_hphp of the transpose (ph' x ph' in its order), the source of B

@@ -276,27 +276,27 @@ __global__ void gen_v_mod_kernel(const ModGen *__restrict__ mods, const int2 *__
   }
 }
 
-// The (particle a, hole i) -> modified-channel lookup that derive_tables_kernel reads, from
-// the ph' (a, i) and hp' (i, a) pair lists of the generated-V path (their ranges checked on the
-// host): slot (a - np) * np + i holds (channel, ph' index, channel, hp' index).  One CTA per
+// The (particle a, hole i) -> modified-channel lookup that derive_tables_kernel and
+// ring_image_kernel read, from the ph' (a, i) and hp' (i, a) pair lists (their ranges checked on
+// the host): slot (a - np) * np + i holds (channel, ph' index, channel, hp' index).  One CTA per
 // active modified channel; the slots start at -1 and each half is claimed once (atomicCAS), so
-// a pair named twice sets kErrBadIndex.
+// a pair named twice sets the error bit `bad`.
 __global__ void mod_lookup_kernel(const ModGen *__restrict__ mods, const int32_t *__restrict__ chan,
                                   const int2 *__restrict__ ph_pairs,
                                   const int2 *__restrict__ hp_pairs, int np, int4 *mlook,
-                                  int32_t *err) {
+                                  int32_t bad, int32_t *err) {
   const ModGen g = mods[blockIdx.x];
   const int c = chan[blockIdx.x];
   for (int k = threadIdx.x; k < g.ph; k += blockDim.x) {
     const int2 ai = ph_pairs[g.ph_off + k];
     int *m = reinterpret_cast<int *>(mlook + (int64_t)(ai.x - np) * np + ai.y);
-    if (atomicCAS(m, -1, c) != -1) atomicOr(err, kErrBadIndex);
+    if (atomicCAS(m, -1, c) != -1) atomicOr(err, bad);
     else m[1] = k;
   }
   for (int k = threadIdx.x; k < g.hp; k += blockDim.x) {
     const int2 ia = hp_pairs[g.hp_off + k];
     int *m = reinterpret_cast<int *>(mlook + (int64_t)(ia.y - np) * np + ia.x) + 2;
-    if (atomicCAS(m, -1, c) != -1) atomicOr(err, kErrBadIndex);
+    if (atomicCAS(m, -1, c) != -1) atomicOr(err, bad);
     else m[1] = k;
   }
 }
@@ -477,6 +477,45 @@ quad_rows_kernel(const ChanInfo *__restrict__ chans, const int32_t *__restrict__
     r.ea = eps[pab.x];
     r.eb = eps[pab.y];
     out[ch.pk_off + u] = r;
+  }
+}
+
+// Records of the hh reduction (one per element of X) and of T X (tx_rows(hk) rows by 16 columns), one
+// CTA per channel, from its hh_first and tx_first on.
+__global__ void __launch_bounds__(256)
+hh_records_kernel(const ChanInfo *__restrict__ chans, const QuadCol *__restrict__ qcols,
+                  HHOut *__restrict__ outs, TXTile *__restrict__ tiles) {
+  const ChanInfo ch = chans[blockIdx.x];
+  if (!ch.nmt) return;
+  auto xt_at = [&](int row, int col) {
+    return ch.nkx ? (int32_t)(ch.xt_base + (int64_t)(row >> 5) * (ch.nbt >> 3) * kTcGroup +
+                              tc_off_mn(col, row & 31))
+                  : -1;
+  };
+  for (int e = threadIdx.x; e < ch.hk * ch.hk; e += blockDim.x) {
+    const int kl = e / ch.hk, ij = e - kl * ch.hk;
+    const QuadCol c = qcols[ch.qcol_off + kl];
+    HHOut o;
+    o.part = ch.part_off + e;
+    o.nslices = ch.nhht;
+    o.stride = ch.hk * ch.hk;
+    o.x = (int32_t)(ch.x_off + kl * ch.hs + ij);
+    o.s = kl == ij ? (int32_t)(ch.qcol_off + ij) : -1;
+    o.xt[0] = xt_at(c.c_ij, ij);
+    o.xt[1] = xt_at(c.c_ji, ij);
+    outs[ch.hh_first + e] = o;
+  }
+  const int rows = tx_rows(ch.hk), nj = (ch.hk + 15) / 16, n = (ch.pk + rows - 1) / rows * nj;
+  for (int e = threadIdx.x; e < n; e += blockDim.x) {
+    const int at = e / nj * rows;
+    TXTile t;
+    t.hk = ch.hk;
+    t.hs = ch.hs;
+    t.rows = min(rows, ch.pk - at);
+    t.j0 = 16 * (e % nj);
+    t.at = ch.q_off + (int64_t)at * ch.hs;
+    t.x = ch.x_off;
+    tiles[ch.tx_first + e] = t;
   }
 }
 
@@ -687,19 +726,34 @@ __global__ void transpose_hpph_kernel(const ModInfo *__restrict__ mods,
 // Operand images and destinations of the fused path's ring (one CTA per pair), from the blocks
 // and the quads of all modified channels.  C[i][k] = V_hpph (held transposed, ph' rows; c_src >= 0:
 // the mean of it and the transpose's at the exchanged pairs),
-// A = V_hphp, B[r][r2] = V_hphp of the transpose at (perm[r2], perm[r]), zero padded, in the order
+// A = V_hphp, B[r][r2] = V_hphp of the transpose at the exchanged pairs, zero padded, in the order
 // in which an m16n8k16 warp takes them: C and B as A operands ([row tile][K step][4][lane][2]), A
 // as accumulators ([row tile][column tile][2][lane][2]), and the destinations alike ([row tile]
 // [column tile][lane][4]).  A destination is 2 * (packed position) + (0 for ab,ij / ba,ji, 1 for
 // ab,ji / ba,ij); -1 outside every quad and on the second of two elements of a quad's sum that lie
 // in one channel.  tp_src: the same position of each element of the T' image (its amplitude is
-// negated where the last bit is set), -1 outside every quad and for the padding.
+// negated where the last bit is set), -1 outside every quad and for the padding.  A pair that is
+// not in the transpose's lists sets the error bit `bad`.
 __global__ void __launch_bounds__(256)
-ring_image_kernel(const RingPair *__restrict__ pairs, const int32_t *__restrict__ perm,
+ring_image_kernel(const RingPair *__restrict__ pairs, const int2 *__restrict__ ph_pairs,
+                  const int2 *__restrict__ hp_pairs, const int4 *__restrict__ mlook, int np,
                   const double *__restrict__ v_hpph, const double *__restrict__ v_hphp,
                   const uint32_t *__restrict__ quads, double *__restrict__ img,
-                  int32_t *__restrict__ tp_src, int32_t *__restrict__ to_img) {
+                  int32_t *__restrict__ tp_src, int32_t *__restrict__ to_img, int32_t bad,
+                  int32_t *err) {
   const RingPair m = pairs[blockIdx.x];
+  __shared__ int pm[kRingMax], pm2[kRingMax];  // hp' (ph') index of each ph' (hp') pair in it
+  for (int k = threadIdx.x; k < m.ph + m.hp; k += blockDim.x) {
+    const bool row = k < m.ph;
+    const int2 q = row ? ph_pairs[m.ph_off + k] : hp_pairs[m.hp_off + k - m.ph];
+    const int a = row ? q.x : q.y, i = row ? q.y : q.x;
+    const int4 l = mlook[(int64_t)(a - np) * np + i];
+    const bool ok = (row ? l.z : l.x) == m.other;
+    if (!ok) atomicOr(err, bad);
+    if (row) pm[k] = ok ? l.w : 0;
+    else pm2[k - m.ph] = ok ? l.y : 0;
+  }
+  __syncthreads();
   const int ph = m.ph, hp = m.hp, P = pad16(ph), H = pad16(hp), n8 = (hp + 7) >> 3;
   auto quad = [&](int r, int c) {
     return r < ph && c < hp ? quads[m.m_off + (int64_t)r * hp + c] : kNoQuad;
@@ -716,14 +770,13 @@ ring_image_kernel(const RingPair *__restrict__ pairs, const int32_t *__restrict_
     row = 16 * (blk / steps) + (lane >> 2) + 8 * (i & 1);
     k = 16 * (blk % steps) + (lane & 3) + 4 * (i >> 1);
   };
-  const int32_t *pm = perm + m.perm_off;
   for (int e = threadIdx.x; e < H * P; e += blockDim.x) {
     int i, k;
     a_elem(e, P / 16, i, k);
     double v = 0.0;
     if (i < hp && k < ph) {
       v = v_hpph[m.m_off + (int64_t)k * hp + i];
-      if (m.c_src >= 0) v = 0.5 * (v + v_hpph[m.c_src + (int64_t)pm[ph + i] * ph + pm[k]]);
+      if (m.c_src >= 0) v = 0.5 * (v + v_hpph[m.c_src + (int64_t)pm2[i] * ph + pm[k]]);
     }
     img[m.c_img + e] = v;
   }

@@ -956,14 +956,17 @@ TcKernel tc_kernel_of(int nt, bool gen) {
 // on the largest bases), later creates only clear them.
 struct BuildScratch {
   std::vector<int32_t> rowmap, kcol, pp_swap, hh_swap, prow, hcol, qrow, list;
-  std::vector<int2> pp_pairs, hh_pairs, mod_ph, mod_hp, mod_dims, mod_look;
+  std::vector<int2> pp_pairs, hh_pairs, mod_ph, mod_hp, mod_dims;
+  std::vector<HHTile> hh_tiles, hh_sorted;
+  std::vector<RingPair> pairs;
+  std::vector<RingUnit> units;
+  std::vector<int32_t> mod_least, mod_owner, mod_partner;
   std::vector<int4> vrows;
   std::vector<QuadCol> quad_cols;
   std::vector<QuadItem> quad_items;
   std::vector<ElemRange> ranges;
   std::vector<int64_t> o_t, o_m, o_m_scratch, list_cnt;
-  std::vector<int4> gv_items, gvt_items, mlook;
-  std::vector<uint64_t> mod_chan;
+  std::vector<int4> gv_items, gvt_items;
   std::vector<int32_t> mod_gen_chan;
 };
 thread_local BuildScratch t_build_scratch;
@@ -1132,11 +1135,12 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   h->tc_tx = h->nt > 0;
   for (int ai = 0; ai < n_act; ai++)
     if (a_hk[ai] && a_pk[ai] > kTcBM) h->tc_tx = false;
-  std::vector<HHTile> hh_tiles;
+  std::vector<HHTile> &hh_tiles = bs.hh_tiles;
+  hh_tiles.clear();
   int64_t vhh_tot = 0, x_tot = 0, q_tot = 0, vt = 0, part_tot = 0, qcol_tot = 0;
   int64_t vraw_tot = 0;
   int64_t vtc = 0, tkttc = 0;
-  std::vector<int64_t> vraw_off, hh_part_off;
+  std::vector<int64_t> vraw_off;
   for (int ai = 0; ai < n_act; ai++) {
     const uint64_t c = act_chan[ai];
     const int64_t pp = D[c].pp, hh = D[c].hh;
@@ -1151,7 +1155,7 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     ci.vhh_off = vhh_tot; ci.x_off = x_tot; ci.q_off = q_tot; ci.vkt_base = vt;
     ci.qcol_off = qcol_tot;
     ci.vtc_base = vtc; ci.tkt_tc_base = tkttc;
-    hh_part_off.push_back(part_tot);
+    ci.part_off = part_tot;
     vhh_tot += hh * hh;
     qcol_tot += hk;
     if (pk && hk) {
@@ -1192,6 +1196,18 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   // 2 x a packed position is 31-bit, 4 x one 32-bit (the ring's tables).  Amplitudes below the limit
   // above reach this only if their padding (rows to 16, 5 hole pairs to 12) quadruples them.
   if (q_tot * 2 >= INT32_MAX) return CCDGPU_ERR_UNSUPPORTED;
+  // Records that the device fills in (hh_records_kernel).  T X: the widest channels first, the short
+  // units fill in behind them.
+  for (ChanInfo &a : chans) {
+    a.hh_first = h->n_hh_out;
+    if (a.nmt) h->n_hh_out += a.hk * a.hk;
+  }
+  for (const int rows : {16, 64, 128})
+    for (ChanInfo &a : chans)
+      if (a.nmt && tx_rows(a.hk) == rows) {
+        a.tx_first = h->n_tx;
+        h->n_tx += (int)(ceil_div(a.pk, rows) * ceil_div(a.hk, 16));
+      }
   h->n_q = q_tot;
   h->n_vhh = vhh_tot;
   h->v_generated = on_the_fly;
@@ -1221,8 +1237,8 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
       if (x.warp != y.warp) return y.warp;
       return x.cost > y.cost;
     });
-    std::vector<HHTile> sorted;
-    sorted.reserve(hh_tiles.size());
+    std::vector<HHTile> &sorted = bs.hh_sorted;
+    sorted.clear();
     for (const Run &r : runs)
       sorted.insert(sorted.end(), hh_tiles.begin() + r.first, hh_tiles.begin() + r.first + r.n);
     hh_tiles.swap(sorted);
@@ -1378,64 +1394,56 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   }
   // Fused-path ring: each channel with its transpose, the channel whose ph' pairs are this one's
   // hp' pairs exchanged (the first of the two in channel order names the pair).
-  // Tables from the host may describe blocks that do not pair up; then (and if their rows and columns
-  // turn out not to be those of the lists) the ring runs channel by channel, as on the table path.
-  std::vector<RingPair> pairs;
-  std::vector<RingUnit> units;
-  std::vector<int32_t> ring_perm;
+  // Named by the smallest pair of each list; that the lists agree in full is checked on the device
+  // (ring_image_kernel).  Tables from the host may describe blocks that do not pair up; then (and if
+  // their rows and columns turn out not to be those of the lists) the ring runs channel by channel,
+  // as on the table path.
+  std::vector<RingPair> &pairs = bs.pairs;
+  std::vector<RingUnit> &units = bs.units;
+  pairs.clear();
+  units.clear();
   int64_t img_tot = 0, tp_tot = 0, to_tot = 0;
   auto pair_up = [&]() {
-    // (hole, particle) pair -> channel, hp' index; and (V_hpph of the transpose, V from the host)
-    // -> channel, ph' index.
-    std::vector<int2> &look = bs.mod_look;
-    look.assign((size_t)np * h->npart, make_int2(-1, -1));
-    std::vector<int2> look_ph(gen_v ? 0 : look.size(), make_int2(-1, -1));
-    for (size_t g = 0; g < mod_gen.size(); g++) {
-      for (int k = 0; k < mod_gen[g].hp; k++) {
-        const int2 ia = mod_hp[mod_gen[g].hp_off + k];
-        if (ia.x < 0) return false;
-        int2 &l = look[(size_t)ia.x * h->npart + (ia.y - np)];
-        if (l.x >= 0) return false;  // in two channels
-        l = make_int2((int)g, k);
-      }
-      for (int k = 0; k < mod_gen[g].ph && !gen_v; k++) {
-        const int2 ai = mod_ph[mod_gen[g].ph_off + k];
-        if (ai.x < 0) return false;
-        look_ph[(size_t)ai.y * h->npart + (ai.x - np)] = make_int2((int)g, k);
-      }
-    }
-    for (size_t g = 0; g < mod_gen.size(); g++) {
+    const int n = (int)mod_gen.size();
+    std::vector<int32_t> &least = bs.mod_least;  // slot of each channel's smallest ph' pair ...
+    std::vector<int32_t> &owner = bs.mod_owner;  // ... and the channel that its hp' list has it in
+    std::vector<int32_t> &partner = bs.mod_partner;
+    least.resize(2 * n);
+    partner.resize(n);
+    owner.assign(np * h->npart, -1);
+#pragma omp parallel for num_threads(host_threads) schedule(static)
+    for (int g = 0; g < n; g++) {
       const ModGen &m = mod_gen[g];
-      const int perm_off = (int)ring_perm.size();
-      int other = -2;
+      int32_t p = INT32_MAX, q = INT32_MAX;  // (a - np) * np + i; -1: an entry is missing
       for (int k = 0; k < m.ph; k++) {
         const int2 ai = mod_ph[m.ph_off + k];
-        if (ai.x < 0) return false;
-        const int2 l = look[(size_t)ai.y * h->npart + (ai.x - np)];
-        if (l.x < 0 || (other >= 0 && l.x != other)) return false;
-        other = l.x;
-        ring_perm.push_back(l.y);
+        p = std::min(p, ai.x < 0 ? -1 : (ai.x - (int)np) * (int)np + ai.y);
       }
-      if (mod_gen[other].hp != m.ph || mod_gen[other].ph != m.hp) return false;
-      if (other < (int)g) {  // named by its transpose
-        ring_perm.resize(perm_off);
-        continue;
+      for (int k = 0; k < m.hp; k++) {
+        const int2 ia = mod_hp[m.hp_off + k];
+        q = std::min(q, ia.x < 0 ? -1 : (ia.y - (int)np) * (int)np + ia.x);
       }
+      least[g] = p;
+      least[n + g] = q;
+    }
+    for (int g = 0; g < n; g++)
+      if (least[n + g] >= 0) owner[least[n + g]] = g;
+    for (int g = 0; g < n; g++) {
+      partner[g] = least[g] >= 0 ? owner[least[g]] : -1;
+      if (partner[g] < 0) return false;
+    }
+    for (int g = 0; g < n; g++) {
+      const int other = partner[g];
+      const ModGen &m = mod_gen[g], &o = mod_gen[other];
+      if (partner[other] != g || o.hp != m.ph || o.ph != m.hp) return false;
+      if (other < g) continue;  // named by its transpose
       RingPair r{};
       r.ph = m.ph; r.hp = m.hp;
-      r.perm_off = perm_off;
-      r.self = other == (int)g;
-      r.m_off = m.m_off; r.a_off = m.y_off; r.b_src = mod_gen[other].y_off;
-      r.c_src = -1;
-      if (!gen_v) {
-        r.c_src = mod_gen[other].m_off;
-        for (int k = 0; k < m.hp; k++) {
-          const int2 ia = mod_hp[m.hp_off + k];
-          const int2 l = look_ph[(size_t)ia.x * h->npart + (ia.y - np)];
-          if (l.x != other) return false;
-          ring_perm.push_back(l.y);
-        }
-      }
+      r.ph_off = (int)m.ph_off; r.hp_off = (int)m.hp_off;
+      r.other = mod_gen_chan[other];
+      r.self = other == g;
+      r.m_off = m.m_off; r.a_off = m.y_off; r.b_src = o.y_off;
+      r.c_src = gen_v ? -1 : o.m_off;
       pairs.push_back(r);
     }
     return true;
@@ -1443,7 +1451,6 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   h->ring_paired = fused && pair_up();
   if (!h->ring_paired) {
     pairs.clear();
-    ring_perm.clear();
     if (fused && derive_tables) return CCDGPU_ERR_BAD_TABLE;  // no tables could fit such lists
   } else {
     // The largest first, so that the short ones fill in behind them.
@@ -1545,8 +1552,6 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   quad_items.clear();
   // Rows: the packed rows with a < b (pk of them per channel), filled in parallel below;
   // columns (i < j) and work items here.
-  std::vector<HHOut> hh_out;
-  std::vector<TXTile> tx_tiles;
   for (int ai = 0; ai < h->n_act; ai++) {
     const ChanInfo &a = chans[ai];
     for (int j = 0; j < a.hh; j++) {
@@ -1562,29 +1567,7 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     for (int64_t q = 0; q < nq; q += kQuadPerItem)
       quad_items.push_back({ai, (int32_t)q, (int32_t)std::min<int64_t>(nq, q + kQuadPerItem),
                             a.hk, a.hs, a.rt_off, a.q_off, a.x_off, a.pk_off, a.qcol_off});
-    const QuadCol *qc = quad_cols.data() + a.qcol_off;
-    auto xt_at = [&](int row, int col) {
-      return a.nkx ? (int32_t)(a.xt_base + (int64_t)(row >> 5) * (a.nbt >> 3) * kTcGroup +
-                               tc_off_mn(col, row & 31))
-                   : -1;
-    };
-    for (int kl = 0; nq && kl < a.hk; kl++)
-      for (int ij = 0; ij < a.hk; ij++)
-        hh_out.push_back({hh_part_off[ai] + kl * a.hk + ij, a.nhht, a.hk * a.hk,
-                          (int32_t)(a.x_off + kl * a.hs + ij),
-                          kl == ij ? (int32_t)(a.qcol_off + ij) : -1,
-                          {xt_at(qc[kl].c_ij, ij), xt_at(qc[kl].c_ji, ij)}});
   }
-  // T X: the widest channels first, the short units fill in behind them.
-  for (const int rows : {16, 64, 128})
-    for (const ChanInfo &a : chans)
-      if (a.nmt && tx_rows(a.hk) == rows)
-        for (int u = 0; u < a.pk; u += rows)
-          for (int j0 = 0; j0 < a.hk; j0 += 16)
-            tx_tiles.push_back({a.hk, a.hs, std::min(rows, a.pk - u), j0,
-                                a.q_off + (int64_t)u * a.hs, a.x_off});
-  h->n_tx = (int)tx_tiles.size();
-  h->n_hh_out = (int)hh_out.size();
   h->n_quad_rows = a_pk_off[n_act];  // built on the device (quad_rows_kernel)
 
   h->host_chans = chans;
@@ -1661,8 +1644,8 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   h->create_ms[0] = ms_since(t_build);
   Arena ar;
   ar.add(&h->chans, chans.size()); ar.add(&h->mods, mods.size());
-  ar.add(&h->hh_tiles, hh_tiles.size()); ar.add(&h->hh_out, hh_out.size());
-  ar.add(&h->tx_tiles, tx_tiles.size());
+  ar.add(&h->hh_tiles, hh_tiles.size()); ar.add(&h->hh_out, h->n_hh_out);
+  ar.add(&h->tx_tiles, h->n_tx);
   ar.add(&h->ranges, ranges.size());
   ar.add(&h->pp_pairs, pp_pairs.size()); ar.add(&h->hh_pairs, hh_pairs.size());
   ar.add(&h->pp_swap, pp_swap.size()); ar.add(&h->hh_swap, hh_swap.size());
@@ -1755,82 +1738,25 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     }
   }
   int64_t *d_vraw_off = nullptr, *d_o_m = nullptr;
-  // Derived tables: per-pair block offsets and the modified-channel lookup of (particle, hole)
-  // pairs, built here from the ph' / hp' maps (O(npart * np)).
+  // Derived tables: per-pair block offsets; and (fused path: for the ring's pairs too) the
+  // modified-channel lookup of (particle, hole) pairs, built on the device from the pair lists.
   int32_t *d_hblk = nullptr, *d_pblk = nullptr;
   int4 *d_mlook = nullptr;
-  std::vector<int4> &mlook = bs.mlook;
-  mlook.clear();
-  // With generated V the ph' / hp' pairs go to the device anyway: the lookup is built there
-  // (mod_lookup_kernel); otherwise here.
-  const bool mlook_dev = derive_tables && gen_v;
-  const uint64_t n_mlook = (nsp - np) * np;
-  if (mlook_dev) {
-    sc.add(&d_mlook, n_mlook);
-  } else if (derive_tables) {
-    const uint64_t npart = nsp - np;
-    mlook.assign(npart * np, make_int4(-1, -1, -1, -1));
-    std::vector<uint64_t> &mc = bs.mod_chan;
-    mc.clear();
-    for (uint64_t c = 0; c < nch; c++) {
-      if (!MD[c].ph || !MD[c].hp) continue;
-      if (!P->chan_mod_maps[c].ph || !P->chan_mod_maps[c].hp) return CCDGPU_ERR_INVALID_ARGUMENT;
-      mc.push_back(c);
-    }
-    // In a valid problem every (particle, hole) slot is named by exactly one ph' entry and one
-    // hp' entry, so the channels fill their slots in parallel (relaxed atomic stores, so that
-    // an invalid problem's duplicates race harmlessly); a second pass checks that each entry's
-    // slot holds that entry, which fails for every duplicate but one.
-    std::atomic<int> bad_m{0};
-    int32_t *ml = reinterpret_cast<int32_t *>(mlook.data());
-    auto each_entry = [&](int64_t g, auto &&f) {
-      const uint64_t c = mc[g];
-      const ccdgpu_pair *phm = P->chan_mod_maps[c].ph, *hpm = P->chan_mod_maps[c].hp;
-      for (uint64_t k = 0; k < MD[c].ph; k++) {
-        const uint64_t a = phm[k].p, i = phm[k].q;
-        if (a < np || a >= nsp || i >= np) bad_m = 1;
-        else f(ml + 4 * ((a - np) * np + i), (int)c, (int)k);
-      }
-      for (uint64_t k = 0; k < MD[c].hp; k++) {
-        const uint64_t i = hpm[k].p, a = hpm[k].q;
-        if (i >= np || a < np || a >= nsp) bad_m = 1;
-        else f(ml + 4 * ((a - np) * np + i) + 2, (int)c, (int)k);
-      }
-    };
-#pragma omp parallel num_threads(host_threads)
-    {
-#pragma omp for schedule(dynamic, 16)
-      for (int64_t g = 0; g < (int64_t)mc.size(); g++)
-        each_entry(g, [](int32_t *m, int c, int k) {
-          __atomic_store_n(m, c, __ATOMIC_RELAXED);
-          __atomic_store_n(m + 1, k, __ATOMIC_RELAXED);
-        });
-#pragma omp for schedule(dynamic, 16)
-      for (int64_t g = 0; g < (int64_t)mc.size(); g++)
-        each_entry(g, [&](int32_t *m, int c, int k) {
-          if (__atomic_load_n(m, __ATOMIC_RELAXED) != c ||
-              __atomic_load_n(m + 1, __ATOMIC_RELAXED) != k)
-            bad_m = 1;
-        });
-    }
-    if (bad_m) return CCDGPU_ERR_BAD_TABLE;
-    sc.add(&d_mlook, mlook.size());
-  } else {
-    sc.add(&raw_idx, (size_t)8 * n_t);
-  }
+  const uint64_t n_mlook = derive_tables || h->ring_paired ? (nsp - np) * np : 0;
+  sc.add(&d_mlook, n_mlook);
+  if (!derive_tables) sc.add(&raw_idx, (size_t)8 * n_t);
   if (derive_tables || gen_v3) {  // block offsets inside hpp(k) and phh(a)
     sc.add(&d_hblk, np * np);
     sc.add(&d_pblk, (nsp - np) * (nsp - np));
   }
-  int32_t *d_ring_perm = nullptr;
   RingPair *d_pairs = nullptr;
-  sc.add(&d_ring_perm, ring_perm.size()); sc.add(&d_pairs, pairs.size());
+  sc.add(&d_pairs, pairs.size());
   ModGen *d_mod_gen = nullptr;
   int2 *d_mod_ph = nullptr, *d_mod_hp = nullptr;
   int32_t *d_mod_chan = nullptr;
   // With tables from the host, the lists that the ring's pairs rest on are checked against them.
   const bool check_lists = h->ring_paired && !derive_tables;
-  const bool lists_on_device = gen_v || check_lists;
+  const bool lists_on_device = gen_v || n_mlook;
   std::vector<int2> mod_at(check_lists ? nch : 0, make_int2(0, 0));
   for (size_t g = 0; g < mod_gen.size() && check_lists; g++)
     mod_at[mod_gen_chan[g]] = make_int2((int)mod_gen[g].ph_off, (int)mod_gen[g].hp_off);
@@ -1838,8 +1764,6 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   sc.add(&d_mod_at, mod_at.size());
   if (lists_on_device) {
     sc.add(&d_mod_ph, mod_ph.size()); sc.add(&d_mod_hp, mod_hp.size());
-  }
-  if (gen_v) {
     sc.add(&d_mod_gen, mod_gen.size()); sc.add(&d_mod_chan, mod_gen_chan.size());
   }
   sc.add(&vraw, vraw_tot); sc.add(&hhpp_raw, gen_v ? 0 : n_t);
@@ -1930,8 +1854,7 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   };
   TRY(put(h->chans, chans)); TRY(put(h->mods, mods));
   TRY(put(d_pairs, pairs)); TRY(put(h->ring_units, units));
-  TRY(put(d_ring_perm, ring_perm));
-  TRY(put(h->hh_tiles, hh_tiles)); TRY(put(h->hh_out, hh_out)); TRY(put(h->tx_tiles, tx_tiles));
+  TRY(put(h->hh_tiles, hh_tiles));
   TRY(put(h->ranges, ranges)); TRY(put(h->quad_items, quad_items));
   TRY(put(h->quad_cols, quad_cols));
 
@@ -1982,13 +1905,10 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     static_assert(sizeof(RawIndex) == sizeof(ccdgpu_chain_index), "ChainIndex layout");
     for (int k = 0; k < 8 && !derive_tables; k++)
       TRY(upload_runs(h, reinterpret_cast<ccdgpu_chain_index *>(raw_idx) + (size_t)k * n_t, sm[k], nm));
-    if (derive_tables && !mlook_dev) TRY(put(d_mlook, mlook));
     TRY(put(d_mod_at, mod_at));
     if (lists_on_device) {
       TRY(put(d_mod_ph, mod_ph));
       TRY(put(d_mod_hp, mod_hp));
-    }
-    if (gen_v) {
       TRY(put(d_mod_gen, mod_gen));
       TRY(put(d_mod_chan, mod_gen_chan));
     }
@@ -2019,6 +1939,9 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   if (h->n_quad_rows) {
     quad_rows_kernel<<<(unsigned)h->n_act, 256, 0, h->s0>>>(
         h->chans, h->kcol, h->pp_swap, h->pp_pairs, h->eps, (int)np, h->quad_rows);
+    CK(cudaGetLastError());
+    hh_records_kernel<<<(unsigned)h->n_act, 256, 0, h->s0>>>(h->chans, h->quad_cols, h->hh_out,
+                                                             h->tx_tiles);
     CK(cudaGetLastError());
   }
   if (gen_v && !mod_gen.empty()) {
@@ -2064,11 +1987,13 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
           (int)h->npart, h->v_h_hpp, h->v_phh_p, h->err);
       CK(cudaGetLastError());
     }
-    if (mlook_dev) {
+    // Lists that contradict each other: bad where the tables come from them, else not to be paired.
+    const int32_t list_err = derive_tables ? kErrBadIndex : kErrRingLists;
+    if (n_mlook) {
       CK(cudaMemsetAsync(d_mlook, 0xff, n_mlook * sizeof(int4), h->s0));  // every field -1
       if (!mod_gen.empty()) {
         mod_lookup_kernel<<<(unsigned)mod_gen.size(), 128, 0, h->s0>>>(
-            d_mod_gen, d_mod_chan, d_mod_ph, d_mod_hp, (int)np, d_mlook, h->err);
+            d_mod_gen, d_mod_chan, d_mod_ph, d_mod_hp, (int)np, d_mlook, list_err, h->err);
         CK(cudaGetLastError());
       }
     }
@@ -2105,8 +2030,8 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     }
     if (!pairs.empty()) {
       ring_image_kernel<<<(unsigned)pairs.size(), 256, 0, h->s0>>>(
-          d_pairs, d_ring_perm, h->v_hpph, h->v_hphp, h->ring_quads, h->ring_img, h->ring_src,
-          h->ring_to);
+          d_pairs, d_mod_ph, d_mod_hp, d_mlook, (int)np, h->v_hpph, h->v_hphp, h->ring_quads,
+          h->ring_img, h->ring_src, h->ring_to, list_err, h->err);
       CK(cudaGetLastError());
     }
   }
