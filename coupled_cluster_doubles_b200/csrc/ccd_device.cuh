@@ -185,6 +185,7 @@ struct ChanInfo {
   int64_t x_off;     // X: hk x hs
   int64_t part_off;  // partials of the hh ladder
   int32_t hh_first, tx_first;  // first of the channel's HHOut and TXTile records
+  int32_t hht_first, hht_last;  // first of its full HHTile slices; the shorter one after them
   int64_t vkt_base;  // A tiles of V
   int64_t pk_off;    // strict particle pairs: offset into kcol / quad rows / r (pk entries)
   int64_t qcol_off;  // strict hole pairs: offset into quad columns / s (hk entries)
@@ -194,12 +195,11 @@ struct ChanInfo {
   int64_t vtc_base, tkt_tc_base;
 };
 
-// hh-ladder unit: `rows` packed rows of channel ch from row r0 of all channels', V and T at `base`,
+// hh-ladder unit: `rows` packed rows of a channel from row r0 of all channels', V and T at `base`,
 // the partial of P at `part`.
 struct __align__(16) HHTile {
-  int32_t hk, hs, rows, ch;
+  int32_t hk, hs, rows, r0;
   int64_t base, part;
-  int32_t r0, pad[3];
 };
 // One element of X = V_hhhh + P: P's partials part[k * stride], k < nslices, where X goes (and the
 // packed V_hhhh comes from) and, on the diagonal, s (s < 0: off the diagonal).
@@ -234,7 +234,7 @@ struct QuadCol {
 struct QuadItem {
   int32_t ch, q0, q1, hk;
   int32_t hs, rt_off;
-  int64_t q_off, x_off, pk_off, qcol_off;
+  int64_t q_off, pk_off, qcol_off;
 };
 
 // Per active modified channel (table path).

@@ -480,13 +480,25 @@ quad_rows_kernel(const ChanInfo *__restrict__ chans, const int32_t *__restrict__
   }
 }
 
-// Records of the hh reduction (one per element of X) and of T X (tx_rows(hk) rows by 16 columns), one
-// CTA per channel, from its hh_first and tx_first on.
+// Records of the hh ladder (a slice of kHHRows rows each), its reduction (one per element of X) and T X
+// (tx_rows(hk) rows by 16 columns), one CTA per channel, from its first of each on.
 __global__ void __launch_bounds__(256)
 hh_records_kernel(const ChanInfo *__restrict__ chans, const QuadCol *__restrict__ qcols,
-                  HHOut *__restrict__ outs, TXTile *__restrict__ tiles) {
+                  HHTile *__restrict__ slices, HHOut *__restrict__ outs,
+                  TXTile *__restrict__ tiles) {
   const ChanInfo ch = chans[blockIdx.x];
   if (!ch.nmt) return;
+  for (int e = threadIdx.x; e < ch.nhht; e += blockDim.x) {
+    const int at = e * kHHRows;
+    HHTile t;
+    t.hk = ch.hk;
+    t.hs = ch.hs;
+    t.rows = min(kHHRows, ch.pk - at);
+    t.r0 = (int32_t)ch.pk_off + at;
+    t.base = ch.q_off + (int64_t)at * ch.hs;
+    t.part = ch.part_off + (int64_t)e * ch.hk * ch.hk;
+    slices[t.rows == kHHRows ? ch.hht_first + e : ch.hht_last] = t;
+  }
   auto xt_at = [&](int row, int col) {
     return ch.nkx ? (int32_t)(ch.xt_base + (int64_t)(row >> 5) * (ch.nbt >> 3) * kTcGroup +
                               tc_off_mn(col, row & 31))

@@ -119,7 +119,7 @@ struct ccdgpu_handle {
   int64_t n_tp = 0;
   bool ring_cols = false;               // the four-warp units hold only their columns of T'
   size_t ring_smem[3] = {0, 0, 0};  // dynamic shared memory of the groups' kernels
-  std::vector<RingPair> host_pairs;
+  double ring_flops[3] = {}, ring_bytes[3] = {};  // of the small, mid and large groups
   bool ring_paired = false;  // else the fused ring runs channel by channel
   double create_ms[5] = {};   // ccdgpu_profile::ms_create
   double loop_graph_ms = 0;   // ccdgpu_profile::ms_loop_graph
@@ -957,10 +957,10 @@ TcKernel tc_kernel_of(int nt, bool gen) {
 struct BuildScratch {
   std::vector<int32_t> rowmap, kcol, pp_swap, hh_swap, prow, hcol, qrow, list;
   std::vector<int2> pp_pairs, hh_pairs, mod_ph, mod_hp, mod_dims;
-  std::vector<HHTile> hh_tiles, hh_sorted;
   std::vector<RingPair> pairs;
   std::vector<RingUnit> units;
-  std::vector<int32_t> mod_least, mod_owner, mod_partner;
+  std::vector<int32_t> mod_owner;
+  std::vector<int2> mod_least, mod_named;
   std::vector<int4> vrows;
   std::vector<QuadCol> quad_cols;
   std::vector<QuadItem> quad_items;
@@ -1135,8 +1135,6 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   h->tc_tx = h->nt > 0;
   for (int ai = 0; ai < n_act; ai++)
     if (a_hk[ai] && a_pk[ai] > kTcBM) h->tc_tx = false;
-  std::vector<HHTile> &hh_tiles = bs.hh_tiles;
-  hh_tiles.clear();
   int64_t vhh_tot = 0, x_tot = 0, q_tot = 0, vt = 0, part_tot = 0, qcol_tot = 0;
   int64_t vraw_tot = 0;
   int64_t vtc = 0, tkttc = 0;
@@ -1164,8 +1162,7 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
       ci.sym = hk <= kSymHK;  // stored V: unless it turns out not to be symmetric
       ci.rt_off = h->n_row_tiles;
       h->n_row_tiles += ci.nmt;
-      const int rows = kHHRows;  // K slice of the hh ladder
-      ci.nhht = (int)ceil_div(pk, rows);
+      ci.nhht = (int)ceil_div(pk, kHHRows);
       ci.nbt = tc_nb(hk);
       ci.nkct = (int)ceil_div(pk, kTcKC);
       vtc += (int64_t)ci.nkct * kTcGroup * ceil_div(pk, 8);
@@ -1181,10 +1178,6 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
       q_tot += (int64_t)ci.nkc * kBK * ci.hs;
       // Stored V: room for the whole of it, should it not be symmetric.
       vt += ladder_chunk(on_the_fly && ci.sym, ci.nkc, ci.nmt - 1, ci.nkc, pk - (ci.nmt - 1) * kMaxBM);
-      for (int t = 0; t < ci.nhht; t++)
-        hh_tiles.push_back({hk, ci.hs, std::min(rows, pk - t * rows), ai,
-                            ci.q_off + (int64_t)t * rows * ci.hs,
-                            part_tot + (int64_t)t * hk * hk, (int32_t)(ci.pk_off + t * rows), {}});
       part_tot += (int64_t)ci.nhht * hk * hk;
     } else if (!on_the_fly) {
       vt += (int64_t)pk * pk;  // row-major, for ccd_general.cuh alone
@@ -1196,8 +1189,37 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   // 2 x a packed position is 31-bit, 4 x one 32-bit (the ring's tables).  Amplitudes below the limit
   // above reach this only if their padding (rows to 16, 5 hole pairs to 12) quadruples them.
   if (q_tot * 2 >= INT32_MAX) return CCDGPU_ERR_UNSUPPORTED;
-  // Records that the device fills in (hh_records_kernel).  T X: the widest channels first, the short
-  // units fill in behind them.
+  // Records that the device fills in (hh_records_kernel): where each channel's start.
+  // hh-ladder units: one per CTA (hk > 8) first, then one per warp; within each the largest
+  // (rows x hk^2) first, so that the short ones fill in behind them: a channel's full slices and
+  // its last, shorter one are sorted as runs, by class and cost.
+  {
+    struct Run {
+      int32_t ai, n;
+      bool warp, full;
+      int64_t cost;
+    };
+    std::vector<Run> runs;
+    runs.reserve(2 * n_act);
+    for (int ai = 0; ai < n_act; ai++) {
+      const ChanInfo &a = chans[ai];
+      const int full = a.nmt ? a.pk / kHHRows : 0, rest = a.nmt ? a.pk % kHHRows : 0;
+      const int64_t hk2 = (int64_t)a.hk * a.hk;
+      if (full) runs.push_back(Run{ai, full, a.hk <= 8, true, kHHRows * hk2});
+      if (rest) runs.push_back(Run{ai, 1, a.hk <= 8, false, rest * hk2});
+      (a.hk > 8 ? h->n_hh_cta : h->n_hh_warp) += full + (rest ? 1 : 0);
+    }
+    std::stable_sort(runs.begin(), runs.end(), [](const Run &x, const Run &y) {
+      if (x.warp != y.warp) return y.warp;
+      return x.cost > y.cost;
+    });
+    int32_t at = 0;
+    for (const Run &r : runs) {
+      (r.full ? chans[r.ai].hht_first : chans[r.ai].hht_last) = at;
+      at += r.n;
+    }
+  }
+  // T X: the widest channels first, the short units fill in behind them.
   for (ChanInfo &a : chans) {
     a.hh_first = h->n_hh_out;
     if (a.nmt) h->n_hh_out += a.hk * a.hk;
@@ -1209,41 +1231,10 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
         h->n_tx += (int)(ceil_div(a.pk, rows) * ceil_div(a.hk, 16));
       }
   h->n_q = q_tot;
+  h->n_act = n_act;
   h->n_vhh = vhh_tot;
   h->v_generated = on_the_fly;
   const int64_t pp_tot = a_pp_off[n_act], hh_tot = a_hh_off[n_act];
-  h->n_act = n_act;
-  // hh-ladder units: one per CTA (hk > 8) first, then one per warp; within each the largest
-  // (rows x hk^2) first, so that the short ones fill in behind them.  A stable sort by (class,
-  // -cost): the units come channel by channel as runs of equal cost (the full slices, then a
-  // shorter last one), so the runs are stably sorted and expanded, which gives the same order as
-  // sorting the units themselves.
-  {
-    struct Run {
-      int32_t first, n;
-      bool warp;
-      int64_t cost;
-    };
-    std::vector<Run> runs;
-    for (int32_t i = 0; i < (int32_t)hh_tiles.size(); i++) {
-      const HHTile &t = hh_tiles[i];
-      const int64_t hk = chans[t.ch].hk, cost = (int64_t)t.rows * hk * hk;
-      if (!runs.empty() && hh_tiles[runs.back().first].ch == t.ch && runs.back().cost == cost)
-        runs.back().n++;
-      else
-        runs.push_back(Run{i, 1, hk <= 8, cost});
-    }
-    std::stable_sort(runs.begin(), runs.end(), [](const Run &x, const Run &y) {
-      if (x.warp != y.warp) return y.warp;
-      return x.cost > y.cost;
-    });
-    std::vector<HHTile> &sorted = bs.hh_sorted;
-    sorted.clear();
-    for (const Run &r : runs)
-      sorted.insert(sorted.end(), hh_tiles.begin() + r.first, hh_tiles.begin() + r.first + r.n);
-    hh_tiles.swap(sorted);
-  }
-  for (const HHTile &t : hh_tiles) (chans[t.ch].hk > 8 ? h->n_hh_cta : h->n_hh_warp)++;
   // Per orbital w, the strict pairs that hold w, in the order of the ordered pairs whose first
   // index is w (particles: rows of r, holes: entries of s): a counting sort.  The pp elements (first index a particle)
   // are split into one contiguous range per host thread: per-thread bucket counts, then each
@@ -1306,8 +1297,7 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   std::vector<int32_t> &mod_gen_chan = bs.mod_gen_chan;  // ... and their channel slots
   mod_gen_chan.clear();
   std::vector<int2> &mod_ph = bs.mod_ph, &mod_hp = bs.mod_hp;  // ... their ph' (b, j), hp' (i, a) pairs
-  mod_ph.clear();
-  mod_hp.clear();
+  std::vector<int2> &mod_least = bs.mod_least;
   const bool fused = h->opt.path == CCDGPU_PATH_FUSED;
   bool mod_maps = true;  // the problem carries the ph' and hp' pair lists
   const bool lists_needed = derive_tables || gen_v;
@@ -1337,11 +1327,27 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     if (w <= kRingSmall) mods.push_back(m);
     else mods_pad[w <= 32 ? 0 : w <= 48 ? 1 : w <= 64 ? 2 : 3].push_back(m);
   }
-  if (!mod_gen.empty()) {
-    mod_ph.resize(mod_gen.back().ph_off + mod_gen.back().ph);
-    mod_hp.resize(mod_gen.back().hp_off + mod_gen.back().hp);
+  const bool lists_used = !mod_gen.empty() && (fused || lists_needed);
+  mod_ph.resize(lists_used ? mod_gen.back().ph_off + mod_gen.back().ph : 0);
+  mod_hp.resize(lists_used ? mod_gen.back().hp_off + mod_gen.back().hp : 0);
+  if (lists_used) {
     const std::vector<int32_t> &mod_chan = mod_gen_chan;
     std::atomic<int> bad_mod{0};
+    // Slots (a - np) * np + i of the smallest ph' and hp' pair; -1: an entry is missing.
+    auto find_least = [&](int64_t g) {
+      const ModGen &m = mod_gen[g];
+      int32_t p = INT32_MAX, q = INT32_MAX;
+      for (int k = 0; k < m.ph; k++) {
+        const int2 ai = mod_ph[m.ph_off + k];
+        p = std::min(p, ai.x < 0 ? -1 : (ai.x - (int)np) * (int)np + ai.y);
+      }
+      for (int k = 0; k < m.hp; k++) {
+        const int2 ia = mod_hp[m.hp_off + k];
+        q = std::min(q, ia.x < 0 ? -1 : (ia.y - (int)np) * (int)np + ia.x);
+      }
+      mod_least[g] = make_int2(p, q);
+    };
+    mod_least.resize(mod_gen.size());
     if (mod_maps) {
 #pragma omp parallel for num_threads(host_threads) schedule(dynamic, 16)
       for (int64_t g = 0; g < (int64_t)mod_gen.size(); g++) {
@@ -1355,6 +1361,7 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
           if (hpm[k].p >= np || hpm[k].q < np || hpm[k].q >= nsp) bad_mod = 1;
           mod_hp[mg.hp_off + k] = make_int2((int)hpm[k].p, (int)hpm[k].q);
         }
+        find_least(g);
       }
       if (bad_mod && lists_needed) return CCDGPU_ERR_BAD_TABLE;
     }
@@ -1390,6 +1397,7 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
         }
       }
       if (rc_maps) return rc_maps;
+      for (size_t g = 0; g < mod_gen.size(); g++) find_least(g);
     }
   }
   // Fused-path ring: each channel with its transpose, the channel whose ph' pairs are this one's
@@ -1405,46 +1413,48 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   int64_t img_tot = 0, tp_tot = 0, to_tot = 0;
   auto pair_up = [&]() {
     const int n = (int)mod_gen.size();
-    std::vector<int32_t> &least = bs.mod_least;  // slot of each channel's smallest ph' pair ...
-    std::vector<int32_t> &owner = bs.mod_owner;  // ... and the channel that its hp' list has it in
-    std::vector<int32_t> &partner = bs.mod_partner;
-    least.resize(2 * n);
-    partner.resize(n);
-    owner.assign(np * h->npart, -1);
-#pragma omp parallel for num_threads(host_threads) schedule(static)
-    for (int g = 0; g < n; g++) {
-      const ModGen &m = mod_gen[g];
-      int32_t p = INT32_MAX, q = INT32_MAX;  // (a - np) * np + i; -1: an entry is missing
-      for (int k = 0; k < m.ph; k++) {
-        const int2 ai = mod_ph[m.ph_off + k];
-        p = std::min(p, ai.x < 0 ? -1 : (ai.x - (int)np) * (int)np + ai.y);
-      }
-      for (int k = 0; k < m.hp; k++) {
-        const int2 ia = mod_hp[m.hp_off + k];
-        q = std::min(q, ia.x < 0 ? -1 : (ia.y - (int)np) * (int)np + ia.x);
-      }
-      least[g] = p;
-      least[n + g] = q;
-    }
+    // The channel whose hp' list has a slot as its smallest; entries of earlier creates are told by
+    // their channel's list.
+    std::vector<int32_t> &owner = bs.mod_owner;
+    std::vector<int2> &named = bs.mod_named;  // channels that name their pair, their transposes
+    owner.resize(np * h->npart);
+    named.clear();
     for (int g = 0; g < n; g++)
-      if (least[n + g] >= 0) owner[least[n + g]] = g;
+      if (mod_least[g].y >= 0) owner[mod_least[g].y] = g;
+    auto partner = [&](int g) {
+      const int slot = mod_least[g].x, o = slot >= 0 ? owner[slot] : -1;
+      return o >= 0 && o < n && mod_least[o].y == slot ? o : -1;
+    };
+    // The largest first, so that the short ones fill in behind them: counted by tiles of 16 x 16.
+    constexpr int kMaxTiles = (kRingMax / 16) * (kRingMax / 16);
+    auto tiles_of = [](const ModGen &m) { return pad16(m.ph) / 16 * (pad16(m.hp) / 16); };
+    int at[kMaxTiles + 1] = {};
     for (int g = 0; g < n; g++) {
-      partner[g] = least[g] >= 0 ? owner[least[g]] : -1;
-      if (partner[g] < 0) return false;
-    }
-    for (int g = 0; g < n; g++) {
-      const int other = partner[g];
+      const int other = partner(g);
+      if (other < 0 || partner(other) != g) return false;
       const ModGen &m = mod_gen[g], &o = mod_gen[other];
-      if (partner[other] != g || o.hp != m.ph || o.ph != m.hp) return false;
+      if (o.hp != m.ph || o.ph != m.hp) return false;
       if (other < g) continue;  // named by its transpose
-      RingPair r{};
+      named.push_back(make_int2(g, other));
+      at[tiles_of(m)]++;
+    }
+    for (int t = kMaxTiles, sum = 0; t >= 0; t--) {
+      const int c = at[t];
+      at[t] = sum;
+      sum += c;
+    }
+    pairs.resize(named.size());
+    for (const int2 &go : named) {
+      const ModGen &m = mod_gen[go.x], &o = mod_gen[go.y];
+      RingPair &r = pairs[at[tiles_of(m)]++];
+      r = RingPair{};
       r.ph = m.ph; r.hp = m.hp;
       r.ph_off = (int)m.ph_off; r.hp_off = (int)m.hp_off;
-      r.other = mod_gen_chan[other];
-      r.self = other == g;
+      r.other = mod_gen_chan[go.y];
+      r.self = go.x == go.y;
       r.m_off = m.m_off; r.a_off = m.y_off; r.b_src = o.y_off;
       r.c_src = gen_v ? -1 : o.m_off;
-      pairs.push_back(r);
+      r.g = ring_group(r.ph, r.hp);
     }
     return true;
   };
@@ -1453,18 +1463,11 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     pairs.clear();
     if (fused && derive_tables) return CCDGPU_ERR_BAD_TABLE;  // no tables could fit such lists
   } else {
-    // The largest first, so that the short ones fill in behind them.
-    std::stable_sort(pairs.begin(), pairs.end(), [](const RingPair &x, const RingPair &y) {
-      return (int64_t)pad16(x.ph) * pad16(x.hp) > (int64_t)pad16(y.ph) * pad16(y.hp);
-    });
     // Warps of a pair's units by its width; a group that does not fill the SMs joins the next wider
     // one: a launch and a graph branch less (pairing: 0.1 ms less in create, mixed 0.2 ms).
     auto units_of = [](const RingPair &r) { return ceil_div((r.hp + 7) / 8, kPairNC); };
     int64_t group_units[5] = {};
-    for (RingPair &r : pairs) {
-      r.g = ring_group(r.ph, r.hp);
-      group_units[r.g] += units_of(r);
-    }
+    for (const RingPair &r : pairs) group_units[r.g] += units_of(r);
     for (int g : {1, 2}) {
       const int to = group_units[2 * g] ? 2 * g : 4;
       if (group_units[g] >= 148 || !group_units[to]) continue;
@@ -1503,10 +1506,13 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
       smem = std::max(smem, (r.g == 1 ? 4 : 1) * sizeof(double) *
                                 ring_unit_smem(r.g, r.g == 4 && h->ring_cols, pad16(r.ph),
                                                pad16(r.hp), nt));
+      const int k = r.g == 1 ? 0 : r.g == 2 ? 1 : 2;
+      const double e = (double)r.ph * r.hp;
+      h->ring_flops[k] += 2.0 * e * (2.0 * r.hp + r.ph);
+      h->ring_bytes[k] += 28.0 * e + 8.0 * ((double)r.hp * r.hp + (double)r.ph * r.ph);
     }
   }
   h->n_tp = tp_tot;
-  h->host_pairs = pairs;
   // Largest channels first within a group, so that the short ones fill in behind them.
   auto by_work = [](const ModInfo &x, const ModInfo &y) {
     return (int64_t)x.ph * x.hp * x.hp > (int64_t)y.ph * y.hp * y.hp;
@@ -1566,7 +1572,7 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     if (nq >= ((int64_t)1 << 31) / 2) return CCDGPU_ERR_UNSUPPORTED;
     for (int64_t q = 0; q < nq; q += kQuadPerItem)
       quad_items.push_back({ai, (int32_t)q, (int32_t)std::min<int64_t>(nq, q + kQuadPerItem),
-                            a.hk, a.hs, a.rt_off, a.q_off, a.x_off, a.pk_off, a.qcol_off});
+                            a.hk, a.hs, a.rt_off, a.q_off, a.pk_off, a.qcol_off});
   }
   h->n_quad_rows = a_pk_off[n_act];  // built on the device (quad_rows_kernel)
 
@@ -1644,7 +1650,7 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   h->create_ms[0] = ms_since(t_build);
   Arena ar;
   ar.add(&h->chans, chans.size()); ar.add(&h->mods, mods.size());
-  ar.add(&h->hh_tiles, hh_tiles.size()); ar.add(&h->hh_out, h->n_hh_out);
+  ar.add(&h->hh_tiles, h->n_hh_cta + h->n_hh_warp); ar.add(&h->hh_out, h->n_hh_out);
   ar.add(&h->tx_tiles, h->n_tx);
   ar.add(&h->ranges, ranges.size());
   ar.add(&h->pp_pairs, pp_pairs.size()); ar.add(&h->hh_pairs, hh_pairs.size());
@@ -1854,7 +1860,6 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   };
   TRY(put(h->chans, chans)); TRY(put(h->mods, mods));
   TRY(put(d_pairs, pairs)); TRY(put(h->ring_units, units));
-  TRY(put(h->hh_tiles, hh_tiles));
   TRY(put(h->ranges, ranges)); TRY(put(h->quad_items, quad_items));
   TRY(put(h->quad_cols, quad_cols));
 
@@ -1940,8 +1945,8 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     quad_rows_kernel<<<(unsigned)h->n_act, 256, 0, h->s0>>>(
         h->chans, h->kcol, h->pp_swap, h->pp_pairs, h->eps, (int)np, h->quad_rows);
     CK(cudaGetLastError());
-    hh_records_kernel<<<(unsigned)h->n_act, 256, 0, h->s0>>>(h->chans, h->quad_cols, h->hh_out,
-                                                             h->tx_tiles);
+    hh_records_kernel<<<(unsigned)h->n_act, 256, 0, h->s0>>>(h->chans, h->quad_cols, h->hh_tiles,
+                                                             h->hh_out, h->tx_tiles);
     CK(cudaGetLastError());
   }
   if (gen_v && !mod_gen.empty()) {
@@ -2143,7 +2148,7 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   if (e & kErrRingLists) {  // the tables' blocks are not those that the lists name
     e &= ~kErrRingLists;
     h->ring_paired = false;
-    h->host_pairs.clear();
+    for (int k = 0; k < 3; k++) h->ring_flops[k] = h->ring_bytes[k] = 0.0;
     h->n_tp = h->n_ring[0] = h->n_ring[1] = h->n_ring[2] = 0;
     if (h->loop64) cudaGraphExecDestroy(h->loop64);
     if (h->loop_tc) cudaGraphExecDestroy(h->loop_tc);
@@ -2492,13 +2497,20 @@ int enqueue_fused_iteration(ccdgpu_handle *h, bool mixed) {
     CK(cudaEventRecord(h->ev_join2, h->s2));
     CK(cudaStreamWaitEvent(h->s1, h->ev_join2, 0));
   }
-  // The groups of units side by side; the first that the system has stays on s1.
+  // The groups of units side by side; the first that the system has stays on s1.  Where the widest
+  // units are many (ring_cols), the one-warp units follow them there: EG N=54 |n|^2 <= 36 150.4 us an
+  // iteration, 151.0 on a branch of their own, PNM N=66 206.5 and 207.6, and the loop graph is built
+  // and torn down 0.1 ms faster; where not, they would end the ring later (|n|^2 <= 20: 52, 47.5).
   CK(cudaEventRecord(h->ev_fork3, h->s1));
   const struct { cudaStream_t st; cudaEvent_t ev; } branch[3] = {
       {h->s1, h->ev_join}, {h->s3, h->ev_join3}, {h->sset.s[4], h->sset.ev[16]}};
   int used = 0;
   for (int k = 0; k < 3; k++) {
     if (!h->n_ring[k]) continue;
+    if (k == 2 && used && h->ring_cols) {
+      if ((rc = launch_ring_units(h, h->s1, gate, k))) return rc;
+      continue;
+    }
     if (used) CK(cudaStreamWaitEvent(branch[used].st, h->ev_fork3, 0));
     if ((rc = launch_ring_units(h, branch[used++].st, gate, k))) return rc;
   }
@@ -3396,11 +3408,9 @@ int ccdgpu_kernel_profile(ccdgpu_handle *h, int32_t reps, double *ms, double *fl
   for (int k = 0; k < 7; k++) ms[k] = flops[k] = bytes[k] = 0;
   // Ring (fused path): S = T' (A + C T') + B T' per pair of channels; reads A, B, C, T' and the
   // destinations, writes S.  The small class is launched with the gather of the T' images.
-  for (const RingPair &m : h->host_pairs) {
-    const int k = m.g == 1 ? 0 : m.g == 2 ? 1 : 2;
-    const double n = (double)m.ph * m.hp;
-    flops[k] += 2.0 * n * (2.0 * m.hp + m.ph);
-    bytes[k] += 28.0 * n + 8.0 * ((double)m.hp * m.hp + (double)m.ph * m.ph);
+  for (int k = 0; k < 3; k++) {
+    flops[k] = h->ring_flops[k];
+    bytes[k] = h->ring_bytes[k];
   }
   // hh ladder: P = V_hhpp T over the packed rows and r = row dots; reads packed V and T, writes
   // the slice partials of P and r.  Reduction: reads the partials and V_hhhh, writes X and s.
