@@ -315,6 +315,7 @@ pp_ladder_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *sch
       const uint64_t v_policy = l2_evict_first();
       int gc = 0;   // stages issued by this CTA
       int nti = 0;  // tiles with a T_I so far
+      int nti_issued = 0;
       bool stop = false;
       // Test-only fault (ccdgpu_inject_wait_timeout): CTA 0 never fills its first stage, so
       // its consumers' bounded waits run out, then this producer's wait for that stage does.
@@ -350,6 +351,7 @@ pp_ladder_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *sch
               const uint32_t bytes = kMaxBM * tile.hs * 8;
               mbar_expect_tx(smem_u32(ti_full), bytes);
               bulk_g2s(smem_u32(Ti), t_q + tile.ti_base, bytes, smem_u32(ti_full));
+              ++nti_issued;
               need_ti = false;
             } else if (c + per > diag_end) {
               atomicOr(err, kErrTimeout);
@@ -374,10 +376,15 @@ pp_ladder_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *sch
         }
         nti += has_ti;
       }
-      if (!stop && free_stage()) {  // the end marker
+      const bool ended = !stop && free_stage();
+      if (ended) {  // the end marker (its stage's last copy has been read)
         info[gc % kStages].nks = 0;
         mbar_arrive(smem_u32(&bars[gc % kStages]));
       }
+      // The copies in flight land before the CTA exits, also where its consumers have given up.
+      for (int k = max(0, gc - kStages + ended); k < gc; ++k)
+        if (!(withhold && k == 0)) mbar_wait(smem_u32(&bars[k % kStages]), (k / kStages) & 1);
+      if (nti_issued) mbar_wait(smem_u32(ti_full), (nti_issued - 1) & 1);
       // The last producer to finish (each has made its last claim) resets the counters for
       // the next launch.
       __threadfence();
@@ -999,7 +1006,10 @@ __device__ __forceinline__ void ring_unit(const RingUnit &m, const double *__res
   const double *Tj = COLS ? Ts : Ts + 8 * m.n0;  // this unit's columns of T'
   bool landed = false;
   auto wait = [&]() {
-    if (!landed && !mbar_wait(bar, parity)) atomicOr(err, kErrTimeout);
+    if (!landed && !mbar_wait(bar, parity)) {
+      atomicOr(err, kErrTimeout);
+      mbar_wait(bar, parity);  // the copies land before the CTA exits
+    }
     landed = true;
   };
   double f[2][8], acc[NC][4];
