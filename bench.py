@@ -519,7 +519,7 @@ def main():
                 ("hh_ladder", "hh_slice_kernel + hh_reduce_kernel",
                  cls_bytes("hh_small", "hh_large", "hh_reduce"),
                  cls_flops("hh_small", "hh_large")),
-                ("onebody", "hh_post_kernel", cls_bytes("onebody"), 0.0),
+                ("onebody", "hh_post_kernel", cls_bytes("onebody"), cls_flops("onebody")),
             ]
             out = {}
             for fam, kname, by, fl in fams:

@@ -3395,9 +3395,8 @@ int ccdgpu_inject_wait_timeout(ccdgpu_handle *h) {
   return CCDGPU_OK;
 }
 
-// Each pp-ladder class launched alone (FP64 thin, mid, wide; tensor-core ladder), `reps` times
-// between CUDA events on the handle's stream; with the executed flops (packed: rows a<=b, K over
-// c<d and hh) and the algorithmic bytes of each class.
+// Each class of the other kernels launched alone, `reps` times between CUDA events on the handle's
+// stream; with the executed flops and the algorithmic bytes of each class.
 int ccdgpu_kernel_profile(ccdgpu_handle *h, int32_t reps, double *ms, double *flops,
                           double *bytes) {
   if (!h || reps < 1 || !ms || !flops || !bytes) return CCDGPU_ERR_INVALID_ARGUMENT;
@@ -3422,9 +3421,14 @@ int ccdgpu_kernel_profile(ccdgpu_handle *h, int32_t reps, double *ms, double *fl
     flops[6] += (double)a.nhht * hk2;
     bytes[6] += 8.0 * a.nhht * hk2 + 16.0 * hk2 + 8.0 * a.hk;
   }
-  // One-body: segmented sums of s and r (one value per pair) into x_k and y_a.
-  flops[5] = (double)h->n_t * 0;  // no arithmetic worth counting
+  // One-body: segmented sums of s and r (one value per pair) into x_k and y_a; and T X (reads T and
+  // X, writes 0.5 T X) where the handle's iterations have it here.
   bytes[5] = 16.0 * (double)(h->nsp) + 12.0 * (double)h->n_list;
+  for (const ChanInfo &a : h->host_chans) {
+    if (!a.nmt || h->tc_tx) continue;
+    flops[5] += 2.0 * a.pk * a.hk * (double)a.hk;
+    bytes[5] += 16.0 * a.pk * a.hk + 8.0 * a.hk * (double)a.hk;
+  }
   for (int k = 0; k < 7; k++) {
     auto launch = [&]() -> int {
       if (k == 0)
@@ -3432,7 +3436,7 @@ int ccdgpu_kernel_profile(ccdgpu_handle *h, int32_t reps, double *ms, double *fl
       if (k <= 2) return launch_ring_units(h, h->s0, 0, 2 - k);
       if (k <= 4) return launch_hh_ladder(h, h->s0, 0, k - 3);
       if (k == 6) return launch_hh_ladder(h, h->s0, 0, 2);
-      return launch_hh_post(h, h->s0, 0, 0);
+      return launch_hh_post(h, h->s0, 0, h->tc_tx ? 0 : -1);
     };
     if ((rc = launch())) return rc;  // warm-up
     CK(cudaEventRecord(h->ev[0], h->s0));
@@ -3447,6 +3451,8 @@ int ccdgpu_kernel_profile(ccdgpu_handle *h, int32_t reps, double *ms, double *fl
   return check_errors(h);
 }
 
+// Each pp-ladder class launched alone (FP64 thin, mid, wide; tensor-core ladder), likewise; flops
+// packed: rows a<b, columns i<j, K over c<d.
 int ccdgpu_ladder_profile(ccdgpu_handle *h, int32_t reps, double *ms, double *flops,
                           double *bytes) {
   if (!h || reps < 1 || !ms || !flops || !bytes) return CCDGPU_ERR_INVALID_ARGUMENT;

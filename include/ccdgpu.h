@@ -355,8 +355,9 @@ int ccdgpu_ladder_profile(ccdgpu_handle *h, int32_t reps, double ms[4], double f
  * per launch, indexed ring small (ph', hp' <= 16; with the phhp gather that precedes the ring
  * on the fused path), ring mid (<= 32), ring large (a class with fewer units than SMs joins the
  * next), hh ladder
- * small (at most 8 strict hole pairs), hh ladder rest, one-body sums, hh-ladder reduction.  Amplitudes are
- * not changed (the kernels write only intermediates).  No counterpart in the reference. */
+ * small (at most 8 strict hole pairs), hh ladder rest, one-body sums and T X (the sums alone on a
+ * mixed handle whose tensor-core ladder does T X), hh-ladder reduction.  Amplitudes are not
+ * changed (the kernels write only intermediates).  No counterpart in the reference. */
 int ccdgpu_kernel_profile(ccdgpu_handle *h, int32_t reps, double ms[7], double flops[7],
                           double bytes[7]);
 
