@@ -922,9 +922,9 @@ __host__ __device__ inline int ring_group(int ph, int hp) {
 // with Y's row stride 8 nt + 4.  Strides are 4 mod 8 doubles.  All of T' is 35 to 54 KB, which
 // leaves room for one CTA of four warps beside the ladder; the columns leave room for two, and T' as
 // the A operand then comes from L2.  Where those units are more than a CTA or two per SM the
-// columns are the better choice (EG N=54 |n|^2 <= 36, 732 units: 160 -> 153 us an iteration, PNM
-// N=66, 1300: 221 -> 210), else all of T' (EG N=54 |n|^2 <= 19, 238 units: 58.8 us an iteration,
-// 60.3 with the columns).
+// columns are the better choice.  All of T' and the columns, FP64 iterations by units, EG N=54: 160
+// 36.7, 37.2 us; 322 58.5, 58.4; 448 91.6, 88.1; 600 118.4, 114.1; 732 156.1, 150.0; PNM N=66: 196
+// 37.6, 39.4; 298 56.3, 55.0; 382 71.8, 71.9; 672 134.9, 132.0; 1218 220.5, 206.3.
 __host__ __device__ inline bool ring_cols(int64_t units4) { return units4 > 2 * 148; }
 __host__ __device__ constexpr int ring_ldy(int g, bool cols, int nt) {
   return g == 1 ? 20 : cols ? 8 * nt + 4 : 8 * kPairNC + 4;

@@ -2483,31 +2483,35 @@ int enqueue_fused_iteration(ccdgpu_handle *h, bool mixed) {
   // Kernels reach the GPU in the order in which they become ready, and the CTAs of one wait behind
   // all CTAs of those before it; of branches that become ready together the one captured last comes
   // first.  So: the ladder (it needs an SM's registers before smaller CTAs take them), the hh
-  // slices and the gather, then the short kernels that follow the hh slices, then the ring.  Where
-  // the ring is more than about a wave of CTAs it waits for X as well as for the gather, which end
-  // together: ahead of T X it would hold that back to the end of the iteration (EG N=54
-  // |n|^2 <= 36: 167 us an iteration, 160 so; a smaller ring leaves room, and would only start
-  // later).
+  // slices and the gather, then the short kernels that follow the hh slices, then the ring.
+  // In a mixed iteration, whose ladder is short, a large ring waits for X as well as for the
+  // gather, which end together: ahead of T X it would hold that back to the end of the iteration.
+  // By its units of four and two warps, not waiting and waiting, us an iteration: EG N=54 752
+  // 55.5, 57.1; 828 67.8, 67.4; 1134 95.2, 92.2; 1632 136.0, 135.0; PNM N=66 680 55.6, 58.8; 1014
+  // 82.2, 80.5; 1416 123.5, 120.6.  In FP64 the ladder covers both, and waiting only starts the
+  // ring later: EG N=54 578 47.2, 50.4; 1632 150.2, 151.0; PNM N=66 2136 206.1, 207.6.
   CK(cudaEventRecord(h->ev_fork, h->s0));
   CK(cudaStreamWaitEvent(h->s1, h->ev_fork, 0));
   CK(cudaStreamWaitEvent(h->s2, h->ev_fork, 0));
   if ((rc = launch_tp_gather(h, h->s1, gate))) return rc;
   if ((rc = launch_hh_ladder(h, h->s2, gate))) return rc;
-  if (h->n_ring[0] + h->n_ring[1] > 2 * 148) {
+  if (mixed && h->n_ring[0] + h->n_ring[1] > 800) {
     CK(cudaEventRecord(h->ev_join2, h->s2));
     CK(cudaStreamWaitEvent(h->s1, h->ev_join2, 0));
   }
   // The groups of units side by side; the first that the system has stays on s1.  Where the widest
-  // units are many (ring_cols), the one-warp units follow them there: EG N=54 |n|^2 <= 36 150.4 us an
-  // iteration, 151.0 on a branch of their own, PNM N=66 206.5 and 207.6, and the loop graph is built
-  // and torn down 0.1 ms faster; where not, they would end the ring later (|n|^2 <= 20: 52, 47.5).
+  // units are many, the one-warp units follow them there: a branch less, which builds and tears the
+  // loop graph down 0.1 ms faster, for iterations that take as long.  By the widest units, FP64 and
+  // mixed, on a branch of their own and following: EG N=54 732 151.0, 135.0 and 150.5, 134.3 us; PNM
+  // N=66 1218 207.6, 185.0 and 206.6, 185.4; but 672 133.0, 120.6 and 134.5, 122.7, and EG N=54 322
+  // 58.8, 57.1 and 63.4, 62.6.
   CK(cudaEventRecord(h->ev_fork3, h->s1));
   const struct { cudaStream_t st; cudaEvent_t ev; } branch[3] = {
       {h->s1, h->ev_join}, {h->s3, h->ev_join3}, {h->sset.s[4], h->sset.ev[16]}};
   int used = 0;
   for (int k = 0; k < 3; k++) {
     if (!h->n_ring[k]) continue;
-    if (k == 2 && used && h->ring_cols) {
+    if (k == 2 && h->n_ring[0] > 700) {
       if ((rc = launch_ring_units(h, h->s1, gate, k))) return rc;
       continue;
     }
