@@ -3,11 +3,11 @@
 // Reference correspondence (calc.cpp / Chain.hpp of justinlietz/coupled_cluster_doubles):
 //   pp_ladder_kernel        V_pppp T part of D = 0.5 T X + 0.5 V T   calc.cpp:162-202
 //                           (antisymmetry-packed; the assembly adds T X)
-//   hh_slice_kernel         X = V_hhhh + 0.5 V_hhpp T                calc.cpp:141-160
-//   ring_pair_kernel        the same as ring_* for the fused path
-//   hh_post_kernel          the same dot products, read from the ladder intermediates, and T X
+//   hh_slice, hh_reduce     X = V_hhhh + 0.5 V_hhpp T                calc.cpp:141-160
 //   ring_small, ring16      Y = V_hphp + 0.5 V_hpph T'; R = T' Y     calc.cpp:264-313
+//   ring_pair_kernel        the same for the fused path, T' from tp_gather_kernel
 //   onebody_tables_kernel   calcChannelT2Diff_h2pp_h1 / _p2_p1hh     calc.cpp:9-25, 73-89
+//   hh_post_kernel          the same dot products, read from the ladder intermediates, and T X
 //   gather8_kernel          Chain::mapFromDistributed x 8            Chain.hpp:710-755
 //   assemble_*_kernel       calcChannelT2_pphh                       calc.cpp:368-421
 //   map_to_kernel           Chain::set + mapToDistributed x 5        Chain.hpp:503-527,757-802
@@ -651,8 +651,10 @@ hh_reduce_kernel(const HHOut *__restrict__ outs, int n, const double *__restrict
 // is the transpose of the first's (t_ab,ij = t_ba,ji), and the assembly needs only the sums
 //   S[ai, jb] = R[ai, jb] + R[bj, ia] = T' (A + C T') + B T'
 // with A = V_hphp of the first channel, C = V_hpph (the same block for both, by the exchange of
-// both pairs; of blocks that come from the host, their mean, which is exact for any) and B[ai, ck] = V_hphp[(k c), (i a)] of the second: three products instead of four
-// and half of the amplitudes, of V_hpph and of the results (ring_unit, below).
+// both pairs; of blocks that come from the host, their mean, which is exact for any) and
+// B[ai, ck] = V_hphp[(k c), (i a)] of the second: three products instead of four and half of the
+// amplitudes, of V_hpph and of the results (ring_unit, below).  Channels that do not pair up
+// (tables from the host) run as on the table path, followed by ring_sums_kernel.
 // ------------------------------------------------------------------------------------------
 constexpr int kRingSmall = 16;
 constexpr int kRingMax = 80;  // largest ph', hp'

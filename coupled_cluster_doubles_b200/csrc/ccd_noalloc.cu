@@ -116,10 +116,11 @@ noalloc_x_sum_kernel(const double *__restrict__ v_hhhh, int hh, int nslices, dou
 // K (pp, then hh) in steps of 16 and their partial tiles are added in a fixed order through
 // shared memory.  C = 8-column tiles.  Operands come
 // straight from global memory: a step reads V once (8 rows of 32 contiguous bytes per load)
-// and T, which all CTAs share, from L2.  Launched programmatically: V T, which needs no X, runs
-// while the X kernels finish.  The whole call at pp = 1796, hh = 54 (369 MFLOP, 28 MB): 37 us,
-// 211 us with one thread per element (two loads a multiply-add); bound by the FP64 MMA of the
-// 113 CTAs (13 us) and the L1 path of their fragment loads.
+// and T, which all CTAs share, from L2.  Launched programmatically: V T, which needs no X, starts
+// with the X kernel in a channel of one slice, else beside the sum of the slices (which waits for
+// the products before it lets this kernel start).  The whole call at pp = 1796, hh = 54 (369
+// MFLOP, 28 MB): 37 us, 211 us with one thread per element (two loads a multiply-add); bound by
+// the FP64 MMA of the 113 CTAs (13 us) and the L1 path of their fragment loads.
 __host__ __device__ constexpr int d_warps(int c) { return c <= 4 ? 16 : 8; }
 template <int C>
 __global__ void __launch_bounds__(d_warps(C) * 32)

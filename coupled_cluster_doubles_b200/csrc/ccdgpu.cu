@@ -2,10 +2,12 @@
 //
 // A handle holds the whole CCD state of one system in device memory, laid out for the
 // kernels in ccd_kernels.cuh:
-//   * amplitudes in the reference t2_pphh layout (two buffers, ping-pong by a device-side
-//     parity bit), plus the ladder operand tiles of T (T^T for V_pppp T, row tiles for T X);
-//   * V_pppp pre-tiled into the swizzled shared-memory image of the pp-ladder kernel;
-//   * V_hhpp transposed to pp x hh so that it streams aligned with T;
+//   * amplitudes packed, one in four (a < b, i < j; two buffers, ping-pong by a device-side parity
+//     bit), and in the reference's layouts for the table path, the stage calls and the readers;
+//   * V_pppp as the pp ladder's chunks in their shared-memory image (of a symmetric channel one
+//     triangle of blocks), for mixed handles also as bf16 terms in the tensor core's layout;
+//   * V_hhpp packed like the amplitudes, and transposed to pp x hh;
+//   * the ring's operands of each pair of transposed modified channels in fragment order;
 //   * the loadMaps tables as int32 flat offsets into the target slabs, validated at create;
 //   * a Control block with the solve loop's state (energy history, stop rule, parity), so a
 //     captured iteration graph can be replayed without host synchronisation.
@@ -62,7 +64,7 @@ struct ccdgpu_handle {
   int n_hh_cta = 0, n_hh_warp = 0;  // hh-ladder units: one per CTA (hk > 8) first, then per warp
   int n_hh_out = 0;    // hh-ladder reduction outputs
   int n_row_tiles = 0;  // row tiles of all channels
-  int n_act = 0, n_mod = 0, n_mod_small = 0, n_mod_mid = 0, n_tiles = 0;
+  int n_act = 0, n_mod = 0, n_mod_small = 0, n_tiles = 0;
   int n_ranges = 0;
   int n_asm_blocks = 0;  // fused assembly CTAs (persistent, striding over quad_items)
   int n_cls[3] = {0, 0, 0};  // FP64 pp-ladder tiles per column class (thin, mid, wide)
@@ -91,7 +93,7 @@ struct ccdgpu_handle {
   int32_t *list = nullptr;
   double *eps = nullptr, *v_pphh = nullptr, *v_hhhh = nullptr, *v_t = nullptr;
   // Packed layout (quads): amplitudes (ping-pong by the control block's parity), V_hhpp, and
-  // the four ring terms of each quad.
+  // the two ring sums of each quad.
   double *tq[2] = {nullptr, nullptr}, *vq = nullptr, *r_quad = nullptr;
   int64_t n_q = 0;
   double *v_hpph = nullptr, *v_hphp = nullptr;
@@ -152,7 +154,7 @@ struct ccdgpu_handle {
   bool profiling = false;
   bool inject_next_step = false;  // ccdgpu_inject_wait_timeout armed for the next step
   ccdgpu_profile prof{};
-  double flops = 0, v_bytes = 0, v_packed_bytes = 0, ladder_flops = 0, ladder_bytes = 0;
+  double flops = 0, ladder_flops = 0, ladder_bytes = 0;
   int64_t launches = 0;
 
   // pp-ladder work lists (make_ladder_tiles), in their own allocation so the autotuner can
@@ -392,7 +394,7 @@ void ctl_release(Control *c) {
   pool.free.push_back(c);
 }
 
-// Process-wide pool of the streams and events a handle uses (four streams, sixteen events per
+// Process-wide pool of the streams and events a handle uses (kStreams streams, kEvents events a
 // set), by device: a create takes a set that a destroyed handle gave back instead of creating
 // twenty objects, and a destroy returns its set (after its streams are idle) instead of
 // destroying them.  Emptied by ccdgpu_release_cached_memory.
@@ -1523,7 +1525,6 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     h->n_mod_pad[k] = (int)mods_pad[k].size();
     mods.insert(mods.end(), mods_pad[k].begin(), mods_pad[k].end());
   }
-  h->n_mod_mid = h->n_mod_pad[0];
   h->n_mod = (int)mods.size();
 
   std::vector<int64_t> o_h(np + 1, 0), o_p(h->npart + 1, 0);
@@ -1583,15 +1584,14 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   h->n_asm_blocks = h->n_act ? std::max(1, std::min(h->n_quad_items, kAsmCTAsPerSM * 148)) : 0;
 
   // Work estimate (reference GEMM flops) for roofline reporting.
-  double fl = 0, lf = 0, vb = 0, vbp = 0;
+  double fl = 0, lf = 0, vbp = 0;
   for (const ChanInfo &a : chans) {
     lf += 2.0 * a.pp * a.pp * a.hh;
     fl += 2.0 * a.pp * a.pp * a.hh + 4.0 * a.pp * a.hh * (double)a.hh;
-    vb += 8.0 * a.pp * a.pp;
     if (a.hk) vbp += 8.0 * a.pk * (double)a.pk;
   }
   for (const ModInfo &m : mods) fl += 4.0 * m.ph * (double)m.hp * m.hp;
-  h->flops = fl; h->ladder_flops = lf; h->v_bytes = vb; h->v_packed_bytes = vbp;
+  h->flops = fl; h->ladder_flops = lf;
   // Bytes one pp-ladder launch must move: packed V (of a symmetric channel one triangle), the
   // packed amplitudes in and D out.
   double lb = vbp;
@@ -2449,9 +2449,10 @@ int launch_pphh(ccdgpu_handle *h) {
   return cuda_status(cudaGetLastError());
 }
 
-// One fused iteration: the pp ladder on s0, the ring on s1 and s3, and the hh ladder with the
-// one-body sums on s2 side by side (each needs only the amplitudes), then the assembly on s0.  The
-// ladder is bound by HBM on one CTA per SM, the others by latency and the L2.
+// One fused iteration: the pp ladder on s0, the ring on s1, s3 and the fifth stream, and the hh
+// ladder with the one-body sums and T X on s2 side by side (each needs only the amplitudes), then
+// the assembly on s0.  The ladder is bound by HBM on one CTA per SM, the others by latency and the
+// L2.
 // mixed: the pp ladder runs on the tensor cores (split bf16) instead of the FP64 pipe.
 int enqueue_fused_iteration(ccdgpu_handle *h, bool mixed) {
   int rc;

@@ -90,10 +90,14 @@ typedef struct ccdgpu_problem {
   const ccdgpu_channel_dims *chan_dims;        /* [n_channels] regular channels, permuted order */
   const ccdgpu_channel_dims *chan_mod_dims;    /* [n_channels] modified (ph') channels */
   const ccdgpu_channel_maps *chan_maps;        /* [n_channels] pp and hh maps are read */
-  const ccdgpu_channel_maps *chan_mod_maps;    /* [n_channels] ph and hp maps are read */
+  const ccdgpu_channel_maps *chan_mod_maps;    /* [n_channels] ph and hp maps are read (optional with
+                                                  tables and V blocks) */
   const ccdgpu_three_body_dims *three_body_dims; /* [n_sp] hpp for holes, phh for particles */
-  /* V blocks.  v_hhhh, v_hhpp, v_hpph_mod and v_hphp_mod may be NULL together when a model is
-   * given: ccdgpu_create then generates them on the device (load.cpp:112-318 elements). */
+  /* V blocks.  V_pppp is antisymmetric in both pairs.  The iterations of the fused path rely on
+   * V_hhpp antisymmetric in both pairs and on V_hhhh antisymmetric in its columns, as matrix
+   * elements are; those of the table path and the stage calls take them as they are.  v_hhhh,
+   * v_hhpp, v_hpph_mod and v_hphp_mod may be NULL together when a model is given: ccdgpu_create
+   * then generates them on the device (load.cpp:112-318 elements). */
   const double *const *v_hhhh;      /* [n_channels] hh x hh  (vnn_hhhh) */
   const double *const *v_hhpp;      /* [n_channels] hh x pp  (vnn_hhpp) */
   const double *const *v_pppp;      /* [n_channels] pp x pp  (vnn_pppp); may be NULL if model given */
@@ -125,8 +129,7 @@ enum ccdgpu_status {
 
 enum ccdgpu_precision {
   CCDGPU_PREC_FP64 = 0,        /* FP64 throughout: FP64 tensor-core MMA (mma.sync f64) for
-                                  the mid/wide pp-ladder classes, the hh ladder and the ring,
-                                  FP64 FMA for the thinnest pp-ladder channels */
+                                  the ladders, T X and the ring */
   CCDGPU_PREC_MIXED_BF16 = 1,  /* pp ladder on tensor cores with 2-term bf16 split operands,
                                   FP32 accumulation; FP64 polish iterations at the end */
   CCDGPU_PREC_MIXED_BF16X3 = 2 /* the same with 3-term bf16 split operands */
@@ -191,10 +194,10 @@ const char *ccdgpu_strerror(int status);
 /* Zero every amplitude chain (main.cpp:497-503). */
 int ccdgpu_reset(ccdgpu_handle *h);
 /* Load / read T2 in t2_pphh order (n = sum of pp*hh).  Loading also refreshes t2Old and
- * the scattered layouts, as main.cpp:660-665 would after an iteration.  The
- * iterations of the fused path take a < b, i < j elements alone (T2 is antisymmetric in (a, b) and
- * in (i, j), as every T2 of the loop is); those of the table path and the stage calls take any T2
- * as it is. */
+ * the scattered layouts, as main.cpp:660-665 would after an iteration.  The iterations
+ * of the fused path take the a < b, i < j elements alone (T2 is antisymmetric in (a, b) and in
+ * (i, j), as every T2 of the loop is); those of the table path and the stage calls take any T2 as
+ * it is. */
 int ccdgpu_set_t2(ccdgpu_handle *h, const double *t2_pphh, uint64_t n);
 int ccdgpu_get_t2(ccdgpu_handle *h, double *t2_pphh, uint64_t n);
 /* Second-order energy on the device, the reference's MBPT2 (MBPT2Corr.cpp:6-38):
