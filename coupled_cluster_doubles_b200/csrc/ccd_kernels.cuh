@@ -135,8 +135,11 @@ __device__ __forceinline__ bool skip_iteration(const Control *ctl, int gate, int
 // and D_J += V_IJ^T T_I.  EG N=54 |n|^2 <= 36: 559 MB of V become 351 (and 32 MB of D planes), in
 // the iteration the ladder's 145 us become 111; PNM N=66: 716 MB to 457, 190 us to 142.  V in full
 // is bound by HBM; halved, as much by each warp's chain of shared-memory loads, MMAs and barriers
-// (DRAM 50 % busy in the thin class, FP64 MMA 40 %).  Wider channels would need twice the FP64 MMA
-// they already wait for.
+// (the whole ladder alone: DRAM 53 %, FP64 MMA 51 % busy; thin class 54 and 41, mid 30 and 57).  Wider
+// channels would need twice the FP64 MMA they already wait for, and more than 80 registers: FP64
+// iterations with the half of V used up to 4, 12, 20 and 36 strict hole pairs, EG N=54
+// |n|^2 <= 36 151.0, 150.1, 148.2, 155.9 us, N=38 105.5, 102.9, 103.5, 107.8, PNM N=66 206.6, 204.6,
+// 205.3, 214.5.
 // One CTA per SM, 80 registers, three 39 KB stages of two chunks: it leaves registers and shared
 // memory for the other streams' kernels (at 94 registers its nine warps kept the ring's CTAs
 // out; with a fourth stage the ladder alone is 5 % faster but the iteration slower, 64 for 56 us at
