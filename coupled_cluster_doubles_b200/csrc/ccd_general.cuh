@@ -44,7 +44,7 @@ antisymmetry_kernel(const ElemRange *__restrict__ ranges, const ChanInfo *__rest
   if (differs) *flag = 1;
 }
 // The same for the columns of V_hhhh, against the largest element of the channel (one CTA each; its
-// rows need not be antisymmetric, see pack_hhhh_kernel).
+// rows need not be antisymmetric, see hh_records_kernel).
 __global__ void __launch_bounds__(256)
 antisymmetry_hhhh_kernel(const ChanInfo *__restrict__ chans, const int32_t *__restrict__ hh_swap,
                          const double *__restrict__ v_hhhh,

@@ -384,10 +384,6 @@ pp_ladder_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *sch
         info[gc % kStages].nks = 0;
         mbar_arrive(smem_u32(&bars[gc % kStages]));
       }
-      // The copies in flight land before the CTA exits, also where its consumers have given up.
-      for (int k = max(0, gc - kStages + ended); k < gc; ++k)
-        if (!(withhold && k == 0)) mbar_wait(smem_u32(&bars[k % kStages]), (k / kStages) & 1);
-      if (nti_issued) mbar_wait(smem_u32(ti_full), (nti_issued - 1) & 1);
       // The last producer to finish (each has made its last claim) resets the counters for
       // the next launch.
       __threadfence();
@@ -396,6 +392,10 @@ pp_ladder_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *sch
         sched[1] = 0;
         __threadfence();
       }
+      // The copies in flight land before the CTA exits, also where its consumers have given up.
+      for (int k = max(0, gc - kStages + ended); k < gc; ++k)
+        if (!(withhold && k == 0)) mbar_wait(smem_u32(&bars[k % kStages]), (k / kStages) & 1);
+      if (nti_issued) mbar_wait(smem_u32(ti_full), (nti_issued - 1) & 1);
     }
     return;
   }
@@ -1579,21 +1579,6 @@ expand_t_kernel(const ElemRange *__restrict__ ranges, const ChanInfo *__restrict
       if (neg) v = -v;
     }
     t2[e] = v;
-  }
-}
-
-// V_hhhh of the strict pairs in the layout of X.  T is antisymmetric in (k, l), so T X takes the
-// antisymmetric part of X's rows alone: of blocks from the host, whatever they hold, exactly.
-__global__ void __launch_bounds__(256)
-pack_hhhh_kernel(const ChanInfo *__restrict__ chans, const QuadCol *__restrict__ qcols,
-                 const double *__restrict__ v_hhhh, double *__restrict__ v_x) {
-  const ChanInfo ch = chans[blockIdx.x];
-  if (!ch.pk) return;  // no X
-  const double *v = v_hhhh + ch.vhh_off;
-  for (int e = threadIdx.x; e < ch.hk * ch.hk; e += blockDim.x) {
-    const int kl = e / ch.hk, ij = e - kl * ch.hk, col = qcols[ch.qcol_off + ij].c_ij;
-    const QuadCol c = qcols[ch.qcol_off + kl];
-    v_x[ch.x_off + kl * ch.hs + ij] = 0.5 * (v[c.c_ij * ch.hh + col] - v[c.c_ji * ch.hh + col]);
   }
 }
 

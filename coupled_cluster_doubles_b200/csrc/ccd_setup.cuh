@@ -481,9 +481,12 @@ quad_rows_kernel(const ChanInfo *__restrict__ chans, const int32_t *__restrict__
 }
 
 // Records of the hh ladder (a slice of kHHRows rows each), its reduction (one per element of X) and T X
-// (tx_rows(hk) rows by 16 columns), one CTA per channel, from its first of each on.
+// (tx_rows(hk) rows by 16 columns), one CTA per channel, from its first of each on; and V_hhhh of the
+// strict pairs in the layout of X.  T is antisymmetric in (k, l), so T X takes the antisymmetric
+// part of X's rows alone: of blocks from the host, whatever they hold, exactly.
 __global__ void __launch_bounds__(256)
 hh_records_kernel(const ChanInfo *__restrict__ chans, const QuadCol *__restrict__ qcols,
+                  const double *__restrict__ v_hhhh, double *__restrict__ v_x,
                   HHTile *__restrict__ slices, HHOut *__restrict__ outs,
                   TXTile *__restrict__ tiles) {
   const ChanInfo ch = chans[blockIdx.x];
@@ -516,6 +519,8 @@ hh_records_kernel(const ChanInfo *__restrict__ chans, const QuadCol *__restrict_
     o.xt[0] = xt_at(c.c_ij, ij);
     o.xt[1] = xt_at(c.c_ji, ij);
     outs[ch.hh_first + e] = o;
+    const double *v = v_hhhh + ch.vhh_off + qcols[ch.qcol_off + ij].c_ij;
+    v_x[o.x] = 0.5 * (v[c.c_ij * ch.hh] - v[c.c_ji * ch.hh]);
   }
   const int rows = tx_rows(ch.hk), nj = (ch.hk + 15) / 16, n = (ch.pk + rows - 1) / rows * nj;
   for (int e = threadIdx.x; e < n; e += blockDim.x) {

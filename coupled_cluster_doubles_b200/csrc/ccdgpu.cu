@@ -1945,9 +1945,6 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     quad_rows_kernel<<<(unsigned)h->n_act, 256, 0, h->s0>>>(
         h->chans, h->kcol, h->pp_swap, h->pp_pairs, h->eps, (int)np, h->quad_rows);
     CK(cudaGetLastError());
-    hh_records_kernel<<<(unsigned)h->n_act, 256, 0, h->s0>>>(h->chans, h->quad_cols, h->hh_tiles,
-                                                             h->hh_out, h->tx_tiles);
-    CK(cudaGetLastError());
   }
   if (gen_v && !mod_gen.empty()) {
     gen_v_mod_kernel<<<(unsigned)mod_gen.size(), 256, 0, h->s0>>>(d_mod_gen, d_mod_ph, d_mod_hp,
@@ -1973,8 +1970,8 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
       pack_quads_kernel<<<h->n_quad_items, kAsmThreads, 0, h->s0>>>(
           h->quad_items, h->chans, h->quad_rows, h->quad_cols, h->v_pphh, h->vq);
       CK(cudaGetLastError());
-      pack_hhhh_kernel<<<(unsigned)h->n_act, 256, 0, h->s0>>>(h->chans, h->quad_cols, h->v_hhhh,
-                                                              h->v_x);
+      hh_records_kernel<<<(unsigned)h->n_act, 256, 0, h->s0>>>(
+          h->chans, h->quad_cols, h->v_hhhh, h->v_x, h->hh_tiles, h->hh_out, h->tx_tiles);
       CK(cudaGetLastError());
     }
     if (derive_tables || gen_v3) {
