@@ -318,7 +318,6 @@ pp_ladder_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *sch
       const uint64_t v_policy = l2_evict_first();
       int gc = 0;   // stages issued by this CTA
       int nti = 0;  // tiles with a T_I so far
-      int nti_issued = 0;
       bool stop = false;
       // Test-only fault (ccdgpu_inject_wait_timeout): CTA 0 never fills its first stage, so
       // its consumers' bounded waits run out, then this producer's wait for that stage does.
@@ -354,7 +353,6 @@ pp_ladder_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *sch
               const uint32_t bytes = kMaxBM * tile.hs * 8;
               mbar_expect_tx(smem_u32(ti_full), bytes);
               bulk_g2s(smem_u32(Ti), t_q + tile.ti_base, bytes, smem_u32(ti_full));
-              ++nti_issued;
               need_ti = false;
             } else if (c + per > diag_end) {
               atomicOr(err, kErrTimeout);
@@ -379,8 +377,7 @@ pp_ladder_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *sch
         }
         nti += has_ti;
       }
-      const bool ended = !stop && free_stage();
-      if (ended) {  // the end marker (its stage's last copy has been read)
+      if (!stop && free_stage()) {  // the end marker
         info[gc % kStages].nks = 0;
         mbar_arrive(smem_u32(&bars[gc % kStages]));
       }
@@ -392,20 +389,17 @@ pp_ladder_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *sch
         sched[1] = 0;
         __threadfence();
       }
-      // The copies in flight land before the CTA exits, also where its consumers have given up.
-      for (int k = max(0, gc - kStages + ended); k < gc; ++k)
-        if (!(withhold && k == 0)) mbar_wait(smem_u32(&bars[k % kStages]), (k / kStages) & 1);
-      if (nti_issued) mbar_wait(smem_u32(ti_full), (nti_issued - 1) & 1);
     }
     return;
   }
   const int tid = threadIdx.x;
   RingPos at;
   int nti = 0;
+  bool gave_up = false;
   for (;;) {
     // The first stage describes the tile.
     if (!mbar_wait(smem_u32(&bars[at.s]), at.phase)) {
-      atomicOr(err, kErrTimeout);
+      gave_up = true;
       break;
     }
     const StageInfo ti = info[at.s];
@@ -433,19 +427,24 @@ pp_ladder_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *sch
       default: ok = consume_mma<5, false>(ti, As, Bs, Ti, bars, tb, tp, tid, at, d); break;
     }
     if (!ok) {  // a timed-out tile leaves its rows unfinished
-      atomicOr(err, kErrTimeout);
+      gave_up = true;
       break;
     }
     if (ti.nseg >= 0) {
       // A warp that had no turn passes T_I's phase all the same before it frees the buffer.
       if (!mbar_wait(tb, tp)) {
-        atomicOr(err, kErrTimeout);
+        gave_up = true;
         break;
       }
       ++nti;
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(ti_free));
     }
+  }
+  if (gave_up) {  // what the producer has issued lands before the CTA exits
+    atomicOr(err, kErrTimeout);
+    for (int s = 0; s < kStages; ++s, at.next()) mbar_wait(smem_u32(&bars[at.s]), at.phase);
+    mbar_wait(smem_u32(ti_full), nti & 1);
   }
   trace_end(ctl, kTrLadderThin);
 }
