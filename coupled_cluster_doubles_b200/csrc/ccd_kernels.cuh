@@ -74,7 +74,7 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t
 }
 // The same for data that an iteration reads once, and from HBM anyway if it is large (V): first to
 // be evicted, so that it does not push out what other kernels read again.  In the FP64 iteration
-// of EG N=54 |n|^2 <= 19 (V 50 MB) 55.0 -> 46.7 us, |n|^2 <= 36 (351 MB) 151.8 -> 148.6, PNM N=66
+// of EG N=54 |n|^2 <= 20 (V 50 MB) 55.0 -> 46.7 us, |n|^2 <= 36 (351 MB) 151.8 -> 148.6, PNM N=66
 // 209.7 -> 206.4, and no change where everything fits (EG N=14).
 __device__ __forceinline__ uint64_t l2_evict_first() {
   uint64_t p;
@@ -143,7 +143,7 @@ __device__ __forceinline__ bool skip_iteration(const Control *ctl, int gate, int
 // One CTA per SM, 80 registers, three 39 KB stages of two chunks: it leaves registers and shared
 // memory for the other streams' kernels (at 94 registers its nine warps kept the ring's CTAs
 // out; with a fourth stage the ladder alone is 5 % faster but the iteration slower, 64 for 56 us at
-// EG N=54 |n|^2 <= 19).  Stages of one chunk, five deep: 51 and 66 us for the thin and the mid
+// EG N=54 |n|^2 <= 20).  Stages of one chunk, five deep: 51 and 66 us for the thin and the mid
 // class alone at EG N=54 |n|^2 <= 36, 46 and 62 now.
 // One producer warp: a lane claims tiles from a launch-wide counter (list sorted by class, wide
 // first, then by decreasing work: longest-first list scheduling that adapts to CTAs starting
@@ -1203,8 +1203,8 @@ __device__ __forceinline__ double block_sum(double v, double *scratch) {
 //   hole k:     x = sum v_h_hpp * t2Old_h2pp_h1;  diff_h2pp_h1 = 0.5 x t2Old_h1pp_h2
 //   particle a: y = sum t2Old_p1_p2hh * v_phh_p;  diff_p2_p1hh = -0.5 y t2Old_p2_p1hh
 // (argument order of main.cpp:591-607).  Bound by latency: the few holes' blocks are long (18000
-// elements at EG N=54 |n|^2 <= 19), so those CTAs have 1024 threads, the particles' 256, four
-// elements each in flight: the call for the holes at EG N=38 |n|^2 <= 15 30 -> 17 us.
+// elements at EG N=54 |n|^2 <= 20), so those CTAs have 1024 threads, the particles' 256, four
+// elements each in flight: the call for the holes at EG N=38 |n|^2 <= 16 30 -> 17 us.
 // ------------------------------------------------------------------------------------------
 constexpr int kOBHoles = 1024, kOBParticles = 256, kOBPer = 4;
 template <int NT>

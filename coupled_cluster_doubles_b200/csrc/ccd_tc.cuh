@@ -191,8 +191,9 @@ constexpr int kTcGrid = 148;          // persistent grid: one CTA on each SM
 // warp on the stage's full barrier, for every chunk); the producer copies only the B planes of
 // those chunks.  No V image is read from HBM.
 // Tiles with nkx > 0 go on with T X from the T image's own operands (small systems, where the
-// ladder is too short to be worth starting before X: their mixed iterations then round D as one
-// sum, and a solve with few FP64 iterations after them depends on that at 1e-8).
+// ladder is too short to be worth starting before X: their mixed iterations round D as one sum;
+// where a solve stops within its threshold depends on that, how far from the FP64 fixed point it
+// stops does not).
 template <int NT, bool GEN>
 __global__ void __launch_bounds__(tc_threads(GEN), GEN ? 2 : 1)
 pp_ladder_tc_kernel(const LadderTile *__restrict__ tiles, int n_tiles, int32_t *sched,
