@@ -23,6 +23,7 @@ namespace ccd {
 // [kBK][as] k-major, as = rows rounded up to 8, plus 4.  hs is 4 mod 8 beyond 4 hole pairs: with
 // strides of 4 mod 8 doubles the 4 k-rows of an m16n8k16 fragment load fall on distinct banks.
 // The last row tile of a channel is stored compact (only its real rows, rounded up to 8).
+constexpr int kSMs = 148;      // SMs of a B200
 constexpr int kBK = 16;        // K depth of one chunk
 constexpr int kStages = 3;     // bulk-copy pipeline depth, stages of two chunks (one if hs > 20)
 constexpr int kMaxHH = 72;     // hole pairs of a channel (ordered)

@@ -929,7 +929,7 @@ __host__ __device__ inline int ring_group(int ph, int hp) {
 // columns are the better choice.  All of T' and the columns, FP64 iterations by units, EG N=54: 160
 // 36.7, 37.2 us; 322 58.5, 58.4; 448 91.6, 88.1; 600 118.4, 114.1; 732 156.1, 150.0; PNM N=66: 196
 // 37.6, 39.4; 298 56.3, 55.0; 382 71.8, 71.9; 672 134.9, 132.0; 1218 220.5, 206.3.
-__host__ __device__ inline bool ring_cols(int64_t units4) { return units4 > 2 * 148; }
+__host__ __device__ inline bool ring_cols(int64_t units4) { return units4 > 2 * kSMs; }
 __host__ __device__ constexpr int ring_ldy(int g, bool cols, int nt) {
   return g == 1 ? 20 : cols ? 8 * nt + 4 : 8 * kPairNC + 4;
 }

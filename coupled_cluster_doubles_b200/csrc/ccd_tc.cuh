@@ -185,7 +185,7 @@ __device__ __forceinline__ void tc_drain(const uint64_t *full, int issued, int s
 // each, plane p at base + p * stride.  A mixed-phase kernel (gate 1 of skip_iteration).
 constexpr uint32_t kTcAccCols = 64;   // columns of one accumulator buffer (nb <= kTcMaxNB)
 constexpr int kTcTQ = 4;              // slots of a CTA's queue of claimed tiles
-constexpr int kTcGrid = 148;          // persistent grid: one CTA on each SM
+constexpr int kTcGrid = kSMs;         // persistent grid: one CTA on each SM
 // GEN (electron gas, V generated in the ladder): warps 6 .. 6 + kTcGenWarps - 1 write the V
 // operand planes of every V T chunk into the stage (fence.proxy.async, then one arrival per
 // warp on the stage's full barrier, for every chunk); the producer copies only the B planes of

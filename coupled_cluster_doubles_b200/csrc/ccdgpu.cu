@@ -811,7 +811,6 @@ int materialize_d(ccdgpu_handle *h);
 int make_ladder_tiles(ccdgpu_handle *h, const ccdgpu_schedule &sch) {
   if (int rc = materialize_d(h)) return rc;  // it reads the planes that go away here
   const std::vector<ChanInfo> &chans = h->host_chans;
-  const int64_t kSMs = 148;
   const int mid_mul = sch.mid_split_mul > 0 ? sch.mid_split_mul : sch.wide_split_mul;
   int64_t chunks = 0, tc_blocks = 0;
   for (const ChanInfo &a : chans) {
@@ -1472,7 +1471,7 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
     for (const RingPair &r : pairs) group_units[r.g] += units_of(r);
     for (int g : {1, 2}) {
       const int to = group_units[2 * g] ? 2 * g : 4;
-      if (group_units[g] >= 148 || !group_units[to]) continue;
+      if (group_units[g] >= kSMs || !group_units[to]) continue;
       for (RingPair &r : pairs)
         if (r.g == g) r.g = to;
       group_units[to] += group_units[g];
@@ -1581,7 +1580,7 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
   h->n_quad_items = (int)quad_items.size();
   // Persistent assembly grid: kAsmCTAsPerSM resident CTAs per SM at most (one CTA if there is no quad,
   // for the energy and the stop rule).
-  h->n_asm_blocks = h->n_act ? std::max(1, std::min(h->n_quad_items, kAsmCTAsPerSM * 148)) : 0;
+  h->n_asm_blocks = h->n_act ? std::max(1, std::min(h->n_quad_items, kAsmCTAsPerSM * kSMs)) : 0;
 
   // Work estimate (reference GEMM flops) for roofline reporting.
   double fl = 0, lf = 0, vbp = 0;
@@ -2016,7 +2015,7 @@ int build(ccdgpu_handle *h, const ccdgpu_problem *P) {
             d_mod_dims, d_mod_at, d_mod_ph, d_mod_hp, h->err);
     }
     CK(cudaGetLastError());
-    const int nb = (int)std::min<int64_t>(ceil_div(5 * n_t, 256), 148 * 32);
+    const int nb = (int)std::min<int64_t>(ceil_div(5 * n_t, 256), kSMs * 32);
     check_counts_kernel<<<std::max(nb, 1), 256, 0, h->s0>>>(counts, 5 * n_t, h->err);
     CK(cudaGetLastError());
     ring_maps_kernel<<<h->n_ranges, 256, 0, h->s0>>>(h->ranges, h->chans, h->pp_swap, h->hh_swap,
@@ -2228,7 +2227,7 @@ int launch_pp_ladder(ccdgpu_handle *h, cudaStream_t st, int cls = -1) {
   if (!n) return CCDGPU_OK;
   h->launches++;
   return cuda_status(launch_pdl(
-      pp_ladder_kernel, std::min(n, 148), kLadderThreads, kLadderSmem, st,
+      pp_ladder_kernel, std::min(n, kSMs), kLadderThreads, kLadderSmem, st,
       (const LadderTile *)(h->tiles + first), n, h->sched, (const double *)h->v_t,
       (const double *)h->tq[0], (const double *)h->tq[1], h->d_planes, (const Control *)h->ctl,
       h->err, 0));
@@ -2265,7 +2264,7 @@ int materialize_t(ccdgpu_handle *h) {
 int launch_antisymmetry(ccdgpu_handle *h, const double *src) {
   if (!h->n_ranges) return CCDGPU_OK;
   CK(cudaMemsetAsync(h->irr, 0, sizeof(*h->irr), h->s0));
-  max_abs_kernel<<<(unsigned)std::min<int64_t>(ceil_div(h->n_t, 1024), 148 * 8), 256, 0, h->s0>>>(
+  max_abs_kernel<<<(unsigned)std::min<int64_t>(ceil_div(h->n_t, 1024), kSMs * 8), 256, 0, h->s0>>>(
       src, h->n_t, h->irr);
   CK(cudaGetLastError());
   antisymmetry_kernel<<<h->n_ranges, 256, 0, h->s0>>>(h->ranges, h->chans, h->pp_swap, h->hh_swap,
@@ -2307,7 +2306,7 @@ int refresh_tc_image(ccdgpu_handle *h) {
 int launch_phhp_gather(ccdgpu_handle *h, cudaStream_t st) {
   if (!h->n_m) return CCDGPU_OK;
   h->launches++;
-  const unsigned blocks = (unsigned)std::min<int64_t>(ceil_div(h->n_m, 256), 148 * 16);
+  const unsigned blocks = (unsigned)std::min<int64_t>(ceil_div(h->n_m, 256), kSMs * 16);
   phhp_gather_kernel<<<blocks, 256, 0, st>>>(h->ring_quads, h->n_m, h->tq[0], h->tq[1],
                                              h->old_phhp, h->ctl);
   return cuda_status(cudaGetLastError());
@@ -2552,7 +2551,7 @@ int stage_onebody_tables(ccdgpu_handle *h, int holes, int particles) {
 }
 int stage_gather(ccdgpu_handle *h) {
   if (!h->have_3body) return CCDGPU_ERR_UNSUPPORTED;
-  const int blocks = (int)std::min<int64_t>(ceil_div(h->n_t, 256), 148 * 16);
+  const int blocks = (int)std::min<int64_t>(ceil_div(h->n_t, 256), kSMs * 16);
   gather8_kernel<<<std::max(blocks, 1), 256, 0, h->s0>>>(h->n_t, h->flat, h->diff_h2pp_h1,
                                                          h->diff_p2_p1hh, h->r_phhp, h->gath);
   h->launches++;
@@ -2976,7 +2975,7 @@ int ccdgpu_build_channels(const ccdgpu_channel_rule *rule, ccdgpu_channel_dims *
     CK(cudaMemcpyAsync(at(o_qn), rule->qn, nsp * rule->qn_stride * 4, cudaMemcpyHostToDevice, st));
     ChannelRuleDev r{reinterpret_cast<const int32_t *>(at(o_qn)), rule->kind, rule->qn_stride,
                      rule->nmax, rule->chan_tz_max, rule->mod_chan_tz_max, nsp, np, nch};
-    const unsigned grid = (unsigned)std::min<uint64_t>((n + 255) / 256, 148 * 16);
+    const unsigned grid = (unsigned)std::min<uint64_t>((n + 255) / 256, kSMs * 16);
     uint32_t *c0 = reinterpret_cast<uint32_t *>(at(o_c0)), *mc0 = reinterpret_cast<uint32_t *>(at(o_mc0));
     pair_channel_kernel<<<grid, 256, 0, st>>>(r, c0, mc0, reinterpret_cast<uint32_t *>(at(o_cnt)),
                                                reinterpret_cast<uint32_t *>(at(o_mcnt)),
