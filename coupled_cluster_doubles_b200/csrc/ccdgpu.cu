@@ -2496,22 +2496,15 @@ int enqueue_fused_iteration(ccdgpu_handle *h, bool mixed) {
     CK(cudaEventRecord(h->ev_join2, h->s2));
     CK(cudaStreamWaitEvent(h->s1, h->ev_join2, 0));
   }
-  // The groups of units side by side; the first that the system has stays on s1.  Where the widest
-  // units are many, the one-warp units follow them there: a branch less, which builds and tears the
-  // loop graph down 0.1 ms faster, for iterations that take as long.  By the widest units, FP64 and
-  // mixed, on a branch of their own and following: EG N=54 732 151.0, 135.0 and 150.5, 134.3 us; PNM
-  // N=66 1218 207.6, 185.0 and 206.6, 185.4; but 672 133.0, 120.6 and 134.5, 122.7, and EG N=54 322
-  // 58.8, 57.1 and 63.4, 62.6.
+  // The groups of units side by side; the first that the system has stays on s1.  (The one-warp units
+  // behind the widest ones, a branch less, build and tear the loop graph down 0.1 ms faster each, but
+  // EG N=54 |n|^2 <= 36 took 0.3 to 0.6 % longer to solve, and |n|^2 <= 21 8 % an iteration.)
   CK(cudaEventRecord(h->ev_fork3, h->s1));
   const struct { cudaStream_t st; cudaEvent_t ev; } branch[3] = {
       {h->s1, h->ev_join}, {h->s3, h->ev_join3}, {h->sset.s[4], h->sset.ev[16]}};
   int used = 0;
   for (int k = 0; k < 3; k++) {
     if (!h->n_ring[k]) continue;
-    if (k == 2 && h->n_ring[0] > 700) {
-      if ((rc = launch_ring_units(h, h->s1, gate, k))) return rc;
-      continue;
-    }
     if (used) CK(cudaStreamWaitEvent(branch[used].st, h->ev_fork3, 0));
     if ((rc = launch_ring_units(h, branch[used++].st, gate, k))) return rc;
   }
