@@ -2430,6 +2430,7 @@ int launch_pphh(ccdgpu_handle *h) {
   if (!h->x_full) {
     void *p = nullptr;
     size_t got = 0;
+    CK(cudaSetDevice(h->opt.device));
     CK(dev_alloc(std::max<int64_t>(h->n_vhh, 1) * sizeof(double), &p, &got));
     h->allocs.push_back({p, got});
     h->x_full = static_cast<double *>(p);
